@@ -217,51 +217,198 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long x) {
     x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
     return x ^ (x >> 31);
 }
+// A weight in fixed point, cut off.  Weights are at most 1: the 24 bits of the number shifted to
+// their place, without the 64-bit conversions, of which an SM makes a sixteenth of what it
+// shifts.  (An infinity or a NaN goes by them.)
 __device__ __forceinline__ unsigned long long to_fixed(float w) {
-    return (unsigned long long)((double)w * FIX_ONE);
+    const unsigned u = __float_as_uint(w);
+    const int e = (int)(u >> 23);                       // (sign clear)
+    if (e > 127) return (unsigned long long)((double)w * FIX_ONE);
+    const unsigned long long m = (u & 0x7fffffu) | 0x800000u;
+    return e >= 110 ? m << (e - 110) : e > 110 - 24 ? m >> (110 - e) : 0ull;
 }
 
+// A row is shared by the C CTAs of a cluster (C = 1, 2, 4 or 8): CTA c owns a contiguous slice of
+// the vocabulary, keeps it in shared memory (SM_RESIDENT values at most; what a larger slice has
+// beyond them is read again from global memory) and answers for it in every pass.  What decides
+// anything crosses the cluster: the maximum, the 256 bins of a radix pass, the slices' sums.
+// All of those are maxima, counts and fixed-point sums, so the token does not depend on C.
+//
+// What bounds it: the passes over the slice and the cluster barriers, not the bytes (64 rows of
+// 262,144 logits are 67 MB, 10 us of HBM).  One CTA a row, every pass over the row in L2 and a
+// 64-bit shared-memory atomic for every value of a bin, took 4,000 us for those 64 rows alone and
+// 6,600 us in a decode step, where the CTAs of the step's next kernel wait on the same SMs.  With
+// slices in shared memory, top-k 64 and top-p 0.95: 334 us when every pass runs over the cluster,
+// 100 us when the few candidates a top-k leaves are finished by one CTA (one row: 3,860, 72 and 33
+// us; top-p 0.9 alone, where every weight takes part: 2,160 -> 326 us).  Eight CTAs of a 262,144
+// row take 128 KB each, so 16 to 18 rows run at a time.
+constexpr int SM_BINS = 256;
+constexpr int SM_RESIDENT = 44 * 1024;         // values of a slice in shared memory (176 KB)
+constexpr int SM_LIST = 2048;                  // candidates of a top-k that one CTA finishes alone
+constexpr int SM_PIECE = 14;                   // bits of a fixed-point weight added at a time
+constexpr int SM_FOLD = 1 << 18;               // values between two folds: SM_PIECE + 18 <= 32 bits
+
 struct SampleShared {
-    unsigned long long hist[256];
-    unsigned long long chunk[SM_THREADS];
+    unsigned long long mass[2][SM_BINS];       // this slice's bins, read by the whole cluster
+    unsigned long long sums[SM_BINS];          // the cluster's
+    unsigned part[3][SM_BINS];                 // (counts in part[0]; the pieces of 64-bit sums)
+    unsigned long long wsum[SM_THREADS / 32];  // kept weight of every warp's range
+    unsigned long long slice_sum;              // read by the whole cluster
+    unsigned long long total_mass;             // read by the whole cluster
     float red[33];
+    float mx;                                  // read by the whole cluster
+    unsigned bound;                            // read by the whole cluster
+    int n_list;                                // read by the whole cluster
+    float list_x[SM_LIST];                     // CTA 0's: written by the whole cluster
+    int list_i[SM_LIST];
     unsigned prefix;
     unsigned long long above;
-    int done;
-    int result;
 };
 
-// Descends the 32-bit key space 8 bits at a time.  COUNT: finds the key of the
-// k-th greatest element (target = k, each element weighs 1).  Otherwise finds
-// the greatest key whose tail mass reaches target (each element weighs its
-// fixed-point weight).
-template <bool COUNT, typename KeyFn, typename MassFn>
-__device__ unsigned radix_descend(SampleShared& sh, int V, unsigned long long target, KeyFn key,
-                                  MassFn mass) {
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// All threads of the cluster meet, and see what the others wrote before.
+__device__ __forceinline__ void cluster_meet() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
+                 ::: "memory");
+}
+__device__ __forceinline__ unsigned peer_address(const void* mine, int rank) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;"
+        : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(mine)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ unsigned long long peer_u64(const unsigned long long* mine, int rank) {
+    unsigned long long v;
+    asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(peer_address(mine, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned peer_u32(const void* mine, int rank) {
+    unsigned v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_address(mine, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// The bin in which a sum over the bins from the greatest downwards, starting at `above`, first
+// reaches `target` (bin 0 if none does), and the sum over the bins above it.  A warp: lane l has
+// bins 8 l .. 8 l + 7 of the cluster's sums.
+__device__ __forceinline__ void pick_bin(const unsigned long long (&m)[8], unsigned long long above,
+                                         unsigned long long target, int& bin,
+                                         unsigned long long& sum_above) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long own = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) own += m[i];
+    unsigned long long tail = own;               // of this lane and the ones above it
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_down_sync(0xffffffffu, tail, o);
+        if (lane + o < 32) tail += t;
+    }
+    unsigned long long acc = above + (tail - own);
+    int mine = -1;
+    unsigned long long before = 0;
+#pragma unroll
+    for (int i = 7; i >= 0; --i) {
+        if (mine < 0 && acc + m[i] >= target) { mine = lane * 8 + i; before = acc; }
+        acc += m[i];
+    }
+    // (acc: with every bin of the lane; lane 0 stops at bin 0 whatever the sum)
+    if (lane == 0 && mine < 0) { mine = 0; before = acc - m[0]; }
+    const unsigned have = __ballot_sync(0xffffffffu, mine >= 0);
+    const int at = 31 - __clz(have);
+    bin = __shfl_sync(0xffffffffu, mine, at);
+    sum_above = __shfl_sync(0xffffffffu, before, at);
+}
+
+// Descends the 32-bit key space 8 bits at a time, over the whole row (C > 1) or this CTA's slice
+// (C = 1).  COUNT: the key of the element at which the count from above reaches target.
+// Otherwise the greatest key whose tail mass reaches target (each element weighs its fixed-point
+// weight).  each(f): calls f(key, weight) for the thread's elements; n: elements of the CTA at
+// most.  Every thread calls it; `turn` counts the passes of the kernel, whose two sets of bins
+// alternate, so one meeting of the cluster a pass suffices: a set is cleared after the meeting
+// of the pass before, when every peer has read it.
+template <bool COUNT, typename EachFn>
+__device__ unsigned radix_descend(SampleShared& sh, int C, int& turn, unsigned long long target,
+                                  int thread_elements, EachFn each) {
     if (threadIdx.x == 0) { sh.prefix = 0; sh.above = 0; }
-    for (int pass = 0; pass < 4; ++pass) {
+    for (int pass = 0; pass < 4; ++pass, ++turn) {
         const int shift = 24 - 8 * pass;
-        for (int i = threadIdx.x; i < 256; i += blockDim.x) sh.hist[i] = 0;
+        unsigned long long* bins = sh.mass[turn & 1];
+        if (threadIdx.x < SM_BINS) {
+            bins[threadIdx.x] = 0;
+            sh.part[0][threadIdx.x] = sh.part[1][threadIdx.x] = sh.part[2][threadIdx.x] = 0;
+        }
         __syncthreads();
         const unsigned prefix = sh.prefix;
         const unsigned himask = pass == 0 ? 0u : (0xffffffffu << (shift + 8));
-        for (int i = threadIdx.x; i < V; i += blockDim.x) {
-            const unsigned kk = key(i);
-            if ((kk & himask) == prefix) {
-                const unsigned long long m = COUNT ? 1ull : mass(i);
-                if (m) atomicAdd(&sh.hist[(kk >> shift) & 255u], m);
+        auto fold = [&]() {
+            __syncthreads();
+            if (threadIdx.x < SM_BINS) {
+                const int b = threadIdx.x;
+                bins[b] += (unsigned long long)sh.part[0][b] +
+                           (COUNT ? 0ull : ((unsigned long long)sh.part[1][b] << SM_PIECE) +
+                                           ((unsigned long long)sh.part[2][b] << (2 * SM_PIECE)));
+                sh.part[0][b] = sh.part[1][b] = sh.part[2][b] = 0;
             }
+            __syncthreads();
+        };
+        // (a CTA adds SM_FOLD values at most before a fold)
+        constexpr int PER = SM_FOLD / SM_THREADS;
+        for (int e0 = 0; e0 < thread_elements; e0 += PER) {
+            each(e0, min(e0 + PER, thread_elements), [&](unsigned key, unsigned long long m) {
+                if ((key & himask) != prefix || m == 0) return;
+                const int b = (key >> shift) & 255u;
+                if (COUNT) {
+                    atomicAdd(&sh.part[0][b], 1u);
+                } else if (m >> (3 * SM_PIECE)) {              // (no weight is above 2^40; a NaN's)
+                    atomicAdd(&bins[b], m);
+                } else {
+                    const unsigned lo = (1u << SM_PIECE) - 1;
+                    const unsigned p0 = (unsigned)m & lo, p1 = (unsigned)(m >> SM_PIECE) & lo,
+                                   p2 = (unsigned)(m >> (2 * SM_PIECE));
+                    if (p0) atomicAdd(&sh.part[0][b], p0);
+                    if (p1) atomicAdd(&sh.part[1][b], p1);
+                    if (p2) atomicAdd(&sh.part[2][b], p2);
+                }
+            });
+            fold();
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned long long acc = sh.above;
-            int bin = 255;
-            for (; bin > 0; --bin) {
-                if (acc + sh.hist[bin] >= target) break;
-                acc += sh.hist[bin];
+        if (C > 1) {
+            // the cluster's sums: a thread a bin, its peers' loads in flight together
+            cluster_meet();
+            if (threadIdx.x < SM_BINS) {
+                unsigned long long v[8];
+#pragma unroll
+                for (int r = 0; r < 8; ++r) v[r] = r < C ? peer_u64(&bins[threadIdx.x], r) : 0ull;
+                unsigned long long m = 0;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) m += v[r];
+                sh.sums[threadIdx.x] = m;
             }
-            sh.above = acc;
-            sh.prefix = prefix | ((unsigned)bin << shift);
+            __syncthreads();
+        }
+        if (threadIdx.x < 32) {
+            const unsigned long long* of = C > 1 ? sh.sums : bins;
+            unsigned long long m[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) m[i] = of[threadIdx.x * 8 + i];
+            int bin;
+            unsigned long long above;
+            pick_bin(m, sh.above, target, bin, above);
+            __syncwarp();
+            if (threadIdx.x == 0) {
+                sh.above = above;
+                sh.prefix = prefix | ((unsigned)bin << shift);
+            }
         }
         __syncthreads();
     }
@@ -269,7 +416,7 @@ __device__ unsigned radix_descend(SampleShared& sh, int V, unsigned long long ta
 }
 
 __global__ void __launch_bounds__(SM_THREADS)
-sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
+sample_kernel(const float* __restrict__ logits, long long row_stride, int V, int C, int slice,
               int* __restrict__ out, float inv_temperature, int top_k, float top_p,
               unsigned long long seed, const long long* __restrict__ seq_ids,
               const int* __restrict__ steps, const int* __restrict__ dev_params) {
@@ -283,79 +430,213 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
                ((unsigned long long)(unsigned)dev_params[SP_SEED_HI] << 32);
     }
     __shared__ SampleShared sh;
-    const float* row = logits + (size_t)blockIdx.x * row_stride;
-    auto xval = [&](int i) { return row[i] * inv_temperature; };
+    extern __shared__ __align__(16) float resident[];
+    float* val = resident;                                // the slice: logits, then weights
+    bool listed = false;                                  // the candidates instead of the slice
+    const int rank = C > 1 ? (int)cluster_rank() : 0;
+    const int row_id = blockIdx.x / C;
+    const float* row = logits + (size_t)row_id * row_stride;
+    const int lo = min(V, rank * slice);
+    int n = min(V, lo + slice) - lo;
+    int held = min(n, SM_RESIDENT);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int elements = (n + SM_THREADS - 1) / SM_THREADS;            // of a thread, SM_THREADS apart
+    int turn = 0;
 
-    // 1. top-k threshold on the scaled logits
-    unsigned kth_key = 0;
-    if (top_k > 0 && top_k < V)
-        kth_key = radix_descend<true>(sh, V, (unsigned long long)top_k,
-                                      [&](int i) { return ordered_key(xval(i)); },
-                                      [&](int) { return 1ull; });
-    // 2. maximum (always kept)
+    // 1. the slice, divided by the temperature; its maximum and the thread's greatest key
     float mx = -INFINITY;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) mx = fmaxf(mx, xval(i));
-    mx = block_max(mx, sh.red);
-    auto weight = [&](int i) -> float {
-        const float x = xval(i);
-        if (ordered_key(x) < kth_key) return 0.f;
-        return expf(x - mx);
+    unsigned best = 0;
+    auto take = [&](int i, float raw) {
+        const float x = raw * inv_temperature;
+        mx = fmaxf(mx, x);
+        best = max(best, ordered_key(x));
+        if (i < SM_RESIDENT) val[i] = x;
     };
-    // 3. top-p threshold on the weights (all >= 0, so their bits order them)
+    if (((uintptr_t)(row + lo) & 15) == 0) {
+        const float4* src = reinterpret_cast<const float4*>(row + lo);
+#pragma unroll 4
+        for (int i = tid; i < n / 4; i += SM_THREADS) {
+            const float4 v = __ldcs(src + i);
+            take(4 * i, v.x); take(4 * i + 1, v.y); take(4 * i + 2, v.z); take(4 * i + 3, v.w);
+        }
+        for (int i = n / 4 * 4 + tid; i < n; i += SM_THREADS) take(i, row[lo + i]);
+    } else {
+#pragma unroll 4
+        for (int i = tid; i < n; i += SM_THREADS) take(i, row[lo + i]);
+    }
+    mx = block_max(mx, sh.red);
+    auto scaled = [&](int i) { return i < held ? val[i] : row[lo + i] * inv_temperature; };
+
+    // 2. top-k threshold on the scaled logits.  The k-th greatest of the threads' greatest keys
+    // is at most the k-th greatest key of the slice, and that at most the row's: only elements
+    // that reach the best such bound of the cluster are counted.
+    const bool by_count = top_k > 0 && top_k < V;
+    unsigned bound = 0;
+    if (by_count && top_k <= SM_THREADS) {
+        bound = radix_descend<true>(sh, 1, turn, (unsigned long long)top_k, 1,
+                                    [&](int, int, auto&& add) { add(best, 1ull); });
+    }
+    if (C > 1) {
+        if (tid == 0) { sh.mx = mx; sh.bound = bound; }
+        cluster_meet();
+        for (int r = 0; r < C; ++r) {
+            mx = fmaxf(mx, __uint_as_float(peer_u32(&sh.mx, r)));
+            bound = max(bound, peer_u32(&sh.bound, r));
+        }
+    }
+    // Where a top-k left few candidates (about C k of them), CTA 0 gets them all, in index order,
+    // and finishes alone: the meetings of the cluster are what the passes below cost.
+    auto index_range = [&](int& a, int& b) {              // a warp's, in whole 32s
+        const int per = ((n + SM_THREADS / 32 - 1) / (SM_THREADS / 32) + 31) / 32 * 32;
+        a = min(n, warp * per);
+        b = min(n, a + per);
+    };
+    if (C > 1 && by_count && top_k <= SM_THREADS) {
+        int a, b, count = 0;
+        index_range(a, b);
+        for (int i = a + lane; i < b; i += 32) count += ordered_key(scaled(i)) >= bound;
+        count = __reduce_add_sync(0xffffffffu, count);
+        if (lane == 0) sh.wsum[warp] = (unsigned long long)count;
+        __syncthreads();
+        const int of_warp = (int)sh.wsum[lane];
+        const int all = __reduce_add_sync(0xffffffffu, of_warp);
+        int at = __reduce_add_sync(0xffffffffu, lane < warp ? of_warp : 0);
+        if (tid == 0) sh.n_list = all;
+        cluster_meet();
+        int total = 0;
+        for (int r = 0; r < C; ++r) {
+            const int c = (int)peer_u32(&sh.n_list, r);
+            if (r < rank) at += c;
+            total += c;
+        }
+        if (total <= SM_LIST) {
+            const unsigned px = peer_address(sh.list_x, 0), pi = peer_address(sh.list_i, 0);
+            for (int i0 = a; i0 < b; i0 += 32) {
+                const int i = i0 + lane;
+                const float x = i < b ? scaled(i) : 0.f;
+                const bool is = i < b && ordered_key(x) >= bound;
+                const unsigned who = __ballot_sync(0xffffffffu, is);
+                if (is) {
+                    const unsigned o = 4u * (unsigned)(at + __popc(who & ((1u << lane) - 1)));
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(px + o), "f"(x) : "memory");
+                    asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(pi + o), "r"(lo + i) : "memory");
+                }
+                at += __popc(who);
+            }
+            cluster_meet();
+            if (rank != 0) return;
+            listed = true;
+            val = sh.list_x;
+            n = held = total;
+            elements = (n + SM_THREADS - 1) / SM_THREADS;
+            bound = 0;
+            C = 1;
+        }
+    }
+    unsigned kth_key = 0;
+    if (by_count)
+        kth_key = radix_descend<true>(sh, C, turn, (unsigned long long)top_k, elements,
+                                      [&](int e0, int e1, auto&& add) {
+            for (int e = e0; e < e1; ++e) {
+                const int i = tid + e * SM_THREADS;
+                if (i >= n) break;
+                const unsigned key = ordered_key(scaled(i));
+                if (key >= bound) add(key, 1ull);
+            }
+        });
+    // 3. the weights take the logits' place; their sum
+    auto weigh = [&](float x) { return ordered_key(x) < kth_key ? 0.f : expf(x - mx); };
+    for (int i = tid; i < held; i += SM_THREADS) val[i] = weigh(val[i]);
+    auto weight = [&](int i) { return i < held ? val[i] : weigh(row[lo + i] * inv_temperature); };
     unsigned cut_bits = 0;
     if (top_p > 0.f && top_p < 1.f) {
+        // top-p threshold (the weights are >= 0, so their bits order them)
         unsigned long long part = 0;
-        for (int i = threadIdx.x; i < V; i += blockDim.x) part += to_fixed(weight(i));
-        if (threadIdx.x == 0) sh.above = 0;
+        for (int i = tid; i < n; i += SM_THREADS) part += to_fixed(weight(i));
+        part = warp_sum_u64(part);
+        if (lane == 0) sh.wsum[warp] = part;
         __syncthreads();
-        atomicAdd(&sh.above, part);
+        if (warp == 0) {
+            part = warp_sum_u64(sh.wsum[lane]);
+            if (lane == 0) sh.total_mass = part;
+        }
         __syncthreads();
-        const unsigned long long total = sh.above;
-        __syncthreads();
+        unsigned long long total = sh.total_mass;
+        if (C > 1) {
+            cluster_meet();
+            total = 0;
+            for (int r = 0; r < C; ++r) total += peer_u64(&sh.total_mass, r);
+        }
         const unsigned long long target = (unsigned long long)((double)top_p * (double)total);
-        cut_bits = radix_descend<false>(sh, V, target > 0 ? target : 1ull,
-                                        [&](int i) { return __float_as_uint(weight(i)); },
-                                        [&](int i) { return to_fixed(weight(i)); });
+        cut_bits = radix_descend<false>(sh, C, turn, target > 0 ? target : 1ull, elements,
+                                        [&](int e0, int e1, auto&& add) {
+            for (int e = e0; e < e1; ++e) {
+                const int i = tid + e * SM_THREADS;
+                if (i >= n) break;
+                const float w = weight(i);
+                if (w != 0.f) add(__float_as_uint(w), to_fixed(w));
+            }
+        });
     }
+    __syncthreads();
     auto kept = [&](int i) -> unsigned long long {
         const float w = weight(i);
         return __float_as_uint(w) >= cut_bits ? to_fixed(w) : 0ull;
     };
-    // 4. draw in index order: contiguous chunk per thread, scan of chunk sums
-    const int per = (V + blockDim.x - 1) / blockDim.x;
-    const int lo = min(V, (int)threadIdx.x * per), hi = min(V, lo + per);
+    // 4. draw in index order: a contiguous range per warp (whole 32s), sums over the ranges
+    int w0, w1;
+    index_range(w0, w1);
     unsigned long long mine = 0;
-    for (int i = lo; i < hi; ++i) mine += kept(i);
-    sh.chunk[threadIdx.x] = mine;
-    if (threadIdx.x == 0) { sh.done = 0; sh.result = V - 1; }
+    for (int i = w0 + lane; i < w1; i += 32) mine += kept(i);
+    mine = warp_sum_u64(mine);
+    if (lane == 0) sh.wsum[warp] = mine;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long run = 0;
-        for (int i = 0; i < (int)blockDim.x; ++i) {
-            const unsigned long long c = sh.chunk[i];
-            sh.chunk[i] = run;
-            run += c;
-        }
-        sh.above = run;
+    unsigned long long upto = sh.wsum[lane];               // inclusive sums over the warps
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += t;
     }
-    __syncthreads();
-    const unsigned long long total = sh.above;
+    unsigned long long total = __shfl_sync(0xffffffffu, upto, 31);
+    unsigned long long before = __shfl_sync(0xffffffffu, upto, warp) - mine;   // ranges before this warp's
+    if (C > 1) {
+        if (tid == 0) sh.slice_sum = total;
+        cluster_meet();
+        total = 0;
+        for (int r = 0; r < C; ++r) {
+            const unsigned long long s = peer_u64(&sh.slice_sum, r);
+            if (r < rank) before += s;
+            total += s;
+        }
+    }
     const unsigned long long h =
         splitmix64(splitmix64(seed ^ 0xA5A5A5A5DEADBEEFull) ^
-                   splitmix64((unsigned long long)seq_ids[blockIdx.x] * 0x100000001B3ull +
-                              (unsigned long long)(unsigned)steps[blockIdx.x]));
+                   splitmix64((unsigned long long)seq_ids[row_id] * 0x100000001B3ull +
+                              (unsigned long long)(unsigned)steps[row_id]));
     const double u = (double)(h >> 11) * (1.0 / 9007199254740992.0);     // [0, 1)
     const unsigned long long thr = (unsigned long long)(u * (double)total);
-    const unsigned long long before = sh.chunk[threadIdx.x];
     if (mine > 0 && before <= thr && thr < before + mine) {
         unsigned long long run = before;
-        for (int i = lo; i < hi; ++i) {
-            run += kept(i);
-            if (thr < run) { sh.result = i; break; }
+        for (int i0 = w0; i0 < w1; i0 += 32) {
+            unsigned long long sum = i0 + lane < w1 ? kept(i0 + lane) : 0ull;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long t = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += t;
+            }
+            const unsigned over = __ballot_sync(0xffffffffu, thr < run + sum);
+            if (over) {
+                const int i = i0 + __ffs(over) - 1;
+                if (lane == 0) out[row_id] = listed ? sh.list_i[i] : lo + i;
+                break;
+            }
+            run += __shfl_sync(0xffffffffu, sum, 31);
         }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) out[blockIdx.x] = sh.result;
+    // (no weight at all, or a sum that rounds up to the total: the last index)
+    if (rank == 0 && tid == 0 && thr >= total) out[row_id] = V - 1;
+    // a CTA's shared memory stays until its peers have read it
+    if (C > 1) cluster_meet();
 }
 
 // One token per row of logits [B, V].  temperature > 0; top_k 0 = off; top_p
@@ -371,9 +652,18 @@ AGV_API int agv_sample(const float* logits, long long row_stride, int B, int V, 
                 "sample: temperature must be positive (0 is arg max)");
     AGV_REQUIRE(top_k >= 0, "sample: top_k must be >= 0");
     if (B == 0) return 0;
-    agv_launch(sample_kernel, B, SM_THREADS, 0, stream, logits, row_stride, V, out,
-               dev_params ? 1.0f : 1.0f / temperature, top_k, top_p, seed, seq_ids, steps,
-               dev_params);
+    // A slice of at most 32,768 values (32 a thread) where eight CTAs can give that; a slice starts
+    // on a multiple of four values, so that a row on a 16-byte boundary is read 16 bytes at a time.
+    int C = 1;
+    while (C < 8 && V > 16384 * C) C *= 2;
+    const int slice = ((V + C - 1) / C + 3) / 4 * 4;
+    AGV_REQUIRE((long long)B * C <= 0x7fffffffLL, "sample: %d rows exceed the grid limit", B);
+    const size_t smem = (size_t)(slice < SM_RESIDENT ? slice : SM_RESIDENT) * sizeof(float);
+    AGV_CUDA_OK(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     SM_RESIDENT * (int)sizeof(float)));
+    agv_launch_cluster(sample_kernel, dim3((unsigned)(B * C)), SM_THREADS, smem, stream, dim3(C), logits,
+                       row_stride, V, C, slice, out, dev_params ? 1.0f : 1.0f / temperature, top_k,
+                       top_p, seed, seq_ids, steps, dev_params);
     AGV_LAUNCH_OK("sample_kernel");
     return 0;
 }

@@ -633,6 +633,58 @@ def test_sampling_matches_the_filtered_distribution():
     assert torch.equal(out2, out[perm])
 
 
+def _splitmix64(x):
+    M = (1 << 64) - 1
+    x = (x + 0x9E3779B97F4A7C15) & M
+    x = ((x ^ (x >> 30)) * 0xBF58476D1CE4E5B9) & M
+    x = ((x ^ (x >> 27)) * 0x94D049BB133111EB) & M
+    return x ^ (x >> 31)
+
+
+@pytest.mark.parametrize("V", [1, 33, 16384, 16385, 65539, 262208, 400003])
+@pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (1, 1.0), (64, 0.95), (1500, 0.9), (0, 0.7)])
+def test_sampling_of_long_rows_against_the_procedure(V, top_k, top_p):
+    """The token of every row lies where the uniform number falls in the running sum, in index
+    order, of the weights that top-k and top-p keep: one CTA a row and a cluster of 2, 4 and 8,
+    slices in shared memory and (400,003) partly beyond it; ordinary rows, equal values, masked
+    ones and a row stride that is not a multiple of four.  The fixed-point weights are those of
+    another exponential, a unit in the last place off: 1e-6 of the sum is allowed for."""
+    from agave_b200 import kernels
+    T, seed, B = 0.8, 77, 6
+    logits = torch.empty((B, V + (V % 2)), dtype=torch.float32, device=DEV)[:, :V]
+    logits.copy_(rnd(B, V, seed=V) * 3.0)
+    logits[1] = 1.25
+    logits[2] = torch.round(logits[2])
+    logits[3, : V // 2] = -math.inf
+    logits[4, V // 3:] = -math.inf if V > 3 else 0.0
+    seq = torch.arange(10, 10 + B, dtype=torch.int64, device=DEV)
+    steps = torch.arange(B, dtype=torch.int32, device=DEV) * 3
+    out = torch.full((B,), -5, dtype=torch.int32, device=DEV)
+    kernels.sample(logits, out, T, top_k, top_p, seed, seq, steps)
+    for b, tok in enumerate(out.tolist()):
+        x = (logits[b] * torch.tensor(1.0 / T, dtype=torch.float32, device=DEV))
+        w = torch.exp((x - x.max()).double())
+        if 0 < top_k < V:
+            w[x < torch.topk(x, top_k).values[-1]] = 0.0
+        if top_p < 1.0:
+            order, _ = torch.sort(w, descending=True)
+            reach = torch.searchsorted(torch.cumsum(order, 0), top_p * order.sum() * (1 - 1e-6))
+            cut = order[min(int(reach), V - 1)]
+        else:
+            cut = torch.zeros((), dtype=torch.float64, device=DEV)
+        assert 0 <= tok < V and float(w[tok]) >= float(cut) * (1 - 1e-6) and float(w[tok]) > 0
+        # (values next to the cut may fall on either side of it: the sums with and without them)
+        h = _splitmix64(_splitmix64(seed ^ 0xA5A5A5A5DEADBEEF) ^
+                        _splitmix64((int(seq[b]) * 0x100000001B3 + int(steps[b])) & ((1 << 64) - 1)))
+        u = (h >> 11) / 2.0 ** 53
+        at_cut = (w >= cut * (1 - 1e-6)) & (w <= cut * (1 + 1e-6)) & (w > 0)
+        sure = torch.where((w >= cut) | at_cut, w, torch.zeros_like(w))
+        total = float(sure.sum())
+        slack = 1e-6 * total + (float(w[at_cut].max()) if int(at_cut.sum()) == 1 else 0.0)
+        upto = float(sure[: tok + 1].sum())
+        assert upto - float(w[tok]) - slack <= u * total <= upto + slack, (b, tok, u)
+
+
 def test_repeat_penalty_per_occurrence_and_history():
     from agave_b200 import kernels
     V = 300
