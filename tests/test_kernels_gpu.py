@@ -234,6 +234,32 @@ def test_linear_simt_plain_and_gated(dtype):
         assert rel_err(o, big.double() @ wb.double().T) < 2e-6
 
 
+@pytest.mark.parametrize("N,K", [(1, 384), (33, 388), (200, 1152), (4200, 500), (13000, 384), (131, 2308)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_linear_simt_rows_do_not_depend_on_their_company(N, K, gated):
+    """The 32-bit products over every number of rows at which another kernel or tile takes over
+    (4, 8, 16, 32, 64), with one, two and four ranges of K a warp, ranges that no piece of 32
+    divides, and strided x and out: against 64 bits, and every row bit for bit what it is alone.
+    A chain of K / 8 roundings of 2^-24 each, added in pairs: 2e-6 of the largest value is far
+    above what they add up to."""
+    from agave_b200 import kernels
+    w, w2 = rnd(N, K, seed=2), rnd(N, K, seed=3) if gated else None
+    x = torch.empty((130, K + 4), device=DEV)[:, :K]
+    x.copy_(rnd(130, K, seed=1))
+    ref = x.double() @ w.double().T
+    if gated:
+        ref = torch.nn.functional.silu(ref) * (x.double() @ w2.double().T)
+    outs = {}
+    for M in (1, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 130):
+        out = torch.full((M, N + 3), float("nan"), device=DEV)
+        kernels.linear_simt(x[130 - M:], w, out[:, :N], w2=w2, activation="silu")
+        assert torch.isnan(out[:, N:]).all()
+        outs[M] = out[:, :N]
+    assert rel_err(outs[130], ref) < (4e-6 if gated else 2e-6)
+    for M, out in outs.items():
+        assert torch.equal(out, outs[130][130 - M:]), M
+
+
 # ---------------------------------------------------------------------- norms
 @pytest.mark.parametrize("H,R", [(48, 7), (1000, 7), (5376, 7), (1152, 300), (2048, 257), (72, 513),
                                  (2560, 300), (5376, 260), (8192, 257), (2052, 258),
