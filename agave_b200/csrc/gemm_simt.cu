@@ -110,7 +110,7 @@ gemm_any_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const TW* __
 // What bounds it: with few rows of x the weight's bytes, so eight warps share a group of 32
 // weight rows where those are few (R = 1: a 1152 x 6912 weight is 36 groups, 288 warps), and a
 // warp takes more of K where there are many and the ends of its walk would cost (R = 2, 4); with
-many rows of x the multiply-adds.  3 rows of x, against tiles of 64 x 64 over all of K:
+// many rows of x the multiply-adds.  3 rows of x, against tiles of 64 x 64 over all of K:
 // 1152 x 6912 603 -> 22.4 us, 6912 x 1152 gated 135 -> 26.7, 262144 x 1152 1,284 -> 240 (5.0 TB/s),
 // 1536 x 1152 101 -> 12.3 (the figures hold about 6 us of launch and events).
 constexpr int GS_ROWS = 32;                    // weight rows of a warp
