@@ -128,6 +128,151 @@ delta_prepare_kernel(RowIn<T> in, DeltaDims dm, DeltaState st, const float* __re
         low_g[(size_t)t * dm.rg + i] = from_f32<T>(rowbuf[C + dm.H + dm.ra + i]);
 }
 
+// The same where the row comes in 32-bit in whole 16-byte pieces, with two to four taps and heads of
+// up to 256: a warp has R tokens of one q or k head, of 128 NJ columns of v, or of 32 of the last
+// columns (b, a1, g1), a lane four neighbouring channels, whose inputs slide through registers.
+// What no kernel of the step writes (weights, the ring, the step's arrays) is asked for before the
+// dependency wait.
+//
+// A decode step is bound by trips to memory one after the other: a CTA a token walked its 3,216
+// columns in a dozen of them, 35 us for 8 tokens (G 4, H 16, heads of 128, eight partial sums);
+// 31 warps a token make two, 4.7 us.  A prompt is bound by its rows (126 MB for 5,120 tokens, 20
+// us): 191 us -> 122 us with R = 8, which reads a row once instead of once a tap.
+template <typename T, int TAPS, int NJ, int R>
+__global__ void __launch_bounds__(128)
+delta_prepare_rows_kernel(RowIn<float> in, DeltaDims dm, DeltaState st, int n_tokens, int n_seg,
+                          const float* __restrict__ conv_w, float eps_unit, float q_mult, int fused_state,
+                          float* __restrict__ qkv, float* __restrict__ beta, T* __restrict__ low_a,
+                          T* __restrict__ low_g) {
+    constexpr int RING = TAPS - 1, SW = NJ * 128;
+    const int lane = threadIdx.x & 31;
+    const long long w = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int tile = (int)(w / n_seg), seg = (int)(w - (long long)tile * n_seg);
+    const int t0 = tile * R;
+    const int C = dm.C(), nq = dm.nq(), nv = dm.nv();
+    const int v_seg = (nv + SW - 1) / SW, conv_seg = 2 * dm.G + v_seg;
+    if (t0 >= n_tokens) return;
+    if (seg >= conv_seg) {
+        pdl_wait();
+        pdl_launch_next();
+        const int e = (seg - conv_seg) * 32 + lane;
+        if (e >= dm.H + dm.ra + dm.rg) return;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int t = t0 + i;
+            if (t >= n_tokens) break;
+            if (st.slots[st.seq_index[t]] < 0) continue;
+            const float x = in.at(t, C + e);
+            if (e < dm.H) beta[(size_t)t * dm.H + e] = sigmoid_f(x);
+            else if (e < dm.H + dm.ra) low_a[(size_t)t * dm.ra + e - dm.H] = from_f32<T>(x);
+            else low_g[(size_t)t * dm.rg + e - dm.H - dm.ra] = from_f32<T>(x);
+        }
+        return;
+    }
+    const bool head = seg < 2 * dm.G;
+    const int c0 = head ? seg * dm.d : 2 * nq + (seg - 2 * dm.G) * SW;
+    const int width = head ? dm.d : min(SW, nv - (seg - 2 * dm.G) * SW);
+    float wv[NJ][4 * TAPS];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+        const int ch = j * 128 + lane * 4;
+#pragma unroll
+        for (int k = 0; k < TAPS; ++k) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (ch < width) v = *reinterpret_cast<const float4*>(conv_w + (size_t)(c0 + ch) * TAPS + 4 * k);
+            wv[j][4 * k] = v.x; wv[j][4 * k + 1] = v.y; wv[j][4 * k + 2] = v.z; wv[j][4 * k + 3] = v.w;
+        }
+    }
+    int pos[R], slot[R], before[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int t = min(t0 + i, n_tokens - 1), b = st.seq_index[t];
+        pos[i] = st.positions[t];
+        slot[i] = st.slots[b];
+        before[i] = t - st.cu[b];
+    }
+    // the ring's rows before the tile's first token (later tokens of the tile that reach further
+    // back than their sequence's first token in the step read it themselves, below)
+    float4 old[NJ][RING];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int k = 1; k <= RING; ++k) {
+            const int ch = j * 128 + lane * 4;
+            old[j][k - 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (ch < width && slot[0] >= 0 && k > before[0] && pos[0] - k >= 0)
+                old[j][k - 1] = *reinterpret_cast<const float4*>(
+                    st.state + (size_t)slot[0] * st.stride + st.conv_off + (size_t)((pos[0] - k) % RING) * C + c0 + ch);
+        }
+    pdl_wait();
+    pdl_launch_next();
+    float4 xs[NJ][R + RING];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < R + RING; ++i) {
+            const int t = t0 - RING + i, ch = j * 128 + lane * 4;
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+            // (one token a tile: earlier tokens of the step are other sequences')
+            if ((R > 1 || i == RING) && t >= 0 && t < n_tokens && ch < width) {
+                if (in.part) {
+                    const float* p = in.part + (size_t)t * in.W + c0 + ch;
+#pragma unroll 8
+                    for (int sp = 0; sp < in.n_splits; ++sp) {
+                        const float4 v = *reinterpret_cast<const float4*>(p + (size_t)sp * in.split_stride);
+                        a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+                    }
+                } else {
+                    a = *reinterpret_cast<const float4*>(in.row + (size_t)t * in.ld + c0 + ch);
+                }
+            }
+            xs[j][i] = a;
+        }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int t = t0 + i;
+        if (t >= n_tokens) break;
+        if (slot[i] < 0) continue;
+        const float* ring = st.state + (size_t)slot[i] * st.stride + st.conv_off + c0;
+        float y[NJ][4], ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const int ch = j * 128 + lane * 4;
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int k = RING; k >= 1; --k) {              // oldest input first
+                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (R > 1 && k <= before[i]) x = xs[j][RING + i - k];
+                else if (i == 0) x = old[j][k - 1];
+                else if (pos[i] - k >= 0 && ch < width)
+                    x = *reinterpret_cast<const float4*>(ring + (size_t)((pos[i] - k) % RING) * C + ch);
+                const float xe[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[e] = fmaf(wv[j][e * TAPS + RING - k], xe[e], acc[e]);
+            }
+            const float4 x = xs[j][RING + i];
+            const float xe[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                y[j][e] = silu_f(fmaf(wv[j][e * TAPS + RING], xe[e], acc[e]));
+                ss = fmaf(y[j][e], y[j][e], ss);
+            }
+            if (fused_state && ch < width)                 // (the row that position p - RING had)
+                *reinterpret_cast<float4*>(st.state + (size_t)slot[i] * st.stride + st.conv_off +
+                                           (size_t)(pos[i] % RING) * C + c0 + ch) = x;
+        }
+        float r = 1.f;
+        if (head) r = (1.0f / sqrtf(warp_sum(ss) + eps_unit)) * (seg < dm.G ? q_mult : 1.0f);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const int ch = j * 128 + lane * 4;
+            if (ch < width)
+                *reinterpret_cast<float4*>(qkv + (size_t)t * C + c0 + ch) =
+                    make_float4(y[j][0] * r, y[j][1] * r, y[j][2] * r, y[j][3] * r);
+        }
+    }
+}
+
 // The convolution's inputs after a step of several tokens a sequence: the step's last
 // taps - 1 positions go to their rows of the ring (fewer, if the step is shorter: the rows of
 // earlier positions stay).  One CTA per sequence, a thread a channel; it runs after the
@@ -379,32 +524,71 @@ delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
 }
 
 // ---------------------------------------------------------------- read-out
-// y[t, h, :] = o[t, h, :] / rms(o[t, h, :]) * w * sigmoid(gate[t, h, :]): one CTA a token,
-// a warp a head.
-template <typename T>
+// y[t, h, :] = o[t, h, :] / rms(o[t, h, :]) * w * sigmoid(gate[t, h, :]): a warp a head, a lane V
+// neighbouring columns at a time, whose o and gate are asked for together.  Bound by the trip to
+// memory when decoding (8 tokens, 16 heads of 128: one warp of four a CTA went through four heads,
+// two trips each, 10.6 us -> 2.6 us), by the bytes in a prompt (5,120 tokens, 105 MB, 16 us:
+// 46 -> 41).
+constexpr int DO_MAX = 16;         // values of a head a lane keeps; the rest is read again
+template <typename T, int V>
 __global__ void __launch_bounds__(128)
 delta_out_kernel(const float* __restrict__ o, const float* __restrict__ gate,
                  const float* __restrict__ w, float eps, int n_tokens, int H, int dv,
                  const int* __restrict__ seq_index, const int* __restrict__ slots,
                  T* __restrict__ y) {
+    constexpr int NJ = DO_MAX / V;
+    const int lane = threadIdx.x & 31;
+    const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (item >= (long long)n_tokens * H) return;
+    const bool pad = slots[seq_index[item / H]] < 0;      // a padding entry's row is zeros
+    const size_t base = (size_t)item * dv;
     pdl_wait();
     pdl_launch_next();
-    const int t = blockIdx.x;
-    const bool pad = slots[seq_index[t]] < 0;      // a padding entry's row is zeros
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int h = warp; h < H; h += nwarps) {
-        const size_t base = ((size_t)t * H + h) * dv;
-        if (pad) {
-            for (int i = lane; i < dv; i += 32) y[base + i] = from_f32<T>(0.f);
-            continue;
+    float ov[DO_MAX], gv[DO_MAX], ss = 0.f;
+    auto load = [&](const float* p, float* to) {
+        if constexpr (V == 4) {
+            const float4 x = *reinterpret_cast<const float4*>(p);
+            to[0] = x.x; to[1] = x.y; to[2] = x.z; to[3] = x.w;
+        } else {
+            to[0] = *p;
         }
-        float ss = 0.f;
-        for (int i = lane; i < dv; i += 32) ss = fmaf(o[base + i], o[base + i], ss);
-        ss = warp_sum(ss);
-        const float r = 1.0f / sqrtf(ss / (float)dv + eps);
-        for (int i = lane; i < dv; i += 32)
-            y[base + i] = from_f32<T>(o[base + i] * r * w[i] * sigmoid_f(gate[base + i]));
+    };
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+        const int i = (j * 32 + lane) * V;
+        if (i < dv) {
+            load(o + base + i, ov + j * V);
+            load(gate + base + i, gv + j * V);
+#pragma unroll
+            for (int e = 0; e < V; ++e) ss = fmaf(ov[j * V + e], ov[j * V + e], ss);
+        }
     }
+    for (int i = (NJ * 32 + lane) * V; i < dv; i += 32 * V)
+#pragma unroll
+        for (int e = 0; e < V; ++e) ss = fmaf(o[base + i + e], o[base + i + e], ss);
+    ss = warp_sum(ss);
+    const float r = 1.0f / sqrtf(ss / (float)dv + eps);
+    auto store = [&](int i, const float* a, const float* g) {
+        float v[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) v[e] = pad ? 0.f : a[e] * r * w[i + e] * sigmoid_f(g[e]);
+        if constexpr (V == 4 && sizeof(T) == 2) {
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+            uint2 b;
+            b.x = *reinterpret_cast<const uint32_t*>(&lo);
+            b.y = *reinterpret_cast<const uint32_t*>(&hi);
+            *reinterpret_cast<uint2*>(y + base + i) = b;
+        } else {
+#pragma unroll
+            for (int e = 0; e < V; ++e) y[base + i + e] = from_f32<T>(v[e]);
+        }
+    };
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+        const int i = (j * 32 + lane) * V;
+        if (i < dv) store(i, ov + j * V, gv + j * V);
+    }
+    for (int i = (NJ * 32 + lane) * V; i < dv; i += 32 * V) store(i, o + base + i, gate + base + i);
 }
 
 }  // namespace
@@ -442,6 +626,40 @@ AGV_API int agv_delta_prepare(const void* row, long long ld, const float* part, 
                 "delta_prepare: the state is too small");
     if (T == 0) return 0;
     const DeltaState st{state, state_stride, conv_off, slots, cu, seq_index, positions};
+    // The rows form; a step of one token a sequence takes a token a warp, which alone has the warps
+    // to hide its trips, others eight.
+    const int W = dm.W(), C = dm.C();
+    if ((part || dtype == AGV_F32) && (part || ld % 4 == 0) && W % 4 == 0 && C % 4 == 0 && d % 4 == 0 &&
+        d <= 256 && taps >= 2 && taps <= 4 && state_stride % 4 == 0 && conv_off % 4 == 0 &&
+        agv_aligned(row, 16) && agv_aligned(part, 16) && agv_aligned(conv_w, 16) && agv_aligned(state, 16) &&
+        agv_aligned(qkv, 16)) {
+        AGV_REQUIRE(dtype == AGV_F32 || dtype == AGV_BF16, "delta_prepare: unknown dtype %d", dtype);
+        const RowIn<float> in{(const float*)row, ld, part, n_splits, (long long)T * W, W};
+        const int NJ = d <= 128 ? 1 : 2, R = several ? 8 : 1;
+        const int n_seg = 2 * G + (dm.nv() + NJ * 128 - 1) / (NJ * 128) + (H + ra + rg + 31) / 32;
+        const long long warps = (long long)((T + R - 1) / R) * n_seg;
+        AGV_REQUIRE((warps + 3) / 4 <= 0x7fffffffLL, "delta_prepare: %d tokens exceed the grid limit", T);
+        auto go = [&](auto kern, auto* la, auto* lg) {
+            agv_launch(kern, (unsigned)((warps + 3) / 4), 128, 0, stream, in, dm, st, T, n_seg, conv_w, eps_unit,
+                       q_mult, several ? 0 : 1, qkv, beta, la, lg);
+        };
+#define AGV_DPR(TT, TAPS, N) do {                                                                        \
+        if (several) go(delta_prepare_rows_kernel<TT, TAPS, N, 8>, (TT*)low_a, (TT*)low_g);              \
+        else go(delta_prepare_rows_kernel<TT, TAPS, N, 1>, (TT*)low_a, (TT*)low_g); } while (0)
+#define AGV_DPT(TT) do {                                                                                 \
+        if (taps == 4) { if (NJ == 1) AGV_DPR(TT, 4, 1); else AGV_DPR(TT, 4, 2); }                       \
+        else if (taps == 3) { if (NJ == 1) AGV_DPR(TT, 3, 1); else AGV_DPR(TT, 3, 2); }                  \
+        else { if (NJ == 1) AGV_DPR(TT, 2, 1); else AGV_DPR(TT, 2, 2); } } while (0)
+        if (dtype == AGV_F32) AGV_DPT(float); else AGV_DPT(__nv_bfloat16);
+#undef AGV_DPT
+#undef AGV_DPR
+        AGV_LAUNCH_OK("delta_prepare_rows_kernel");
+        if (several) {
+            agv_launch(delta_conv_state_kernel<float>, (unsigned)B, 256, 0, stream, in, dm, st);
+            AGV_LAUNCH_OK("delta_conv_state_kernel");
+        }
+        return 0;
+    }
     const size_t smem = (size_t)(dm.C() + dm.W()) * sizeof(float);
 #define AGV_DP(TT)                                                                              \
     do {                                                                                        \
@@ -523,14 +741,14 @@ AGV_API int agv_delta_out(const float* o, const float* gate, const float* w, flo
                           int dtype, cudaStream_t stream) {
     AGV_REQUIRE(T >= 0 && H > 0 && dv > 0, "delta_out: bad sizes");
     if (T == 0) return 0;
-    if (dtype == AGV_F32)
-        agv_launch(delta_out_kernel<float>, (unsigned)T, 128, 0, stream, o, gate, w, eps, T, H, dv,
-                   seq_index, slots, (float*)y);
-    else if (dtype == AGV_BF16)
-        agv_launch(delta_out_kernel<__nv_bfloat16>, (unsigned)T, 128, 0, stream, o, gate, w, eps, T,
-                   H, dv, seq_index, slots, (__nv_bfloat16*)y);
-    else
-        return agv_fail(-1, "delta_out: unknown dtype %d", dtype);
+    const bool four = dv % 4 == 0 && agv_aligned(o, 16) && agv_aligned(gate, 16) && agv_aligned(y, 8);
+    const unsigned grid = (unsigned)(((long long)T * H + 3) / 4);
+#define AGV_DO(TT, VV) agv_launch(delta_out_kernel<TT, VV>, grid, 128, 0, stream, o, gate, w, eps, T, H, dv, \
+                                  seq_index, slots, (TT*)y)
+    if (dtype == AGV_F32) { if (four) AGV_DO(float, 4); else AGV_DO(float, 1); }
+    else if (dtype == AGV_BF16) { if (four) AGV_DO(__nv_bfloat16, 4); else AGV_DO(__nv_bfloat16, 1); }
+    else return agv_fail(-1, "delta_out: unknown dtype %d", dtype);
+#undef AGV_DO
     AGV_LAUNCH_OK("delta_out_kernel");
     return 0;
 }

@@ -1,0 +1,154 @@
+"""Kernels that move a token's row four values or 16 bytes at a time, against their general forms
+(which a weight off its 16-byte boundary selects), at the edges of their warps, tiles and pieces."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+BF, F32 = torch.bfloat16, torch.float32
+
+
+def rnd(*shape, dtype=F32, seed=0, scale=1.0):
+    g = torch.Generator(device="cpu").manual_seed(seed)
+    return (torch.randn(*shape, generator=g) * scale).to(dtype).to(DEV)
+
+
+def off(t):
+    """The same values one element off a 16-byte boundary."""
+    return torch.cat([t.reshape(-1)[:1], t.reshape(-1)])[1:].view(t.shape)
+
+
+def same(a, b, dtype=F32):
+    # (sums in another order: a few roundings of the largest value; bfloat16 results may fall on
+    # either side of a rounding of 2^-9)
+    tol = 3e-6 if dtype == F32 else 2.0 ** -8
+    a, b = a.double(), b.double()
+    assert torch.isfinite(a).all()
+    assert float((a - b).abs().max()) <= tol * float(b.abs().max().clamp_min(1e-30))
+
+
+def step(counts, starts, slots):
+    i = dict(dtype=torch.int32, device=DEV)
+    cu = [0]
+    for n in counts:
+        cu.append(cu[-1] + n)
+    return SimpleNamespace(
+        batch=len(counts), mode="decode" if max(counts) == 1 else "prefill",
+        cu_seqlens=torch.tensor(cu, **i), slots=torch.tensor(slots, **i),
+        seq_index=torch.tensor([b for b, n in enumerate(counts) for _ in range(n)], **i),
+        positions=torch.tensor([s + k for s, n in zip(starts, counts) for k in range(n)], **i))
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("G,H,d,dv,splits,dtype", [(2, 4, 128, 128, 3, BF), (1, 3, 36, 20, 1, BF),
+                                                   (2, 2, 256, 200, 1, F32), (3, 3, 132, 4, 2, F32)])
+@pytest.mark.parametrize("counts,starts", [([1, 1, 1], [5, 0, 2]), ([17, 1, 30], [0, 0, 0]),
+                                           ([9, 3, 2], [4, 1, 0])])
+def test_delta_prepare_rows(taps, G, H, d, dv, splits, dtype, counts, starts):
+    """One token a warp and eight, sequences that begin and end inside a tile or go on from the
+    ring, a padding entry."""
+    from agave_b200 import kernels
+    T, ra, rg = sum(counts), 8, 12
+    C = 2 * G * d + H * dv
+    W = (C + H + ra + rg + 3) // 4 * 4
+    ra += W - (C + H + ra + rg)
+    ctx = step(counts, starts, [2, -1, 0] if max(counts) == 1 else [2, 1, 0])
+    part = rnd(splits, T, W, seed=1)
+    conv_w = rnd(C, taps, seed=2, scale=0.5)
+    off0 = H * dv * d + (-H * dv * d) % 4
+    state0 = rnd(3, off0 + (taps - 1) * C, seed=3)
+    outs = []
+    for w in (conv_w, off(conv_w)):
+        state = state0.clone()
+        qkv, beta = torch.zeros(T, C, device=DEV), torch.zeros(T, H, device=DEV)
+        la, lg = (torch.zeros(T, r, dtype=dtype, device=DEV) for r in (ra, rg))
+        kernels.delta_prepare(None, part, T, ctx, state, off0, G, H, d, dv, taps, ra, rg, w, 1e-6,
+                              0.3, qkv, beta, la, lg)
+        outs.append((qkv, beta, la, lg, state))
+    for a, b in zip(*outs):
+        same(a, b)
+
+
+@pytest.mark.parametrize("T,H,dv", [(1, 3, 128), (9, 16, 128), (5, 2, 516), (4, 1, 700), (130, 3, 4)])
+@pytest.mark.parametrize("dtype", [BF, F32])
+def test_delta_out_by_fours(T, H, dv, dtype):
+    from agave_b200 import kernels
+    ctx = step([1] * T, [1] * T, [-1 if t == 3 else t for t in range(T)])
+    o, gate, w = rnd(T, H * dv, seed=1), rnd(T, H * dv, seed=2), rnd(dv, seed=3)
+    ys = []
+    for g in (gate, off(gate)):
+        y = torch.full((T, H * dv), float("nan"), dtype=dtype, device=DEV)
+        kernels.delta_out(o, g, w, 1e-6, H, dv, ctx, y)
+        ys.append(y)
+    same(*ys, dtype)
+    if T > 3:
+        assert not ys[0][3].any()
+
+
+@pytest.mark.parametrize("T,K,H", [(1, 8, 4), (9, 2048, 2048), (3, 2056, 2052), (2, 4104, 4100)])
+@pytest.mark.parametrize("dtype", [BF, F32])
+def test_row_gate_by_pieces(T, K, H, dtype):
+    from agave_b200 import kernels
+    x, w, y0 = rnd(T, K, dtype=dtype, seed=1), rnd(K, dtype=dtype, seed=2, scale=0.05), rnd(T, H, seed=3)
+    ys = []
+    for v in (w, off(w)):
+        y = y0.clone()
+        kernels.row_gate(x, v, y)
+        ys.append(y)
+    same(*ys)
+
+
+@pytest.mark.parametrize("T,H,E,top", [(1, 8, 4, 2), (64, 2048, 32, 4), (3, 2056, 33, 3), (5, 4616, 70, 6)])
+@pytest.mark.parametrize("dtype", [BF, F32])
+def test_route_of_few_tokens(T, H, E, top, dtype):
+    """A warp an expert: one round of experts and several, rows of one round of pieces and more."""
+    from agave_b200 import kernels
+    x, w = rnd(T, H, dtype=dtype, seed=1), rnd(E, H, dtype=dtype, seed=2, scale=0.05)
+    got = []
+    for v in (w, off(w)):
+        ids = torch.empty(T, top, dtype=torch.int32, device=DEV)
+        wts = torch.empty(T, top, device=DEV)
+        kernels.moe_route(x, v, None, 1, 1, top, ids, wts, softmax_top=True)
+        got.append((ids, wts))
+    assert torch.equal(got[0][0], got[1][0])
+    same(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("T", [3, 70])
+@pytest.mark.parametrize("nq,nk,nv,splits", [(4, 4, 4, 1), (2048, 512, 512, 3), (260, 516, 8, 2), (4000, 2000, 1004, 1)])
+@pytest.mark.parametrize("dtype", [BF, F32])
+def test_proj_norm_by_fours(T, nq, nk, nv, splits, dtype):
+    from agave_b200 import kernels
+    part = rnd(splits, T, nq + nk + nv, seed=1)
+    wq, wk, vf = rnd(nq, seed=2), rnd(nk, seed=3), rnd(T, nv, dtype=dtype, seed=4)
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+    for first in (None, vf):
+        outs = []
+        for w in (wq, off(wq)):
+            out = torch.full((T, nq + nk + nv), float("nan"), dtype=dtype, device=DEV)
+            kernels.proj_norm_store(out, nq, nk, nv, w, wk, 1e-6, pos, partial=part, v_first=first, v_mix=0.3)
+            outs.append(out)
+        same(*outs, dtype)
+
+
+@pytest.mark.parametrize("T", [3, 70])
+@pytest.mark.parametrize("latent", [False, True])
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("A,d,r,R,G", [(16, 128, 64, 192, 16), (3, 4, 8, 4, 0), (2, 20, 24, 36, 40)])
+@pytest.mark.parametrize("dtype", [BF, F32])
+def test_latent_prepare_by_fours(T, latent, interleaved, A, d, r, R, G, dtype):
+    from agave_b200 import kernels
+    Q = 60 if latent else A * (d + r)
+    part = rnd(2, T, Q + R + r + G, seed=1)
+    wq, wc = (rnd(Q, seed=2) if latent else None), rnd(R, seed=3)
+    cos, sin = rnd(T, r // 2, seed=4), rnd(T, r // 2, seed=5)
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+    outs = []
+    for w in (wc, off(wc)):
+        out = torch.full((T, Q + R + r + G), float("nan"), dtype=dtype, device=DEV)
+        kernels.latent_prepare(out, Q, latent, A, d, r, R, G, wq, w, 1e-6, cos, sin, interleaved, pos, partial=part)
+        outs.append(out)
+    same(*outs, dtype)
