@@ -549,8 +549,10 @@ struct PTile {
                                      TMEM_USED <= 128 ? 128 : TMEM_USED <= 256 ? 256 : 512;
     static constexpr int STAGES_RAW = (200 * 1024) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
-    static constexpr int EPI_BYTES = PERSISTENT_EPI_WARPS * 16 * 32 * 4;   // per-warp staging, f32
+    // per-warp staging, f32: 16 x 32 values, in the q/k/v form twice as many
+    static constexpr int EPI_BYTES = PERSISTENT_EPI_WARPS * 16 * 32 * 4 * (MODE == 3 ? 2 : 1);
     static constexpr int SMEM = STAGES * STAGE_BYTES + EPI_BYTES + 1024 + 256;
+    static_assert(SMEM <= 227 * 1024, "stages and staging must fit shared memory");
     static_assert(TMEM_USED <= 512, "accumulators must fit tensor memory");
 };
 
@@ -573,12 +575,37 @@ struct QkvEpilogue {
     VtWrite vw;
 };
 
-__device__ __forceinline__ void st_bf16x16(__nv_bfloat16* dst, const float (&v)[16]) {
-    __nv_bfloat16 tmp[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) tmp[j] = __float2bfloat16_rn(v[j]);
-    reinterpret_cast<uint4*>(dst)[0] = reinterpret_cast<const uint4*>(tmp)[0];
-    reinterpret_cast<uint4*>(dst)[1] = reinterpret_cast<const uint4*>(tmp)[1];
+// Where a token's key and value go.
+struct QkvPlace {
+    long long row = -1;        // row of the pools, or none
+    long long vt_col = -1;     // column of the transposed values, or none
+    int vt_pad = 0;            // zero columns after it (a sequence's last token)
+};
+__device__ __forceinline__ QkvPlace qkv_place(const QkvEpilogue& qe, int tok) {
+    QkvPlace o;
+    const int b = qe.cw.seq_index ? qe.cw.seq_index[tok] : qe.vw.seq_index[tok];
+    const int p = qe.positions[tok];
+    if (qe.cw.k_pool) {
+        const int slot = qe.cw.slots[b], len = qe.cw.lens[b];
+        if (slot >= 0 && p >= len - qe.cw.cap) {
+            const int r = p % qe.cw.cap;
+            o.row = (long long)qe.cw.page_table[(size_t)slot * qe.cw.max_pages + r / qe.cw.page] * qe.cw.page +
+                    r % qe.cw.page;
+        }
+    }
+    if (qe.vw.vt) {
+        int start = 0;
+        for (int i = 0; i < b; ++i) start += (qe.vw.cu[i + 1] - qe.vw.cu[i] + 63) & ~63;
+        o.vt_col = start + p;
+        const int len = qe.vw.cu[b + 1] - qe.vw.cu[b];
+        if (p == len - 1) o.vt_pad = ((len + 63) & ~63) - len;
+    }
+    return o;
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
 }
 
 // One epilogue warp's share of one accumulator [128 tokens x 256 columns]: lanes are tokens
@@ -586,16 +613,24 @@ __device__ __forceinline__ void st_bf16x16(__nv_bfloat16* dst, const float (&v)[
 // the lanes (half 0 and 1) each take half of every head's rotation pairs (i, i + hd / 2);
 // both add up the whole head's squares, which costs a few tensor-memory loads and saves an
 // exchange.
+//
+// Pairs go P at a time through the warp's staging (st, 4 KB): a lane writes its token's P pairs, and
+// LP = P / 4 neighbouring lanes read a token back, four pairs each, so that the tables are read and
+// q, k, v and the cache rows written in lines of a token.  With every lane at its own token's row
+// (each access 32 rows apart) the epilogue took 28 us a tile, and the product (1,152 or 2,560 long)
+// 5 to 11.  8,696 tokens of eight
+// sequences x 1,536 x 1,152: 84 us, 73 with the lookups under the products and the zeros behind a sequence's
+// end by the whole warp (one lane wrote them all), 68 so; 2,048 tokens 26, 25, 20; 4,001 x 4,096 x 2,560 101
+// before and after.
+// (swizzled by the row: neither side has bank conflicts, and no padding is needed)
+template <int P>
 __device__ __forceinline__ void qkv_epilogue(uint32_t lane_base, int m0, int tok, int half, int T,
-                                             const QkvEpilogue& qe) {
+                                             const QkvEpilogue& qe, const QkvPlace& at_row, float* st) {
+    constexpr int LP = P / 4, ROWS = 512 / P, PER = 32 / LP;       // lanes a token, tokens staged, a pass
     const int hd = qe.hd, H2 = hd / 2, heads = qe.nh + 2 * qe.nkv;
-    const bool live = tok < T;
+    const int lane = threadIdx.x & 31, tok0 = tok - lane;
     const int share = H2 / 2;                       // pairs per warp and head: 16, 32 or 64
-    // where this token's key and value go: looked up when the first k or v head comes
-    bool looked = false;
-    int c_page = -1, c_row = 0;
-    long long vt_col = -1;
-    int vt_pad = 0;
+    const long long c_row = at_row.row, vt_col = at_row.vt_col;
     for (int hh = 0; hh * hd < 2 * TILE_M; ++hh) {
         const int head = m0 / hd + hh;
         if (head >= heads) break;
@@ -606,107 +641,119 @@ __device__ __forceinline__ void qkv_epilogue(uint32_t lane_base, int m0, int tok
         float rs = 1.f;
         if (w) {
             float ss = 0.f;
+            uint32_t a[16], b[16];
+            tc_ld16(base, a);
 #pragma unroll 1
             for (int c = 0; c < hd; c += 32) {
-                uint32_t a[16], b[16];
-                tc_ld16(base + c, a);
-                tc_ld16(base + c + 16, b);
                 tc_wait_ld();
+                tc_ld16(base + c + 16, b);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float x = __uint_as_float(a[j]), y = __uint_as_float(b[j]);
-                    ss = fmaf(x, x, ss);
-                    ss = fmaf(y, y, ss);
-                }
+                for (int j = 0; j < 16; ++j) ss = fmaf(__uint_as_float(a[j]), __uint_as_float(a[j]), ss);
+                tc_wait_ld();
+                if (c + 32 < hd) tc_ld16(base + c + 32, a);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) ss = fmaf(__uint_as_float(b[j]), __uint_as_float(b[j]), ss);
             }
             rs = 1.0f / sqrtf(ss / (float)hd + qe.eps);
         }
-        if (!is_q && !looked && live) {
-            looked = true;
-            const int b = qe.cw.seq_index ? qe.cw.seq_index[tok] : qe.vw.seq_index[tok];
-            const int p = qe.positions[tok];
-            if (qe.cw.k_pool) {
-                const int slot = qe.cw.slots[b], len = qe.cw.lens[b];
-                if (slot >= 0 && p >= len - qe.cw.cap) {
-                    c_row = p % qe.cw.cap;
-                    c_page = qe.cw.page_table[(size_t)slot * qe.cw.max_pages + c_row / qe.cw.page];
-                }
-            }
-            if (qe.vw.vt) {
-                int start = 0;
-                for (int i = 0; i < b; ++i) start += (qe.vw.cu[i + 1] - qe.vw.cu[i] + 63) & ~63;
-                vt_col = start + p;
-                const int len = qe.vw.cu[b + 1] - qe.vw.cu[b];
-                if (p == len - 1) vt_pad = ((len + 63) & ~63) - len;
-            }
-        }
         const int g = is_k ? head - qe.nh : head - qe.nh - qe.nkv;
-        __nv_bfloat16* row_dst = qe.qkv + (size_t)tok * qe.row_stride + (size_t)head * hd;
-        __nv_bfloat16* pool_dst = nullptr;
-        if (!is_q && c_page >= 0)
-            pool_dst = (__nv_bfloat16*)(is_k ? qe.cw.k_pool : qe.cw.v_pool) +
-                       (((size_t)c_page * qe.cw.page + c_row % qe.cw.page) * qe.nkv + g) * hd;
+        __nv_bfloat16* pool = is_q || !qe.cw.k_pool ? nullptr
+                                                    : (__nv_bfloat16*)(is_k ? qe.cw.k_pool : qe.cw.v_pool);
         const bool rotate = qe.cosv && !is_v;
+        const int mine = (lane % LP) * 4;                          // of the P pairs, when reading back
 #pragma unroll 1
-        for (int i = half * share; i < (half + 1) * share; i += 16) {
-            uint32_t a[16], b[16];
-            tc_ld16(base + i, a);
-            tc_ld16(base + H2 + i, b);
-            tc_wait_ld();
-            if (!live) continue;
-            float x[16], y[16];
+        for (int i = half * share; i < (half + 1) * share; i += P) {
+            uint32_t x[P], y[P];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                x[j] = __uint_as_float(a[j]);
-                y[j] = __uint_as_float(b[j]);
+            for (int j = 0; j < P; j += 16) {
+                tc_ld16(base + i + j, *reinterpret_cast<uint32_t(*)[16]>(x + j));
+                tc_ld16(base + H2 + i + j, *reinterpret_cast<uint32_t(*)[16]>(y + j));
             }
+            float4 wa = make_float4(1.f, 1.f, 1.f, 1.f), wb = wa;
             if (w) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float4 wa = *reinterpret_cast<const float4*>(w + i + 4 * q);
-                    const float4 wb = *reinterpret_cast<const float4*>(w + H2 + i + 4 * q);
-                    x[4 * q] *= rs * wa.x, x[4 * q + 1] *= rs * wa.y;
-                    x[4 * q + 2] *= rs * wa.z, x[4 * q + 3] *= rs * wa.w;
-                    y[4 * q] *= rs * wb.x, y[4 * q + 1] *= rs * wb.y;
-                    y[4 * q + 2] *= rs * wb.z, y[4 * q + 3] *= rs * wb.w;
-                }
+                wa = *reinterpret_cast<const float4*>(w + i + mine);
+                wb = *reinterpret_cast<const float4*>(w + H2 + i + mine);
             }
-            if (rotate) {
-                const float* cs = qe.cosv + (size_t)tok * H2 + i;
-                const float* sn = qe.sinv + (size_t)tok * H2 + i;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float4 c4 = *reinterpret_cast<const float4*>(cs + 4 * q);
-                    const float4 s4 = *reinterpret_cast<const float4*>(sn + 4 * q);
-                    const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, sv[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float re = x[4 * q + e], im = y[4 * q + e];
-                        x[4 * q + e] = re * cc[e] - im * sv[e];
-                        y[4 * q + e] = re * sv[e] + im * cc[e];
-                    }
-                }
-            }
-            st_bf16x16(row_dst + i, x);
-            st_bf16x16(row_dst + H2 + i, y);
-            if (pool_dst) {
-                st_bf16x16(pool_dst + i, x);
-                st_bf16x16(pool_dst + H2 + i, y);
-            }
+            tc_wait_ld();
             if (is_v && vt_col >= 0) {
                 __nv_bfloat16* v0 = qe.vw.vt + (size_t)(g * hd + i) * qe.vw.ld + vt_col;
                 __nv_bfloat16* v1 = qe.vw.vt + (size_t)(g * hd + H2 + i) * qe.vw.ld + vt_col;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    v0[(size_t)j * qe.vw.ld] = __float2bfloat16_rn(x[j]);
-                    v1[(size_t)j * qe.vw.ld] = __float2bfloat16_rn(y[j]);
+                for (int j = 0; j < P; ++j) {
+                    v0[(size_t)j * qe.vw.ld] = __float2bfloat16_rn(__uint_as_float(x[j]));
+                    v1[(size_t)j * qe.vw.ld] = __float2bfloat16_rn(__uint_as_float(y[j]));
                 }
-                for (int pc = 1; pc <= vt_pad; ++pc)        // the sequence's last token: zero padding
+            }
+            // after a sequence's last token zeros up to the next multiple of 64 columns, by the whole warp
+            for (unsigned ends = __ballot_sync(0xffffffffu, is_v && at_row.vt_pad > 0); ends; ends &= ends - 1) {
+                const int l = __ffs(ends) - 1, pad = __shfl_sync(0xffffffffu, at_row.vt_pad, l);
+                const long long col = __shfl_sync(0xffffffffu, vt_col, l) + 1;
+                for (int j = 0; j < 2 * P; ++j) {
+                    __nv_bfloat16* v0 = qe.vw.vt + (size_t)(g * hd + i + (j < P ? j : H2 + j - P)) * qe.vw.ld + col;
+                    for (int pc = lane; pc < pad; pc += 32) v0[pc] = __float2bfloat16_rn(0.f);
+                }
+            }
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        v0[(size_t)j * qe.vw.ld + pc] = __float2bfloat16_rn(0.f);
-                        v1[(size_t)j * qe.vw.ld + pc] = __float2bfloat16_rn(0.f);
+            for (int r0 = 0; r0 < 32; r0 += ROWS) {
+                // the tables' pieces of this round's tokens are under way while it is staged
+                float4 c4[ROWS / PER], s4[ROWS / PER];
+#pragma unroll
+                for (int q = 0; q < ROWS / PER; ++q) {
+                    const int t = tok0 + r0 + q * PER + lane / LP;
+                    c4[q] = make_float4(1.f, 1.f, 1.f, 1.f);
+                    s4[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (rotate && t < T) {
+                        c4[q] = *reinterpret_cast<const float4*>(qe.cosv + (size_t)t * H2 + i + mine);
+                        s4[q] = *reinterpret_cast<const float4*>(qe.sinv + (size_t)t * H2 + i + mine);
                     }
+                }
+                if (lane >= r0 && lane < r0 + ROWS) {
+                    const int r = lane - r0;
+                    uint4* row = reinterpret_cast<uint4*>(st) + r * (P / 2);
+#pragma unroll
+                    for (int j = 0; j < P / 4; ++j) {
+                        row[j ^ (r & (P / 2 - 1))] = make_uint4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+                        row[(P / 4 + j) ^ (r & (P / 2 - 1))] =
+                            make_uint4(y[4 * j], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < ROWS / PER; ++q) {
+                    const int r = q * PER + lane / LP, t = tok0 + r0 + r;
+                    const float4* row = reinterpret_cast<const float4*>(st) + r * (P / 2);
+                    const float4 u = row[(lane % LP) ^ (r & (P / 2 - 1))];
+                    const float4 v = row[(P / 4 + lane % LP) ^ (r & (P / 2 - 1))];
+                    const float scale = __shfl_sync(0xffffffffu, rs, r0 + r);
+                    const long long at = __shfl_sync(0xffffffffu, c_row, r0 + r);
+                    float re[4] = {u.x, u.y, u.z, u.w}, im[4] = {v.x, v.y, v.z, v.w};
+                    const float we[4] = {wa.x, wa.y, wa.z, wa.w}, wi[4] = {wb.x, wb.y, wb.z, wb.w};
+                    const float cc[4] = {c4[q].x, c4[q].y, c4[q].z, c4[q].w};
+                    const float sv[4] = {s4[q].x, s4[q].y, s4[q].z, s4[q].w};
+                    float ox[4], oy[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if (w) {
+                            re[e] *= scale * we[e];
+                            im[e] *= scale * wi[e];
+                        }
+                        ox[e] = rotate ? re[e] * cc[e] - im[e] * sv[e] : re[e];
+                        oy[e] = rotate ? re[e] * sv[e] + im[e] * cc[e] : im[e];
+                    }
+                    if (t < T) {
+                        const uint2 px = make_uint2(pack_bf16(ox[0], ox[1]), pack_bf16(ox[2], ox[3]));
+                        const uint2 py = make_uint2(pack_bf16(oy[0], oy[1]), pack_bf16(oy[2], oy[3]));
+                        __nv_bfloat16* dst = qe.qkv + (size_t)t * qe.row_stride + (size_t)head * hd + i + mine;
+                        *reinterpret_cast<uint2*>(dst) = px;
+                        *reinterpret_cast<uint2*>(dst + H2) = py;
+                        if (pool && at >= 0) {
+                            dst = pool + ((size_t)at * qe.nkv + g) * hd + i + mine;
+                            *reinterpret_cast<uint2*>(dst) = px;
+                            *reinterpret_cast<uint2*>(dst + H2) = py;
+                        }
+                    }
+                }
+                __syncwarp();
             }
         }
     }
@@ -873,6 +920,13 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w,
             int m0, n0, kb_begin, n_kb, split;
             decode_item(item, m0, n0, kb_begin, n_kb, split);
             const int as = li & 1;
+            // (the way to a token's cache rows is four trips one after the other: made while the
+            // products run)
+            [[maybe_unused]] QkvPlace place;
+            if constexpr (QKV) {
+                const int t = n0 + quarter * 32 + lane;
+                if (t < T && (m0 + M_STEP - 1) / qe.hd >= qe.nh) place = qkv_place(qe, t);
+            }
             bool ok = !*abort_flag && mbar_wait(&acc_full[as], (li >> 1) & 1);
             if (!ok) {
                 if (!*abort_flag) atomicCAS(&g_gemm_status, 0, (3 << 8) | as);
@@ -966,7 +1020,8 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w,
                 continue;
             }
             if constexpr (QKV) {
-                qkv_epilogue(lane_base, m0, tok, half, T, qe);
+                if (qe.hd == 64) qkv_epilogue<16>(lane_base, m0, tok, half, T, qe, place, (float*)wst);
+                else qkv_epilogue<32>(lane_base, m0, tok, half, T, qe, place, (float*)wst);
                 release();
                 continue;
             }
