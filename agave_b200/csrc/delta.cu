@@ -396,32 +396,54 @@ __host__ __device__ inline size_t scan_buf_floats(int TCH, int Dp, int CC) {
     return ((size_t)TCH * (4 * Dp + CC + 2) + 3) / 4 * 4;      // (16-byte rows in the next buffer)
 }
 
-template <int L>
-__global__ void __launch_bounds__(256)
+// A lane's rows of CPT columns (CC apart), two rows to a register pair: a piece of a token's row read
+// once serves them all.  The pieces of k, g, g k and g q are what bounds the kernel: 16 reads of 16
+// bytes a lane and token, 256 cycles of an SM's shared memory for the four warps of a CTA.
+// 8 sequences of 256 to 1,024 tokens, 16 heads of 128 x 128: one column a lane 905 us, two MEASURED_D.
+template <int L, int CPT>
+__global__ void __launch_bounds__(128)
 delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
     pdl_wait();
     extern __shared__ float smem[];
-    const int b = blockIdx.z;
+    // the longest sequences of a prompt step begin first: this CTA's is the blockIdx.z-th longest
+    int b = blockIdx.z;
+    if (a.TCH > 1 && gridDim.z <= blockDim.x) {
+        __shared__ int ranked;
+        const int e = threadIdx.x, B = gridDim.z;
+        if (e < B) {
+            const int mine = st.cu[e + 1] - st.cu[e];
+            int rank = 0;
+            for (int j = 0; j < B; ++j) {
+                const int other = st.cu[j + 1] - st.cu[j];
+                rank += other > mine || (other == mine && j < e);
+            }
+            if (rank == (int)blockIdx.z) ranked = e;
+        }
+        __syncthreads();
+        b = ranked;
+    }
     const int slot = st.slots[b];
     if (slot < 0) return;
     const int t0 = st.cu[b], n = st.cu[b + 1] - t0;
     if (n <= 0) return;
     const int h = blockIdx.y;
     const int d = dm.d, dv = dm.dv, C = dm.C(), nq = dm.nq();
-    constexpr int Dp = L * DL_R;
-    const int CC = a.CC, TCH = a.TCH;
+    constexpr int Dp = L * DL_R, P = DL_R / 2;
+    const int CC = a.CC, CW = CC * CPT, TCH = a.TCH;
     const int l = threadIdx.x & (L - 1);
     const int jc = threadIdx.x / L;
-    const int j = blockIdx.x * CC + jc;
-    const bool live = jc < CC && j < dv;
-    const size_t per = scan_buf_floats(TCH, Dp, CC);
+    const int j0 = blockIdx.x * CW + jc;               // and j0 + CC, ...
+    bool live[CPT];
+#pragma unroll
+    for (int x = 0; x < CPT; ++x) live[x] = jc < CC && j0 + x * CC < dv;
+    const size_t per = scan_buf_floats(TCH, Dp, CW);
     // (columns of v past dv are never copied: zero them once)
     for (size_t i = threadIdx.x; i < 2 * per; i += blockDim.x) smem[i] = 0.f;
     __syncthreads();
 
     auto fetch = [&](int c0, float* base) {
         const int m = min(TCH, n - c0);
-        const ScanBuf sb(base, TCH, Dp, CC);
+        const ScanBuf sb(base, TCH, Dp, CW);
         // rows of Dp floats a token: tokens of a head lie H * Dp apart
         constexpr int Q = Dp / 4;
         for (int idx = threadIdx.x; idx < m * Q; idx += blockDim.x) {
@@ -433,9 +455,9 @@ delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
             cp_async_16(sb.gk + dst, a.wgk + src);
             cp_async_16(sb.gq + dst, a.wgq + src);
         }
-        for (int idx = threadIdx.x; idx < m * CC; idx += blockDim.x) {
-            const int tt = idx / CC, c = idx - tt * CC;
-            const int col = blockIdx.x * CC + c;
+        for (int idx = threadIdx.x; idx < m * CW; idx += blockDim.x) {
+            const int tt = idx / CW, c = idx - tt * CW;
+            const int col = blockIdx.x * CW + c;
             if (col < dv)
                 cp_async_f32(sb.v + idx, a.qkv + (size_t)(t0 + c0 + tt) * C + 2 * nq + (size_t)h * dv + col);
         }
@@ -446,18 +468,22 @@ delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
         cp_async_commit();
     };
 
-    float S[DL_R];
-    float* srow = st.state + (size_t)slot * st.stride + ((size_t)h * dv + (live ? j : 0)) * d;
+    f32x2 S[CPT][P];
+    float* srow[CPT];
     fetch(0, smem);
 #pragma unroll
-    for (int i = 0; i < DL_R; ++i) {
-        const int r = ((i >> 2) * L + l) * 4 + (i & 3);
-        S[i] = live && r < d ? srow[r] : 0.f;
+    for (int x = 0; x < CPT; ++x) {
+        srow[x] = st.state + (size_t)slot * st.stride + ((size_t)h * dv + (live[x] ? j0 + x * CC : 0)) * d;
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+            const int r = ((i >> 1) * L + l) * 4 + (i & 1) * 2;
+            S[x][i] = pack2(live[x] && r < d ? srow[x][r] : 0.f, live[x] && r + 1 < d ? srow[x][r + 1] : 0.f);
+        }
     }
     int cur = 0;
     for (int c0 = 0; c0 < n; c0 += TCH, cur ^= 1) {
         const int m = min(TCH, n - c0);
-        const ScanBuf sb(smem + (size_t)cur * per, TCH, Dp, CC);
+        const ScanBuf sb(smem + (size_t)cur * per, TCH, Dp, CW);
         // (the other buffer was read in the round before, which ended with a barrier)
         if (c0 + TCH < n) {
             fetch(c0 + TCH, smem + (size_t)(cur ^ 1) * per);
@@ -471,56 +497,75 @@ delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
         const float* pgq = sb.gq + l * 4;
         const float* pg = sb.g + l * 4;
         const float* pv = sb.v + (jc < CC ? jc : 0);
-        float* po = a.out + (size_t)(t0 + c0) * dm.H * dv + (size_t)h * dv + (live ? j : 0);
+        float* po = a.out + (size_t)(t0 + c0) * dm.H * dv + (size_t)h * dv + j0;
 #pragma unroll 2
         for (int tt = 0; tt < m; ++tt) {
-            float gk[DL_R], gq[DL_R], kk[DL_R], gg[DL_R];
+            f32x2 ac[CPT][2], rc[CPT][2];
+#pragma unroll
+            for (int x = 0; x < CPT; ++x) ac[x][0] = ac[x][1] = rc[x][0] = rc[x][1] = 0;
 #pragma unroll
             for (int i = 0; i < DL_R / 4; ++i) {
-                const float4 x = reinterpret_cast<const float4*>(pgk)[i * L];
-                const float4 y = reinterpret_cast<const float4*>(pgq)[i * L];
-                gk[4 * i] = x.x; gk[4 * i + 1] = x.y; gk[4 * i + 2] = x.z; gk[4 * i + 3] = x.w;
-                gq[4 * i] = y.x; gq[4 * i + 1] = y.y; gq[4 * i + 2] = y.z; gq[4 * i + 3] = y.w;
-            }
-            float ac[4] = {0.f, 0.f, 0.f, 0.f}, rc[4] = {0.f, 0.f, 0.f, 0.f};
+                const ulonglong2 gk = reinterpret_cast<const ulonglong2*>(pgk)[i * L];
+                const ulonglong2 gq = reinterpret_cast<const ulonglong2*>(pgq)[i * L];
 #pragma unroll
-            for (int i = 0; i < DL_R; ++i) {
-                ac[i & 3] = fmaf(S[i], gk[i], ac[i & 3]);
-                rc[i & 3] = fmaf(S[i], gq[i], rc[i & 3]);
+                for (int x = 0; x < CPT; ++x) {
+                    ac[x][0] = fma2(S[x][2 * i], gk.x, ac[x][0]);
+                    ac[x][1] = fma2(S[x][2 * i + 1], gk.y, ac[x][1]);
+                    rc[x][0] = fma2(S[x][2 * i], gq.x, rc[x][0]);
+                    rc[x][1] = fma2(S[x][2 * i + 1], gq.y, rc[x][1]);
+                }
+            }
+            float acc[CPT], rr[CPT];
+#pragma unroll
+            for (int x = 0; x < CPT; ++x) {
+                float a0, a1, a2, a3, r0, r1, r2, r3;
+                unpack2(ac[x][0], a0, a1); unpack2(ac[x][1], a2, a3);
+                unpack2(rc[x][0], r0, r1); unpack2(rc[x][1], r2, r3);
+                acc[x] = (a0 + a1) + (a2 + a3);
+                rr[x] = (r0 + r1) + (r2 + r3);
+            }
+#pragma unroll
+            for (int o = 1; o < L; o <<= 1)
+#pragma unroll
+                for (int x = 0; x < CPT; ++x) {
+                    acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], o);
+                    rr[x] += __shfl_xor_sync(0xffffffffu, rr[x], o);
+                }
+            const float beta = sb.beta[tt], kq = sb.kq[tt];
+            f32x2 uu[CPT];
+#pragma unroll
+            for (int x = 0; x < CPT; ++x) {
+                const float u = beta * (pv[x * CC] - acc[x]);
+                if (live[x] && l == 0) po[x * CC] = fmaf(kq, u, rr[x]);
+                uu[x] = pack2(u, u);
             }
 #pragma unroll
             for (int i = 0; i < DL_R / 4; ++i) {
-                const float4 x = reinterpret_cast<const float4*>(pk)[i * L];
-                const float4 y = reinterpret_cast<const float4*>(pg)[i * L];
-                kk[4 * i] = x.x; kk[4 * i + 1] = x.y; kk[4 * i + 2] = x.z; kk[4 * i + 3] = x.w;
-                gg[4 * i] = y.x; gg[4 * i + 1] = y.y; gg[4 * i + 2] = y.z; gg[4 * i + 3] = y.w;
+                const ulonglong2 kk = reinterpret_cast<const ulonglong2*>(pk)[i * L];
+                const ulonglong2 gg = reinterpret_cast<const ulonglong2*>(pg)[i * L];
+#pragma unroll
+                for (int x = 0; x < CPT; ++x) {
+                    S[x][2 * i] = fma2(kk.x, uu[x], mul2(gg.x, S[x][2 * i]));
+                    S[x][2 * i + 1] = fma2(kk.y, uu[x], mul2(gg.y, S[x][2 * i + 1]));
+                }
             }
-            float acc = (ac[0] + ac[1]) + (ac[2] + ac[3]);
-            float rr = (rc[0] + rc[1]) + (rc[2] + rc[3]);
-#pragma unroll
-            for (int o = 1; o < L; o <<= 1) {
-                acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                rr += __shfl_xor_sync(0xffffffffu, rr, o);
-            }
-#pragma unroll
-            for (int i = 0; i < DL_R; ++i) gg[i] *= S[i];          // g S: needs no u
-            const float u = sb.beta[tt] * (*pv - acc);
-            if (live && l == 0) *po = fmaf(sb.kq[tt], u, rr);
-#pragma unroll
-            for (int i = 0; i < DL_R; ++i) S[i] = fmaf(kk[i], u, gg[i]);
-            pk += Dp; pgk += Dp; pgq += Dp; pg += Dp; pv += CC;
+            pk += Dp; pgk += Dp; pgq += Dp; pg += Dp; pv += CW;
             po += (size_t)dm.H * dv;
         }
         __syncthreads();
     }
     pdl_launch_next();
-    if (live) {
 #pragma unroll
-        for (int i = 0; i < DL_R; ++i) {
-            const int r = ((i >> 2) * L + l) * 4 + (i & 3);
-            if (r < d) srow[r] = S[i];
-        }
-    }
+    for (int x = 0; x < CPT; ++x)
+        if (live[x])
+#pragma unroll
+            for (int i = 0; i < P; ++i) {
+                const int r = ((i >> 1) * L + l) * 4 + (i & 1) * 2;
+                float lo, hi;
+                unpack2(S[x][i], lo, hi);
+                if (r < d) srow[x][r] = lo;
+                if (r + 1 < d) srow[x][r + 1] = hi;
+            }
 }
 
 // ---------------------------------------------------------------- read-out
@@ -708,10 +753,15 @@ AGV_API int agv_delta_scan(const float* qkv, const float* beta, const float* a,
     while (CC > 32 / L && CC / 2 >= dv) CC >>= 1;
     if (CC < 1) CC = 1;
     const int Dp = L * DL_R;
-    // two buffers of TCH tokens and the decay's bias, within the 48 KB every launch may have
+    // Two columns a lane where one would put more than two CTAs on every SM, in a step whose sequences
+    // bring several tokens; a decode step is a read and a write of the state.
+    const long long ctas = (long long)((dv + CC - 1) / CC) * H * B;
+    const int CPT = T > B && dv >= 2 * CC && ctas > 296 ? 2 : 1;
+    const int CW = CC * CPT;
+    // two buffers of TCH tokens, within the 48 KB every launch may have
     int TCH = T <= B ? 1 : 16;             // (a decode step brings a token a sequence)
-    while (TCH > 1 && 2 * scan_buf_floats(TCH, Dp, CC) * sizeof(float) > 46 * 1024) TCH >>= 1;
-    const size_t smem = 2 * scan_buf_floats(TCH, Dp, CC) * sizeof(float);
+    while (TCH > 1 && 2 * scan_buf_floats(TCH, Dp, CW) * sizeof(float) > 46 * 1024) TCH >>= 1;
+    const size_t smem = 2 * scan_buf_floats(TCH, Dp, CW) * sizeof(float);
     AGV_REQUIRE(smem <= 48 * 1024, "delta_scan: key heads of %d need too much shared memory", d);
     AGV_REQUIRE(work && ((size_t)work & 15) == 0, "delta_scan: no scratch, or not 16-byte aligned");
     const size_t row = (size_t)T * H * Dp;
@@ -723,14 +773,17 @@ AGV_API int agv_delta_scan(const float* qkv, const float* beta, const float* a,
         AGV_LAUNCH_OK("delta_decay_kernel");
     }
     const DeltaState st{state, state_stride, 0, slots, cu, nullptr, nullptr};
-    dim3 grid((unsigned)((dv + CC - 1) / CC), (unsigned)H, (unsigned)B);
+    dim3 grid((unsigned)((dv + CW - 1) / CW), (unsigned)H, (unsigned)B);
+#define AGV_SCAN(LL)                                                                                              \
+    case LL:                                                                                                      \
+        if (CPT == 1) agv_launch_after(delta_scan_kernel<LL, 1>, grid, (unsigned)(CC * L), smem, stream, sa, dm, st); \
+        else agv_launch_after(delta_scan_kernel<LL, 2>, grid, (unsigned)(CC * L), smem, stream, sa, dm, st);      \
+        break
     switch (L) {
-#define AGV_SCAN(LL) case LL: agv_launch_after(delta_scan_kernel<LL>, grid, (unsigned)(CC * L), smem, \
-                                               stream, sa, dm, st); break
         AGV_SCAN(1); AGV_SCAN(2); AGV_SCAN(4); AGV_SCAN(8); AGV_SCAN(16); AGV_SCAN(32);
-#undef AGV_SCAN
         default: return agv_fail(-1, "delta_scan: %d lanes a column", L);
     }
+#undef AGV_SCAN
     AGV_LAUNCH_OK("delta_scan_kernel");
     return 0;
 }
