@@ -352,6 +352,394 @@ mlstm_scan_kernel(ScanIn in, float* __restrict__ num, float* __restrict__ den, i
     }
 }
 
+// ---------------------------------------------- the scan without normaliser, by chunks
+// S_t = a_t S_(t-1) + b_t k_t v_t^T and o_t = S_t^T q_t are linear in S, so a sequence can be cut into
+// chunks of CK tokens, each a few small products.  With A(r, t) = a_r ... a_t (1 if r > t), S_0 what
+// the chunk begins from and tokens counted from the chunk's first:
+//   o_t = A(1, t) S_0^T q_t + sum_(s <= t) (q_t . k_s) b_s A(s + 1, t) v_s
+//   S_end = A(1, CK) S_0 + sum_t b_t A(t + 1, CK) k_t v_t^T
+// q . k is the same for all heads of a group and made once; the sums of S_end run over all chunks at
+// once (from nothing), a pass over the chunks turns them into what every chunk begins from, and the
+// outputs again run over all chunks at once.  Decays are products of the a's themselves, as in the
+// token-by-token scan, never quotients or exponentials of differences.
+constexpr int CK = 128;            // tokens of a chunk
+constexpr int CK_C = 64;           // columns of S a CTA has
+
+struct Chunks {
+    int n_seq;
+    const int* cu;
+    float* states;             // [chunks, H, d, dv]
+    float* decays;             // [chunks, H]
+    float* scores;             // [chunks, groups, CK, CK]: q_t . k_s for s <= t
+};
+
+// Chunk z of the step: its first token and how many it has; false: there is none.
+__device__ __forceinline__ bool chunk_of(const Chunks& ck, int z, int& t0, int& nt) {
+    int at = 0;
+    for (int e = 0; e < ck.n_seq; ++e) {
+        const int from = ck.cu[e], n = ck.cu[e + 1] - from, c = (n + CK - 1) / CK;
+        if (z < at + c) {
+            t0 = from + (z - at) * CK;
+            nt = min(CK, from + n - t0);
+            return true;
+        }
+        at += c;
+    }
+    return false;
+}
+
+// ROWS x COLS values (columns a multiple of 4) into shared memory, 256 threads, their loads issued
+// together: row r, columns c .. are src(r) + c, zeros from n_rows and n_cols on; times scale[r] where given.
+template <int ROWS, int COLS, typename RowFn>
+__device__ __forceinline__ void chunk_fill(float* dst, int pitch, int n_rows, int n_cols, bool vec,
+                                           const float* scale, RowFn src) {
+    constexpr int PER = COLS / 4, ALL = ROWS * PER / 256, U = ALL < 8 ? ALL : 8;
+    static_assert(ROWS * PER % 256 == 0 && ALL % U == 0, "whole rounds of 256 threads");
+#pragma unroll 1
+    for (int i0 = 0; i0 < ALL; i0 += U) {
+        float4 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = threadIdx.x + (i0 + u) * 256, r = i / PER, c = (i % PER) * 4;
+            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r < n_rows) {
+                const float* p = src(r) + c;
+                if (vec && c + 4 <= n_cols) {
+                    v[u] = __ldg(reinterpret_cast<const float4*>(p));
+                } else {
+                    if (c < n_cols) v[u].x = __ldg(p);
+                    if (c + 1 < n_cols) v[u].y = __ldg(p + 1);
+                    if (c + 2 < n_cols) v[u].z = __ldg(p + 2);
+                    if (c + 3 < n_cols) v[u].w = __ldg(p + 3);
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = threadIdx.x + (i0 + u) * 256, r = i / PER, c = (i % PER) * 4;
+            if (scale) {
+                const float f = scale[r];
+                v[u].x *= f; v[u].y *= f; v[u].z *= f; v[u].w *= f;
+            }
+            *reinterpret_cast<float4*>(dst + r * pitch + c) = v[u];
+        }
+    }
+}
+
+// grid (lower 64 x 64 tiles of a chunk's scores, groups, chunks)
+__global__ void __launch_bounds__(256)
+chunk_scores_kernel(ScanIn in, int d, Chunks ck, int vec) {
+    pdl_wait();
+    pdl_launch_next();
+    __shared__ __align__(16) float qs[64 * 36], ks[64 * 36];
+    int t0, nt;
+    if (!chunk_of(ck, blockIdx.z, t0, nt)) return;
+    const int g = blockIdx.y, tq = blockIdx.x > 0 ? 64 : 0, tk = blockIdx.x == 2 ? 64 : 0;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    float acc[4][4] = {};
+    for (int k0 = 0; k0 < d; k0 += 32) {
+        __syncthreads();
+        chunk_fill<64, 32>(qs, 36, nt - tq, d - k0, vec, nullptr, [&](int r) {
+            return in.q + (size_t)(t0 + tq + r) * in.ld + (size_t)g * d + k0; });
+        chunk_fill<64, 32>(ks, 36, nt - tk, d - k0, vec, nullptr, [&](int r) {
+            return in.k + (size_t)(t0 + tk + r) * in.ld + (size_t)g * d + k0; });
+        __syncthreads();
+        float part[4][4] = {};
+#pragma unroll
+        for (int k = 0; k < 32; k += 4) {
+            if (k == 16)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { acc[i][j] += part[i][j]; part[i][j] = 0.f; }
+            float4 x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(qs + (ty + 16 * i) * 36 + k);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 y = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * 36 + k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    part[i][j] = fmaf(x[i].x, y.x, part[i][j]);
+                    part[i][j] = fmaf(x[i].y, y.y, part[i][j]);
+                    part[i][j] = fmaf(x[i].z, y.z, part[i][j]);
+                    part[i][j] = fmaf(x[i].w, y.w, part[i][j]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
+    }
+    float* out = ck.scores + ((size_t)blockIdx.z * gridDim.y + g) * CK * CK;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) out[(size_t)(tq + ty + 16 * i) * CK + tk + tx + 16 * j] = acc[i][j];
+}
+
+// grid (tiles of 128 rows x 64 columns of S, heads, chunks): S_end from nothing; a thread 8 x 4 of it.
+__global__ void __launch_bounds__(256)
+chunk_states_kernel(ScanIn in, int H, int d, int dv, Chunks ck, int c_tiles, int vec_q, int vec_v) {
+    pdl_wait();
+    pdl_launch_next();
+    __shared__ __align__(16) float ks[32 * 128], vs[32 * CK_C];
+    __shared__ float w[CK];
+    int t0, nt;
+    if (!chunk_of(ck, blockIdx.z, t0, nt)) return;
+    const int h = blockIdx.y, hg = h / in.shared, n0 = blockIdx.x / c_tiles * 128, c0 = blockIdx.x % c_tiles * CK_C;
+    if (threadIdx.x < 32) {
+        // w_t = b_t A(t + 1, end): products from the last token on, 32 tokens at a time
+        const int l = threadIdx.x;
+        float run = 1.f;
+        for (int x = CK - 32; x >= 0; x -= 32) {
+            const int t = x + 31 - l;                   // lane 0: the last
+            const float2 ab = t < nt ? *reinterpret_cast<const float2*>(in.gates + ((size_t)(t0 + t) * H + h) * 2)
+                                     : make_float2(1.f, 0.f);
+            float p = ab.x;                             // of this token and the ones after it
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float q = __shfl_up_sync(0xffffffffu, p, o);
+                if (l >= o) p *= q;
+            }
+            float after = __shfl_up_sync(0xffffffffu, p, 1);
+            if (l == 0) after = 1.f;
+            w[t] = ab.y * (after * run);
+            run *= __shfl_sync(0xffffffffu, p, 31);
+        }
+        if (l == 0 && blockIdx.x == 0) ck.decays[(size_t)blockIdx.z * H + h] = run;
+    }
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    float acc[8][4] = {};
+    for (int x = 0; x < nt; x += 32) {
+        __syncthreads();                                // (the first: w is there)
+        chunk_fill<32, 128>(ks, 128, nt - x, d - n0, vec_q, nullptr, [&](int r) {
+            return in.k + (size_t)(t0 + x + r) * in.ld + (size_t)hg * d + n0; });
+        chunk_fill<32, CK_C>(vs, CK_C, nt - x, dv - c0, vec_v, w + x, [&](int r) {
+            return in.v + (size_t)(t0 + x + r) * in.ld + (size_t)h * dv + c0; });
+        __syncthreads();
+        float part[8][4] = {};                          // (see chunk_outputs_kernel)
+#pragma unroll 8
+        for (int t = 0; t < 32; ++t) {
+            if (t == 16)
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { acc[i][j] += part[i][j]; part[i][j] = 0.f; }
+            const float4 ka = *reinterpret_cast<const float4*>(ks + t * 128 + ty * 8);
+            const float4 kb = *reinterpret_cast<const float4*>(ks + t * 128 + ty * 8 + 4);
+            const float4 y = *reinterpret_cast<const float4*>(vs + t * CK_C + tx * 4);
+            const float kk[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                part[i][0] = fmaf(kk[i], y.x, part[i][0]);
+                part[i][1] = fmaf(kk[i], y.y, part[i][1]);
+                part[i][2] = fmaf(kk[i], y.z, part[i][2]);
+                part[i][3] = fmaf(kk[i], y.w, part[i][3]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
+    }
+    float* out = ck.states + ((size_t)blockIdx.z * H + h) * d * dv;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int n = n0 + ty * 8 + i, c = c0 + tx * 4;
+        if (n >= d) continue;
+        if (c + 4 <= dv && dv % 4 == 0) {
+            *reinterpret_cast<float4*>(out + (size_t)n * dv + c) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (c + j < dv) out[(size_t)n * dv + c + j] = acc[i][j];
+        }
+    }
+}
+
+// grid (pieces of S, heads, sequences): a thread takes four values of S through its sequence's chunks,
+// from the state and back to it; `states` becomes what every chunk begins from.
+__global__ void __launch_bounds__(256)
+chunk_pass_kernel(Chunks ck, int H, int dn, float* __restrict__ state, long long state_stride,
+                  long long state_off, const int* __restrict__ slots) {
+    pdl_wait();
+    pdl_launch_next();
+    const int e = blockIdx.z, h = blockIdx.y, slot = slots[e], i = (blockIdx.x * 256 + threadIdx.x) * 4;
+    const int n = (ck.cu[e + 1] - ck.cu[e] + CK - 1) / CK;
+    if (i >= dn || n == 0 || slot < 0) return;
+    int z = 0;
+    for (int j = 0; j < e; ++j) z += (ck.cu[j + 1] - ck.cu[j] + CK - 1) / CK;
+    float* S = state + (size_t)slot * state_stride + state_off + (size_t)h * dn + i;     // (any alignment)
+    float4 run = make_float4(S[0], S[1], S[2], S[3]);
+    float4* at = reinterpret_cast<float4*>(ck.states + ((size_t)z * H + h) * dn + i);
+    const size_t step = (size_t)H * dn / 4;
+    const float* decays = ck.decays + (size_t)z * H + h;
+    constexpr int AHEAD = 4;                              // trips under way
+    float4 own[AHEAD];
+    float by[AHEAD];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j)
+        if (j < n) { own[j] = at[j * step]; by[j] = decays[(size_t)j * H]; }
+    for (int s0 = 0; s0 < n; s0 += AHEAD)
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j) {
+            const int s = s0 + j;
+            if (s >= n) break;
+            at[s * step] = run;
+            const float a = by[j];
+            run = make_float4(fmaf(a, run.x, own[j].x), fmaf(a, run.y, own[j].y), fmaf(a, run.z, own[j].z),
+                              fmaf(a, run.w, own[j].w));
+            if (s + AHEAD < n) { own[j] = at[(s + AHEAD) * step]; by[j] = decays[(size_t)(s + AHEAD) * H]; }
+        }
+    S[0] = run.x; S[1] = run.y; S[2] = run.z; S[3] = run.w;
+}
+
+// grid (tiles of 64 columns, heads, chunks): the outputs of a chunk's tokens, a thread 8 x 4 of them
+// (tokens ty + 16 i).  First q S_0, then the scores with their decays times v; both left operands use
+// the same shared memory.
+constexpr int CO_PITCH = CK + 4;
+constexpr int CO_SMEM = (CK * CO_PITCH + CK * CK_C) * 4;
+// Tokens ty + 16 i, i >= FROM, times 16 of the common dimension from k0 on.
+template <int FROM>
+__device__ __forceinline__ void chunk_product(float (&part)[8][4], const float* X, const float* Y, int k0, int tx,
+                                              int ty) {
+#pragma unroll 2
+    for (int k = k0; k < k0 + 16; k += 4) {
+        float4 y[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j] = *reinterpret_cast<const float4*>(Y + (k + j) * CK_C + tx * 4);
+#pragma unroll
+        for (int i = FROM; i < 8; ++i) {
+            const float4 x = *reinterpret_cast<const float4*>(X + (ty + 16 * i) * CO_PITCH + k);
+            const float xe[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                part[i][0] = fmaf(xe[j], y[j].x, part[i][0]);
+                part[i][1] = fmaf(xe[j], y[j].y, part[i][1]);
+                part[i][2] = fmaf(xe[j], y[j].z, part[i][2]);
+                part[i][3] = fmaf(xe[j], y[j].w, part[i][3]);
+            }
+        }
+    }
+}
+__global__ void __launch_bounds__(256, 2)
+chunk_outputs_kernel(ScanIn in, float* __restrict__ num, int H, int d, int dv, Chunks ck, int vec_q, int vec_v,
+                     int vec_s) {
+    pdl_wait();
+    pdl_launch_next();
+    extern __shared__ __align__(16) float sm[];
+    float* X = sm;                                       // [CK][CO_PITCH]
+    float* Y = sm + CK * CO_PITCH;                       // [CK][CK_C]
+    __shared__ float as[CK], bs[CK], pre[CK];
+    int t0, nt;
+    if (!chunk_of(ck, blockIdx.z, t0, nt)) return;
+    const int h = blockIdx.y, hg = h / in.shared, groups = H / in.shared, c0 = blockIdx.x * CK_C;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    if (tid < CK) {
+        const float2 ab = tid < nt ? *reinterpret_cast<const float2*>(in.gates + ((size_t)(t0 + tid) * H + h) * 2)
+                                   : make_float2(1.f, 0.f);
+        as[tid] = ab.x;
+        bs[tid] = ab.y;
+    }
+    float acc[8][4] = {};
+    const float* S = ck.states + ((size_t)blockIdx.z * H + h) * d * dv;
+    for (int n0 = 0; n0 < d; n0 += CK) {
+        __syncthreads();
+        chunk_fill<CK, CK>(X, CO_PITCH, nt, d - n0, vec_q, nullptr, [&](int r) {
+            return in.q + (size_t)(t0 + r) * in.ld + (size_t)hg * d + n0; });
+        chunk_fill<CK, CK_C>(Y, CK_C, d - n0, dv - c0, vec_s, nullptr, [&](int r) {
+            return S + (size_t)(n0 + r) * dv + c0; });
+        __syncthreads();
+        // (sums of 16 terms, then added: a chain of 128 would round three times as far)
+        for (int kb = 0; kb < CK && n0 + kb < d; kb += 16) {
+            float part[8][4] = {};
+            chunk_product<0>(part, X, Y, kb, tx, ty);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
+        }
+    }
+    __syncthreads();
+    if (tid < 32) {
+        float run = 1.f;
+        for (int x = 0; x < CK; x += 32) {
+            float p = as[x + tid];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float q = __shfl_up_sync(0xffffffffu, p, o);
+                if (tid >= o) p *= q;
+            }
+            pre[x + tid] = p * run;
+            run *= __shfl_sync(0xffffffffu, p, 31);
+        }
+    }
+    {
+        // column s of the scores with its decays: half the threads have tokens 0 .. 63, half the rest
+        const int s = tid & (CK - 1), first = tid >> 7 << 6;
+        const float* G = ck.scores + ((size_t)blockIdx.z * groups + hg) * CK * CK + s;
+        const float b = bs[s];
+        float run = 1.f;
+        for (int r = s + 1; r < first; ++r) run *= as[r];
+#pragma unroll 1
+        for (int ta = first; ta < first + 64; ta += 16) {
+            float sc[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) sc[u] = ta + u >= s ? __ldg(G + (size_t)(ta + u) * CK) : 0.f;
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                const int t = ta + u;
+                if (t > s) run *= as[t];
+                X[t * CO_PITCH + s] = t >= s ? sc[u] * (b * run) : 0.f;
+            }
+        }
+    }
+    chunk_fill<CK, CK_C>(Y, CK_C, nt, dv - c0, vec_v, nullptr, [&](int r) {
+        return in.v + (size_t)(t0 + r) * in.ld + (size_t)h * dv + c0; });
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float p = pre[ty + 16 * i];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] *= p;
+    }
+    // (tokens ty + 16 i see nothing of s >= 16 (i + 1))
+#pragma unroll
+    for (int blk = 0; blk < CK / 16; ++blk) {
+        if (blk * 16 >= nt) break;
+        float part[8][4] = {};
+        switch (blk) {                                   // (unrolled: a constant)
+            case 0: chunk_product<0>(part, X, Y, 0, tx, ty); break;
+            case 1: chunk_product<1>(part, X, Y, 16, tx, ty); break;
+            case 2: chunk_product<2>(part, X, Y, 32, tx, ty); break;
+            case 3: chunk_product<3>(part, X, Y, 48, tx, ty); break;
+            case 4: chunk_product<4>(part, X, Y, 64, tx, ty); break;
+            case 5: chunk_product<5>(part, X, Y, 80, tx, ty); break;
+            case 6: chunk_product<6>(part, X, Y, 96, tx, ty); break;
+            default: chunk_product<7>(part, X, Y, 112, tx, ty); break;
+        }
+#pragma unroll
+        for (int i = blk; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int t = ty + 16 * i, c = c0 + tx * 4;
+        if (t >= nt) continue;
+        float* out = num + (size_t)(t0 + t) * H * dv + (size_t)h * dv + c;
+        if (c + 4 <= dv && dv % 4 == 0) {
+            *reinterpret_cast<float4*>(out) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (c + j < dv) out[j] = acc[i][j];
+        }
+    }
+}
+
 // One warp per (token, head): the read-out o = num / (max(|n . q|, exp(-m)) + den_eps), over
 // its root mean square, times the weight, times sigmoid(g).
 template <typename T>
@@ -465,10 +853,27 @@ AGV_API int agv_mlstm_scan(const float* qkv, const float* gates, float* num, flo
 // The scan without normaliser.  q, k: [T, groups * d] and v: [T, H * dv], 32-bit, with row stride
 // ld (parts of one row each); head h reads the q and k of group h / (H / groups); coef [T, H, 2]:
 // a_t, b_t; out [T, H * dv] receives S_t^T q_t; state: S [H, d, dv] per slot from state_off on.
+// max_new: the longest sequence of the step; work: scratch of agv_head_scan_work floats (null: none,
+// and the tokens are taken one by one).
+//
+// By chunks where sequences have some: a token of a head costs an SM 200 ns of issue in the scan, and
+// 230 ns of waiting where few heads and sequences leave it one CTA.  333 + 1,501 tokens, 64 heads of 128
+// x 64: 345 us token by token, 281 token by token in segments of 256 side by side with their states
+// added afterwards, 198 by chunks (scores 10, states 70, pass 9, outputs 109).  At least 192 tokens in the
+// longest and 64 on average, so that chunks are not mostly padding; narrow states stay with the scan,
+// whose tiles are 16 x 32.
+constexpr long long HS_MOST_WORK = 128LL << 20;      // floats of scratch (512 MB)
+AGV_API long long agv_head_scan_work(int T, int B, int H, int groups, int d, int dv, int max_new) {
+    if (max_new < 192 || T < 64 * B || d < 64 || d > 256 || dv < 32 || d * dv % 4 != 0) return 0;
+    const long long n = T / CK + B;                  // chunks at most
+    const long long need = n * ((long long)H * d * dv + (long long)groups * CK * CK + H);
+    return n > 65535 || need > HS_MOST_WORK ? 0 : need;
+}
 AGV_API int agv_head_scan(const float* q, const float* k, const float* v, long long ld,
                           const float* coef, float* out, int T, int B, int H, int groups, int d,
                           int dv, float* state, long long state_stride, long long state_off,
-                          const int* slots, const int* cu_seqlens, cudaStream_t stream) {
+                          const int* slots, const int* cu_seqlens, int max_new, float* work,
+                          cudaStream_t stream) {
     AGV_REQUIRE(T >= 0 && B > 0 && H > 0 && groups > 0 && H % groups == 0 && d > 0 && dv > 0,
                 "head_scan: bad sizes");
     AGV_REQUIRE(d <= 256, "head_scan: state size %d exceeds 256", d);
@@ -476,6 +881,27 @@ AGV_API int agv_head_scan(const float* q, const float* k, const float* v, long l
     AGV_REQUIRE(B <= 65535 && H <= 65535, "head_scan: batch or head count exceeds the grid limit");
     if (T == 0) return 0;
     const ScanIn in{q, k, v, ld, H / groups, coef};
+    if (work && agv_aligned(work, 16) && agv_aligned(coef, 8) && agv_aligned(out, 16) &&
+        agv_head_scan_work(T, B, H, groups, d, dv, max_new) > 0) {
+        const int n = T / CK + B, c_tiles = (dv + CK_C - 1) / CK_C;
+        float* scores = work + (size_t)n * H * d * dv;
+        const Chunks ck{B, cu_seqlens, work, scores + (size_t)n * groups * CK * CK, scores};
+        const int vec_q = ld % 4 == 0 && d % 4 == 0 && agv_aligned(q, 16) && agv_aligned(k, 16);
+        const int vec_v = ld % 4 == 0 && dv % 4 == 0 && agv_aligned(v, 16), vec_s = dv % 4 == 0;
+        agv_launch(chunk_scores_kernel, dim3(3, groups, n), 256, 0, stream, in, d, ck, vec_q);
+        AGV_LAUNCH_OK("chunk_scores_kernel");
+        agv_launch(chunk_states_kernel, dim3((d + 127) / 128 * c_tiles, H, n), 256, 0, stream, in, H, d, dv, ck,
+                   c_tiles, vec_q, vec_v);
+        AGV_LAUNCH_OK("chunk_states_kernel");
+        agv_launch(chunk_pass_kernel, dim3((d * dv / 4 + 255) / 256, H, B), 256, 0, stream, ck, H, d * dv, state,
+                   state_stride, state_off, slots);
+        AGV_LAUNCH_OK("chunk_pass_kernel");
+        AGV_CUDA_OK(cudaFuncSetAttribute(chunk_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CO_SMEM));
+        agv_launch(chunk_outputs_kernel, dim3(c_tiles, H, n), 256, CO_SMEM, stream, in, out, H, d, dv, ck, vec_q,
+                   vec_v, vec_s);
+        AGV_LAUNCH_OK("chunk_outputs_kernel");
+        return 0;
+    }
     // Two columns a lane halve the reads of k and q but also the warps that hide a token's
     // latencies: taken where one column a lane would put a second CTA on most SMs anyway (2,048
     // tokens, 128 heads of 128 x 64: 475 us against 555; 64 such heads: 475 against 367), and

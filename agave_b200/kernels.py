@@ -1188,12 +1188,18 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, coef: torch.Ten
     _dense(coef, "coef"); _dense(out, "out")
     assert coef.shape == (T, H, 2) and out.shape == (T, H * dv)
     sp, ss = _state_args(state)
+    # long sequences are taken by chunks, whose states need scratch
+    max_new = int(getattr(ctx, "max_new", 1))
+    lib = library()
+    lib.agv_head_scan_work.restype = ctypes.c_longlong
+    n = int(lib.agv_head_scan_work(T, ctx.batch, H, n_groups, N, dv, max_new))
+    work = torch.empty(n, dtype=torch.float32, device=out.device) if n else None
     with _span("head_scan", _nbytes(q, k, v, coef, out) + 8 * ctx.batch * H * N * dv,
                5 * T * H * N * dv):
         _check(library().agv_head_scan(
             _ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(v.stride(0)), _ptr(coef), _ptr(out), T,
             ctx.batch, H, n_groups, N, dv, sp, ss, ctypes.c_longlong(state_off), _ptr(ctx.slots),
-            _ptr(ctx.cu_seqlens), _stream()))
+            _ptr(ctx.cu_seqlens), max_new, _ptr(work), _stream()))
 
 
 def ssd_out(num: torch.Tensor, u: torch.Tensor, d: torch.Tensor, row: Optional[torch.Tensor],

@@ -152,3 +152,42 @@ def test_latent_prepare_by_fours(T, latent, interleaved, A, d, r, R, G, dtype):
         kernels.latent_prepare(out, Q, latent, A, d, r, R, G, wq, w, 1e-6, cos, sin, interleaved, pos, partial=part)
         outs.append(out)
     same(*outs, dtype)
+
+
+@pytest.mark.parametrize("H,G,d,dv", [(4, 1, 128, 64), (2, 2, 64, 32), (3, 1, 200, 100), (2, 1, 256, 34)])
+@pytest.mark.parametrize("counts", [[192], [1, 300, 64, 3], [129, 128, 127, 515]])
+@pytest.mark.parametrize("strong", [False, True])
+def test_head_scan_by_chunks(H, G, d, dv, counts, strong):
+    """Chunks that end inside, at and after a sequence's end, states that go on from another step,
+    decays near one and near (and at) zero: against the recurrence in 64 bits, no further from it than the
+    scan token by token (with room for the order of the sums)."""
+    from agave_b200 import kernels
+    T, B, W = sum(counts), len(counts), 2 * G * d + H * dv + 4
+    ctx = step(counts, [0] * B, list(range(B)))
+    row = rnd(T, W, seed=1)
+    q, k, v = row[:, :G * d], row[:, G * d:2 * G * d], row[:, 2 * G * d:2 * G * d + H * dv]
+    a = torch.exp(-torch.exp(rnd(T, H, seed=2, scale=2.0) + (1.0 if strong else -5.0)))
+    if strong:
+        a[T // 2] = 0.0
+    coef = torch.stack([a, rnd(T, H, seed=3).abs()], -1).contiguous()
+    state0 = rnd(B, 5 + H * d * dv, seed=4)
+    S = state0[:, 5:].view(B, H, d, dv).double()
+    want = torch.empty(T, H, dv, dtype=torch.float64, device=DEV)
+    q8, k8 = (t.double().view(T, G, d).repeat_interleave(H // G, 1) for t in (q, k))
+    v8, c8 = v.double().view(T, H, dv), coef.double()
+    at = 0
+    for b, n in enumerate(counts):
+        for t in range(at, at + n):
+            S[b] = c8[t, :, 0, None, None] * S[b] + c8[t, :, 1, None, None] * k8[t, :, :, None] * v8[t, :, None]
+            want[t] = torch.einsum("hd,hdv->hv", q8[t], S[b])
+        at += n
+    err = {}
+    for max_new in (1, max(counts)):
+        ctx.max_new = max_new
+        state, out = state0.clone(), torch.full((T, H * dv), float("nan"), device=DEV)
+        kernels.head_scan(q, k, v, coef, out, ctx, state, 5, H, G, d, dv)
+        err[max_new] = [float((g.double() - r).norm() / r.norm()) for g, r in
+                        ((out.view(T, H, dv), want), (state[:, 5:].view(B, H, d, dv), S))]
+        assert torch.equal(state[:, :5], state0[:, :5])
+    for token, chunk in zip(err[1], err[max(counts)]):
+        assert chunk <= 1.5 * token + 1e-7 and chunk < 2e-6, err
