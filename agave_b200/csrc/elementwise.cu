@@ -364,10 +364,15 @@ norm_residual_warp_kernel(float* __restrict__ h, const float* __restrict__ y, in
     }
 }
 
-// The same with one CTA of 256 threads per row, 16-byte loads issued up front, two
-// block-wide sums: for rows too wide for a warp's registers (above 2,048 values), and for
-// 32 to 256 rows of any width (decoding many sequences: too few rows for a warp each).
-template <typename TX, int NV>
+// The same with one CTA per row, 16-byte loads issued up front, two block-wide sums: for prompts'
+// rows of more than 512 values, and for 32 to 256 rows of any width (decoding many sequences).  U partial
+// sums are loaded together: four where a step has up to sixteen, one in long prompts, whose one or two
+// do not pay for 16 NV registers more a thread, i.e. two CTAs an SM instead of five.
+// Bound by the bytes (h in and out, y, x) and by how many rows' loads an SM has in flight.  With an event's
+// 6 us, against four partial sums at a time (a warp a row up to 2,048 values): 4,001 rows of 2,560, 22 us of
+// HBM, 43.0 -> 30.7; of 5,376, 46 us, 92.1 -> 59.4; 2,048 rows of 2,048 25.6 -> 18.5; 8,696 of 1,152
+// 31.7 -> 29.7, with two partial sums 42.0 -> 37.8.
+template <typename TX, int NV, int U, int TH>
 __global__ void __launch_bounds__(256)
 norm_residual_row_kernel(float* __restrict__ h, const float* __restrict__ y, int n_splits,
                           size_t split_stride, const float* __restrict__ w_post,
@@ -376,35 +381,35 @@ norm_residual_row_kernel(float* __restrict__ h, const float* __restrict__ y, int
     pdl_wait();
     pdl_launch_next();
     __shared__ float red[33];
-    const int lane = threadIdx.x;                   // 256 threads share the row
+    const int lane = threadIdx.x, n = TH ? TH : blockDim.x;         // n threads share the row
     const int row = blockIdx.x;
     const int H4 = H >> 2;
     const size_t base = (size_t)row * H;
     float4 v[NV], hv[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        const int idx = lane + 256 * i;
+        const int idx = lane + n * i;
         const bool in = idx < H4;
         v[i] = in ? reinterpret_cast<const float4*>(y + base)[idx] : make_float4(0, 0, 0, 0);
         hv[i] = (in && add_residual) ? reinterpret_cast<const float4*>(h + base)[idx]
                                      : make_float4(0, 0, 0, 0);
     }
-    // the other partial sums, four at a time: their loads are issued together (a rolled
+    // the other partial sums, U at a time: their loads are issued together (a rolled
     // loop would make one trip to memory per partial sum)
-    for (int s = 1; s < n_splits; s += 4) {
-        float4 t[4][NV];
+    for (int s = 1; s < n_splits; s += U) {
+        float4 t[U][NV];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
             const float* src = y + (size_t)min(s + u, n_splits - 1) * split_stride + base;
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
-                const int idx = lane + 256 * i;
+                const int idx = lane + n * i;
                 t[u][i] = idx < H4 ? reinterpret_cast<const float4*>(src)[idx]
                                    : make_float4(0, 0, 0, 0);
             }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
             if (s + u < n_splits) {
 #pragma unroll
                 for (int i = 0; i < NV; ++i) {
@@ -426,7 +431,7 @@ norm_residual_row_kernel(float* __restrict__ h, const float* __restrict__ y, int
     float ss2 = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        const int idx = lane + 256 * i;
+        const int idx = lane + n * i;
         if (idx < H4) {
             if (w_post) {
                 const float4 w = reinterpret_cast<const float4*>(w_post)[idx];
@@ -445,7 +450,7 @@ norm_residual_row_kernel(float* __restrict__ h, const float* __restrict__ y, int
         const float r2 = 1.0f / sqrtf(ss2 / (float)H + eps_next);
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            const int idx = lane + 256 * i;
+            const int idx = lane + n * i;
             if (idx < H4) {
                 const float4 w = reinterpret_cast<const float4*>(w_next)[idx];
                 Pack4<TX>::store(x + base + 4 * idx,
@@ -456,7 +461,7 @@ norm_residual_row_kernel(float* __restrict__ h, const float* __restrict__ y, int
     } else if (x) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            const int idx = lane + 256 * i;
+            const int idx = lane + n * i;
             if (idx < H4) Pack4<TX>::store(x + base + 4 * idx, v[i]);
         }
     }
@@ -474,11 +479,7 @@ static bool launch_norm_warp(float* h, const float* y, int n_splits, size_t spli
                split_stride, w_post, w_next, x, R, H, eps_post, eps_next, add_residual)
     if (nv <= 2) AGV_WARP(2);
     else if (nv <= 4) AGV_WARP(4);
-    else if (nv <= 6) AGV_WARP(6);
-    else if (nv <= 8) AGV_WARP(8);
     else if (nv <= 10) AGV_WARP(10);
-    else if (nv <= 12) AGV_WARP(12);
-    else if (nv <= 16) AGV_WARP(16);
     else return false;
 #undef AGV_WARP
     return true;
@@ -491,9 +492,16 @@ static bool launch_norm_row(float* h, const float* y, int n_splits, size_t split
                             cudaStream_t stream) {
     const int nv = (H / 4 + 255) / 256;
 #define AGV_ROW(NV)                                                                             \
-    agv_launch(norm_residual_row_kernel<TX, NV>, (unsigned)R, 256, 0, stream, h, y, n_splits,   \
-               split_stride, w_post, w_next, x, R, H, eps_post, eps_next, add_residual)
+    do {                                                                                        \
+        const int threads = R <= 256 ? 256 : ((H / 4 + NV - 1) / NV + 31) / 32 * 32;            \
+        auto kern = R <= 256       ? norm_residual_row_kernel<TX, NV, 4, 256>                   \
+                    : n_splits > 2 ? norm_residual_row_kernel<TX, NV, 4, 0>                     \
+                                   : norm_residual_row_kernel<TX, NV, 1, 0>;                    \
+        agv_launch(kern, (unsigned)R, threads, 0, stream, h, y, n_splits, split_stride, w_post, w_next, x, R, H, \
+                   eps_post, eps_next, add_residual);                                           \
+    } while (0)
     if (nv <= 2) AGV_ROW(2);
+    else if (nv <= 3) AGV_ROW(3);
     else if (nv <= 4) AGV_ROW(4);
     else if (nv <= 6) AGV_ROW(6);
     else if (nv <= 8) AGV_ROW(8);
@@ -507,9 +515,11 @@ static int launch_norm(float* h, const void* y, int n_splits, size_t split_strid
                        const float* w_post, const float* w_next, void* x, const int* rows, int R,
                        int H, float eps_post, float eps_next, int add_residual,
                        cudaStream_t stream) {
-    // many rows with a 32-bit branch input: one warp per row
+    // many rows with a 32-bit branch input: one warp per row while a row is a few loads a lane, and
+    // for rows of up to 1,280 values where their number gives every SM 7 to 20 warps (2,048 of 1,152: 14.4 us
+    // alone either way, but 0.4 us a launch less in a step, whose next kernel finds room earlier)
     if constexpr (std::is_same<TY, float>::value) {
-        if (R > 256 && y && !rows && H % 4 == 0 && H <= 2048 && agv_aligned(y, 16) &&
+        if (R > 256 && (H <= 512 || (H <= 1280 && R > 1024 && R <= 3072)) && y && !rows && H % 4 == 0 && agv_aligned(y, 16) &&
             agv_aligned(h, 16) && agv_aligned(x, 16) && split_stride % 4 == 0 &&
             (!w_post || agv_aligned(w_post, 16)) && (!w_next || agv_aligned(w_next, 16)) &&
             (add_residual || !h || true)) {
@@ -519,7 +529,7 @@ static int launch_norm(float* h, const void* y, int n_splits, size_t split_strid
                 return 0;
             }
         }
-        if (((R > 256 && H > 2048) || (R >= 32 && R <= 256)) && y && !rows && H % 4 == 0 && H <= 8192 && agv_aligned(y, 16) &&
+        if (((R > 256 && H > 512) || (R >= 32 && R <= 256)) && y && !rows && H % 4 == 0 && H <= 8192 && agv_aligned(y, 16) &&
             agv_aligned(h, 16) && agv_aligned(x, 16) && split_stride % 4 == 0 &&
             (!w_post || agv_aligned(w_post, 16)) && (!w_next || agv_aligned(w_next, 16))) {
             if (launch_norm_row<TX>(h, (const float*)y, n_splits, split_stride, w_post, w_next,
