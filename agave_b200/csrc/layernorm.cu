@@ -176,13 +176,17 @@ layer_norm_rows_kernel(float* __restrict__ h, const float* __restrict__ y, int n
     if (row >= R) return;                          // (whole warps, or nobody, leave)
     const int H4 = H >> 2;
     const size_t base = (size_t)row * H;
-    float4 v[NV];
+    constexpr bool EARLY = NV <= 4;                // the stream's row is asked for with the branch's
+    float4 v[NV], early[EARLY ? NV : 1];
     if (y) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int idx = lane + GT * i;
             v[i] = idx < H4 ? reinterpret_cast<const float4*>(y + base)[idx]
                             : make_float4(0, 0, 0, 0);
+            if constexpr (EARLY)
+                early[i] = add_residual && idx < H4 ? reinterpret_cast<const float4*>(h + base)[idx]
+                                                    : make_float4(0, 0, 0, 0);
         }
         for (int s = 1; s < n_splits; ++s) {
 #pragma unroll
@@ -198,10 +202,11 @@ layer_norm_rows_kernel(float* __restrict__ h, const float* __restrict__ y, int n
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int idx = lane + GT * i;
-            // (the stream's row is asked for here, not up front: with both in registers the
-            // widest rows spill, and a prompt has rows enough to hide the trip)
+            // (wide rows a thread ask for the stream's row here, not up front: with both in
+            // registers they spill, and a prompt has rows enough to hide the trip)
             float4 hv = make_float4(0, 0, 0, 0);
-            if (add_residual && idx < H4) hv = reinterpret_cast<const float4*>(h + base)[idx];
+            if constexpr (EARLY) hv = early[i];
+            else if (add_residual && idx < H4) hv = reinterpret_cast<const float4*>(h + base)[idx];
             v[i].x = v[i].x * mult + hv.x; v[i].y = v[i].y * mult + hv.y;
             v[i].z = v[i].z * mult + hv.z; v[i].w = v[i].w * mult + hv.w;
             if (idx >= H4) v[i] = make_float4(0, 0, 0, 0);
@@ -238,8 +243,10 @@ bool launch_layer_norm_rows(float* h, const float* y, int n_splits, size_t split
         if (nv <= 2) AGV_LNR(2, 32);
         else if (nv <= 4) AGV_LNR(4, 32);
         else if (nv <= 8) AGV_LNR(8, 32);
-        else if (nv <= 12) AGV_LNR(12, 32);
-        else AGV_LNR(16, 32);
+        // (a warp a row has too few rows' loads in flight: 2,048 rows of 2,048 26.6 us, 20.5 with a CTA; of
+        // 1,152, where a third of a CTA's threads would idle, 16.4 and 18.4, but 512 rows 14.4 and 9.1)
+        else if (R <= 1024 || nv > 12) AGV_LNR(2, 256);
+        else AGV_LNR(12, 32);
     } else {
         const int nv = (H / 4 + 255) / 256;
         if (nv <= 4) AGV_LNR(4, 256);
