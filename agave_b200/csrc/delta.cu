@@ -228,6 +228,43 @@ delta_prepare_rows_kernel(RowIn<float> in, DeltaDims dm, DeltaState st, int n_to
             }
             xs[j][i] = a;
         }
+    // a tile whose every token finds its whole past in the step: products and sums alone
+    bool plain = R > 1 && t0 + R <= n_tokens && !fused_state;
+#pragma unroll
+    for (int i = 0; i < R; ++i) plain = plain && slot[i] >= 0 && before[i] >= RING;
+    if (R > 1 && plain) {
+        const float mult = seg < dm.G ? q_mult : 1.0f;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            float y[NJ][4], ss = 0.f;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int k = RING; k >= 0; --k) {          // oldest input first
+                    const float4 x = xs[j][RING + i - k];
+                    acc[0] = fmaf(wv[j][RING - k], x.x, acc[0]);
+                    acc[1] = fmaf(wv[j][TAPS + RING - k], x.y, acc[1]);
+                    acc[2] = fmaf(wv[j][2 * TAPS + RING - k], x.z, acc[2]);
+                    acc[3] = fmaf(wv[j][3 * TAPS + RING - k], x.w, acc[3]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    y[j][e] = silu_f(acc[e]);
+                    ss = fmaf(y[j][e], y[j][e], ss);
+                }
+            }
+            const float r = head ? (1.0f / sqrtf(warp_sum(ss) + eps_unit)) * mult : 1.f;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                const int ch = j * 128 + lane * 4;
+                if (ch < width)
+                    *reinterpret_cast<float4*>(qkv + (size_t)(t0 + i) * C + c0 + ch) =
+                        make_float4(y[j][0] * r, y[j][1] * r, y[j][2] * r, y[j][3] * r);
+            }
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < R; ++i) {
         const int t = t0 + i;
@@ -397,9 +434,11 @@ __host__ __device__ inline size_t scan_buf_floats(int TCH, int Dp, int CC) {
 }
 
 // A lane's rows of CPT columns (CC apart), two rows to a register pair: a piece of a token's row read
-// once serves them all.  The pieces of k, g, g k and g q are what bounds the kernel: 16 reads of 16
-// bytes a lane and token, 256 cycles of an SM's shared memory for the four warps of a CTA.
-// 8 sequences of 256 to 1,024 tokens, 16 heads of 128 x 128: one column a lane 905 us, two MEASURED_D.
+// once serves them all.  What bounds it are a token's reads of k, g, g k and g q (16 of 16 bytes a
+// lane), the sums over the lanes and the wait for u, token after token, behind the longest sequence.
+// 8 sequences of 256 to 1,024 tokens, 16 heads of 128 x 128: 905 us with one column a lane, a value a
+// register and the sequences as they come; 856 with pairs and the longest first; 644 with two columns (four:
+// 620, but a step of 287 tokens lost what that gained).
 template <int L, int CPT>
 __global__ void __launch_bounds__(128)
 delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {

@@ -62,14 +62,20 @@ ssm_conv_kernel(RowIn<float> in, int n_tokens, int off, int C, StepArgs st,
     __shared__ int s_pos[R], s_in[R], s_slot[R], s_keep[R];
     const int c = blockIdx.x * 128 + threadIdx.x;
     const int t0 = blockIdx.y * R;
-    if (threadIdx.x < R && t0 + threadIdx.x < n_tokens) {
-        const int t = t0 + threadIdx.x, e = st.seq_index[t], p = st.positions[t];
-        s_pos[threadIdx.x] = p;
-        s_in[threadIdx.x] = t - st.cu[e];
-        s_slot[threadIdx.x] = st.slots[e];
-        s_keep[threadIdx.x] = p >= st.lens[e] - RING;
+    bool past = true;
+    if (threadIdx.x < R) {
+        past = t0 + threadIdx.x < n_tokens;
+        if (past) {
+            const int t = t0 + threadIdx.x, e = st.seq_index[t], p = st.positions[t];
+            s_pos[threadIdx.x] = p;
+            s_in[threadIdx.x] = t - st.cu[e];
+            s_slot[threadIdx.x] = st.slots[e];
+            s_keep[threadIdx.x] = p >= st.lens[e] - RING;
+            past = s_in[threadIdx.x] >= RING && s_slot[threadIdx.x] >= 0 && !s_keep[threadIdx.x];
+        }
     }
-    __syncthreads();
+    // whether every token of the tile finds its whole past in the step and none is kept
+    const bool plain = __syncthreads_and(past);
     if (c >= C + n_dt) return;
     if (c >= C) {
         const int h = c - C;
@@ -101,6 +107,20 @@ ssm_conv_kernel(RowIn<float> in, int n_tokens, int off, int C, StepArgs st,
             const int t = t0 - RING + i;
             xs[i] = t >= 0 && t < n_tokens ? in.at(t, off + c) : 0.f;
         }
+    }
+    if (plain) {
+        // (products and sums alone: the places to look for an input cost more than all the rest.  1,834
+        // tokens of 4,352 channels, 64 MB: 41.5 us -> 24.8)
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            float acc = b;
+#pragma unroll
+            for (int k = RING; k >= 0; --k) acc = fmaf(wv[RING - k], xs[RING + i - k], acc);
+            const float y = silu_f(acc);
+            out[(size_t)(t0 + i) * C + c] = y;
+            if (rounded) rounded[(size_t)(t0 + i) * C + c] = from_f32<T>(y);
+        }
+        return;
     }
 #pragma unroll
     for (int i = 0; i < R; ++i) {
