@@ -137,7 +137,7 @@ delta_prepare_kernel(RowIn<T> in, DeltaDims dm, DeltaState st, const float* __re
 // A decode step is bound by trips to memory one after the other: a CTA a token walked its 3,216
 // columns in a dozen of them, 35 us for 8 tokens (G 4, H 16, heads of 128, eight partial sums);
 // 31 warps a token make two, 4.7 us.  A prompt is bound by its rows (126 MB for 5,120 tokens, 20
-// us): 191 us -> 122 us with R = 8, which reads a row once instead of once a tap.
+// us): 191 us -> 108 with R = 8, which reads a row once instead of once a tap.
 template <typename T, int TAPS, int NJ, int R>
 __global__ void __launch_bounds__(128)
 delta_prepare_rows_kernel(RowIn<float> in, DeltaDims dm, DeltaState st, int n_tokens, int n_seg,

@@ -227,14 +227,40 @@ struct SelectiveArgs {
     int inner, N, z_off;       // z: columns z_off .. of the stacked projection
 };
 
-// grid (channel blocks, sequences), 128 threads: 128 / L channels a CTA, L lanes a channel, NS
+// Sequences cut into segments of `len` tokens (0: whole ones), which run side by side: a first pass
+// leaves the state at every segment's end but a sequence's last, from nothing, and the sum of its step
+// sizes; segment_begins_kernel makes of them what every segment begins from, since the decays over a
+// segment are exp(A sum dt); the second pass is the scan itself.
+struct Segments {
+    int len, n_seq;
+    float* ends;               // [segments, inner, N]
+    float* sums;               // [segments, inner]
+};
+__device__ __forceinline__ bool segment_of(const Segments& sg, const int* __restrict__ cu, int z, int& seq,
+                                           int& part, int& parts) {
+    int at = 0;
+    for (int e = 0; e < sg.n_seq; ++e) {
+        const int n = (cu[e + 1] - cu[e] + sg.len - 1) / sg.len;
+        if (z < at + n) {
+            seq = e;
+            part = z - at;
+            parts = n;
+            return true;
+        }
+        at += n;
+    }
+    return false;
+}
+
+// grid (channel blocks, sequences or segments), 128 threads: 128 / L channels a CTA, L lanes a channel, NS
 // states a lane.  Tokens come SS_CH at a time through two buffers filled by asynchronous copies;
 // after a chunk has landed the CTA turns its step sizes into (dt, dt u) once, runs the
 // recurrence (four tokens' read-outs are reduced over the lanes together), and finishes the
 // chunk's outputs with the gate.  A token beyond the chunk has dt = 0 and changes nothing.
-template <typename T, int NS, int L>
+// PASS 0: whole sequences; 1, 2: the passes over segments.
+template <typename T, int NS, int L, int PASS>
 __global__ void __launch_bounds__(SS_THREADS)
-selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restrict__ out) {
+selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restrict__ out, Segments sg) {
     pdl_wait();
     extern __shared__ __align__(16) float sm[];
     constexpr int CC = SS_THREADS / L, Np = NS * L, CH = SS_CH;
@@ -242,8 +268,12 @@ selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restri
     constexpr int ZN = CH * CC / SS_THREADS > 0 ? CH * CC / SS_THREADS : 1;
     float2* dd = reinterpret_cast<float2*>(sm + 2 * BUF);     // [CH][CC] (dt, dt u)
     float* ys = reinterpret_cast<float*>(dd + CH * CC);       // [CH][CC]
-    const int e = blockIdx.y, slot = st.slots[e];
-    const int t0 = st.cu[e], n = st.cu[e + 1] - t0;
+    int e = blockIdx.y, part = 0, parts = 1;
+    if (PASS && !segment_of(sg, st.cu, blockIdx.y, e, part, parts)) return;
+    if (PASS == 1 && part == parts - 1) return;
+    const int slot = st.slots[e];
+    const int t0 = st.cu[e] + (PASS ? part * sg.len : 0);
+    const int n = PASS ? min(st.cu[e + 1] - t0, sg.len) : st.cu[e + 1] - t0;
     const int tid = threadIdx.x, l = tid % L, jc = tid / L;
     const int cb = blockIdx.x * CC, c = cb + jc;
     const bool live = c < a.inner;
@@ -257,7 +287,7 @@ selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restri
     __syncthreads();
     // z comes with the tokens where it is one sum, else its partial sums are added up below
     long long zld;
-    const float* zrow = in.single(zld);
+    const float* zrow = PASS == 1 ? nullptr : in.single(zld);
     if (zrow) zrow += a.z_off;
     const bool vec = a.inner % 4 == 0 && CC % 4 == 0 &&
                      (!zrow || (zld % 4 == 0 && ((uintptr_t)zrow & 15) == 0));
@@ -298,7 +328,8 @@ selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restri
     for (int s = 0; s < NS; ++s) {
         const int k = l * NS + s;
         const bool ok = live && k < a.N;
-        S[s] = ok ? srow[k] : 0.f;
+        if (PASS == 0) S[s] = ok ? srow[k] : 0.f;
+        else S[s] = PASS == 2 && ok ? sg.ends[((size_t)blockIdx.y * a.inner + c) * a.N + k] : 0.f;
         a2[s] = ok ? a.a2[(size_t)c * a.N + k] : 0.f;
     }
     // outside the recurrence a thread's places of a chunk all have one channel
@@ -306,6 +337,7 @@ selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restri
     const bool mine = my_c < a.inner;
     const float my_bias = mine ? a.dt_bias[my_c] : 0.f, my_d = mine ? a.D[my_c] : 0.f;
     const int n_chunks = (n + CH - 1) / CH;
+    float steps = 0.f;                                   // (PASS 1: of the thread's channel)
     for (int ch = 0; ch < n_chunks; ++ch) {
         const int c0 = ch * CH, m = min(CH, n - c0);
         const float* base = sm + (ch & 1) * BUF;
@@ -329,6 +361,7 @@ selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restri
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float2 d = dd[(tt + q) * CC + jc];
+                if (PASS == 1) steps += d.x;
                 const float* row = bs + (tt + q) * 2 * Np + l * NS;
                 float B[NS], Cv[NS];
                 if constexpr (NS % 4 == 0) {
@@ -348,10 +381,11 @@ selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restri
 #pragma unroll
                 for (int s = 0; s < NS; ++s) {
                     S[s] = fmaf(d.y, B[s], ex2_ftz(d.x * a2[s]) * S[s]);
-                    acc = fmaf(S[s], Cv[s], acc);
+                    if (PASS != 1) acc = fmaf(S[s], Cv[s], acc);
                 }
                 y[q] = acc;
             }
+            if constexpr (PASS == 1) continue;
             // sum over the channel's lanes: each exchange halves the tokens a lane answers for
             if constexpr (L == 1) {
 #pragma unroll
@@ -374,6 +408,7 @@ selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restri
                 }
             }
         }
+        if constexpr (PASS == 1) continue;
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < ZN; ++i) {
@@ -386,11 +421,40 @@ selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restri
         }
     }
     pdl_launch_next();
-    if (live) {
+    if (PASS == 1) {
+        srow = sg.ends + ((size_t)blockIdx.y * a.inner + (live ? c : 0)) * a.N;
+        if (live && l == 0) sg.sums[(size_t)blockIdx.y * a.inner + c] = steps;
+    }
+    if (live && (PASS != 2 || part == parts - 1)) {
 #pragma unroll
         for (int s = 0; s < NS; ++s)
             if (l * NS + s < a.N) srow[l * NS + s] = S[s];
     }
+}
+
+// grid (values of S, sequences): `ends` becomes what every segment begins from.
+__global__ void __launch_bounds__(256)
+segment_begins_kernel(SelectiveArgs a, StepArgs st, Segments sg) {
+    pdl_wait();
+    pdl_launch_next();
+    const int e = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x, slot = st.slots[e];
+    const int n = (st.cu[e + 1] - st.cu[e] + sg.len - 1) / sg.len;
+    if (i >= a.inner * a.N || n == 0 || slot < 0) return;
+    int z = 0;
+    for (int j = 0; j < e; ++j) z += (st.cu[j + 1] - st.cu[j] + sg.len - 1) / sg.len;
+    const int c = i / a.N;
+    const float a2 = a.a2[i];
+    float run = st.state[(size_t)slot * st.stride + st.off + i];
+    float* at = sg.ends + (size_t)z * a.inner * a.N + i;
+    const float* sum = sg.sums + (size_t)z * a.inner + c;
+    const size_t step = (size_t)a.inner * a.N;
+#pragma unroll 4
+    for (int s = 0; s < n - 1; ++s) {
+        const float own = at[s * step], d = ex2_ftz(sum[(size_t)s * a.inner] * a2);
+        at[s * step] = run;
+        run = fmaf(d, run, own);
+    }
+    at[(n - 1) * step] = run;
 }
 
 // ------------------------------------------------------ read-out of the head scan
@@ -491,21 +555,40 @@ void launch_conv(const RowIn<float>& in, int n_tokens, int off, int C, const Ste
                    off, C, st, w, bias, out, rounded, dt_off, n_dt, dt_bias, neg_a, coef);
 }
 
+// Tokens of a segment (0: the sequences are not cut).  A CTA's chain takes 148 ns a token with two CTAs
+// an SM and the step's tokens times its CTAs are what there is to spread: about six CTAs an SM.  333 +
+// 1,501 tokens, 4,096 channels of 16 states: 223 us whole, 136 so (50 + 8 + 78).
+constexpr int SS_CTAS = 6 * 148;
+int selective_segment(int T, int B, int inner, int N, int max_new) {
+    if (T <= B) return 0;
+    const int Np = ss_pad(N), L = Np <= 8 ? 2 : Np <= 16 ? 4 : Np <= 64 ? 8 : Np <= 128 ? 16 : 32;
+    const int CC = SS_THREADS / L;
+    const long long blocks = (inner + CC - 1) / CC;
+    long long len = (T * blocks / SS_CTAS + 15) / 16 * 16;
+    if (len < 96) len = 96;
+    return 2LL * max_new >= 3 * len ? (int)len : 0;
+}
+
 template <typename T, int NS, int L>
 int launch_selective(const SelectiveArgs& a, const RowIn<float>& in, const StepArgs& st, int B,
-                     T* out, cudaStream_t stream) {
-    auto kern = selective_scan_kernel<T, NS, L>;
+                     T* out, const Segments& sg, int n_seg, cudaStream_t stream) {
     constexpr int CC = SS_THREADS / L;
     constexpr int smem = (2 * SS_CH * (3 * CC + 2 * NS * L) + 3 * SS_CH * CC) * (int)sizeof(float);
-    static bool configured = false;
-    if (smem > 48 * 1024 && !configured) {
-        AGV_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured = true;
-    }
-    // (as with the other scans: few CTAs, each a long dependent chain, spread over the SMs)
-    agv_launch_after(kern, dim3((a.inner + CC - 1) / CC, B), SS_THREADS, smem, stream, a, in, st, out);
-    AGV_LAUNCH_OK("selective_scan_kernel");
-    return 0;
+    const unsigned blocks = (unsigned)((a.inner + CC - 1) / CC);
+    auto run = [&](auto kern, int rows) -> int {
+        if (smem > 48 * 1024)
+            AGV_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        // (as with the other scans: few CTAs, each a long dependent chain, spread over the SMs)
+        agv_launch_after(kern, dim3(blocks, (unsigned)rows), SS_THREADS, smem, stream, a, in, st, out, sg);
+        AGV_LAUNCH_OK("selective_scan_kernel");
+        return 0;
+    };
+    if (!sg.len) return run(selective_scan_kernel<T, NS, L, 0>, B);
+    if (int rc = run(selective_scan_kernel<T, NS, L, 1>, n_seg)) return rc;
+    agv_launch(segment_begins_kernel, dim3((unsigned)((a.inner * a.N + 255) / 256), (unsigned)B), 256, 0, stream, a,
+               st, sg);
+    AGV_LAUNCH_OK("segment_begins_kernel");
+    return run(selective_scan_kernel<T, NS, L, 2>, n_seg);
 }
 
 }  // namespace
@@ -581,15 +664,23 @@ AGV_API int agv_selective_low(const void* row, long long ld, const float* part, 
     return 0;
 }
 
+AGV_API long long agv_selective_scan_work(int T, int B, int inner, int N, int max_new) {
+    const int len = selective_segment(T, B, inner, N, max_new);
+    if (!len || T / len + B > 65535) return 0;
+    return (long long)(T / len + B) * ((long long)inner * N + inner);
+}
 // u, dt [T, inner], dt_bias, D [inner], bc [T, 2 Np] (agv_selective_low), a2 [inner, N] = A *
 // log2(e), all 32-bit; z: columns z_off .. z_off + inner of the stacked projection (row / part as
 // in agv_ssm_conv); out [T, inner] in dtype; state: S [inner, N] per slot from state_off on.
+// max_new: the longest sequence of the step; work: scratch of agv_selective_scan_work floats (null: none, and
+// the sequences are not cut).
 AGV_API int agv_selective_scan(const float* u, const float* dt, const float* dt_bias,
                                const float* bc, const float* a2, const float* D, const float* row,
                                long long ld, const float* part, int n_splits, int T, int W,
                                int z_off, int B, int inner, int N, void* out, int dtype,
                                float* state, long long state_stride, long long state_off,
-                               const int* slots, const int* cu, cudaStream_t stream) {
+                               const int* slots, const int* cu, int max_new, float* work,
+                               cudaStream_t stream) {
     AGV_REQUIRE(T >= 0 && B >= 0 && inner > 0 && N > 0 && N <= SS_MAX_N && z_off >= 0 &&
                 z_off + inner <= W, "selective_scan: bad sizes");
     AGV_REQUIRE(B <= 65535, "selective_scan: batch %d exceeds the grid limit", B);
@@ -602,11 +693,14 @@ AGV_API int agv_selective_scan(const float* u, const float* dt, const float* dt_
     if (int rc = row_of(in, row, ld, part, n_splits, T, W)) return rc;
     const SelectiveArgs a{u, dt, dt_bias, bc, a2, D, inner, N, z_off};
     const StepArgs st{state, state_stride, state_off, slots, cu, nullptr, nullptr, nullptr};
-    const int Np = ss_pad(N);
+    const int Np = ss_pad(N), len = work ? selective_segment(T, B, inner, N, max_new) : 0;
+    const int n_seg = len ? T / len + B : 0;             // (at most: a sequence rounds up by less than one)
+    AGV_REQUIRE(n_seg <= 65535, "selective_scan: %d segments exceed the grid limit", n_seg);
+    const Segments sg{len, B, work, len ? work + (size_t)n_seg * inner * N : nullptr};
 #define AGV_SS(NS, L)                                                                            \
-    return dtype == AGV_F32 ? launch_selective<float, NS, L>(a, in, st, B, (float*)out, stream)  \
-                            : launch_selective<__nv_bfloat16, NS, L>(a, in, st, B,               \
-                                                                     (__nv_bfloat16*)out, stream)
+    return dtype == AGV_F32                                                                      \
+               ? launch_selective<float, NS, L>(a, in, st, B, (float*)out, sg, n_seg, stream)    \
+               : launch_selective<__nv_bfloat16, NS, L>(a, in, st, B, (__nv_bfloat16*)out, sg, n_seg, stream)
     AGV_REQUIRE(dtype == AGV_F32 || dtype == AGV_BF16, "selective_scan: unknown dtype %d", dtype);
     switch (Np) {
         case 4: AGV_SS(2, 2);

@@ -1164,12 +1164,18 @@ def selective_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, bc:
     lib = library()
     assert lib.agv_selective_pad(N) == selective_pad(N)
     sp, ss = _state_args(state)
+    # long sequences are cut into segments, whose states need scratch
+    max_new = int(getattr(ctx, "max_new", 1))
+    lib.agv_selective_scan_work.restype = ctypes.c_longlong
+    n = int(lib.agv_selective_scan_work(T, ctx.batch, inner, N, max_new))
+    work = torch.empty(n, dtype=torch.float32, device=out.device) if n else None
     with _span("selective_scan", _nbytes(u, dt, bc, out) + T * inner * 4 * max(ns, 1) +
                8 * ctx.batch * inner * N, 7 * T * inner * N):
         _check(lib.agv_selective_scan(
             _ptr(u), _ptr(dt), _ptr(dt_bias), _ptr(bc), _ptr(a2), _ptr(d), rp, ld, pp, ns, T, W,
             z_offset, ctx.batch, inner, N, _ptr(out), dtype_code(out.dtype), sp, ss,
-            ctypes.c_longlong(state_off), _ptr(ctx.slots), _ptr(ctx.cu_seqlens), _stream()))
+            ctypes.c_longlong(state_off), _ptr(ctx.slots), _ptr(ctx.cu_seqlens), max_new, _ptr(work),
+            _stream()))
 
 
 def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, coef: torch.Tensor,

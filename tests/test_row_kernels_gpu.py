@@ -191,3 +191,29 @@ def test_head_scan_by_chunks(H, G, d, dv, counts, strong):
         assert torch.equal(state[:, :5], state0[:, :5])
     for token, chunk in zip(err[1], err[max(counts)]):
         assert chunk <= 1.5 * token + 1e-7 and chunk < 2e-6, err
+
+
+@pytest.mark.parametrize("inner,N", [(96, 16), (130, 4), (64, 7), (33, 128), (48, 200)])
+@pytest.mark.parametrize("counts", [[150], [1, 700, 96, 3], [192, 191, 97, 515]])
+@pytest.mark.parametrize("dtype", [BF, F32])
+def test_selective_scan_by_segments(inner, N, counts, dtype):
+    """Segments that end inside, at and after a sequence's end, states that go on from another step:
+    against the scan of whole sequences (2^-21 a decay, over a segment once instead of a token)."""
+    from agave_b200 import kernels
+    T, B, Np = sum(counts), len(counts), kernels.selective_pad(N)
+    ctx = step(counts, [0] * B, list(range(B)))
+    u, dt, z = rnd(T, inner, seed=1), rnd(T, inner, seed=2) - 1.0, rnd(T, inner, seed=3)
+    bc = torch.zeros(T, 2, Np, device=DEV)
+    bc[:, :, :N] = rnd(T, 2, N, seed=4)
+    a2 = -torch.exp(rnd(inner, N, seed=5, scale=2.0) - 2.0)
+    bias, d, state0 = rnd(inner, seed=6), rnd(inner, seed=7), rnd(B, 3 + inner * N, seed=8)
+    got = []
+    for max_new in (1, max(counts)):
+        ctx.max_new = max_new
+        state, out = state0.clone(), torch.full((T, inner), float("nan"), dtype=dtype, device=DEV)
+        kernels.selective_scan(u, dt, bias, bc.view(T, -1), a2, d, z, None, inner, 0, out, ctx, state, 3)
+        got.append((out, state))
+    assert float((got[0][1] - got[1][1]).abs().max()) <= 4e-6 * float(got[0][1].abs().max())
+    assert torch.equal(got[0][1][:, :3], got[1][1][:, :3])
+    tol = 4e-6 if dtype == F32 else 2.0 ** -8
+    assert float((got[0][0].double() - got[1][0].double()).abs().max()) <= tol * float(got[0][0].abs().max())
