@@ -711,6 +711,29 @@ def test_sampling_of_long_rows_against_the_procedure(V, top_k, top_p):
         assert upto - float(w[tok]) - slack <= u * total <= upto + slack, (b, tok, u)
 
 
+@pytest.mark.parametrize("V", [40, 5000, 16384])
+@pytest.mark.parametrize("top_k,top_p", [(1, 1.0), (7, 0.9), (39, 1.0), (1024, 0.95), (1025, 0.5), (0, 0.8)])
+def test_sampling_token_does_not_depend_on_the_ctas_of_a_row(V, top_k, top_p):
+    """One CTA a row (the bound's descent directly before the k-th key's) and, with masked values
+    behind the row, clusters of 2, 4 and 8: the same tokens, since what decides is exact."""
+    from agave_b200 import kernels
+    if top_k >= V:
+        pytest.skip("the cut has to be there at every length")
+    B = 33
+    seq = torch.arange(B, dtype=torch.int64, device=DEV)
+    steps = torch.zeros(B, dtype=torch.int32, device=DEV)
+    row = torch.round(rnd(B, V, seed=V) * 8.0) / 4.0      # (equal values at every cut)
+    tokens = []
+    for length in (V, 16388, 32772, 70000):
+        logits = torch.full((B, length), -math.inf, device=DEV)
+        logits[:, :V] = row
+        out = torch.full((B,), -5, dtype=torch.int32, device=DEV)
+        kernels.sample(logits, out, 0.7, top_k, top_p, 5, seq, steps)
+        tokens.append(out.tolist())
+    assert all(t == tokens[0] for t in tokens), tokens
+    assert all(0 <= t < V for t in tokens[0])
+
+
 def test_repeat_penalty_per_occurrence_and_history():
     from agave_b200 import kernels
     V = 300
