@@ -601,8 +601,10 @@ chunk_pass_kernel(Chunks ck, int H, int dn, float* __restrict__ state, long long
 // the same shared memory.
 constexpr int CO_PITCH = CK + 4;
 constexpr int CO_SMEM = (CK * CO_PITCH + CK * CK_C) * 4;
-// Tokens ty + 16 i, i >= FROM, times 16 of the common dimension from k0 on.
-template <int FROM>
+// Tokens ty + 16 i, i >= FROM, times 16 of the common dimension from k0 on.  DIAG: the common dimension are
+// tokens too, and the first of the thread's (block FROM) takes no later one than itself: a product with zero
+// would hand it the infinities and NaNs of tokens that it must not see.
+template <int FROM, bool DIAG>
 __device__ __forceinline__ void chunk_product(float (&part)[8][4], const float* X, const float* Y, int k0, int tx,
                                               int ty) {
 #pragma unroll 2
@@ -616,6 +618,7 @@ __device__ __forceinline__ void chunk_product(float (&part)[8][4], const float* 
             const float xe[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
+                if (DIAG && i == FROM && k + j - k0 > ty) continue;
                 part[i][0] = fmaf(xe[j], y[j].x, part[i][0]);
                 part[i][1] = fmaf(xe[j], y[j].y, part[i][1]);
                 part[i][2] = fmaf(xe[j], y[j].z, part[i][2]);
@@ -655,7 +658,7 @@ chunk_outputs_kernel(ScanIn in, float* __restrict__ num, int H, int d, int dv, C
         // (sums of 16 terms, then added: a chain of 128 would round three times as far)
         for (int kb = 0; kb < CK && n0 + kb < d; kb += 16) {
             float part[8][4] = {};
-            chunk_product<0>(part, X, Y, kb, tx, ty);
+            chunk_product<0, false>(part, X, Y, kb, tx, ty);
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -711,14 +714,14 @@ chunk_outputs_kernel(ScanIn in, float* __restrict__ num, int H, int d, int dv, C
         if (blk * 16 >= nt) break;
         float part[8][4] = {};
         switch (blk) {                                   // (unrolled: a constant)
-            case 0: chunk_product<0>(part, X, Y, 0, tx, ty); break;
-            case 1: chunk_product<1>(part, X, Y, 16, tx, ty); break;
-            case 2: chunk_product<2>(part, X, Y, 32, tx, ty); break;
-            case 3: chunk_product<3>(part, X, Y, 48, tx, ty); break;
-            case 4: chunk_product<4>(part, X, Y, 64, tx, ty); break;
-            case 5: chunk_product<5>(part, X, Y, 80, tx, ty); break;
-            case 6: chunk_product<6>(part, X, Y, 96, tx, ty); break;
-            default: chunk_product<7>(part, X, Y, 112, tx, ty); break;
+            case 0: chunk_product<0, true>(part, X, Y, 0, tx, ty); break;
+            case 1: chunk_product<1, true>(part, X, Y, 16, tx, ty); break;
+            case 2: chunk_product<2, true>(part, X, Y, 32, tx, ty); break;
+            case 3: chunk_product<3, true>(part, X, Y, 48, tx, ty); break;
+            case 4: chunk_product<4, true>(part, X, Y, 64, tx, ty); break;
+            case 5: chunk_product<5, true>(part, X, Y, 80, tx, ty); break;
+            case 6: chunk_product<6, true>(part, X, Y, 96, tx, ty); break;
+            default: chunk_product<7, true>(part, X, Y, 112, tx, ty); break;
         }
 #pragma unroll
         for (int i = blk; i < 8; ++i)

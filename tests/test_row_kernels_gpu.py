@@ -193,6 +193,35 @@ def test_head_scan_by_chunks(H, G, d, dv, counts, strong):
         assert chunk <= 1.5 * token + 1e-7 and chunk < 2e-6, err
 
 
+@pytest.mark.parametrize("H,G,d,dv", [(2, 1, 64, 64), (3, 3, 200, 100)])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_head_scan_values_reach_no_earlier_token(H, G, d, dv, bad):
+    """A value that is infinite or NaN, at the first, a middle and the last token of a chunk's
+    block of sixteen: every earlier token's output is bit for bit what it is without it, and its
+    own and later ones in that column are not finite."""
+    from agave_b200 import kernels
+    T, W = 300, 2 * G * d + H * dv
+    ctx = step([T], [0], [0])
+    ctx.max_new = T
+    assert kernels.library().agv_head_scan_work(T, 1, H, G, d, dv, T)          # (chunks are taken)
+    row = rnd(T, W, seed=1)
+    coef = torch.stack([torch.sigmoid(rnd(T, H, seed=2) + 4.0), rnd(T, H, seed=3).abs() + 0.1], -1).contiguous()
+    got = []
+    for at in (None, 128, 137, 143, 255, 299):
+        r = row.clone()
+        if at is not None:
+            r[at, 2 * G * d + 5] = bad                       # head 0, column 5
+        q, k, v = r[:, :G * d], r[:, G * d:2 * G * d], r[:, 2 * G * d:]
+        out = torch.empty(T, H * dv, device=DEV)
+        kernels.head_scan(q, k, v, coef, out, ctx, torch.zeros(1, H * d * dv, device=DEV), 0, H, G, d, dv)
+        got.append(out)
+        if at is not None:
+            assert torch.equal(out[:at], got[0][:at]), at
+            assert not torch.isfinite(out[at:, 5]).any()
+            others = torch.arange(H * dv, device=DEV) != 5
+            assert torch.equal(out[:, others], got[0][:, others])
+
+
 @pytest.mark.parametrize("inner,N", [(96, 16), (130, 4), (64, 7), (33, 128), (48, 200)])
 @pytest.mark.parametrize("counts", [[150], [1, 700, 96, 3], [192, 191, 97, 515]])
 @pytest.mark.parametrize("dtype", [BF, F32])
