@@ -367,20 +367,21 @@ constexpr int CK_C = 64;           // columns of S a CTA has
 
 struct Chunks {
     int n_seq;
-    const int* cu;
+    const int *cu, *slots;
     float* states;             // [chunks, H, d, dv]
     float* decays;             // [chunks, H]
     float* scores;             // [chunks, groups, CK, CK]: q_t . k_s for s <= t
 };
 
-// Chunk z of the step: its first token and how many it has; false: there is none.
-__device__ __forceinline__ bool chunk_of(const Chunks& ck, int z, int& t0, int& nt) {
+// Chunk z of the step: its first token, how many it has and its sequence's slot; false: there is none.
+__device__ __forceinline__ bool chunk_of(const Chunks& ck, int z, int& t0, int& nt, int& slot) {
     int at = 0;
     for (int e = 0; e < ck.n_seq; ++e) {
         const int from = ck.cu[e], n = ck.cu[e + 1] - from, c = (n + CK - 1) / CK;
         if (z < at + c) {
             t0 = from + (z - at) * CK;
             nt = min(CK, from + n - t0);
+            slot = ck.slots[e];
             return true;
         }
         at += c;
@@ -432,8 +433,8 @@ chunk_scores_kernel(ScanIn in, int d, Chunks ck, int vec) {
     pdl_wait();
     pdl_launch_next();
     __shared__ __align__(16) float qs[64 * 36], ks[64 * 36];
-    int t0, nt;
-    if (!chunk_of(ck, blockIdx.z, t0, nt)) return;
+    int t0, nt, slot;
+    if (!chunk_of(ck, blockIdx.z, t0, nt, slot) || slot < 0) return;
     const int g = blockIdx.y, tq = blockIdx.x > 0 ? 64 : 0, tk = blockIdx.x == 2 ? 64 : 0;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     float acc[4][4] = {};
@@ -486,8 +487,8 @@ chunk_states_kernel(ScanIn in, int H, int d, int dv, Chunks ck, int c_tiles, int
     pdl_launch_next();
     __shared__ __align__(16) float ks[32 * 128], vs[32 * CK_C];
     __shared__ float w[CK];
-    int t0, nt;
-    if (!chunk_of(ck, blockIdx.z, t0, nt)) return;
+    int t0, nt, slot;
+    if (!chunk_of(ck, blockIdx.z, t0, nt, slot) || slot < 0) return;
     const int h = blockIdx.y, hg = h / in.shared, n0 = blockIdx.x / c_tiles * 128, c0 = blockIdx.x % c_tiles * CK_C;
     if (threadIdx.x < 32) {
         // w_t = b_t A(t + 1, end): products from the last token on, 32 tokens at a time
@@ -563,10 +564,10 @@ chunk_states_kernel(ScanIn in, int H, int d, int dv, Chunks ck, int c_tiles, int
 // from the state and back to it; `states` becomes what every chunk begins from.
 __global__ void __launch_bounds__(256)
 chunk_pass_kernel(Chunks ck, int H, int dn, float* __restrict__ state, long long state_stride,
-                  long long state_off, const int* __restrict__ slots) {
+                  long long state_off) {
     pdl_wait();
     pdl_launch_next();
-    const int e = blockIdx.z, h = blockIdx.y, slot = slots[e], i = (blockIdx.x * 256 + threadIdx.x) * 4;
+    const int e = blockIdx.z, h = blockIdx.y, slot = ck.slots[e], i = (blockIdx.x * 256 + threadIdx.x) * 4;
     const int n = (ck.cu[e + 1] - ck.cu[e] + CK - 1) / CK;
     if (i >= dn || n == 0 || slot < 0) return;
     int z = 0;
@@ -636,10 +637,16 @@ chunk_outputs_kernel(ScanIn in, float* __restrict__ num, int H, int d, int dv, C
     float* X = sm;                                       // [CK][CO_PITCH]
     float* Y = sm + CK * CO_PITCH;                       // [CK][CK_C]
     __shared__ float as[CK], bs[CK], pre[CK];
-    int t0, nt;
-    if (!chunk_of(ck, blockIdx.z, t0, nt)) return;
+    int t0, nt, slot;
+    if (!chunk_of(ck, blockIdx.z, t0, nt, slot)) return;
     const int h = blockIdx.y, hg = h / in.shared, groups = H / in.shared, c0 = blockIdx.x * CK_C;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    if (slot < 0) {                                      // a padding entry: its rows are written, with zeros
+        const int cols = min(CK_C, dv - c0);
+        for (int i = tid; i < nt * cols; i += 256)
+            num[(size_t)(t0 + i / cols) * H * dv + (size_t)h * dv + c0 + i % cols] = 0.f;
+        return;
+    }
     if (tid < CK) {
         const float2 ab = tid < nt ? *reinterpret_cast<const float2*>(in.gates + ((size_t)(t0 + tid) * H + h) * 2)
                                    : make_float2(1.f, 0.f);
@@ -888,7 +895,7 @@ AGV_API int agv_head_scan(const float* q, const float* k, const float* v, long l
         agv_head_scan_work(T, B, H, groups, d, dv, max_new) > 0) {
         const int n = T / CK + B, c_tiles = (dv + CK_C - 1) / CK_C;
         float* scores = work + (size_t)n * H * d * dv;
-        const Chunks ck{B, cu_seqlens, work, scores + (size_t)n * groups * CK * CK, scores};
+        const Chunks ck{B, cu_seqlens, slots, work, scores + (size_t)n * groups * CK * CK, scores};
         const int vec_q = ld % 4 == 0 && d % 4 == 0 && agv_aligned(q, 16) && agv_aligned(k, 16);
         const int vec_v = ld % 4 == 0 && dv % 4 == 0 && agv_aligned(v, 16), vec_s = dv % 4 == 0;
         agv_launch(chunk_scores_kernel, dim3(3, groups, n), 256, 0, stream, in, d, ck, vec_q);
@@ -897,7 +904,7 @@ AGV_API int agv_head_scan(const float* q, const float* k, const float* v, long l
                    c_tiles, vec_q, vec_v);
         AGV_LAUNCH_OK("chunk_states_kernel");
         agv_launch(chunk_pass_kernel, dim3((d * dv / 4 + 255) / 256, H, B), 256, 0, stream, ck, H, d * dv, state,
-                   state_stride, state_off, slots);
+                   state_stride, state_off);
         AGV_LAUNCH_OK("chunk_pass_kernel");
         AGV_CUDA_OK(cudaFuncSetAttribute(chunk_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CO_SMEM));
         agv_launch(chunk_outputs_kernel, dim3(c_tiles, H, n), 256, CO_SMEM, stream, in, out, H, d, dv, ck, vec_q,

@@ -222,6 +222,36 @@ def test_head_scan_values_reach_no_earlier_token(H, G, d, dv, bad):
             assert torch.equal(out[:, others], got[0][:, others])
 
 
+@pytest.mark.parametrize("pad", [0, 1, 2])
+@pytest.mark.parametrize("H,G,d,dv", [(2, 1, 64, 64), (3, 3, 200, 100)])
+def test_head_scan_padding_entries_are_zeros(H, G, d, dv, pad):
+    """A padding entry of a prompt step gets rows of zeros and touches no state, by chunks as token by
+    token, and the other entries are bit for bit what they are without one."""
+    from agave_b200 import kernels
+    counts = [130, 400, 65]
+    T, W = sum(counts), 2 * G * d + H * dv
+    row = rnd(T, W, seed=1)
+    q, k, v = row[:, :G * d], row[:, G * d:2 * G * d], row[:, 2 * G * d:]
+    coef = torch.stack([torch.sigmoid(rnd(T, H, seed=2) + 2.0), rnd(T, H, seed=3).abs()], -1).contiguous()
+    state0 = rnd(3, H * d * dv, seed=4)
+    assert kernels.library().agv_head_scan_work(T, 3, H, G, d, dv, max(counts))
+    for max_new in (1, max(counts)):
+        got = []
+        for s in ([0, 1, 2], [b if b != pad else -1 for b in range(3)]):
+            ctx = step(counts, [0] * 3, s)
+            ctx.max_new = max_new
+            state, out = state0.clone(), torch.full((T, H * dv), float("nan"), device=DEV)
+            kernels.head_scan(q, k, v, coef, out, ctx, state, 0, H, G, d, dv)
+            got.append((out, state))
+        rows = torch.zeros(T, dtype=torch.bool, device=DEV)
+        rows[sum(counts[:pad]):sum(counts[:pad + 1])] = True
+        assert not got[1][0][rows].any()
+        assert torch.equal(got[1][0][~rows], got[0][0][~rows])
+        assert torch.equal(got[1][1][pad], state0[pad])
+        keep = [b for b in range(3) if b != pad]
+        assert torch.equal(got[1][1][keep], got[0][1][keep])
+
+
 @pytest.mark.parametrize("inner,N", [(96, 16), (130, 4), (64, 7), (33, 128), (48, 200)])
 @pytest.mark.parametrize("counts", [[150], [1, 700, 96, 3], [192, 191, 97, 515]])
 @pytest.mark.parametrize("dtype", [BF, F32])
