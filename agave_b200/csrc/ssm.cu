@@ -664,10 +664,12 @@ AGV_API int agv_selective_low(const void* row, long long ld, const float* part, 
     return 0;
 }
 
+constexpr long long SS_MOST_WORK = 128LL << 20;      // floats of scratch (512 MB)
 AGV_API long long agv_selective_scan_work(int T, int B, int inner, int N, int max_new) {
     const int len = selective_segment(T, B, inner, N, max_new);
     if (!len || T / len + B > 65535) return 0;
-    return (long long)(T / len + B) * ((long long)inner * N + inner);
+    const long long need = (long long)(T / len + B) * ((long long)inner * N + inner);
+    return need > SS_MOST_WORK ? 0 : need;
 }
 // u, dt [T, inner], dt_bias, D [inner], bc [T, 2 Np] (agv_selective_low), a2 [inner, N] = A *
 // log2(e), all 32-bit; z: columns z_off .. z_off + inner of the stacked projection (row / part as
@@ -693,9 +695,9 @@ AGV_API int agv_selective_scan(const float* u, const float* dt, const float* dt_
     if (int rc = row_of(in, row, ld, part, n_splits, T, W)) return rc;
     const SelectiveArgs a{u, dt, dt_bias, bc, a2, D, inner, N, z_off};
     const StepArgs st{state, state_stride, state_off, slots, cu, nullptr, nullptr, nullptr};
-    const int Np = ss_pad(N), len = work ? selective_segment(T, B, inner, N, max_new) : 0;
+    const bool cut = work && agv_selective_scan_work(T, B, inner, N, max_new) > 0;
+    const int Np = ss_pad(N), len = cut ? selective_segment(T, B, inner, N, max_new) : 0;
     const int n_seg = len ? T / len + B : 0;             // (at most: a sequence rounds up by less than one)
-    AGV_REQUIRE(n_seg <= 65535, "selective_scan: %d segments exceed the grid limit", n_seg);
     const Segments sg{len, B, work, len ? work + (size_t)n_seg * inner * N : nullptr};
 #define AGV_SS(NS, L)                                                                            \
     return dtype == AGV_F32                                                                      \

@@ -1119,6 +1119,17 @@ def ssm_conv(row: Optional[torch.Tensor], partial: Optional[torch.Tensor], T: in
             _ptr(ctx.lens), _stream()))
 
 
+def _scratch(n: int, device) -> Optional[torch.Tensor]:
+    """``n`` 32-bit values for a form of a kernel that has another without scratch; None for none,
+    and where the device has no room for them."""
+    if n == 0:
+        return None
+    try:
+        return torch.empty(n, dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 SELECTIVE_MAX_STATE = 256
 
 
@@ -1167,8 +1178,7 @@ def selective_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, bc:
     # long sequences are cut into segments, whose states need scratch
     max_new = int(getattr(ctx, "max_new", 1))
     lib.agv_selective_scan_work.restype = ctypes.c_longlong
-    n = int(lib.agv_selective_scan_work(T, ctx.batch, inner, N, max_new))
-    work = torch.empty(n, dtype=torch.float32, device=out.device) if n else None
+    work = _scratch(int(lib.agv_selective_scan_work(T, ctx.batch, inner, N, max_new)), out.device)
     with _span("selective_scan", _nbytes(u, dt, bc, out) + T * inner * 4 * max(ns, 1) +
                8 * ctx.batch * inner * N, 7 * T * inner * N):
         _check(lib.agv_selective_scan(
@@ -1198,8 +1208,7 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, coef: torch.Ten
     max_new = int(getattr(ctx, "max_new", 1))
     lib = library()
     lib.agv_head_scan_work.restype = ctypes.c_longlong
-    n = int(lib.agv_head_scan_work(T, ctx.batch, H, n_groups, N, dv, max_new))
-    work = torch.empty(n, dtype=torch.float32, device=out.device) if n else None
+    work = _scratch(int(lib.agv_head_scan_work(T, ctx.batch, H, n_groups, N, dv, max_new)), out.device)
     with _span("head_scan", _nbytes(q, k, v, coef, out) + 8 * ctx.batch * H * N * dv,
                5 * T * H * N * dv):
         _check(library().agv_head_scan(

@@ -276,3 +276,55 @@ def test_selective_scan_by_segments(inner, N, counts, dtype):
     assert torch.equal(got[0][1][:, :3], got[1][1][:, :3])
     tol = 4e-6 if dtype == F32 else 2.0 ** -8
     assert float((got[0][0].double() - got[1][0].double()).abs().max()) <= tol * float(got[0][0].abs().max())
+
+
+def test_scans_run_without_room_for_scratch(monkeypatch):
+    """Where the device has no room for the chunks' and the segments' states, the scans take the
+    form that needs none: the results of a step that asks for none."""
+    from agave_b200 import kernels
+    counts = [300, 80]
+    T, H, G, d, dv, inner, N = sum(counts), 2, 1, 64, 64, 128, 16
+    row = rnd(T, 2 * G * d + H * dv, seed=1)
+    q, k, v = row[:, :G * d], row[:, G * d:2 * G * d], row[:, 2 * G * d:]
+    coef = torch.stack([torch.sigmoid(rnd(T, H, seed=2) + 2.0), rnd(T, H, seed=3).abs()], -1).contiguous()
+    u, dt, z, bc = (rnd(T, n, seed=4 + i) for i, n in enumerate((inner, inner, inner, 2 * N)))
+    a2, bias, D = -torch.exp(rnd(inner, N, seed=8)), rnd(inner, seed=9), rnd(inner, seed=10)
+    lib, ctx = kernels.library(), step(counts, [0, 0], [0, 1])
+    assert lib.agv_head_scan_work(T, 2, H, G, d, dv, max(counts)) > 0
+    assert lib.agv_selective_scan_work(T, 2, inner, N, max(counts)) > 0
+
+    def both(out, y, S, state):
+        kernels.head_scan(q, k, v, coef, out, ctx, S, 0, H, G, d, dv)
+        kernels.selective_scan(u, dt, bias, bc, a2, D, z, None, inner, 0, y, ctx, state, 0)
+        return out, y, S, state
+    fresh = [(torch.empty(T, H * dv, device=DEV), torch.empty(T, inner, device=DEV), torch.zeros(2, H * d * dv, device=DEV),
+              torch.zeros(2, inner * N, device=DEV)) for _ in range(2)]
+    ctx.max_new = 1
+    want = both(*fresh[0])
+    ctx.max_new = max(counts)
+
+    def full(*a, **k):
+        raise torch.OutOfMemoryError("no room")
+    monkeypatch.setattr(torch, "empty", full)
+    got = both(*fresh[1])
+    monkeypatch.undo()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+def test_scratch_of_the_scans_is_bounded():
+    """Whatever the batch, the states, the heads and the lengths: at most 512 MB."""
+    import ctypes
+    from agave_b200 import kernels
+    lib = kernels.library()
+    lib.agv_head_scan_work.restype = lib.agv_selective_scan_work.restype = ctypes.c_longlong
+    some = 0
+    for B in (1, 8, 64, 1024):
+        for longest in (150, 2000, 100000):
+            T = longest + (B - 1) * 64
+            for wide in (1, 8, 64):
+                n = lib.agv_selective_scan_work(T, B, 128 * wide, 256, longest)
+                m = lib.agv_head_scan_work(T, B, 2 * wide, 1, 128, 64, longest)
+                assert 0 <= n <= 1 << 27 and 0 <= m <= 1 << 27
+                some += (n > 0) + (m > 0)
+    assert some > 20
