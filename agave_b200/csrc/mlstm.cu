@@ -25,6 +25,7 @@
 //  * agv_mlstm_out: the division, every head's o over its root mean square, times a weight
 //    per channel, times sigmoid(g), rounded to the compute dtype for the output product.
 #include "common.cuh"
+#include "pieces.cuh"
 #include "row_in.cuh"
 
 namespace {
@@ -375,18 +376,12 @@ struct Chunks {
 
 // Chunk z of the step: its first token, how many it has and its sequence's slot; false: there is none.
 __device__ __forceinline__ bool chunk_of(const Chunks& ck, int z, int& t0, int& nt, int& slot) {
-    int at = 0;
-    for (int e = 0; e < ck.n_seq; ++e) {
-        const int from = ck.cu[e], n = ck.cu[e + 1] - from, c = (n + CK - 1) / CK;
-        if (z < at + c) {
-            t0 = from + (z - at) * CK;
-            nt = min(CK, from + n - t0);
-            slot = ck.slots[e];
-            return true;
-        }
-        at += c;
-    }
-    return false;
+    Piece p;
+    if (!piece_of(ck.cu, ck.n_seq, CK, z, p)) return false;
+    t0 = ck.cu[p.seq] + p.part * CK;
+    nt = min(CK, ck.cu[p.seq + 1] - t0);
+    slot = ck.slots[p.seq];
+    return true;
 }
 
 // ROWS x COLS values (columns a multiple of 4) into shared memory, 256 threads, their loads issued
@@ -569,9 +564,8 @@ chunk_pass_kernel(Chunks ck, int H, int dn, float* __restrict__ state, long long
     pdl_launch_next();
     const int e = blockIdx.z, h = blockIdx.y, slot = ck.slots[e], i = (blockIdx.x * 256 + threadIdx.x) * 4;
     const int n = (ck.cu[e + 1] - ck.cu[e] + CK - 1) / CK;
+    const int z = first_piece(ck.cu, e, CK);
     if (i >= dn || n == 0 || slot < 0) return;
-    int z = 0;
-    for (int j = 0; j < e; ++j) z += (ck.cu[j + 1] - ck.cu[j] + CK - 1) / CK;
     float* S = state + (size_t)slot * state_stride + state_off + (size_t)h * dn + i;     // (any alignment)
     float4 run = make_float4(S[0], S[1], S[2], S[3]);
     float4* at = reinterpret_cast<float4*>(ck.states + ((size_t)z * H + h) * dn + i);
@@ -863,18 +857,35 @@ AGV_API int agv_mlstm_scan(const float* qkv, const float* gates, float* num, flo
 // The scan without normaliser.  q, k: [T, groups * d] and v: [T, H * dv], 32-bit, with row stride
 // ld (parts of one row each); head h reads the q and k of group h / (H / groups); coef [T, H, 2]:
 // a_t, b_t; out [T, H * dv] receives S_t^T q_t; state: S [H, d, dv] per slot from state_off on.
-// max_new: the longest sequence of the step; work: scratch of agv_head_scan_work floats (null: none,
-// and the tokens are taken one by one).
+// work: scratch of agv_head_scan_work floats (null: none, and the tokens are taken one by one).
 //
-// By chunks where sequences have some: a token of a head costs an SM 200 ns of issue in the scan, and
-// 230 ns of waiting where few heads and sequences leave it one CTA.  333 + 1,501 tokens, 64 heads of 128
-// x 64: 345 us token by token, 281 token by token in segments of 256 side by side with their states
-// added afterwards, 198 by chunks (scores 10, states 70, pass 9, outputs 109).  At least 192 tokens in the
-// longest and 64 on average, so that chunks are not mostly padding; narrow states stay with the scan,
-// whose tiles are 16 x 32.
+// By chunks where that is faster by what the two forms take (us, one B200, launches in a row; 2,000 calls of 1
+// to 128 heads, 1 to 256 sequences of equal, spread and mixed lengths):
+//   token by token, the longer of the longest sequence's chain (160 to 267 ns a token where CTAs have an SM
+//     alone, 190 to 385 where they share one) and the issue of all tokens' CTAs (60 to 195 ns an SM each);
+//   by chunks, four launches and 24.5 to 47.5 us of an SM for a chunk's tile of 64 columns of a head, and its
+//     group's scores.  A sequence's last chunk is full or nearly empty: half a chunk each on average.
+// 333 + 1,501 tokens, 64 heads of 128 x 64: 345 us token by token, 281 token by token in segments of 256 side
+// by side with their states added afterwards, 198 by chunks (scores 10, states 70, pass 9, outputs 109).  One
+// sequence: 256 tokens of 24 heads 48 and 45, 1,024 181 and 68; sixteen of 192 of 48 heads of 64 x 64 144
+// and 248 (token by token).  Of the 2,000 calls 26 lose by the rule, 18 % at most; by lengths alone (192
+// in the longest, 64 on average) 405 lost, up to eight times.  Narrow states stay with the scan, whose
+// tiles are 16 x 32.
 constexpr long long HS_MOST_WORK = 128LL << 20;      // floats of scratch (512 MB)
+static bool chunks_pay(int T, int B, int H, int groups, int d, int dv, int max_new) {
+    const int k = d <= 64 ? 0 : d <= 128 ? 1 : 2;
+    const double alone[] = {0.160, 0.172, 0.267}, sharing[] = {0.190, 0.230, 0.385}, busy[] = {0.060, 0.116, 0.195},
+                 tile[] = {24.5, 28.0, 47.5};
+    const double columns = (double)H * ((dv + 31) / 32), tiles = (double)H * ((dv + CK_C - 1) / CK_C);
+    const double chain = max_new * (B * columns > 148 ? sharing[k] : alone[k]), issue = T * columns * busy[k] / 148;
+    const double chunks = T / (double)CK + 0.5 * B;
+    return 34 + chunks * (tiles * tile[k] + groups * (6 + 0.11 * d)) / 148 < 1.15 * (chain > issue ? chain : issue);
+}
+// Floats of scratch for the form by chunks, 0 where it does not take the sizes or, with max_new > 0 (the longest
+// sequence of the step), where it is the slower one.
 AGV_API long long agv_head_scan_work(int T, int B, int H, int groups, int d, int dv, int max_new) {
-    if (max_new < 192 || T < 64 * B || d < 64 || d > 256 || dv < 32 || d * dv % 4 != 0) return 0;
+    if (d < 64 || d > 256 || dv < 32 || d * dv % 4 != 0) return 0;
+    if (max_new && (max_new < 2 * CK || T < 64 * B || !chunks_pay(T, B, H, groups, d, dv, max_new))) return 0;
     const long long n = T / CK + B;                  // chunks at most
     const long long need = n * ((long long)H * d * dv + (long long)groups * CK * CK + H);
     return n > 65535 || need > HS_MOST_WORK ? 0 : need;
@@ -882,7 +893,7 @@ AGV_API long long agv_head_scan_work(int T, int B, int H, int groups, int d, int
 AGV_API int agv_head_scan(const float* q, const float* k, const float* v, long long ld,
                           const float* coef, float* out, int T, int B, int H, int groups, int d,
                           int dv, float* state, long long state_stride, long long state_off,
-                          const int* slots, const int* cu_seqlens, int max_new, float* work,
+                          const int* slots, const int* cu_seqlens, float* work,
                           cudaStream_t stream) {
     AGV_REQUIRE(T >= 0 && B > 0 && H > 0 && groups > 0 && H % groups == 0 && d > 0 && dv > 0,
                 "head_scan: bad sizes");
@@ -892,7 +903,7 @@ AGV_API int agv_head_scan(const float* q, const float* k, const float* v, long l
     if (T == 0) return 0;
     const ScanIn in{q, k, v, ld, H / groups, coef};
     if (work && agv_aligned(work, 16) && agv_aligned(coef, 8) && agv_aligned(out, 16) &&
-        agv_head_scan_work(T, B, H, groups, d, dv, max_new) > 0) {
+        agv_head_scan_work(T, B, H, groups, d, dv, 0) > 0) {
         const int n = T / CK + B, c_tiles = (dv + CK_C - 1) / CK_C;
         float* scores = work + (size_t)n * H * d * dv;
         const Chunks ck{B, cu_seqlens, slots, work, scores + (size_t)n * groups * CK * CK, scores};

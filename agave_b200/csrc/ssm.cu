@@ -20,6 +20,7 @@
 // 32-bit throughout: sums over partial products, convolution, silu, softplus, decays, states.
 // Prompts and decoded tokens run the same kernels.
 #include "common.cuh"
+#include "pieces.cuh"
 #include "row_in.cuh"
 
 namespace {
@@ -236,21 +237,6 @@ struct Segments {
     float* ends;               // [segments, inner, N]
     float* sums;               // [segments, inner]
 };
-__device__ __forceinline__ bool segment_of(const Segments& sg, const int* __restrict__ cu, int z, int& seq,
-                                           int& part, int& parts) {
-    int at = 0;
-    for (int e = 0; e < sg.n_seq; ++e) {
-        const int n = (cu[e + 1] - cu[e] + sg.len - 1) / sg.len;
-        if (z < at + n) {
-            seq = e;
-            part = z - at;
-            parts = n;
-            return true;
-        }
-        at += n;
-    }
-    return false;
-}
 
 // grid (channel blocks, sequences or segments), 128 threads: 128 / L channels a CTA, L lanes a channel, NS
 // states a lane.  Tokens come SS_CH at a time through two buffers filled by asynchronous copies;
@@ -268,11 +254,11 @@ selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restri
     constexpr int ZN = CH * CC / SS_THREADS > 0 ? CH * CC / SS_THREADS : 1;
     float2* dd = reinterpret_cast<float2*>(sm + 2 * BUF);     // [CH][CC] (dt, dt u)
     float* ys = reinterpret_cast<float*>(dd + CH * CC);       // [CH][CC]
-    int e = blockIdx.y, part = 0, parts = 1;
-    if (PASS && !segment_of(sg, st.cu, blockIdx.y, e, part, parts)) return;
-    if (PASS == 1 && part == parts - 1) return;
-    const int slot = st.slots[e];
-    const int t0 = st.cu[e] + (PASS ? part * sg.len : 0);
+    Piece at{(int)blockIdx.y, 0, 1};
+    if (PASS && !piece_of(st.cu, sg.n_seq, sg.len, blockIdx.y, at)) return;
+    if (PASS == 1 && at.part == at.parts - 1) return;
+    const int e = at.seq, slot = st.slots[e];
+    const int t0 = st.cu[e] + (PASS ? at.part * sg.len : 0);
     const int n = PASS ? min(st.cu[e + 1] - t0, sg.len) : st.cu[e + 1] - t0;
     const int tid = threadIdx.x, l = tid % L, jc = tid / L;
     const int cb = blockIdx.x * CC, c = cb + jc;
@@ -425,7 +411,7 @@ selective_scan_kernel(SelectiveArgs a, RowIn<float> in, StepArgs st, T* __restri
         srow = sg.ends + ((size_t)blockIdx.y * a.inner + (live ? c : 0)) * a.N;
         if (live && l == 0) sg.sums[(size_t)blockIdx.y * a.inner + c] = steps;
     }
-    if (live && (PASS != 2 || part == parts - 1)) {
+    if (live && (PASS != 2 || at.part == at.parts - 1)) {
 #pragma unroll
         for (int s = 0; s < NS; ++s)
             if (l * NS + s < a.N) srow[l * NS + s] = S[s];
@@ -439,9 +425,8 @@ segment_begins_kernel(SelectiveArgs a, StepArgs st, Segments sg) {
     pdl_launch_next();
     const int e = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x, slot = st.slots[e];
     const int n = (st.cu[e + 1] - st.cu[e] + sg.len - 1) / sg.len;
+    const int z = first_piece(st.cu, e, sg.len);
     if (i >= a.inner * a.N || n == 0 || slot < 0) return;
-    int z = 0;
-    for (int j = 0; j < e; ++j) z += (st.cu[j + 1] - st.cu[j] + sg.len - 1) / sg.len;
     const int c = i / a.N;
     const float a2 = a.a2[i];
     float run = st.state[(size_t)slot * st.stride + st.off + i];
@@ -555,18 +540,22 @@ void launch_conv(const RowIn<float>& in, int n_tokens, int off, int C, const Ste
                    off, C, st, w, bias, out, rounded, dt_off, n_dt, dt_bias, neg_a, coef);
 }
 
-// Tokens of a segment (0: the sequences are not cut).  A CTA's chain takes 148 ns a token with two CTAs
-// an SM and the step's tokens times its CTAs are what there is to spread: about six CTAs an SM.  333 +
-// 1,501 tokens, 4,096 channels of 16 states: 223 us whole, 136 so (50 + 8 + 78).
+// Tokens of a segment (0: the sequences are not cut; max_new 0: whatever the lengths).  A CTA's chain takes 134 ns a token alone on an SM, 146
+// with a second (160 and 210 with 64 states), and the step's tokens times its CTAs are what there is to
+// spread: about six CTAs an SM.  Two passes cost about half a chain's time for every CTA's worth of tokens an
+// SM has (0.6 from 32 states on) and two launches more, 160 tokens' time: taken where the longest sequence is
+// above that.  4,096 channels of 16 states: 333 + 1,501 tokens 223 us whole, 136 so (50 + 8 + 78); one
+// sequence of 256 37 and 33, of 4,096 554 and 286; two of 4,096 603 and 544, of 384 60 and 65 (whole), four of
+// 4,096 776 and 1,089 (whole).  Of 1,969 calls (1 to 256 sequences, 128 to 8,192 channels of 4 to 128 states)
+// 6 lose by the rule, 13 % at most; by lengths alone 235 lost, up to 14 times.
 constexpr int SS_CTAS = 6 * 148;
 int selective_segment(int T, int B, int inner, int N, int max_new) {
-    if (T <= B) return 0;
     const int Np = ss_pad(N), L = Np <= 8 ? 2 : Np <= 16 ? 4 : Np <= 64 ? 8 : Np <= 128 ? 16 : 32;
     const int CC = SS_THREADS / L;
     const long long blocks = (inner + CC - 1) / CC;
-    long long len = (T * blocks / SS_CTAS + 15) / 16 * 16;
-    if (len < 96) len = 96;
-    return 2LL * max_new >= 3 * len ? (int)len : 0;
+    if (max_new && (T <= B || max_new - (L <= 4 ? 0.45 : 0.60) * T * blocks / 148 <= 160)) return 0;
+    const long long len = (T * blocks / SS_CTAS + 15) / 16 * 16;
+    return len < 96 ? 96 : (int)len;
 }
 
 template <typename T, int NS, int L>
@@ -665,6 +654,8 @@ AGV_API int agv_selective_low(const void* row, long long ld, const float* part, 
 }
 
 constexpr long long SS_MOST_WORK = 128LL << 20;      // floats of scratch (512 MB)
+// Floats of scratch for the form by segments, 0 where it does not take the sizes or, with max_new > 0 (the
+// longest sequence of the step), where it is the slower one.
 AGV_API long long agv_selective_scan_work(int T, int B, int inner, int N, int max_new) {
     const int len = selective_segment(T, B, inner, N, max_new);
     if (!len || T / len + B > 65535) return 0;
@@ -674,14 +665,13 @@ AGV_API long long agv_selective_scan_work(int T, int B, int inner, int N, int ma
 // u, dt [T, inner], dt_bias, D [inner], bc [T, 2 Np] (agv_selective_low), a2 [inner, N] = A *
 // log2(e), all 32-bit; z: columns z_off .. z_off + inner of the stacked projection (row / part as
 // in agv_ssm_conv); out [T, inner] in dtype; state: S [inner, N] per slot from state_off on.
-// max_new: the longest sequence of the step; work: scratch of agv_selective_scan_work floats (null: none, and
-// the sequences are not cut).
+// work: scratch of agv_selective_scan_work floats (null: none, and the sequences are not cut).
 AGV_API int agv_selective_scan(const float* u, const float* dt, const float* dt_bias,
                                const float* bc, const float* a2, const float* D, const float* row,
                                long long ld, const float* part, int n_splits, int T, int W,
                                int z_off, int B, int inner, int N, void* out, int dtype,
                                float* state, long long state_stride, long long state_off,
-                               const int* slots, const int* cu, int max_new, float* work,
+                               const int* slots, const int* cu, float* work,
                                cudaStream_t stream) {
     AGV_REQUIRE(T >= 0 && B >= 0 && inner > 0 && N > 0 && N <= SS_MAX_N && z_off >= 0 &&
                 z_off + inner <= W, "selective_scan: bad sizes");
@@ -695,8 +685,8 @@ AGV_API int agv_selective_scan(const float* u, const float* dt, const float* dt_
     if (int rc = row_of(in, row, ld, part, n_splits, T, W)) return rc;
     const SelectiveArgs a{u, dt, dt_bias, bc, a2, D, inner, N, z_off};
     const StepArgs st{state, state_stride, state_off, slots, cu, nullptr, nullptr, nullptr};
-    const bool cut = work && agv_selective_scan_work(T, B, inner, N, max_new) > 0;
-    const int Np = ss_pad(N), len = cut ? selective_segment(T, B, inner, N, max_new) : 0;
+    const bool cut = work && agv_selective_scan_work(T, B, inner, N, 0) > 0;
+    const int Np = ss_pad(N), len = cut ? selective_segment(T, B, inner, N, 0) : 0;
     const int n_seg = len ? T / len + B : 0;             // (at most: a sequence rounds up by less than one)
     const Segments sg{len, B, work, len ? work + (size_t)n_seg * inner * N : nullptr};
 #define AGV_SS(NS, L)                                                                            \

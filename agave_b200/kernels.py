@@ -1130,6 +1130,19 @@ def _scratch(n: int, device) -> Optional[torch.Tensor]:
         return None
 
 
+def _scan_scratch(form: str, wants: str, without: str, ctx, device, need) -> Optional[torch.Tensor]:
+    """Scratch of a scan whose form ``wants`` needs some and whose form ``without`` does not; ``need``
+    takes the step's longest sequence, 0 for whatever the lengths."""
+    if form == "auto":
+        return _scratch(int(need(max(1, int(getattr(ctx, "max_new", 1))))), device)
+    if form == without:
+        return None
+    n = int(need(0)) if form == wants else 0
+    if n == 0:
+        raise KernelError(f"the scan has no form {form!r} for these sizes")
+    return torch.empty(n, dtype=torch.float32, device=device)
+
+
 SELECTIVE_MAX_STATE = 256
 
 
@@ -1159,11 +1172,12 @@ def selective_low(row: Optional[torch.Tensor], partial: Optional[torch.Tensor], 
 def selective_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, bc: torch.Tensor,
                    a2: torch.Tensor, d: torch.Tensor, row: Optional[torch.Tensor],
                    partial: Optional[torch.Tensor], W: int, z_offset: int, out: torch.Tensor, ctx,
-                   state: torch.Tensor, state_off: int) -> None:
+                   state: torch.Tensor, state_off: int, form: str = "auto") -> None:
     """S[c, n] <- exp(dt_c A[c, n]) S[c, n] + dt_c u_c B_n;  y_c = sum_n S[c, n] C_n + D_c u_c  over
     the step's tokens, sequence by sequence, with dt_c = softplus(dt_c + dt_bias_c) and ``a2`` =
     A * log2(e); out = y * silu(z), z the columns ``z_offset`` .. of the stacked projection.  S
-    [inner, N] of each sequence is read from and written to ``state`` at ``state_off``."""
+    [inner, N] of each sequence is read from and written to ``state`` at ``state_off``.  ``form``:
+    "auto", or one of the two forms, "whole" (sequences) and "segments" (which needs scratch)."""
     T, inner = u.shape
     N = a2.shape[1]
     rp, ld, pp, ns = _f32_row_input(row, partial, T, W)
@@ -1176,25 +1190,26 @@ def selective_scan(u: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, bc:
     assert lib.agv_selective_pad(N) == selective_pad(N)
     sp, ss = _state_args(state)
     # long sequences are cut into segments, whose states need scratch
-    max_new = int(getattr(ctx, "max_new", 1))
     lib.agv_selective_scan_work.restype = ctypes.c_longlong
-    work = _scratch(int(lib.agv_selective_scan_work(T, ctx.batch, inner, N, max_new)), out.device)
+    work = _scan_scratch(form, "segments", "whole", ctx, out.device,
+                         lambda max_new: lib.agv_selective_scan_work(T, ctx.batch, inner, N, max_new))
     with _span("selective_scan", _nbytes(u, dt, bc, out) + T * inner * 4 * max(ns, 1) +
                8 * ctx.batch * inner * N, 7 * T * inner * N):
         _check(lib.agv_selective_scan(
             _ptr(u), _ptr(dt), _ptr(dt_bias), _ptr(bc), _ptr(a2), _ptr(d), rp, ld, pp, ns, T, W,
             z_offset, ctx.batch, inner, N, _ptr(out), dtype_code(out.dtype), sp, ss,
-            ctypes.c_longlong(state_off), _ptr(ctx.slots), _ptr(ctx.cu_seqlens), max_new, _ptr(work),
+            ctypes.c_longlong(state_off), _ptr(ctx.slots), _ptr(ctx.cu_seqlens), _ptr(work),
             _stream()))
 
 
 def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, coef: torch.Tensor,
               out: torch.Tensor, ctx, state: torch.Tensor, state_off: int, n_heads: int,
-              n_groups: int, state_dim: int, value_dim: int) -> None:
+              n_groups: int, state_dim: int, value_dim: int, form: str = "auto") -> None:
     """S <- a S + b k v^T;  o = S^T q  per head over the step's tokens, sequence by sequence, with
     (a, b) = coef[t, h]; q, k [T, n_groups * state_dim] and v [T, n_heads * value_dim] are column
     ranges of one 32-bit tensor, head h reads the q and k of group h // (n_heads / n_groups).  S
-    [H, state_dim, value_dim] of each sequence is in ``state`` at ``state_off``."""
+    [H, state_dim, value_dim] of each sequence is in ``state`` at ``state_off``.  ``form``: "auto",
+    or one of the two forms, "tokens" (one by one) and "chunks" (which needs scratch)."""
     T = v.shape[0]
     H, N, dv = n_heads, state_dim, value_dim
     for t, n in ((q, "q"), (k, "k"), (v, "v"), (coef, "coef"), (out, "out")):
@@ -1205,16 +1220,16 @@ def head_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, coef: torch.Ten
     assert coef.shape == (T, H, 2) and out.shape == (T, H * dv)
     sp, ss = _state_args(state)
     # long sequences are taken by chunks, whose states need scratch
-    max_new = int(getattr(ctx, "max_new", 1))
     lib = library()
     lib.agv_head_scan_work.restype = ctypes.c_longlong
-    work = _scratch(int(lib.agv_head_scan_work(T, ctx.batch, H, n_groups, N, dv, max_new)), out.device)
+    work = _scan_scratch(form, "chunks", "tokens", ctx, out.device,
+                         lambda max_new: lib.agv_head_scan_work(T, ctx.batch, H, n_groups, N, dv, max_new))
     with _span("head_scan", _nbytes(q, k, v, coef, out) + 8 * ctx.batch * H * N * dv,
                5 * T * H * N * dv):
         _check(library().agv_head_scan(
             _ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(v.stride(0)), _ptr(coef), _ptr(out), T,
             ctx.batch, H, n_groups, N, dv, sp, ss, ctypes.c_longlong(state_off), _ptr(ctx.slots),
-            _ptr(ctx.cu_seqlens), max_new, _ptr(work), _stream()))
+            _ptr(ctx.cu_seqlens), _ptr(work), _stream()))
 
 
 def ssd_out(num: torch.Tensor, u: torch.Tensor, d: torch.Tensor, row: Optional[torch.Tensor],

@@ -182,14 +182,13 @@ def test_head_scan_by_chunks(H, G, d, dv, counts, strong):
             want[t] = torch.einsum("hd,hdv->hv", q8[t], S[b])
         at += n
     err = {}
-    for max_new in (1, max(counts)):
-        ctx.max_new = max_new
+    for form in ("tokens", "chunks"):
         state, out = state0.clone(), torch.full((T, H * dv), float("nan"), device=DEV)
-        kernels.head_scan(q, k, v, coef, out, ctx, state, 5, H, G, d, dv)
-        err[max_new] = [float((g.double() - r).norm() / r.norm()) for g, r in
+        kernels.head_scan(q, k, v, coef, out, ctx, state, 5, H, G, d, dv, form=form)
+        err[form] = [float((g.double() - r).norm() / r.norm()) for g, r in
                         ((out.view(T, H, dv), want), (state[:, 5:].view(B, H, d, dv), S))]
         assert torch.equal(state[:, :5], state0[:, :5])
-    for token, chunk in zip(err[1], err[max(counts)]):
+    for token, chunk in zip(err["tokens"], err["chunks"]):
         assert chunk <= 1.5 * token + 1e-7 and chunk < 2e-6, err
 
 
@@ -202,8 +201,6 @@ def test_head_scan_values_reach_no_earlier_token(H, G, d, dv, bad):
     from agave_b200 import kernels
     T, W = 300, 2 * G * d + H * dv
     ctx = step([T], [0], [0])
-    ctx.max_new = T
-    assert kernels.library().agv_head_scan_work(T, 1, H, G, d, dv, T)          # (chunks are taken)
     row = rnd(T, W, seed=1)
     coef = torch.stack([torch.sigmoid(rnd(T, H, seed=2) + 4.0), rnd(T, H, seed=3).abs() + 0.1], -1).contiguous()
     got = []
@@ -213,7 +210,8 @@ def test_head_scan_values_reach_no_earlier_token(H, G, d, dv, bad):
             r[at, 2 * G * d + 5] = bad                       # head 0, column 5
         q, k, v = r[:, :G * d], r[:, G * d:2 * G * d], r[:, 2 * G * d:]
         out = torch.empty(T, H * dv, device=DEV)
-        kernels.head_scan(q, k, v, coef, out, ctx, torch.zeros(1, H * d * dv, device=DEV), 0, H, G, d, dv)
+        kernels.head_scan(q, k, v, coef, out, ctx, torch.zeros(1, H * d * dv, device=DEV), 0, H, G, d, dv,
+                          form="chunks")
         got.append(out)
         if at is not None:
             assert torch.equal(out[:at], got[0][:at]), at
@@ -234,14 +232,12 @@ def test_head_scan_padding_entries_are_zeros(H, G, d, dv, pad):
     q, k, v = row[:, :G * d], row[:, G * d:2 * G * d], row[:, 2 * G * d:]
     coef = torch.stack([torch.sigmoid(rnd(T, H, seed=2) + 2.0), rnd(T, H, seed=3).abs()], -1).contiguous()
     state0 = rnd(3, H * d * dv, seed=4)
-    assert kernels.library().agv_head_scan_work(T, 3, H, G, d, dv, max(counts))
-    for max_new in (1, max(counts)):
+    for form in ("tokens", "chunks"):
         got = []
         for s in ([0, 1, 2], [b if b != pad else -1 for b in range(3)]):
             ctx = step(counts, [0] * 3, s)
-            ctx.max_new = max_new
             state, out = state0.clone(), torch.full((T, H * dv), float("nan"), device=DEV)
-            kernels.head_scan(q, k, v, coef, out, ctx, state, 0, H, G, d, dv)
+            kernels.head_scan(q, k, v, coef, out, ctx, state, 0, H, G, d, dv, form=form)
             got.append((out, state))
         rows = torch.zeros(T, dtype=torch.bool, device=DEV)
         rows[sum(counts[:pad]):sum(counts[:pad + 1])] = True
@@ -267,10 +263,9 @@ def test_selective_scan_by_segments(inner, N, counts, dtype):
     a2 = -torch.exp(rnd(inner, N, seed=5, scale=2.0) - 2.0)
     bias, d, state0 = rnd(inner, seed=6), rnd(inner, seed=7), rnd(B, 3 + inner * N, seed=8)
     got = []
-    for max_new in (1, max(counts)):
-        ctx.max_new = max_new
+    for form in ("whole", "segments"):
         state, out = state0.clone(), torch.full((T, inner), float("nan"), dtype=dtype, device=DEV)
-        kernels.selective_scan(u, dt, bias, bc.view(T, -1), a2, d, z, None, inner, 0, out, ctx, state, 3)
+        kernels.selective_scan(u, dt, bias, bc.view(T, -1), a2, d, z, None, inner, 0, out, ctx, state, 3, form=form)
         got.append((out, state))
     assert float((got[0][1] - got[1][1]).abs().max()) <= 4e-6 * float(got[0][1].abs().max())
     assert torch.equal(got[0][1][:, :3], got[1][1][:, :3])
@@ -282,7 +277,7 @@ def test_scans_run_without_room_for_scratch(monkeypatch):
     """Where the device has no room for the chunks' and the segments' states, the scans take the
     form that needs none: the results of a step that asks for none."""
     from agave_b200 import kernels
-    counts = [300, 80]
+    counts = [900, 80]
     T, H, G, d, dv, inner, N = sum(counts), 2, 1, 64, 64, 128, 16
     row = rnd(T, 2 * G * d + H * dv, seed=1)
     q, k, v = row[:, :G * d], row[:, G * d:2 * G * d], row[:, 2 * G * d:]
@@ -313,7 +308,7 @@ def test_scans_run_without_room_for_scratch(monkeypatch):
 
 
 def test_scratch_of_the_scans_is_bounded():
-    """Whatever the batch, the states, the heads and the lengths: at most 512 MB."""
+    """Whatever the batch, the states, the heads and the lengths, chosen or asked for: at most 512 MB."""
     import ctypes
     from agave_b200 import kernels
     lib = kernels.library()
@@ -323,8 +318,60 @@ def test_scratch_of_the_scans_is_bounded():
         for longest in (150, 2000, 100000):
             T = longest + (B - 1) * 64
             for wide in (1, 8, 64):
-                n = lib.agv_selective_scan_work(T, B, 128 * wide, 256, longest)
-                m = lib.agv_head_scan_work(T, B, 2 * wide, 1, 128, 64, longest)
-                assert 0 <= n <= 1 << 27 and 0 <= m <= 1 << 27
-                some += (n > 0) + (m > 0)
+                for lengths in (longest, 0):
+                    n = lib.agv_selective_scan_work(T, B, 128 * wide, 256, lengths)
+                    m = lib.agv_head_scan_work(T, B, 2 * wide, 1, 128, 64, lengths)
+                    assert 0 <= n <= 1 << 27 and 0 <= m <= 1 << 27
+                    some += (n > 0) + (m > 0)
     assert some > 20
+
+
+# lengths, heads, groups, state, values: whether the chunks are the faster form (both measured)
+@pytest.mark.parametrize("counts,H,G,d,dv,chunks", [
+    ([333, 1501], 64, 1, 128, 64, True), ([1024], 24, 1, 128, 64, True), ([4096], 8, 1, 64, 32, True),
+    ([1], 64, 1, 128, 64, False), ([192] * 16, 48, 1, 64, 64, False), ([256] * 32, 16, 16, 64, 64, False),
+    ([64] * 255 + [192], 16, 16, 64, 64, False), ([128] * 32, 64, 1, 128, 64, False), ([192], 32, 1, 256, 128, False)])
+def test_head_scan_rule(counts, H, G, d, dv, chunks):
+    import ctypes
+    from agave_b200 import kernels
+    lib = kernels.library()
+    lib.agv_head_scan_work.restype = ctypes.c_longlong
+    assert (lib.agv_head_scan_work(sum(counts), len(counts), H, G, d, dv, max(counts)) > 0) == chunks
+
+
+@pytest.mark.parametrize("counts,inner,N,segments", [
+    ([333, 1501], 4096, 16, True), ([4096], 512, 16, True), ([1024] * 4, 128, 16, True), ([512], 1024, 4, True),
+    ([1], 4096, 16, False), ([384] * 2, 4096, 16, False), ([20] * 500 + [400], 512, 16, False),
+    ([150], 2048, 128, False), ([256] * 32, 512, 16, False), ([400] * 2, 8192, 16, False)])
+def test_selective_scan_rule(counts, inner, N, segments):
+    import ctypes
+    from agave_b200 import kernels
+    lib = kernels.library()
+    lib.agv_selective_scan_work.restype = ctypes.c_longlong
+    assert (lib.agv_selective_scan_work(sum(counts), len(counts), inner, N, max(counts)) > 0) == segments
+
+
+@pytest.mark.parametrize("B", [1, 31, 32, 33, 97])
+def test_scans_find_their_pieces_in_any_batch(B):
+    """Empty, short and long sequences in batches around a warp's 32: chunks and segments against the
+    forms that take every sequence by itself."""
+    from agave_b200 import kernels
+    g = torch.Generator().manual_seed(B)
+    counts = torch.randint(0, 3, (B,), generator=g).mul_(97).tolist()
+    counts[-1] = 300
+    T, H, G, d, dv, inner, N = sum(counts), 2, 1, 64, 32, 64, 16
+    ctx = step(counts, [0] * B, list(range(B)))
+    row = rnd(T, 2 * G * d + H * dv, seed=1)
+    q, k, v = row[:, :G * d], row[:, G * d:2 * G * d], row[:, 2 * G * d:]
+    coef = torch.stack([torch.sigmoid(rnd(T, H, seed=2) + 2.0), rnd(T, H, seed=3).abs()], -1).contiguous()
+    u, dt, z, bc = (rnd(T, n, seed=4 + i) for i, n in enumerate((inner, inner, inner, 2 * N)))
+    a2, bias, D = -torch.exp(rnd(inner, N, seed=8)), rnd(inner, seed=9), rnd(inner, seed=10)
+    S0, s0 = rnd(B, H * d * dv, seed=11), rnd(B, inner * N, seed=12)
+    got = []
+    for head, sel in (("tokens", "whole"), ("chunks", "segments")):
+        S, s, out, y = S0.clone(), s0.clone(), torch.empty(T, H * dv, device=DEV), torch.empty(T, inner, device=DEV)
+        kernels.head_scan(q, k, v, coef, out, ctx, S, 0, H, G, d, dv, form=head)
+        kernels.selective_scan(u, dt, bias, bc, a2, D, z, None, inner, 0, y, ctx, s, 0, form=sel)
+        got.append((out, S, y, s))
+    for a, b in zip(*got):
+        same(b, a)
