@@ -433,20 +433,27 @@ __host__ __device__ inline size_t scan_buf_floats(int TCH, int Dp, int CC) {
     return ((size_t)TCH * (4 * Dp + CC + 2) + 3) / 4 * 4;      // (16-byte rows in the next buffer)
 }
 
-// A lane's rows of CPT columns (CC apart), two rows to a register pair: a piece of a token's row read
-// once serves them all.  What bounds it are a token's reads of k, g, g k and g q (16 of 16 bytes a
-// lane), the sums over the lanes and the wait for u, token after token, behind the longest sequence.
-// 8 sequences of 256 to 1,024 tokens, 16 heads of 128 x 128: 905 us with one column a lane, a value a
-// register and the sequences as they come; 856 with pairs and the longest first; 644 with two columns (four:
-// 620, but a step of 287 tokens lost what that gained).
-template <int L, int CPT>
-__global__ void __launch_bounds__(128)
+// A lane's rows of CPT columns (CC apart): a piece of a token's row read once serves them all.  One column's
+// rows are single values; two columns' are pairs, two rows to a register pair.  What bounds it are a token's
+// reads of k, g, g k and g q (16 of 16 bytes a lane), the sums over the lanes and the wait for u, token after
+// token, behind the longest sequence; a step of one token a sequence (STEP) is bound by the trip to memory.
+//
+// 8 sequences of 256 to 1,024 tokens, 16 heads of 128 x 128: 905 us with one column a lane and the sequences
+// as they come; 644 with two columns and the longest first (four: 620, but a step of 287 tokens lost what that
+// gained).  One column in pairs is slower, a chain of half as many but slower operations: one sequence of
+// 1,024 tokens, 8 heads of 64 x 64 310 us against 224.  Registers: a prompt's loads of a token are asked for
+// together where there are enough (the compiler, left alone, kept to 72 and 80: 705 us for the eight sequences
+// above, 670 with 128); a STEP has no second token and wants warps instead (64 sequences, 32 heads of 128 x
+// 128: 92 us with 100 registers, 76 with 64).
+constexpr int scan_ctas(int cpt, bool step) { return step ? 7 : cpt == 1 ? 1 : 4; }
+template <int L, int CPT, bool STEP>
+__global__ void __launch_bounds__(128, scan_ctas(CPT, STEP))
 delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
     pdl_wait();
     extern __shared__ float smem[];
     // the longest sequences of a prompt step begin first: this CTA's is the blockIdx.z-th longest
     int b = blockIdx.z;
-    if (a.TCH > 1 && gridDim.z <= blockDim.x) {
+    if (!STEP && gridDim.z <= blockDim.x) {
         __shared__ int ranked;
         const int e = threadIdx.x, B = gridDim.z;
         if (e < B) {
@@ -467,7 +474,7 @@ delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
     if (n <= 0) return;
     const int h = blockIdx.y;
     const int d = dm.d, dv = dm.dv, C = dm.C(), nq = dm.nq();
-    constexpr int Dp = L * DL_R, P = DL_R / 2;
+    constexpr int Dp = L * DL_R, P = DL_R / 2, TOKENS = STEP ? 1 : 2;
     const int CC = a.CC, CW = CC * CPT, TCH = a.TCH;
     const int l = threadIdx.x & (L - 1);
     const int jc = threadIdx.x / L;
@@ -507,7 +514,9 @@ delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
         cp_async_commit();
     };
 
-    f32x2 S[CPT][P];
+    // S: single values where a lane has one column, else pairs
+    float S1[CPT == 1 ? DL_R : 1];
+    f32x2 S[CPT == 1 ? 1 : CPT][P];
     float* srow[CPT];
     fetch(0, smem);
 #pragma unroll
@@ -516,7 +525,9 @@ delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
 #pragma unroll
         for (int i = 0; i < P; ++i) {
             const int r = ((i >> 1) * L + l) * 4 + (i & 1) * 2;
-            S[x][i] = pack2(live[x] && r < d ? srow[x][r] : 0.f, live[x] && r + 1 < d ? srow[x][r + 1] : 0.f);
+            const float lo = live[x] && r < d ? srow[x][r] : 0.f, hi = live[x] && r + 1 < d ? srow[x][r + 1] : 0.f;
+            if constexpr (CPT == 1) { S1[2 * i] = lo; S1[2 * i + 1] = hi; }
+            else S[x][i] = pack2(lo, hi);
         }
     }
     int cur = 0;
@@ -537,55 +548,92 @@ delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
         const float* pg = sb.g + l * 4;
         const float* pv = sb.v + (jc < CC ? jc : 0);
         float* po = a.out + (size_t)(t0 + c0) * dm.H * dv + (size_t)h * dv + j0;
-#pragma unroll 2
+#pragma unroll TOKENS
         for (int tt = 0; tt < m; ++tt) {
-            f32x2 ac[CPT][2], rc[CPT][2];
+            if constexpr (CPT == 1) {
+                float gk[DL_R], gq[DL_R], kk[DL_R], gg[DL_R];
 #pragma unroll
-            for (int x = 0; x < CPT; ++x) ac[x][0] = ac[x][1] = rc[x][0] = rc[x][1] = 0;
-#pragma unroll
-            for (int i = 0; i < DL_R / 4; ++i) {
-                const ulonglong2 gk = reinterpret_cast<const ulonglong2*>(pgk)[i * L];
-                const ulonglong2 gq = reinterpret_cast<const ulonglong2*>(pgq)[i * L];
-#pragma unroll
-                for (int x = 0; x < CPT; ++x) {
-                    ac[x][0] = fma2(S[x][2 * i], gk.x, ac[x][0]);
-                    ac[x][1] = fma2(S[x][2 * i + 1], gk.y, ac[x][1]);
-                    rc[x][0] = fma2(S[x][2 * i], gq.x, rc[x][0]);
-                    rc[x][1] = fma2(S[x][2 * i + 1], gq.y, rc[x][1]);
+                for (int i = 0; i < DL_R / 4; ++i) {
+                    const float4 x = reinterpret_cast<const float4*>(pgk)[i * L];
+                    const float4 y = reinterpret_cast<const float4*>(pgq)[i * L];
+                    gk[4 * i] = x.x; gk[4 * i + 1] = x.y; gk[4 * i + 2] = x.z; gk[4 * i + 3] = x.w;
+                    gq[4 * i] = y.x; gq[4 * i + 1] = y.y; gq[4 * i + 2] = y.z; gq[4 * i + 3] = y.w;
                 }
-            }
-            float acc[CPT], rr[CPT];
+                float ac[4] = {0.f, 0.f, 0.f, 0.f}, rc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int x = 0; x < CPT; ++x) {
-                float a0, a1, a2, a3, r0, r1, r2, r3;
-                unpack2(ac[x][0], a0, a1); unpack2(ac[x][1], a2, a3);
-                unpack2(rc[x][0], r0, r1); unpack2(rc[x][1], r2, r3);
-                acc[x] = (a0 + a1) + (a2 + a3);
-                rr[x] = (r0 + r1) + (r2 + r3);
-            }
-#pragma unroll
-            for (int o = 1; o < L; o <<= 1)
-#pragma unroll
-                for (int x = 0; x < CPT; ++x) {
-                    acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], o);
-                    rr[x] += __shfl_xor_sync(0xffffffffu, rr[x], o);
+                for (int i = 0; i < DL_R; ++i) {
+                    ac[i & 3] = fmaf(S1[i], gk[i], ac[i & 3]);
+                    rc[i & 3] = fmaf(S1[i], gq[i], rc[i & 3]);
                 }
-            const float beta = sb.beta[tt], kq = sb.kq[tt];
-            f32x2 uu[CPT];
 #pragma unroll
-            for (int x = 0; x < CPT; ++x) {
-                const float u = beta * (pv[x * CC] - acc[x]);
-                if (live[x] && l == 0) po[x * CC] = fmaf(kq, u, rr[x]);
-                uu[x] = pack2(u, u);
-            }
+                for (int i = 0; i < DL_R / 4; ++i) {
+                    const float4 x = reinterpret_cast<const float4*>(pk)[i * L];
+                    const float4 y = reinterpret_cast<const float4*>(pg)[i * L];
+                    kk[4 * i] = x.x; kk[4 * i + 1] = x.y; kk[4 * i + 2] = x.z; kk[4 * i + 3] = x.w;
+                    gg[4 * i] = y.x; gg[4 * i + 1] = y.y; gg[4 * i + 2] = y.z; gg[4 * i + 3] = y.w;
+                }
+                float acc = (ac[0] + ac[1]) + (ac[2] + ac[3]);
+                float rr = (rc[0] + rc[1]) + (rc[2] + rc[3]);
 #pragma unroll
-            for (int i = 0; i < DL_R / 4; ++i) {
-                const ulonglong2 kk = reinterpret_cast<const ulonglong2*>(pk)[i * L];
-                const ulonglong2 gg = reinterpret_cast<const ulonglong2*>(pg)[i * L];
+                for (int o = 1; o < L; o <<= 1) {
+                    acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                    rr += __shfl_xor_sync(0xffffffffu, rr, o);
+                }
+#pragma unroll
+                for (int i = 0; i < DL_R; ++i) gg[i] *= S1[i];         // g S: needs no u
+                const float u = sb.beta[tt] * (*pv - acc);
+                if (live[0] && l == 0) *po = fmaf(sb.kq[tt], u, rr);
+#pragma unroll
+                for (int i = 0; i < DL_R; ++i) S1[i] = fmaf(kk[i], u, gg[i]);
+            } else {
+                f32x2 ac[CPT][2], rc[CPT][2];
+#pragma unroll
+                for (int x = 0; x < CPT; ++x) ac[x][0] = ac[x][1] = rc[x][0] = rc[x][1] = 0;
+#pragma unroll
+                for (int i = 0; i < DL_R / 4; ++i) {
+                    const ulonglong2 gk = reinterpret_cast<const ulonglong2*>(pgk)[i * L];
+                    const ulonglong2 gq = reinterpret_cast<const ulonglong2*>(pgq)[i * L];
+#pragma unroll
+                    for (int x = 0; x < CPT; ++x) {
+                        ac[x][0] = fma2(S[x][2 * i], gk.x, ac[x][0]);
+                        ac[x][1] = fma2(S[x][2 * i + 1], gk.y, ac[x][1]);
+                        rc[x][0] = fma2(S[x][2 * i], gq.x, rc[x][0]);
+                        rc[x][1] = fma2(S[x][2 * i + 1], gq.y, rc[x][1]);
+                    }
+                }
+                float acc[CPT], rr[CPT];
 #pragma unroll
                 for (int x = 0; x < CPT; ++x) {
-                    S[x][2 * i] = fma2(kk.x, uu[x], mul2(gg.x, S[x][2 * i]));
-                    S[x][2 * i + 1] = fma2(kk.y, uu[x], mul2(gg.y, S[x][2 * i + 1]));
+                    float a0, a1, a2, a3, r0, r1, r2, r3;
+                    unpack2(ac[x][0], a0, a1); unpack2(ac[x][1], a2, a3);
+                    unpack2(rc[x][0], r0, r1); unpack2(rc[x][1], r2, r3);
+                    acc[x] = (a0 + a1) + (a2 + a3);
+                    rr[x] = (r0 + r1) + (r2 + r3);
+                }
+#pragma unroll
+                for (int o = 1; o < L; o <<= 1)
+#pragma unroll
+                    for (int x = 0; x < CPT; ++x) {
+                        acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], o);
+                        rr[x] += __shfl_xor_sync(0xffffffffu, rr[x], o);
+                    }
+                const float beta = sb.beta[tt], kq = sb.kq[tt];
+                f32x2 uu[CPT];
+#pragma unroll
+                for (int x = 0; x < CPT; ++x) {
+                    const float u = beta * (pv[x * CC] - acc[x]);
+                    if (live[x] && l == 0) po[x * CC] = fmaf(kq, u, rr[x]);
+                    uu[x] = pack2(u, u);
+                }
+#pragma unroll
+                for (int i = 0; i < DL_R / 4; ++i) {
+                    const ulonglong2 kk = reinterpret_cast<const ulonglong2*>(pk)[i * L];
+                    const ulonglong2 gg = reinterpret_cast<const ulonglong2*>(pg)[i * L];
+#pragma unroll
+                    for (int x = 0; x < CPT; ++x) {
+                        S[x][2 * i] = fma2(kk.x, uu[x], mul2(gg.x, S[x][2 * i]));
+                        S[x][2 * i + 1] = fma2(kk.y, uu[x], mul2(gg.y, S[x][2 * i + 1]));
+                    }
                 }
             }
             pk += Dp; pgk += Dp; pgq += Dp; pg += Dp; pv += CW;
@@ -601,7 +649,8 @@ delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
             for (int i = 0; i < P; ++i) {
                 const int r = ((i >> 1) * L + l) * 4 + (i & 1) * 2;
                 float lo, hi;
-                unpack2(S[x][i], lo, hi);
+                if constexpr (CPT == 1) { lo = S1[2 * i]; hi = S1[2 * i + 1]; }
+                else unpack2(S[x][i], lo, hi);
                 if (r < d) srow[x][r] = lo;
                 if (r + 1 < d) srow[x][r + 1] = hi;
             }
@@ -813,10 +862,13 @@ AGV_API int agv_delta_scan(const float* qkv, const float* beta, const float* a,
     }
     const DeltaState st{state, state_stride, 0, slots, cu, nullptr, nullptr};
     dim3 grid((unsigned)((dv + CW - 1) / CW), (unsigned)H, (unsigned)B);
-#define AGV_SCAN(LL)                                                                                              \
-    case LL:                                                                                                      \
-        if (CPT == 1) agv_launch_after(delta_scan_kernel<LL, 1>, grid, (unsigned)(CC * L), smem, stream, sa, dm, st); \
-        else agv_launch_after(delta_scan_kernel<LL, 2>, grid, (unsigned)(CC * L), smem, stream, sa, dm, st);      \
+    // (a STEP's tokens are a buffer each and its columns one a lane)
+    auto go = [&](auto kern) { agv_launch_after(kern, grid, (unsigned)(CC * L), smem, stream, sa, dm, st); };
+#define AGV_SCAN(LL)                                         \
+    case LL:                                                 \
+        if (T <= B) go(delta_scan_kernel<LL, 1, true>);      \
+        else if (CPT == 1) go(delta_scan_kernel<LL, 1, false>); \
+        else go(delta_scan_kernel<LL, 2, false>);            \
         break
     switch (L) {
         AGV_SCAN(1); AGV_SCAN(2); AGV_SCAN(4); AGV_SCAN(8); AGV_SCAN(16); AGV_SCAN(32);

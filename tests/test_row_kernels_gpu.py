@@ -72,6 +72,73 @@ def test_delta_prepare_rows(taps, G, H, d, dv, splits, dtype, counts, starts):
         same(a, b)
 
 
+@pytest.mark.parametrize("G,H,d,dv,counts", [
+    (4, 16, 128, 128, [70, 1, 0, 33, 17]),              # two columns a lane: 2, 8 and 16 lanes a column,
+    (2, 16, 128, 36, [5, 40, 1, 9, 18, 2, 33, 16]),     # last groups of columns that are not whole,
+    (16, 48, 20, 130, [20] * 5), (1, 24, 256, 68, [3, 21, 34, 2]),
+    (4, 16, 128, 100, [2] * 140),                       # more sequences than a CTA has threads to rank
+    (2, 4, 64, 40, [50, 1, 20]), (3, 3, 500, 12, [18, 3]), (1, 2, 8, 3, [40]),      # one column
+    (4, 16, 128, 128, [1] * 9), (2, 4, 300, 70, [1, 1])])                           # one token a sequence
+def test_delta_scan(G, H, d, dv, counts):
+    """Against the recurrence in 64 bits, with a padding entry, and bit for bit what the same form
+    gives in another order of the sequences; the sequences one by one take one column a lane."""
+    from agave_b200 import kernels
+    T, B, C = sum(counts), len(counts), 2 * G * d + H * dv
+    qkv = rnd(T, C, seed=1)
+    for h in range(2 * G):                              # (q and k are unit vectors)
+        qkv[:, h * d:(h + 1) * d] /= qkv[:, h * d:(h + 1) * d].norm(dim=1, keepdim=True)
+    beta, a = torch.sigmoid(rnd(T, H, seed=2)), rnd(T, H * d, seed=3)
+    bias, neg_a = rnd(H * d, seed=4), -torch.exp(rnd(H, seed=5) - 1.0)
+    state0 = rnd(B + 1, H * dv * d + 4, seed=6)
+    slots = [B - b for b in range(B)]
+    pad = 1 if B > 2 else None
+    if pad is not None:
+        slots[pad] = -1
+
+    def run(counts, rows, slots, state):
+        ctx = step(counts, [0] * len(counts), slots)
+        ctx.new = lambda *s, dtype: torch.empty(s, dtype=dtype, device=DEV)
+        out = torch.full((len(rows), H * dv), float("nan"), device=DEV)
+        kernels.delta_scan(qkv[rows].contiguous(), beta[rows].contiguous(), a[rows].contiguous(), bias, neg_a, out,
+                           ctx, state, G, H, d, dv)
+        return out
+    state = state0.clone()
+    every = torch.arange(T, device=DEV)
+    out = run(counts, every, slots, state)
+    # in 64 bits
+    g = torch.exp(neg_a.double()[:, None] * torch.nn.functional.softplus((a + bias).double().view(T, H, d), threshold=1e9))
+    q, k = (t.double().view(T, G, d).repeat_interleave(H // G, 1) for t in (qkv[:, :G * d], qkv[:, G * d:2 * G * d]))
+    v = qkv[:, 2 * G * d:].double().view(T, H, dv)
+    want, ends = torch.zeros(T, H, dv, dtype=torch.float64, device=DEV), state0.double()
+    cuts = [sum(counts[:b]) for b in range(B + 1)]
+    for b in range(B):
+        if slots[b] < 0:
+            continue
+        S = state0[slots[b], :H * dv * d].double().view(H, dv, d)
+        for t in range(cuts[b], cuts[b + 1]):
+            S = S * g[t][:, None, :]
+            u = beta[t].double()[:, None] * (v[t] - torch.einsum("hvd,hd->hv", S, k[t]))
+            S = S + u[:, :, None] * k[t][:, None, :]
+            want[t] = torch.einsum("hvd,hd->hv", S, q[t])
+        ends[slots[b], :H * dv * d] = S.reshape(-1)
+    live = torch.cat([torch.arange(cuts[b], cuts[b + 1], device=DEV) for b in range(B) if slots[b] >= 0])
+    assert float((out.double().view(T, H, dv) - want)[live].norm() / want[live].norm()) < 2e-6
+    assert float((state.double() - ends).norm() / ends.norm()) < 2e-6
+    assert torch.equal(state[:, H * dv * d:], state0[:, H * dv * d:]) and torch.equal(state[0], state0[0])
+    # the sequences in reverse
+    order = [b for b in range(B)][::-1]
+    again = state0.clone()
+    rows = torch.cat([every[cuts[b]:cuts[b + 1]] for b in order])
+    back = run([counts[b] for b in order], rows, [slots[b] for b in order], again)
+    keep = torch.isin(rows, live)
+    assert torch.equal(back[keep], out[rows[keep]]) and torch.equal(again, state)
+    # one by one: the same numbers but for the order of a column's sums
+    for b in range(min(B, 8)):
+        if slots[b] >= 0 and counts[b]:
+            own = every[cuts[b]:cuts[b + 1]]
+            same(run([counts[b]], own, [slots[b]], state0.clone()), out[own])
+
+
 @pytest.mark.parametrize("T,H,dv", [(1, 3, 128), (9, 16, 128), (5, 2, 516), (4, 1, 700), (130, 3, 4)])
 @pytest.mark.parametrize("dtype", [BF, F32])
 def test_delta_out_by_fours(T, H, dv, dtype):
