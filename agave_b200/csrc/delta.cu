@@ -131,8 +131,8 @@ delta_prepare_kernel(RowIn<T> in, DeltaDims dm, DeltaState st, const float* __re
 // The same where the row comes in 32-bit in whole 16-byte pieces, with two to four taps and heads of
 // up to 256: a warp has R tokens of one q or k head, of 128 NJ columns of v, or of 32 of the last
 // columns (b, a1, g1), a lane four neighbouring channels, whose inputs slide through registers.
-// What no kernel of the step writes (weights, the ring, the step's arrays) is asked for before the
-// dependency wait.
+// Weights and the step's arrays are asked for before the dependency wait, the ring after it: the kernel
+// before may be the one that writes it (another step's, a call apart).
 //
 // A decode step is bound by trips to memory one after the other: a CTA a token walked its 3,216
 // columns in a dozen of them, 35 us for 8 tokens (G 4, H 16, heads of 128, eight partial sums);
@@ -191,6 +191,8 @@ delta_prepare_rows_kernel(RowIn<float> in, DeltaDims dm, DeltaState st, int n_to
         slot[i] = st.slots[b];
         before[i] = t - st.cu[b];
     }
+    pdl_wait();
+    pdl_launch_next();
     // the ring's rows before the tile's first token (later tokens of the tile that reach further
     // back than their sequence's first token in the step read it themselves, below)
     float4 old[NJ][RING];
@@ -204,8 +206,6 @@ delta_prepare_rows_kernel(RowIn<float> in, DeltaDims dm, DeltaState st, int n_to
                 old[j][k - 1] = *reinterpret_cast<const float4*>(
                     st.state + (size_t)slot[0] * st.stride + st.conv_off + (size_t)((pos[0] - k) % RING) * C + c0 + ch);
         }
-    pdl_wait();
-    pdl_launch_next();
     float4 xs[NJ][R + RING];
 #pragma unroll
     for (int j = 0; j < NJ; ++j)

@@ -72,6 +72,47 @@ def test_delta_prepare_rows(taps, G, H, d, dv, splits, dtype, counts, starts):
         same(a, b)
 
 
+@pytest.mark.parametrize("taps", [2, 4])
+@pytest.mark.parametrize("starts", [0, 3])
+def test_delta_prepare_of_steps_one_after_the_other(taps, starts):
+    """Steps that follow each other with no other kernel between them, a prompt and then single tokens,
+    recorded together: each finds in the ring what the one before wrote there."""
+    from agave_b200 import kernels
+    G, H, d, dv, ra, rg, B, N = 2, 4, 128, 64, 8, 12, 3, 9
+    C = 2 * G * d + H * dv
+    W = C + H + ra + rg
+    rows, conv_w = rnd(1, B * (7 + N), W, seed=1), rnd(C, taps, seed=2, scale=0.5)
+    off0 = H * dv * d
+    state0 = rnd(B, off0 + (taps - 1) * C, seed=3)
+    part = rows.view(B, 7 + N, W)
+    steps = [(step([7] * B, [starts] * B, list(range(B))), part[:, :7].reshape(1, B * 7, W).contiguous())]
+    steps += [(step([1] * B, [starts + 7 + i] * B, list(range(B))), part[:, 7 + i].reshape(1, B, W).contiguous())
+              for i in range(N)]
+    outs = [(torch.zeros(x.shape[1], C, device=DEV), torch.zeros(x.shape[1], H, device=DEV),
+             torch.zeros(x.shape[1], ra, device=DEV), torch.zeros(x.shape[1], rg, device=DEV)) for _, x in steps]
+
+    def run(state):
+        for (ctx, x), o in zip(steps, outs):
+            kernels.delta_prepare(None, x, x.shape[1], ctx, state, off0, G, H, d, dv, taps, ra, rg, conv_w, 1e-6,
+                                  0.3, *o)
+    state = state0.clone()
+    run(state)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run(state)
+    # all tokens in one step
+    whole = torch.zeros(B * (7 + N), C, device=DEV)
+    kernels.delta_prepare(None, rows, B * (7 + N), step([7 + N] * B, [starts] * B, list(range(B))), state0.clone(), off0,
+                          G, H, d, dv, taps, ra, rg, conv_w, 1e-6, 0.3, whole, torch.zeros(B * (7 + N), H, device=DEV),
+                          torch.zeros(B * (7 + N), ra, device=DEV), torch.zeros(B * (7 + N), rg, device=DEV))
+    for _ in range(20):
+        state.copy_(state0)
+        graph.replay()
+        got = torch.cat([outs[0][0].view(B, 7, C)] + [o[0].view(B, 1, C) for o in outs[1:]], 1)
+        same(got, whole.view(B, 7 + N, C))
+
+
 @pytest.mark.parametrize("G,H,d,dv,counts", [
     (4, 16, 128, 128, [70, 1, 0, 33, 17]),              # two columns a lane: 2, 8 and 16 lanes a column,
     (2, 16, 128, 36, [5, 40, 1, 9, 18, 2, 33, 16]),     # last groups of columns that are not whole,
