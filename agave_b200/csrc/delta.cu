@@ -657,27 +657,29 @@ delta_scan_kernel(ScanArgs a, DeltaDims dm, DeltaState st) {
 }
 
 // ---------------------------------------------------------------- read-out
-// y[t, h, :] = o[t, h, :] / rms(o[t, h, :]) * w * sigmoid(gate[t, h, :]): a warp a head, a lane V
-// neighbouring columns at a time, whose o and gate are asked for together.  Bound by the trip to
-// memory when decoding (8 tokens, 16 heads of 128: one warp of four a CTA went through four heads,
-// two trips each, 10.6 us -> 2.6 us), by the bytes in a prompt (5,120 tokens, 105 MB, 16 us:
-// 46 -> 41).
-constexpr int DO_MAX = 16;         // values of a head a lane keeps; the rest is read again
-template <typename T, int V>
+// y[t, h, :] = o[t, h, :] / rms(o[t, h, :]) * w * sigmoid(gate[t, h, :]): L lanes a head (a warp, or
+// eight for heads of up to 32 values), a lane V neighbouring columns at a time, whose o and gate are asked
+// for together; it keeps NJ V of them and reads the rest again.  Bound by the trip to memory when decoding
+// (8 tokens, 16 heads of 128: one warp of four a CTA went through four heads, two trips each, 7.4 us -> 2.4
+// us), by the instructions in a prompt (5,120 tokens, 105 MB, 16 us of HBM: 46 -> 27).  There every head costs
+// its warp's address, and columns that are not there their predicates: with the token by a 64-bit division and
+// NJ = 4 it took 42; heads of 16 on a warp each 31, now 7.6.
+template <typename T, int V, int NJ, int L>
 __global__ void __launch_bounds__(128)
 delta_out_kernel(const float* __restrict__ o, const float* __restrict__ gate,
                  const float* __restrict__ w, float eps, int n_tokens, int H, int dv,
                  const int* __restrict__ seq_index, const int* __restrict__ slots,
                  T* __restrict__ y) {
-    constexpr int NJ = DO_MAX / V;
-    const int lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (item >= (long long)n_tokens * H) return;
-    const bool pad = slots[seq_index[item / H]] < 0;      // a padding entry's row is zeros
-    const size_t base = (size_t)item * dv;
+    constexpr int HEADS = 128 / L;                       // of a CTA
+    const int lane = threadIdx.x % L;
+    const unsigned h_ctas = (unsigned)(H + HEADS - 1) / HEADS, t = blockIdx.x / h_ctas;
+    const int at = (int)(blockIdx.x - t * h_ctas) * HEADS + threadIdx.x / L;
+    const int h = min(at, H - 1);                        // (lanes behind the last head store nothing)
+    const bool pad = slots[seq_index[t]] < 0;            // a padding entry's row is zeros
+    const size_t base = ((size_t)t * H + h) * dv;
     pdl_wait();
     pdl_launch_next();
-    float ov[DO_MAX], gv[DO_MAX], ss = 0.f;
+    float ov[NJ * V], gv[NJ * V], ss = 0.f;
     auto load = [&](const float* p, float* to) {
         if constexpr (V == 4) {
             const float4 x = *reinterpret_cast<const float4*>(p);
@@ -688,7 +690,7 @@ delta_out_kernel(const float* __restrict__ o, const float* __restrict__ gate,
     };
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
-        const int i = (j * 32 + lane) * V;
+        const int i = (j * L + lane) * V;
         if (i < dv) {
             load(o + base + i, ov + j * V);
             load(gate + base + i, gv + j * V);
@@ -696,10 +698,12 @@ delta_out_kernel(const float* __restrict__ o, const float* __restrict__ gate,
             for (int e = 0; e < V; ++e) ss = fmaf(ov[j * V + e], ov[j * V + e], ss);
         }
     }
-    for (int i = (NJ * 32 + lane) * V; i < dv; i += 32 * V)
+    for (int i = (NJ * L + lane) * V; i < dv; i += L * V)
 #pragma unroll
         for (int e = 0; e < V; ++e) ss = fmaf(o[base + i + e], o[base + i + e], ss);
-    ss = warp_sum(ss);
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (at >= H) return;
     const float r = 1.0f / sqrtf(ss / (float)dv + eps);
     auto store = [&](int i, const float* a, const float* g) {
         float v[V];
@@ -718,10 +722,10 @@ delta_out_kernel(const float* __restrict__ o, const float* __restrict__ gate,
     };
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
-        const int i = (j * 32 + lane) * V;
+        const int i = (j * L + lane) * V;
         if (i < dv) store(i, ov + j * V, gv + j * V);
     }
-    for (int i = (NJ * 32 + lane) * V; i < dv; i += 32 * V) store(i, o + base + i, gate + base + i);
+    for (int i = (NJ * L + lane) * V; i < dv; i += L * V) store(i, o + base + i, gate + base + i);
 }
 
 }  // namespace
@@ -886,12 +890,19 @@ AGV_API int agv_delta_out(const float* o, const float* gate, const float* w, flo
     AGV_REQUIRE(T >= 0 && H > 0 && dv > 0, "delta_out: bad sizes");
     if (T == 0) return 0;
     const bool four = dv % 4 == 0 && agv_aligned(o, 16) && agv_aligned(gate, 16) && agv_aligned(y, 8);
-    const unsigned grid = (unsigned)(((long long)T * H + 3) / 4);
-#define AGV_DO(TT, VV) agv_launch(delta_out_kernel<TT, VV>, grid, 128, 0, stream, o, gate, w, eps, T, H, dv, \
-                                  seq_index, slots, (TT*)y)
-    if (dtype == AGV_F32) { if (four) AGV_DO(float, 4); else AGV_DO(float, 1); }
-    else if (dtype == AGV_BF16) { if (four) AGV_DO(__nv_bfloat16, 4); else AGV_DO(__nv_bfloat16, 1); }
+    const int L = dv <= 32 ? 8 : 32, heads = 128 / L;
+    const long long grid = (long long)T * ((H + heads - 1) / heads);
+    AGV_REQUIRE(grid <= 0x7fffffffLL, "delta_out: %d tokens exceed the grid limit", T);
+#define AGV_DO(TT, VV, NN, LL) agv_launch(delta_out_kernel<TT, VV, NN, LL>, (unsigned)grid, 128, 0, stream, o, gate, w, \
+                                          eps, T, H, dv, seq_index, slots, (TT*)y)
+#define AGV_DOT(TT) do {                                                                \
+        if (L == 8) { if (four) AGV_DO(TT, 4, 1, 8); else AGV_DO(TT, 1, 4, 8); }        \
+        else if (dv <= 128) { if (four) AGV_DO(TT, 4, 1, 32); else AGV_DO(TT, 1, 4, 32); } \
+        else { if (four) AGV_DO(TT, 4, 4, 32); else AGV_DO(TT, 1, 16, 32); } } while (0)
+    if (dtype == AGV_F32) AGV_DOT(float);
+    else if (dtype == AGV_BF16) AGV_DOT(__nv_bfloat16);
     else return agv_fail(-1, "delta_out: unknown dtype %d", dtype);
+#undef AGV_DOT
 #undef AGV_DO
     AGV_LAUNCH_OK("delta_out_kernel");
     return 0;

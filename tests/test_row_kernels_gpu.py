@@ -196,6 +196,25 @@ def test_delta_out_by_fours(T, H, dv, dtype):
         assert not ys[0][3].any()
 
 
+@pytest.mark.parametrize("T,H,dv", [(5, 3, 4), (7, 17, 20), (3, 16, 32), (6, 5, 33), (9, 33, 30), (2, 2, 132), (4, 3, 513),
+                                     (2000, 5, 16)])
+@pytest.mark.parametrize("dtype", [BF, F32])
+def test_delta_out(T, H, dv, dtype):
+    """Eight lanes a head and a warp a head, heads that fill no CTA, columns kept and read again, in fours and
+    one by one, in 64 bits; a padding entry's row."""
+    from agave_b200 import kernels
+    ctx = step([1] * T, [1] * T, [-1 if t == 2 else t for t in range(T)])
+    o, gate, w = rnd(T, H * dv, seed=1), rnd(T, H * dv, seed=2), rnd(dv, seed=3)
+    x = o.double().view(T, H, dv)
+    want = (x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6) * w.double()).view(T, -1) * torch.sigmoid(gate.double())
+    if T > 2:
+        want[2] = 0.0
+    for g in (gate, off(gate)):
+        y = torch.full((T, H * dv), float("nan"), dtype=dtype, device=DEV)
+        kernels.delta_out(o, g, w, 1e-6, H, dv, ctx, y)
+        same(y, want, dtype)
+
+
 @pytest.mark.parametrize("T,K,H", [(1, 8, 4), (9, 2048, 2048), (3, 2056, 2052), (2, 4104, 4100)])
 @pytest.mark.parametrize("dtype", [BF, F32])
 def test_row_gate_by_pieces(T, K, H, dtype):
