@@ -745,6 +745,7 @@ static int check_dims(const DeltaDims& dm) {
 // 2 G d + H dv + H + ra + rg.  conv_w: [2 G d + H dv, taps] 32-bit.  state: [n_slots,
 // state_stride] 32-bit, the convolution's inputs [taps - 1, 2 G d + H dv] at conv_off (a ring:
 // position pp in row pp % (taps - 1)).
+// form: 0 the faster one, 1 the rows form, 2 a CTA a token.
 // several != 0: sequences may bring more than one token (a prompt step); the convolution's
 // inputs are then renewed by a launch of its own.  Outputs: qkv [T, 2 G d + H dv] and beta
 // [T, H] 32-bit, low_a [T, ra] and low_g [T, rg] in dtype.
@@ -753,7 +754,7 @@ AGV_API int agv_delta_prepare(const void* row, long long ld, const float* part, 
                               int ra, int rg, const float* conv_w, float eps_unit, float q_mult,
                               float* state, long long state_stride, long long conv_off,
                               const int* slots, const int* cu, const int* seq_index,
-                              const int* positions, int several, float* qkv, float* beta,
+                              const int* positions, int several, int form, float* qkv, float* beta,
                               void* low_a, void* low_g, cudaStream_t stream) {
     const DeltaDims dm{G, H, d, dv, taps, ra, rg};
     if (int rc = check_dims(dm)) return rc;
@@ -763,13 +764,24 @@ AGV_API int agv_delta_prepare(const void* row, long long ld, const float* part, 
                 "delta_prepare: the state is too small");
     if (T == 0) return 0;
     const DeltaState st{state, state_stride, conv_off, slots, cu, seq_index, positions};
-    // The rows form; a step of one token a sequence takes a token a warp, which alone has the warps
-    // to hide its trips, others eight.
+    // The rows form: a step of one token a sequence takes a token a warp, which alone has the warps to hide its
+    // trips, others eight.  Those want whole lanes, since a head's channels have a warp to themselves: taken
+    // for heads of up to 128 whose channels fill three quarters of the lanes, and enough channels or tokens
+    // that the longer walk of a warp is hidden (or many channels and few tokens).  Against a CTA a token (us): 5,120 tokens, 16 heads of 128 213 and
+    // 125, of 96 170 and 136, of 64 228 and 227, 8 of 64 118 and 128, 16 of 16 85 and 174, 4 of 256 213 and 229 (two
+    // pieces a lane, too many registers); 300 tokens of 768 channels 14.6 and 16.3, 600 20.7 and 16.3, 300 of 2,304
+    // 26.5 and 25.8, of 3,072 channels, heads of 64, 34.7 and 29.6.
     const int W = dm.W(), C = dm.C();
-    if ((part || dtype == AGV_F32) && (part || ld % 4 == 0) && W % 4 == 0 && C % 4 == 0 && d % 4 == 0 &&
-        d <= 256 && taps >= 2 && taps <= 4 && state_stride % 4 == 0 && conv_off % 4 == 0 &&
-        agv_aligned(row, 16) && agv_aligned(part, 16) && agv_aligned(conv_w, 16) && agv_aligned(state, 16) &&
-        agv_aligned(qkv, 16)) {
+    const bool rows_can = (part || dtype == AGV_F32) && (part || ld % 4 == 0) && W % 4 == 0 && C % 4 == 0 && d % 4 == 0 &&
+                          d <= (several ? 128 : 256) && taps >= 2 && taps <= 4 && state_stride % 4 == 0 &&
+                          conv_off % 4 == 0 && agv_aligned(row, 16) && agv_aligned(part, 16) && agv_aligned(conv_w, 16) &&
+                          agv_aligned(state, 16) && agv_aligned(qkv, 16);
+    const long long lanes = 128LL * (2 * G + (dm.nv() + 127) / 128);
+    const bool rows_pay = !several || (4LL * C >= 3 * lanes && (C >= 1536 || T >= 512)) ||
+                          (5LL * C >= 3 * lanes && C >= 3072 && T <= 1024);
+    AGV_REQUIRE(form >= 0 && form <= 2, "delta_prepare: no form %d", form);
+    AGV_REQUIRE(form != 1 || rows_can, "delta_prepare: the rows form does not take these rows");
+    if (form == 1 || (form == 0 && rows_can && rows_pay)) {
         AGV_REQUIRE(dtype == AGV_F32 || dtype == AGV_BF16, "delta_prepare: unknown dtype %d", dtype);
         const RowIn<float> in{(const float*)row, ld, part, n_splits, (long long)T * W, W};
         const int NJ = d <= 128 ? 1 : 2, R = several ? 8 : 1;
@@ -780,13 +792,12 @@ AGV_API int agv_delta_prepare(const void* row, long long ld, const float* part, 
             agv_launch(kern, (unsigned)((warps + 3) / 4), 128, 0, stream, in, dm, st, T, n_seg, conv_w, eps_unit,
                        q_mult, several ? 0 : 1, qkv, beta, la, lg);
         };
-#define AGV_DPR(TT, TAPS, N) do {                                                                        \
-        if (several) go(delta_prepare_rows_kernel<TT, TAPS, N, 8>, (TT*)low_a, (TT*)low_g);              \
-        else go(delta_prepare_rows_kernel<TT, TAPS, N, 1>, (TT*)low_a, (TT*)low_g); } while (0)
-#define AGV_DPT(TT) do {                                                                                 \
-        if (taps == 4) { if (NJ == 1) AGV_DPR(TT, 4, 1); else AGV_DPR(TT, 4, 2); }                       \
-        else if (taps == 3) { if (NJ == 1) AGV_DPR(TT, 3, 1); else AGV_DPR(TT, 3, 2); }                  \
-        else { if (NJ == 1) AGV_DPR(TT, 2, 1); else AGV_DPR(TT, 2, 2); } } while (0)
+#define AGV_DPR(TT, TAPS) do {                                                                               \
+        if (several) go(delta_prepare_rows_kernel<TT, TAPS, 1, 8>, (TT*)low_a, (TT*)low_g);                      \
+        else if (NJ == 1) go(delta_prepare_rows_kernel<TT, TAPS, 1, 1>, (TT*)low_a, (TT*)low_g);                 \
+        else go(delta_prepare_rows_kernel<TT, TAPS, 2, 1>, (TT*)low_a, (TT*)low_g); } while (0)
+#define AGV_DPT(TT) do {                                                                                     \
+        if (taps == 4) AGV_DPR(TT, 4); else if (taps == 3) AGV_DPR(TT, 3); else AGV_DPR(TT, 2); } while (0)
         if (dtype == AGV_F32) AGV_DPT(float); else AGV_DPT(__nv_bfloat16);
 #undef AGV_DPT
 #undef AGV_DPR

@@ -858,13 +858,15 @@ def delta_prepare(row: Optional[torch.Tensor], partial: Optional[torch.Tensor], 
                   state: torch.Tensor, conv_off: int, n_qk_heads: int, n_heads: int,
                   head_dim: int, value_dim: int, taps: int, decay_rank: int, gate_rank: int,
                   conv_w: torch.Tensor, unit_eps: float, q_mult: float, qkv: torch.Tensor,
-                  beta: torch.Tensor, low_a: torch.Tensor, low_g: torch.Tensor) -> None:
+                  beta: torch.Tensor, low_a: torch.Tensor, low_g: torch.Tensor,
+                  form: str = "auto") -> None:
     """From a token's row  q | k | v | b | a1 | g1  of the stacked projection ([T, W] in the
     compute dtype or ``partial`` [S, T, W] 32-bit sums): the causal convolution over ``taps``
     tokens and silu on q, k and v (its earlier inputs come from the step's rows or, before
     the step, from ``state`` at ``conv_off``, which is brought up to date), unit q and k heads
     (q times ``q_mult``), beta = sigmoid(b).  qkv [T, 2 G d + H dv] and beta [T, H] are 32-bit;
-    low_a [T, ra] and low_g [T, rg] are the two bottlenecks in the compute dtype."""
+    low_a [T, ra] and low_g [T, rg] are the two bottlenecks in the compute dtype.  ``form``: "auto", or
+    one of the two forms, "rows" (a warp a head or piece of a row) and "token" (a CTA a token)."""
     C = 2 * n_qk_heads * head_dim + n_heads * value_dim
     W = C + n_heads + decay_rank + gate_rank
     rp, ld, pp, ns = _row_input(row, partial, T, W)
@@ -881,8 +883,8 @@ def delta_prepare(row: Optional[torch.Tensor], partial: Optional[torch.Tensor], 
             head_dim, value_dim, taps, decay_rank, gate_rank, _ptr(conv_w),
             ctypes.c_float(unit_eps), ctypes.c_float(q_mult), sp, ss, ctypes.c_longlong(conv_off),
             _ptr(ctx.slots), _ptr(ctx.cu_seqlens), _ptr(ctx.seq_index), _ptr(ctx.positions),
-            0 if ctx.mode == "decode" else 1, _ptr(qkv), _ptr(beta), _ptr(low_a), _ptr(low_g),
-            _stream()))
+            0 if ctx.mode == "decode" else 1, ("auto", "rows", "token").index(form), _ptr(qkv),
+            _ptr(beta), _ptr(low_a), _ptr(low_g), _stream()))
 
 
 def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, a: torch.Tensor, dt_bias: torch.Tensor,

@@ -61,15 +61,21 @@ def test_delta_prepare_rows(taps, G, H, d, dv, splits, dtype, counts, starts):
     off0 = H * dv * d + (-H * dv * d) % 4
     state0 = rnd(3, off0 + (taps - 1) * C, seed=3)
     outs = []
-    for w in (conv_w, off(conv_w)):
+    for w, form in ((conv_w, "token"), (off(conv_w), "auto"), (conv_w, "rows"), (conv_w, "auto")):
+        if form == "rows" and d > 128 and ctx.mode != "decode":
+            with pytest.raises(kernels.KernelError, match="rows form"):
+                kernels.delta_prepare(None, part, T, ctx, state0.clone(), off0, G, H, d, dv, taps, ra, rg, w, 1e-6,
+                                      0.3, qkv, beta, la, lg, form=form)
+            continue
         state = state0.clone()
         qkv, beta = torch.zeros(T, C, device=DEV), torch.zeros(T, H, device=DEV)
         la, lg = (torch.zeros(T, r, dtype=dtype, device=DEV) for r in (ra, rg))
         kernels.delta_prepare(None, part, T, ctx, state, off0, G, H, d, dv, taps, ra, rg, w, 1e-6,
-                              0.3, qkv, beta, la, lg)
+                              0.3, qkv, beta, la, lg, form=form)
         outs.append((qkv, beta, la, lg, state))
-    for a, b in zip(*outs):
-        same(a, b)
+    for got in outs[1:]:
+        for a, b in zip(outs[0], got):
+            same(b, a)
 
 
 @pytest.mark.parametrize("taps", [2, 4])
@@ -94,7 +100,7 @@ def test_delta_prepare_of_steps_one_after_the_other(taps, starts):
     def run(state):
         for (ctx, x), o in zip(steps, outs):
             kernels.delta_prepare(None, x, x.shape[1], ctx, state, off0, G, H, d, dv, taps, ra, rg, conv_w, 1e-6,
-                                  0.3, *o)
+                                  0.3, *o, form="rows")
     state = state0.clone()
     run(state)
     torch.cuda.synchronize()
@@ -105,7 +111,8 @@ def test_delta_prepare_of_steps_one_after_the_other(taps, starts):
     whole = torch.zeros(B * (7 + N), C, device=DEV)
     kernels.delta_prepare(None, rows, B * (7 + N), step([7 + N] * B, [starts] * B, list(range(B))), state0.clone(), off0,
                           G, H, d, dv, taps, ra, rg, conv_w, 1e-6, 0.3, whole, torch.zeros(B * (7 + N), H, device=DEV),
-                          torch.zeros(B * (7 + N), ra, device=DEV), torch.zeros(B * (7 + N), rg, device=DEV))
+                          torch.zeros(B * (7 + N), ra, device=DEV), torch.zeros(B * (7 + N), rg, device=DEV),
+                          form="token")
     for _ in range(20):
         state.copy_(state0)
         graph.replay()
