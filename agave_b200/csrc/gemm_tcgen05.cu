@@ -618,10 +618,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 // LP = P / 4 neighbouring lanes read a token back, four pairs each, so that the tables are read and
 // q, k, v and the cache rows written in lines of a token.  With every lane at its own token's row
 // (each access 32 rows apart) the epilogue took 28 us a tile, and the product (1,152 or 2,560 long)
-// 5 to 11.  8,696 tokens of eight
-// sequences x 1,536 x 1,152: 84 us, 73 with the lookups under the products and the zeros behind a sequence's
-// end by the whole warp (one lane wrote them all), 68 so; 2,048 tokens 26, 25, 20; 4,001 x 4,096 x 2,560 101
-// before and after.
+// 5 to 11.  In lines, with the lookups under the products and the zeros behind a sequence's end 16 bytes at
+// a time, a lane a row (us; before, and with those zeros by the whole warp a row at a time): 8,696 tokens of
+// eight sequences x 1,536 x 1,152 58 (61) -> 45, 2,048 26 -> 18, 2,049 50 (39) -> 19; 4,001 x 4,096 x 2,560 99 (92)
+// -> 79.
 // (swizzled by the row: neither side has bank conflicts, and no padding is needed)
 template <int P>
 __device__ __forceinline__ void qkv_epilogue(uint32_t lane_base, int m0, int tok, int half, int T,
@@ -684,13 +684,19 @@ __device__ __forceinline__ void qkv_epilogue(uint32_t lane_base, int m0, int tok
                     v1[(size_t)j * qe.vw.ld] = __float2bfloat16_rn(__uint_as_float(y[j]));
                 }
             }
-            // after a sequence's last token zeros up to the next multiple of 64 columns, by the whole warp
+            // after a sequence's last token zeros up to the next multiple of 64 columns, by the whole warp: a
+            // lane a row, single values up to a 16-byte boundary, then eight at a time
             for (unsigned ends = __ballot_sync(0xffffffffu, is_v && at_row.vt_pad > 0); ends; ends &= ends - 1) {
                 const int l = __ffs(ends) - 1, pad = __shfl_sync(0xffffffffu, at_row.vt_pad, l);
                 const long long col = __shfl_sync(0xffffffffu, vt_col, l) + 1;
-                for (int j = 0; j < 2 * P; ++j) {
-                    __nv_bfloat16* v0 = qe.vw.vt + (size_t)(g * hd + i + (j < P ? j : H2 + j - P)) * qe.vw.ld + col;
-                    for (int pc = lane; pc < pad; pc += 32) v0[pc] = __float2bfloat16_rn(0.f);
+#pragma unroll 1
+                for (int j = 0; j < 2 * P / 32; ++j) {
+                    const int r = j * 32 + lane;
+                    __nv_bfloat16* z = qe.vw.vt + (size_t)(g * hd + i + (r < P ? r : H2 + r - P)) * qe.vw.ld + col;
+                    __nv_bfloat16* const end = z + pad;
+                    while (z < end && ((uintptr_t)z & 15)) *z++ = __float2bfloat16_rn(0.f);
+                    for (; z + 8 <= end; z += 8) *reinterpret_cast<uint4*>(z) = make_uint4(0, 0, 0, 0);
+                    while (z < end) *z++ = __float2bfloat16_rn(0.f);
                 }
             }
 #pragma unroll

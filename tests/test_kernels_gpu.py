@@ -449,6 +449,33 @@ def test_qkv_product_with_norm_rotation_and_stores_in_its_epilogue(nh, nkv, hd, 
     assert torch.equal(qkv2, qkv)
 
 
+@pytest.mark.parametrize("nkv,hd", [(1, 256), (2, 128), (3, 64)])
+def test_qkv_prefill_zeros_behind_every_end(nkv, hd):
+    """The transposed values of sequences of many lengths: every sequence's columns, zeros up to the next
+    multiple of 64, nothing behind them; ends in one tile of tokens and in several."""
+    from agave_b200 import kernels
+    lens = [1, 2, 7, 8, 9, 31, 33, 55, 56, 57, 63, 64, 65, 120, 127, 128, 129, 200]
+    T, K, nh, B = sum(lens), 64, 2, len(lens)
+    x = rnd(T, K, dtype=torch.bfloat16, seed=1)
+    w = rnd((nh + 2 * nkv) * hd, K, dtype=torch.bfloat16, seed=2)
+    i32 = dict(dtype=torch.int32, device=DEV)
+    cuts = [sum(lens[:b]) for b in range(B + 1)]
+    pos = torch.cat([torch.arange(n) for n in lens]).to(**i32)
+    seq = torch.cat([torch.full((n,), b) for b, n in enumerate(lens)]).to(**i32)
+    cols = [(n + 63) // 64 * 64 for n in lens]
+    vt = torch.full((nkv * hd, sum(cols) + 64), 7.0, dtype=torch.bfloat16, device=DEV)
+    qkv = torch.empty((T, (nh + 2 * nkv) * hd), dtype=torch.bfloat16, device=DEV)
+    kernels.qkv_prefill(x, w, qkv, nh, nkv, hd, None, None, 1e-6, None, None, pos, seq, vt=vt,
+                        cu_seqlens=torch.tensor(cuts, **i32))
+    assert kernels.linear_tc_status() == 0
+    v, at = qkv[:, (nh + nkv) * hd:], 0
+    for b, n in enumerate(lens):
+        assert torch.equal(vt[:, at:at + n], v[cuts[b]:cuts[b + 1]].T), n
+        assert not vt[:, at + n:at + cols[b]].any(), n
+        at += cols[b]
+    assert (vt[:, at:] == 7.0).all()
+
+
 def ref_attention(q, k, v, scale, window):
     """q [Tq, nh, hd] at positions pos (last Tq of the keys), k/v [Tk, nkv, hd]."""
     Tq, nh, hd = q.shape
