@@ -367,7 +367,9 @@ norm_residual_warp_kernel(float* __restrict__ h, const float* __restrict__ y, in
 // The same with one CTA per row, 16-byte loads issued up front, two block-wide sums: for prompts'
 // rows of more than 512 values, and for 32 to 256 rows of any width (decoding many sequences).  U partial
 // sums are loaded together: four where a step has up to sixteen, one in long prompts, whose one or two
-// do not pay for 16 NV registers more a thread, i.e. two CTAs an SM instead of five.
+// do not pay for 16 NV registers more a thread, i.e. two CTAs an SM instead of five.  TH: 256 threads, or 0
+// for as many as the row needs (one or two partial sums, and rows of up to 1,024 values: with four sums and wider
+// rows what the fixed number saves in addresses is worth more; 512 rows of 5,376, four sums, 25 us against 29).
 // Bound by the bytes (h in and out, y, x) and by how many rows' loads an SM has in flight.  With an event's
 // 6 us, against four partial sums at a time (a warp a row up to 2,048 values): 4,001 rows of 2,560, 22 us of
 // HBM, 43.0 -> 30.7; of 5,376, 46 us, 92.1 -> 59.4; 2,048 rows of 2,048 25.6 -> 18.5; 8,696 of 1,152
@@ -479,7 +481,6 @@ static bool launch_norm_warp(float* h, const float* y, int n_splits, size_t spli
                split_stride, w_post, w_next, x, R, H, eps_post, eps_next, add_residual)
     if (nv <= 2) AGV_WARP(2);
     else if (nv <= 4) AGV_WARP(4);
-    else if (nv <= 10) AGV_WARP(10);
     else return false;
 #undef AGV_WARP
     return true;
@@ -493,8 +494,9 @@ static bool launch_norm_row(float* h, const float* y, int n_splits, size_t split
     const int nv = (H / 4 + 255) / 256;
 #define AGV_ROW(NV)                                                                             \
     do {                                                                                        \
-        const int threads = R <= 256 ? 256 : ((H / 4 + NV - 1) / NV + 31) / 32 * 32;            \
-        auto kern = R <= 256       ? norm_residual_row_kernel<TX, NV, 4, 256>                   \
+        const bool whole = R <= 256 || (n_splits > 2 && H > 1024);                              \
+        const int threads = whole ? 256 : ((H / 4 + NV - 1) / NV + 31) / 32 * 32;               \
+        auto kern = whole          ? norm_residual_row_kernel<TX, NV, 4, 256>                   \
                     : n_splits > 2 ? norm_residual_row_kernel<TX, NV, 4, 0>                     \
                                    : norm_residual_row_kernel<TX, NV, 1, 0>;                    \
         agv_launch(kern, (unsigned)R, threads, 0, stream, h, y, n_splits, split_stride, w_post, w_next, x, R, H, \
@@ -515,14 +517,13 @@ static int launch_norm(float* h, const void* y, int n_splits, size_t split_strid
                        const float* w_post, const float* w_next, void* x, const int* rows, int R,
                        int H, float eps_post, float eps_next, int add_residual,
                        cudaStream_t stream) {
-    // many rows with a 32-bit branch input: one warp per row while a row is a few loads a lane, and
-    // for rows of up to 1,280 values where their number gives every SM 7 to 20 warps (2,048 of 1,152: 14.4 us
-    // alone either way, but 0.4 us a launch less in a step, whose next kernel finds room earlier)
+    // many rows with a 32-bit branch input: a warp a row while a row is a few loads a lane (up to 512
+    // values), else a CTA a row.  (516 to 1,280 values, 1,025 to 3,073 rows, a warp a row against a CTA: 2,048
+    // rows of 1,152 11.2 us and 11.0, everything else 4.2 to 22 us and 0.67 to 0.98 of it.)
     if constexpr (std::is_same<TY, float>::value) {
-        if (R > 256 && (H <= 512 || (H <= 1280 && R > 1024 && R <= 3072)) && y && !rows && H % 4 == 0 && agv_aligned(y, 16) &&
+        if (R > 256 && H <= 512 && y && !rows && H % 4 == 0 && agv_aligned(y, 16) &&
             agv_aligned(h, 16) && agv_aligned(x, 16) && split_stride % 4 == 0 &&
-            (!w_post || agv_aligned(w_post, 16)) && (!w_next || agv_aligned(w_next, 16)) &&
-            (add_residual || !h || true)) {
+            (!w_post || agv_aligned(w_post, 16)) && (!w_next || agv_aligned(w_next, 16))) {
             if (launch_norm_warp<TX>(h, (const float*)y, n_splits, split_stride, w_post, w_next,
                                      (TX*)x, R, H, eps_post, eps_next, add_residual, stream)) {
                 AGV_LAUNCH_OK("norm_residual_warp_kernel");

@@ -300,6 +300,27 @@ def test_norm_family(H, R):
     assert rel_err(xb, norm(href, wn, eps_n)) < 5e-3
 
 
+@pytest.mark.parametrize("S", [1, 2, 4])
+@pytest.mark.parametrize("H,R", [(512, 1030), (516, 257), (1024, 300), (1028, 300), (1152, 300), (1152, 1025), (1152, 3073),
+                                 (1280, 2000), (2048, 1025), (2560, 300), (3076, 513), (8192, 300)])
+def test_norm_of_prompts(H, R, S):
+    """A warp a row and a CTA a row, one, two and four partial sums, threads that follow the row and 256, two to
+    eight pieces a thread: with both norms and with neither."""
+    from agave_b200 import kernels
+    h, y = rnd(R, H, seed=1), rnd(S, R, H, seed=2)
+    wp, wn = rnd(H, seed=3) * 0.2 + 1, rnd(H, seed=4) * 0.2 + 1
+
+    def norm(v, w, eps):
+        return v / torch.sqrt((v * v).mean(-1, keepdim=True) + eps) * w.double()
+    total = y.double().sum(0)
+    for post, nxt in ((wp, wn), (None, None)):
+        got, x = h.clone(), torch.empty((R, H), device=DEV)
+        kernels.norm_residual(got, y, post, nxt, x, eps_post=1e-5, eps_next=1e-6)
+        want = h.double() + (norm(total, post, 1e-5) if post is not None else total)
+        assert rel_err(got, want) < 1e-6
+        assert rel_err(x, norm(want, nxt, 1e-6) if nxt is not None else want) < 2e-6
+
+
 # ------------------------------------------------------ embedding and rotation
 def test_embed_and_rope_table():
     from agave_b200 import kernels
