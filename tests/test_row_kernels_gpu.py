@@ -222,6 +222,27 @@ def test_delta_out(T, H, dv, dtype):
         same(y, want, dtype)
 
 
+@pytest.mark.parametrize("H,R,S", [(256, 70, 1), (512, 300, 2), (1000, 65, 1), (1028, 65, 2), (1028, 1024, 1), (1152, 1024, 2),
+                                   (1152, 1025, 1), (1536, 1025, 2), (1540, 1025, 1), (2048, 65, 2), (2048, 1025, 1),
+                                   (2560, 70, 2), (5000, 66, 1)])
+@pytest.mark.parametrize("rms", [False, True])
+def test_layer_norm_of_prompts(H, R, S, rms):
+    """A warp a row and a CTA a row on both sides of every size at which they change places, the stream's row asked
+    for early and late: branch norm, multiplier, residual sum and next norm in 64 bits."""
+    from agave_b200 import kernels
+    h, y = rnd(R, H, seed=1), rnd(S, R, H, seed=2)
+    w1, b1, w2, b2 = (rnd(H, seed=3 + i) for i in range(4))
+
+    def norm(v, w, b, eps):
+        c = v if rms else v - v.mean(-1, keepdim=True)
+        return c / torch.sqrt((c * c).mean(-1, keepdim=True) + eps) * w.double() + b.double()
+    got, x = h.clone(), torch.empty(R, H, device=DEV)
+    kernels.layer_norm_join(got, y, w1, b1, w2, b2, x, eps_post=1e-5, eps_next=1e-6, mult=0.7, rms=rms)
+    want = h.double() + 0.7 * norm(y.double().sum(0), w1, b1, 1e-5)
+    same(got, want)
+    same(x, norm(want, w2, b2, 1e-6))
+
+
 @pytest.mark.parametrize("T,K,H", [(1, 8, 4), (9, 2048, 2048), (3, 2056, 2052), (2, 4104, 4100)])
 @pytest.mark.parametrize("dtype", [BF, F32])
 def test_row_gate_by_pieces(T, K, H, dtype):
