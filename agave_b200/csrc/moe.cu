@@ -265,7 +265,8 @@ template <> struct Row16<__nv_bfloat16> {
 // The same for rows that move in 16-byte pieces: a CTA of RT_VW warps takes RT_TOK tokens,
 // warp w the experts w, w + RT_VW, ...; a lane's piece of a router row meets the same piece
 // of every token of the CTA, so the router's matrix is read once per RT_TOK tokens, and the
-// loads of a row are independent of one another.  Then warp t chooses for token t.
+// loads of a row are independent of one another.  Then warp t chooses for token t.  Few
+// tokens (decoding) take a CTA of sixteen warps each, many (prompts) share CTAs of eight by fours.
 template <typename T, int RT_TOK, int RT_VW>
 __global__ void __launch_bounds__(RT_VW * 32)
 moe_route_tiled_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ wr,
@@ -571,7 +572,11 @@ AGV_API int agv_moe_route_mode(const void* x, long long ldx, const void* wr,
     agv_launch(moe_route_tiled_kernel<TT, TOK, VW>, (unsigned)((T + TOK - 1) / TOK), VW * 32,   \
                (size_t)TOK * 3 * E * sizeof(float), stream, (const TT*)x, ldx, (const TT*)wr,   \
                correction, T, H, E, n_groups, keep, top, ids, wts, rs)
-        if (T <= 64) {
+        // A warp an expert from the seventeenth expert on, where sixteen warps would walk twice, and with rows
+        // of four pieces a lane at least (8 tokens, us, sixteen warps and 32: bfloat16 rows of 2,048, 16 experts 4.6 and
+        // 5.2, 24 6.1 and 5.1, 256 28 and 20; of 512 32 experts 4.5 and 5.0, 256 14 and 19; 32-bit rows of 512 256
+        // experts 19 and 12).
+        if (T <= 64 && E > 16 && H / piece >= 128) {
             const size_t smem = (size_t)3 * E * sizeof(float);
             if (dtype == AGV_F32)
                 agv_launch(moe_route_few_kernel<float>, (unsigned)T, RF_VW * 32, smem, stream, (const float*)x,
@@ -580,6 +585,12 @@ AGV_API int agv_moe_route_mode(const void* x, long long ldx, const void* wr,
                 agv_launch(moe_route_few_kernel<__nv_bfloat16>, (unsigned)T, RF_VW * 32, smem, stream,
                            (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)wr, correction, H, E, n_groups,
                            keep, top, ids, wts, rs);
+            AGV_LAUNCH_OK("moe_route_few_kernel");
+            return 0;
+        }
+        if (T <= 64) {
+            if (dtype == AGV_F32) AGV_ROUTE(float, 1, 16);
+            else AGV_ROUTE(__nv_bfloat16, 1, 16);
         } else {
             if (dtype == AGV_F32) AGV_ROUTE(float, 4, 8);
             else AGV_ROUTE(__nv_bfloat16, 4, 8);

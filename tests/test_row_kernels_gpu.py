@@ -256,10 +256,13 @@ def test_row_gate_by_pieces(T, K, H, dtype):
     same(*ys)
 
 
-@pytest.mark.parametrize("T,H,E,top", [(1, 8, 4, 2), (64, 2048, 32, 4), (3, 2056, 33, 3), (5, 4616, 70, 6)])
+@pytest.mark.parametrize("T,H,E,top", [(1, 8, 4, 2), (64, 2048, 32, 4), (3, 2056, 33, 3), (5, 4616, 70, 6),
+                                       (64, 1024, 17, 2), (65, 1024, 17, 2), (3, 1024, 16, 2), (3, 1016, 17, 2),
+                                       (3, 512, 40, 2), (3, 508 * 2, 200, 5)])
 @pytest.mark.parametrize("dtype", [BF, F32])
 def test_route_of_few_tokens(T, H, E, top, dtype):
-    """A warp an expert: one round of experts and several, rows of one round of pieces and more."""
+    """A warp an expert: one round of experts and several, rows of one round of pieces and more; the sizes at
+    which sixteen warps and shared CTAs take over."""
     from agave_b200 import kernels
     x, w = rnd(T, H, dtype=dtype, seed=1), rnd(E, H, dtype=dtype, seed=2, scale=0.05)
     got = []
