@@ -217,7 +217,8 @@ proj_norm_store4_kernel(RowIn<float> in, T* __restrict__ out, long long ldo, int
 
 // latent_prepare, four values at a time (see proj_norm_store4_kernel): the pieces that are rotated also
 // go to shared memory, where a piece of one half of a rotated part finds the other's.  2,048 tokens,
-// rows of 3,072 + 192 + 64 + 2,048 and of 512 + 192 + 64 + 16 values: 31 and 12 us, two of each 99.7 -> 85.1.
+// rows of 2,048 + 192 + 64 + 2,048 and of 512 + 192 + 64 + 16 values: 28 and 12 us, two of each 99.7 -> 85.1 with
+// three pieces a thread.
 template <typename T>
 __global__ void __launch_bounds__(1024)
 latent_prepare4_kernel(RowIn<float> in, T* __restrict__ out, long long ldo, int q_width, int q_latent, int d,
@@ -597,12 +598,20 @@ __global__ void rope_table_freqs_kernel(const int* __restrict__ positions,
 // Threads of a one-CTA-per-token kernel: a decode step has few tokens, and what hides a
 // load's latency there is more threads per row; a prompt has rows enough.
 int row_threads(int T) { return T <= 64 ? 1024 : 256; }
-// Threads of a row of W values in pieces of four: few rows, a piece a thread; many, up to three, and no
+// Threads of a row of W values in pieces of four: few rows, a piece a thread; many, up to `each` and no
 // idle warps.
-int row4_threads(int T, int W) {
-    const int pieces = (W + 3) / 4, n = T <= 64 ? pieces : (pieces + 2) / 3;
+int row4_threads(int T, int W, int each) {
+    const int pieces = (W + 3) / 4, n = T <= 64 ? pieces : (pieces + each - 1) / each;
     return n >= 1024 ? 1024 : n <= 128 ? 128 : (n + 31) / 32 * 32;
 }
+// Prompts' rows of many values have CTAs of many threads, few to an SM and waiting for one another in the middle
+// of a row: from 3,073 values on a thread has four pieces instead of three, and the widest go through shared
+// memory.  (us, through shared memory, three and four pieces: 2,048 rows of 2,320 values 22.2, 19.9, 18.4, 512 6.6,
+// 5.0, 5.8; 2,048 of 3,664 25.9, 25.4, 23.9, 512 8.4, 9.1, 6.8; 2,048 of 4,352 28.9, 32.6, 28.0, 512 9.4, 9.9, 10.7;
+// 2,048 of 5,376 31, 35, 39; 2,048 of 6,752 42, 68, 43, 256 9.4, 9.4, 6.3; 2,048 of 8,512 52, 75, 84, 256 11.7,
+// 11.2, 13.0.)
+bool latent4_pays(int T, int W) { return T <= 256 || W <= 4096 || (W <= 4608 && T > 512); }
+int latent4_threads(int T, int W) { return row4_threads(T, W, T > 256 && W > 3072 ? 4 : 3); }
 
 unsigned flat_grid(long long n, int threads) {
     long long b = (n + threads - 1) / threads;
@@ -646,7 +655,7 @@ AGV_API int agv_proj_norm_store(const void* row, long long ld, const float* part
     AGV_REQUIRE(ld >= W || !row, "proj_norm: row stride shorter than the row");
     AGV_REQUIRE((size_t)W * 4 <= 200 * 1024, "proj_norm: rows of %d values do not fit", W);
     if (T == 0) return 0;
-    const int threads = row4_threads(T, W);
+    const int threads = row4_threads(T, W, 3);
     if ((part || (dtype == AGV_F32 && ld % 4 == 0)) && nq % 4 == 0 && nk % 4 == 0 && nv % 4 == 0 &&
         W <= threads * 4 * PN_PIECES && ldo % 4 == 0 && (!v_first || ldvf % 4 == 0) && agv_aligned(row, 16) &&
         agv_aligned(part, 16) && agv_aligned(out, 16) && agv_aligned(wq, 16) && agv_aligned(wk, 16) &&
@@ -707,8 +716,8 @@ AGV_API int agv_latent_prepare(const void* row, long long ld, const float* part,
     AGV_REQUIRE(ld >= W || !row, "latent_prepare: row stride shorter than the row");
     AGV_REQUIRE((size_t)W * 4 <= 200 * 1024, "latent_prepare: rows of %d values do not fit", W);
     if (T == 0) return 0;
-    const int threads = row4_threads(T, W);
-    if ((part || (dtype == AGV_F32 && ld % 4 == 0)) && q_width % 4 == 0 && R % 4 == 0 && G % 4 == 0 && d % 4 == 0 &&
+    const int threads = latent4_threads(T, W);
+    if (latent4_pays(T, W) && (part || (dtype == AGV_F32 && ld % 4 == 0)) && q_width % 4 == 0 && R % 4 == 0 && G % 4 == 0 && d % 4 == 0 &&
         r % (interleaved ? 4 : 8) == 0 && W <= threads * 4 * PN_PIECES && ldo % 4 == 0 && agv_aligned(row, 16) &&
         agv_aligned(part, 16) && agv_aligned(out, 16) && agv_aligned(w_q, 16) && agv_aligned(w_c, 16) &&
         agv_aligned(cosv, 16) && agv_aligned(sinv, 16) && agv_aligned(k_pool, 16) &&

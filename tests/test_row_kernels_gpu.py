@@ -312,6 +312,71 @@ def test_latent_prepare_by_fours(T, latent, interleaved, A, d, r, R, G, dtype):
     same(*outs, dtype)
 
 
+def paged(counts, slots, width, cap, dtype, page=4):
+    """A cache of rings of `cap` rows in scattered pages, and the step that whole sequences of these lengths make."""
+    ctx = step(counts, [0] * len(counts), slots)
+    ctx.lens = torch.tensor(counts, dtype=torch.int32, device=DEV)
+    per = cap // page
+    g = torch.Generator().manual_seed(cap)
+    table = torch.randperm(len(counts) * per, generator=g).int().view(len(counts), per).contiguous().to(DEV)
+    pool = torch.full((len(counts) * per, page, 1, width), 7.0, dtype=dtype, device=DEV)
+    return ctx, SimpleNamespace(k_pool=pool, v_pool=pool, page_table=table, page=page, cap=cap)
+
+
+def in_cache(view, counts, slots, rows):
+    """What the pool holds when each sequence's last `cap` rows are in their ring."""
+    want, at = torch.full_like(view.k_pool, 7.0), 0
+    for n, slot in zip(counts, slots):
+        for p in range(max(0, n - view.cap), n):
+            if slot >= 0:
+                r = p % view.cap
+                want[int(view.page_table[slot, r // view.page]), r % view.page, 0] = rows[at + p]
+        at += n
+    return want
+
+
+@pytest.mark.parametrize("counts,slots", [([5, 1, 9], [2, 0, 1]), ([40, 3, 60], [1, -1, 0]), ([200, 90, 30], [0, 2, 1])])
+@pytest.mark.parametrize("nq,nk,nv", [(64, 16, 16), (2048, 512, 512)])
+@pytest.mark.parametrize("dtype", [BF, F32])
+def test_proj_norm_by_fours_into_the_cache(counts, slots, nq, nk, nv, dtype):
+    """Keys and values of few and of many tokens into rings that keep a sequence's end, beside a padding entry."""
+    from agave_b200 import kernels
+    T = sum(counts)
+    part, wq, wk = rnd(2, T, nq + nk + nv, seed=1), rnd(nq, seed=2), rnd(nk, seed=3)
+    for w in (wq, off(wq)):
+        ctx, view = paged(counts, slots, nk, 32, dtype)
+        view.v_pool = torch.full((*view.k_pool.shape[:3], nv), 7.0, dtype=dtype, device=DEV)
+        out = torch.full((T, nq + nk + nv), float("nan"), dtype=dtype, device=DEV)
+        kernels.proj_norm_store(out, nq, nk, nv, w, wk, 1e-6, ctx.positions, view, ctx, partial=part)
+        assert torch.equal(view.k_pool, in_cache(view, counts, slots, out[:, nq:nq + nk]))
+        both = SimpleNamespace(**{**vars(view), "k_pool": view.v_pool})
+        assert torch.equal(view.v_pool, in_cache(both, counts, slots, out[:, nq + nk:]))
+
+
+@pytest.mark.parametrize("counts,slots", [([5, 1, 9], [2, 0, 1]), ([40, 3, 60], [1, -1, 0]), ([200, 90, 30], [0, 2, 1]),
+                                          ([300, 100, 150], [2, 0, 1])])
+@pytest.mark.parametrize("latent", [False, True])
+@pytest.mark.parametrize("A,d,r,R,G", [(2, 20, 24, 36, 40), (16, 128, 64, 512, 16), (16, 64, 64, 192, 2048), (32, 128, 64, 512, 32)])
+@pytest.mark.parametrize("dtype", [BF, F32])
+def test_latent_prepare_by_fours_into_the_cache(counts, slots, latent, A, d, r, R, G, dtype):
+    """Latent and key part of few and of many tokens into rings, at the widths and row counts at which threads and
+    forms change places: the same rows as the general form's."""
+    from agave_b200 import kernels
+    T, Q = sum(counts), 60 if latent else A * (d + r)
+    part = rnd(1, T, Q + R + r + G, seed=1)
+    wq, wc = (rnd(Q, seed=2) if latent else None), rnd(R, seed=3)
+    cos, sin = rnd(T, r // 2, seed=4), rnd(T, r // 2, seed=5)
+    outs = []
+    for w in (wc, off(wc)):
+        ctx, view = paged(counts, slots, R + r, 32, dtype)
+        out = torch.full((T, Q + R + r + G), float("nan"), dtype=dtype, device=DEV)
+        kernels.latent_prepare(out, Q, latent, A, d, r, R, G, wq, w, 1e-6, cos, sin, latent, ctx.positions, view, ctx,
+                               partial=part)
+        assert torch.equal(view.k_pool, in_cache(view, counts, slots, out[:, Q:Q + R + r]))
+        outs.append(out)
+    same(*outs, dtype)
+
+
 @pytest.mark.parametrize("H,G,d,dv", [(4, 1, 128, 64), (2, 2, 64, 32), (3, 1, 200, 100), (2, 1, 256, 34)])
 @pytest.mark.parametrize("counts", [[192], [1, 300, 64, 3], [129, 128, 127, 515]])
 @pytest.mark.parametrize("strong", [False, True])
