@@ -3,7 +3,7 @@
 // (plain FFMA, no reduced-precision mode) and the fallback of the bfloat16 path
 // for shapes the tensor-core kernel refuses.  A plain product may carry the squared relu or the erf GELU.
 //
-// In 32-bit K (from GS_MIN_K on) is cut into eight ranges whose bounds follow from K alone (the last may be short or empty).
+// In 32-bit K (from GS_MIN_K on, rows in whole 16-byte pieces) is cut into eight ranges whose bounds follow from K alone (the last may be short or empty).
 // A range is one chain of 32-bit fused multiply-adds in ascending k, and the eight sums are added
 // in pairs, ((0+1)+(2+3))+((4+5)+(6+7)), whatever M and N are and however the work is spread: a
 // row's result does not depend on which other rows share the launch.
@@ -358,8 +358,7 @@ gemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* xs = gs_smem + (t % GT_STAGES) * GT_STAGE + tm * GT_PITCH;
         const float* ws = gs_smem + (t % GT_STAGES) * GT_STAGE + (GT_M + tn) * GT_PITCH;
-#pragma unroll
-        for (int k = 0; k < GT_K; k += 4) {
+        auto four = [&](int k) {
             float4 x[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(xs + 8 * i * GT_PITCH + k);
@@ -373,6 +372,14 @@ gemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const
                     a = fmaf(x[i].z, w.z, a); a = fmaf(x[i].w, w.w, a);
                 }
             }
+        };
+        const int len = k_to - (k_from + t * GT_K);
+        if (len >= GT_K) {
+#pragma unroll
+            for (int k = 0; k < GT_K; k += 4) four(k);
+        } else {                                       // (a range's end: what is behind it is zeros)
+#pragma unroll 1
+            for (int k = 0; k < len; k += 4) four(k);
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -430,7 +437,7 @@ static int launch_f32(const GsArgs& a) {
     agv_launch_cluster(kern, dim3((unsigned)(m_tiles * n_tiles * CL)), TILE ? GT_THREADS : GS_WARPS * 32, smem,
                        a.stream, dim3(CL), (const float*)a.A, (const float*)a.W, (const float*)a.W2, (float*)a.C,
                        a.M, a.N, a.K, a.lda, a.ldc, a.act, (int)m_tiles, range);
-    AGV_LAUNCH_OK("gemm_rows_kernel");
+    AGV_LAUNCH_OK(TILE ? "gemm_tile_kernel" : "gemm_rows_kernel");
     return 0;
 }
 
@@ -457,16 +464,17 @@ static int launch_any(const GsArgs& a) {
 }
 
 // A K below this has ranges too short for a ring to fill (2048 x 256, 2,048 rows: 107 us either way;
-// x 64: 34 us with one chain, 83 with eight).  Which kernels a weight goes to follows from K and the
-// alignment alone, so that a row's sums have one order whatever the number of rows.
-constexpr int GS_MIN_K = 384;
+// x 64: 34 us with one chain, 83 with eight; gated, 4,096 x 384, 1,024 rows 1.08 times as long as in one chain, x 512
+// 0.98).  Which kernels a weight goes to follows from K, the form of the product and the alignment alone, so
+// that a row's sums have one order whatever the number of rows.
+template <bool GATED> constexpr int GS_MIN_K = GATED ? 512 : 384;
 
 template <bool GATED>
 static int launch_gemm(const GsArgs& a, int in_dtype, int out_dtype) {
     if (in_dtype == AGV_F32 && out_dtype == AGV_F32) {
         const bool pieces = a.K % 4 == 0 && a.lda % 4 == 0 && agv_aligned(a.A, 16) && agv_aligned(a.W, 16) &&
                             agv_aligned(a.W2, 16);
-        if (!pieces || a.K < GS_MIN_K) return launch_any<float, float, float, GATED>(a);
+        if (!pieces || a.K < GS_MIN_K<GATED>) return launch_any<float, float, float, GATED>(a);
         if (a.M <= 4) return launch_rows<GATED, 4>(a);
         if (a.M <= 8) return launch_rows<GATED, 8>(a);
         if (a.M <= 16) return launch_rows<GATED, 16>(a);

@@ -260,6 +260,27 @@ def test_linear_simt_rows_do_not_depend_on_their_company(N, K, gated):
         assert torch.equal(out, outs[130][130 - M:]), M
 
 
+@pytest.mark.parametrize("K", [380, 384, 400, 508, 512, 516])
+@pytest.mark.parametrize("gated", [False, True])
+def test_linear_simt_short_sums(K, gated):
+    """Where the eight ranges of K begin, and ranges that end inside a piece of sixteen: every kernel, in 64
+    bits, a row bit for bit the same in any company."""
+    from agave_b200 import kernels
+    N = 70
+    w, w2 = rnd(N, K, seed=2), rnd(N, K, seed=3) if gated else None
+    x = rnd(70, K, seed=1)
+    ref = x.double() @ w.double().T
+    if gated:
+        ref = torch.nn.functional.silu(ref) * (x.double() @ w2.double().T)
+    whole = torch.empty((70, N), device=DEV)
+    kernels.linear_simt(x, w, whole, w2=w2, activation="silu")
+    assert rel_err(whole, ref) < 4e-6
+    for M in (1, 6, 20, 33):
+        out = torch.empty((M, N), device=DEV)
+        kernels.linear_simt(x[:M], w, out, w2=w2, activation="silu")
+        assert torch.equal(out, whole[:M]), M
+
+
 # ---------------------------------------------------------------------- norms
 @pytest.mark.parametrize("H,R", [(48, 7), (1000, 7), (5376, 7), (1152, 300), (2048, 257), (72, 513),
                                  (2560, 300), (5376, 260), (8192, 257), (2052, 258),
