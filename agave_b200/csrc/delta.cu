@@ -16,12 +16,12 @@
 // weight [dv] and by sigmoid(gate), and rounded to the compute dtype for the output product.
 //
 // The columns of S are independent recurrences over d-vectors, so the scan gives every column
-// to a group of L lanes that hold 16 rows of it each in registers; the two dot products of a
+// (or two) to a group of L lanes that hold 16 rows of it each in registers; the two dot products of a
 // token are finished with L-wide shuffles.  A sequence's tokens run in order; sequences,
 // heads and groups of columns run side by side.  The state of a sequence (S of every head,
 // and the last taps - 1 inputs of the convolution) lives in 32-bit in the sequence's slot of
 // the fixed-size state and is read at the start of a step and written at its end, so a
-// prompt and a decoded token run the same code.
+// prompt and a decoded token differ only in the form of the kernels that does their work fastest.
 //
 // 32-bit throughout: sums over partial products, the convolution, silu, unit norms, beta, the
 // decay, the state and the recurrence, the output norm and the gate's sigmoid.
@@ -59,6 +59,7 @@ __device__ __forceinline__ float softplus_f(float t) {
 }
 
 // ------------------------------------------------------------------ prepare
+// Two forms, a CTA a token (any sizes) and a warp a head's or a piece of a row's channels (below).
 // The convolution's inputs of a sequence are a ring by position: the input of position pp is
 // row pp % (taps - 1) of the slot's [taps - 1, C] block, so a step writes the rows of its own
 // last taps - 1 positions and moves nothing.
@@ -136,7 +137,7 @@ delta_prepare_kernel(RowIn<T> in, DeltaDims dm, DeltaState st, const float* __re
 //
 // A decode step is bound by trips to memory one after the other: a CTA a token walked its 3,216
 // columns in a dozen of them, 35 us for 8 tokens (G 4, H 16, heads of 128, eight partial sums);
-// 31 warps a token make two, 4.7 us.  A prompt is bound by its rows (126 MB for 5,120 tokens, 20
+// 29 warps a token make two, 4.7 us.  A prompt is bound by its rows (126 MB for 5,120 tokens, 20
 // us): 191 us -> 108 with R = 8, which reads a row once instead of once a tap.
 template <typename T, int TAPS, int NJ, int R>
 __global__ void __launch_bounds__(128)

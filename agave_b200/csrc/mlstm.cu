@@ -9,7 +9,8 @@
 //     o_t = S_t^T q_t / (max(|n_t . q_t|, exp(-m_t)) + den_eps)
 // S, n and m of a sequence live in 32-bit in its slot of the cache's fixed-size state
 // ([H, d, dv] | [H, d] | [H, ceil(dv / 8)]), zero when the slot is taken, read at the start of a step and
-// written at its end.  A prompt and a decoded token run the same kernels.
+// written at its end.  A prompt and a decoded token run the same kernels (agv_head_scan's prompts
+// may go by chunks).
 //
 //  * agv_mlstm_prepare: from a token's row  q | k | v | g | i | f  of the stacked projection
 //    (32-bit, or 32-bit partial sums over ranges of K): q times q_mult, k, v and the two log
@@ -19,9 +20,10 @@
 //    token are read by a whole warp at once; the row blocks' parts of a column's dot product
 //    with q meet in shared memory after a chunk of tokens.  It leaves S_t^T q_t, n_t . q_t
 //    and exp(-m_t).
-//  * agv_head_scan: the same kernel without n and m, for other recurrences S_t = a_t S_(t-1) +
+//  * agv_head_scan: without n and m, for other recurrences S_t = a_t S_(t-1) +
 //    b_t k_t v_t^T, o_t = S_t^T q_t with a pair (a_t, b_t) per head and token that is given; the
-//    heads of a group may share q and k (the state-space form of Mamba-2).
+//    heads of a group may share q and k (the state-space form of Mamba-2).  The same kernel token by
+//    token, or chunks of 128 tokens as small products that run side by side.
 //  * agv_mlstm_out: the division, every head's o over its root mean square, times a weight
 //    per channel, times sigmoid(g), rounded to the compute dtype for the output product.
 #include "common.cuh"

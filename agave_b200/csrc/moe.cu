@@ -626,8 +626,8 @@ AGV_API int agv_moe_route(const void* x, long long ldx, const void* wr, const fl
 // product and the sigmoid are 32-bit.
 namespace {
 // V: values a load.  y's first two pieces a thread are asked for with x and w, so that a row is one
-// trip to memory (8 rows of 2,048, a load at a time in turn: 13.5 us, now 2.2; 5,120 rows, 105
-// MB, 16 us: 38 -> 13.6).
+// trip to memory (8 rows of 2,048, a load at a time in turn: 13.5 us, now 2.2; 5,120 rows, 105 MB, 16 us of
+// HBM: 38 -> 13.6 with rows that the kernel before left in L2, 55 -> 22.6 without and with an event's 6).
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 row_gate_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ w,

@@ -18,7 +18,8 @@
 //    part's root mean square, times a weight per channel.
 //
 // 32-bit throughout: sums over partial products, convolution, silu, softplus, decays, states.
-// Prompts and decoded tokens run the same kernels.
+// Prompts and decoded tokens run the same recurrences; long sequences are cut into segments that run
+// side by side where that is faster (see the selective scan).
 #include "common.cuh"
 #include "pieces.cuh"
 #include "row_in.cuh"
