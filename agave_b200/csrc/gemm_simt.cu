@@ -308,7 +308,9 @@ constexpr int GT_M = 64, GT_N = 128, GT_K = 16, GT_PITCH = GT_K + 4, GT_STAGES =
 constexpr int GT_STAGE = (GT_M + GT_N) * GT_PITCH;
 static_assert(GT_STAGES * GT_STAGE >= GT_M * GT_N, "the sums take the ring's place");
 
-template <bool GATED>
+// RAGGED: ranges that no piece divides, whose last piece stops at the range's end instead of multiplying zeros
+// (K = 400 in ranges of 52: 8 to 10 % less; the second loop costs the other ranges 2 to 5 %).
+template <bool GATED, bool RAGGED>
 __global__ void __launch_bounds__(GT_THREADS)
 gemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ W2,
                  float* __restrict__ C, int M, int N, int K, long long lda, long long ldc, GateAct act,
@@ -374,10 +376,10 @@ gemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const
             }
         };
         const int len = k_to - (k_from + t * GT_K);
-        if (len >= GT_K) {
+        if (!RAGGED || len >= GT_K) {
 #pragma unroll
             for (int k = 0; k < GT_K; k += 4) four(k);
-        } else {                                       // (a range's end: what is behind it is zeros)
+        } else {
 #pragma unroll 1
             for (int k = 0; k < len; k += 4) four(k);
         }
@@ -430,7 +432,7 @@ static int launch_f32(const GsArgs& a) {
     const int range = ((a.K + 7) / 8 + 3) / 4 * 4;
     void (*kern)(const float*, const float*, const float*, float*, int, int, int, long long, long long, GateAct,
                  int, int);
-    if constexpr (TILE) kern = gemm_tile_kernel<GATED>;
+    if constexpr (TILE) kern = range % GT_K ? gemm_tile_kernel<GATED, true> : gemm_tile_kernel<GATED, false>;
     else kern = gemm_rows_kernel<GATED, BM, R>;
     if (smem > 48 * 1024)
         AGV_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -464,17 +466,17 @@ static int launch_any(const GsArgs& a) {
 }
 
 // A K below this has ranges too short for a ring to fill (2048 x 256, 2,048 rows: 107 us either way;
-// x 64: 34 us with one chain, 83 with eight; gated, 4,096 x 384, 1,024 rows 1.08 times as long as in one chain, x 512
-// 0.98).  Which kernels a weight goes to follows from K, the form of the product and the alignment alone, so
-// that a row's sums have one order whatever the number of rows.
-template <bool GATED> constexpr int GS_MIN_K = GATED ? 512 : 384;
+// x 64: 34 us with one chain, 83 with eight).  At 384 many rows of a gated pair lose up to 9 % (4,096 outputs,
+// 2,048 rows) and few rows take a seventh (three rows 46 -> 7 us).  Which kernels a weight goes to follows
+// from K and the alignment alone, so that a row's sums have one order whatever the number of rows.
+constexpr int GS_MIN_K = 384;
 
 template <bool GATED>
 static int launch_gemm(const GsArgs& a, int in_dtype, int out_dtype) {
     if (in_dtype == AGV_F32 && out_dtype == AGV_F32) {
         const bool pieces = a.K % 4 == 0 && a.lda % 4 == 0 && agv_aligned(a.A, 16) && agv_aligned(a.W, 16) &&
                             agv_aligned(a.W2, 16);
-        if (!pieces || a.K < GS_MIN_K<GATED>) return launch_any<float, float, float, GATED>(a);
+        if (!pieces || a.K < GS_MIN_K) return launch_any<float, float, float, GATED>(a);
         if (a.M <= 4) return launch_rows<GATED, 4>(a);
         if (a.M <= 8) return launch_rows<GATED, 8>(a);
         if (a.M <= 16) return launch_rows<GATED, 16>(a);

@@ -1,8 +1,8 @@
 """Projections: a weight [out, in] and the kernel choice for it.
 
 The 32-bit path always runs the FFMA kernels (the order of an output's sum follows
-from K, the form of the product and the alignment of its operands, not from the number
-of rows: a token's result does not depend on its company at all).  The
+from K and the alignment of its operands, not from the number of rows: a token's result
+does not depend on its company at all).  The
 bfloat16 path runs the tcgen05 kernel when the shape qualifies and otherwise
 the FFMA kernel on bfloat16 data.  On the tcgen05 path the number of ranges K
 is cut into follows the number of tokens, so a token's 32-bit sums are added in
