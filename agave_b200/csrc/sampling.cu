@@ -229,7 +229,7 @@ __device__ __forceinline__ unsigned long long to_fixed(float w) {
 }
 
 // A row is shared by the C CTAs of a cluster (C = 1, 2, 4 or 8): CTA c owns a contiguous slice of
-// the vocabulary, keeps it in shared memory (SM_RESIDENT values at most; what a larger slice has
+// the vocabulary, keeps it in shared memory (`resident` values at most; what a larger slice has
 // beyond them is read again from global memory) and answers for it in every pass.  What decides
 // anything crosses the cluster: the maximum, the 256 bins of a radix pass, the slices' sums.
 // All of those are maxima, counts and fixed-point sums, so the token does not depend on C.
@@ -241,7 +241,9 @@ __device__ __forceinline__ unsigned long long to_fixed(float w) {
 // slices in shared memory, top-k 64 and top-p 0.95: 334 us when every pass runs over the cluster,
 // 100 us when the few candidates a top-k leaves are finished by one CTA (one row: 3,860, 72 and 33
 // us; top-p 0.9 alone, where every weight takes part: 2,160 -> 326 us).  Eight CTAs of a 262,144
-// row take 128 KB each, so 16 to 18 rows run at a time.
+// row take 128 KB each, so 16 to 18 rows run at a time.  CTAS: how many an SM is to hold; two have 32 registers
+// a thread, which costs a lone CTA its spills (one row of 65,536, top-k 64 21.9 -> 25.4 us) and gains where
+// there are more than SMs and their slices leave room (256 rows of 20,000, temperature alone 42 -> 30).
 constexpr int SM_RESIDENT = 44 * 1024;         // values of a slice in shared memory (176 KB)
 constexpr int SM_LIST = 2048;                  // candidates of a top-k that one CTA finishes alone
 
@@ -291,8 +293,9 @@ struct SampleShared : RadixShared {
     int list_i[SM_LIST];
 };
 
-__global__ void __launch_bounds__(SM_THREADS)
-sample_kernel(const float* __restrict__ logits, long long row_stride, int V, int C, int slice,
+template <int CTAS>
+__global__ void __launch_bounds__(SM_THREADS, CTAS)
+sample_kernel(const float* __restrict__ logits, long long row_stride, int V, int C, int slice, int resident,
               int* __restrict__ out, float inv_temperature, int top_k, float top_p,
               unsigned long long seed, const long long* __restrict__ seq_ids,
               const int* __restrict__ steps, const int* __restrict__ dev_params) {
@@ -306,15 +309,15 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V, int
                ((unsigned long long)(unsigned)dev_params[SP_SEED_HI] << 32);
     }
     __shared__ SampleShared sh;
-    extern __shared__ __align__(16) float resident[];
-    float* val = resident;                                // the slice: logits, then weights
+    extern __shared__ __align__(16) float sm_slice[];
+    float* val = sm_slice;                                // the slice: logits, then weights
     bool listed = false;                                  // the candidates instead of the slice
     const int rank = C > 1 ? (int)cluster_rank() : 0;
     const int row_id = blockIdx.x / C;
     const float* row = logits + (size_t)row_id * row_stride;
     const int lo = min(V, rank * slice);
     int n = min(V, lo + slice) - lo;
-    int held = min(n, SM_RESIDENT);
+    int held = min(n, resident);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int elements = (n + SM_THREADS - 1) / SM_THREADS;            // of a thread, SM_THREADS apart
     int turn = 0;
@@ -326,7 +329,7 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V, int
         const float x = raw * inv_temperature;
         mx = fmaxf(mx, x);
         best = max(best, ordered_key(x));
-        if (i < SM_RESIDENT) val[i] = x;
+        if (i < resident) val[i] = x;
     };
     if (((uintptr_t)(row + lo) & 15) == 0) {
         const float4* src = reinterpret_cast<const float4*>(row + lo);
@@ -529,16 +532,21 @@ AGV_API int agv_sample(const float* logits, long long row_stride, int B, int V, 
     AGV_REQUIRE(top_k >= 0, "sample: top_k must be >= 0");
     if (B == 0) return 0;
     // A slice of at most 32,768 values (32 a thread) where eight CTAs can give that; a slice starts
-    // on a multiple of four values, so that a row on a 16-byte boundary is read 16 bytes at a time.
+    // on a multiple of four values, so that a row on a 16-byte boundary is read 16 bytes at a time.  Rows for
+    // every SM that have only a temperature make no passes over bins: a CTA for up to 40,960 values (256 rows of
+    // 40,000: 54 us, 87 with clusters of four).
+    const bool plain = !dev_params && top_k == 0 && !(top_p > 0.f && top_p < 1.f) && B > 148;
     int C = 1;
-    while (C < 8 && V > 16384 * C) C *= 2;
-    const int slice = ((V + C - 1) / C + 3) / 4 * 4;
+    while (C < 8 && V > (plain ? 40960 : 16384) * C) C *= 2;
+    const int slice = ((V + C - 1) / C + 3) / 4 * 4, resident = slice < SM_RESIDENT ? slice : SM_RESIDENT;
     AGV_REQUIRE((long long)B * C <= 0x7fffffffLL, "sample: %d rows exceed the grid limit", B);
-    const size_t smem = (size_t)(slice < SM_RESIDENT ? slice : SM_RESIDENT) * sizeof(float);
-    AGV_CUDA_OK(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const size_t smem = (size_t)resident * sizeof(float);
+    const bool two = (long long)B * C > 148 && 2 * (smem + sizeof(SampleShared) + 1024) <= 227 * 1024;
+    auto kern = two ? sample_kernel<2> : sample_kernel<1>;
+    AGV_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      SM_RESIDENT * (int)sizeof(float)));
-    agv_launch_cluster(sample_kernel, dim3((unsigned)(B * C)), SM_THREADS, smem, stream, dim3(C), logits,
-                       row_stride, V, C, slice, out, dev_params ? 1.0f : 1.0f / temperature, top_k,
+    agv_launch_cluster(kern, dim3((unsigned)(B * C)), SM_THREADS, smem, stream, dim3(C), logits,
+                       row_stride, V, C, slice, resident, out, dev_params ? 1.0f : 1.0f / temperature, top_k,
                        top_p, seed, seq_ids, steps, dev_params);
     AGV_LAUNCH_OK("sample_kernel");
     return 0;

@@ -803,6 +803,29 @@ def test_sampling_token_does_not_depend_on_the_ctas_of_a_row(V, top_k, top_p):
     assert all(0 <= t < V for t in tokens[0])
 
 
+@pytest.mark.parametrize("V", [300, 16384, 20001, 70000])
+@pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (0, 0.8), (20, 0.9)])
+def test_sampling_of_many_rows(V, top_k, top_p):
+    """More rows than SMs: two CTAs an SM, and with a temperature alone a CTA a row, most of a long one read again;
+    the same tokens as the rows a few at a time, and with the options on the device."""
+    from agave_b200 import kernels
+    B = 300
+    logits = rnd(B, V, seed=V) * 3.0
+    seq = torch.arange(B, dtype=torch.int64, device=DEV)
+    steps = torch.full((B,), 4, dtype=torch.int32, device=DEV)
+    out = torch.full((B,), -5, dtype=torch.int32, device=DEV)
+    kernels.sample(logits, out, 0.5, top_k, top_p, 5, seq, steps)
+    words = torch.tensor(kernels.sampling_words(0.5, top_k, top_p, 5, 1.0), dtype=torch.int32, device=DEV)
+    again = torch.full_like(out, -5)
+    kernels.sample(logits, again, 1.0, 0, 1.0, 0, seq, steps, dev_params=words)
+    assert torch.equal(out, again)
+    for at in (0, 149, 293):
+        few = torch.full((7,), -5, dtype=torch.int32, device=DEV)
+        kernels.sample(logits[at:at + 7], few, 0.5, top_k, top_p, 5, seq[at:at + 7].contiguous(), steps[:7].contiguous())
+        assert torch.equal(few, out[at:at + 7])
+    assert len(set(out.tolist())) > 50
+
+
 def test_repeat_penalty_per_occurrence_and_history():
     from agave_b200 import kernels
     V = 300
