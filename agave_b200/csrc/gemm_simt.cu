@@ -309,7 +309,7 @@ constexpr int GT_STAGE = (GT_M + GT_N) * GT_PITCH;
 static_assert(GT_STAGES * GT_STAGE >= GT_M * GT_N, "the sums take the ring's place");
 
 // RAGGED: ranges that no piece divides, whose last piece stops at the range's end instead of multiplying zeros
-// (K = 400 in ranges of 52: 8 to 10 % less; the second loop costs the other ranges 2 to 5 %).
+// (K = 400 in ranges of 52: 8 to 10 % less; the tests cost the other ranges 2 to 5 %).
 template <bool GATED, bool RAGGED>
 __global__ void __launch_bounds__(GT_THREADS)
 gemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ W2,
@@ -360,7 +360,10 @@ gemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* xs = gs_smem + (t % GT_STAGES) * GT_STAGE + tm * GT_PITCH;
         const float* ws = gs_smem + (t % GT_STAGES) * GT_STAGE + (GT_M + tn) * GT_PITCH;
-        auto four = [&](int k) {
+        const int len = RAGGED ? k_to - (k_from + t * GT_K) : GT_K;
+#pragma unroll
+        for (int k = 0; k < GT_K; k += 4) {
+            if (RAGGED && k >= len) break;
             float4 x[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(xs + 8 * i * GT_PITCH + k);
@@ -374,14 +377,6 @@ gemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const
                     a = fmaf(x[i].z, w.z, a); a = fmaf(x[i].w, w.w, a);
                 }
             }
-        };
-        const int len = k_to - (k_from + t * GT_K);
-        if (!RAGGED || len >= GT_K) {
-#pragma unroll
-            for (int k = 0; k < GT_K; k += 4) four(k);
-        } else {
-#pragma unroll 1
-            for (int k = 0; k < len; k += 4) four(k);
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -467,7 +462,7 @@ static int launch_any(const GsArgs& a) {
 
 // A K below this has ranges too short for a ring to fill (2048 x 256, 2,048 rows: 107 us either way;
 // x 64: 34 us with one chain, 83 with eight).  At 384 many rows of a gated pair lose up to 9 % (4,096 outputs,
-// 2,048 rows) and few rows take a seventh (three rows 46 -> 7 us).  Which kernels a weight goes to follows
+// 2,048 rows; at 400, whose ranges end inside a piece, a third) and few rows take a seventh (three rows 46 -> 7 us).  Which kernels a weight goes to follows
 // from K and the alignment alone, so that a row's sums have one order whatever the number of rows.
 constexpr int GS_MIN_K = 384;
 
