@@ -308,8 +308,24 @@ constexpr int GT_M = 64, GT_N = 128, GT_K = 16, GT_PITCH = GT_K + 4, GT_STAGES =
 constexpr int GT_STAGE = (GT_M + GT_N) * GT_PITCH;
 static_assert(GT_STAGES * GT_STAGE >= GT_M * GT_N, "the sums take the ring's place");
 
+__device__ __forceinline__ void gt_four(float (&acc)[8][8], const float* xs, const float* ws, int k) {
+    float4 x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(xs + 8 * i * GT_PITCH + k);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float4 w = *reinterpret_cast<const float4*>(ws + 16 * j * GT_PITCH + k);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float& a = acc[i][j];
+            a = fmaf(x[i].x, w.x, a); a = fmaf(x[i].y, w.y, a);
+            a = fmaf(x[i].z, w.z, a); a = fmaf(x[i].w, w.w, a);
+        }
+    }
+}
+
 // RAGGED: ranges that no piece divides, whose last piece stops at the range's end instead of multiplying zeros
-// (K = 400 in ranges of 52: 8 to 10 % less; the tests cost the other ranges 2 to 5 %).
+// (K = 400 in ranges of 52: 8 to 10 % less; the second loop costs the other ranges 2 to 5 %).
 template <bool GATED, bool RAGGED>
 __global__ void __launch_bounds__(GT_THREADS)
 gemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ W2,
@@ -360,23 +376,13 @@ gemm_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* xs = gs_smem + (t % GT_STAGES) * GT_STAGE + tm * GT_PITCH;
         const float* ws = gs_smem + (t % GT_STAGES) * GT_STAGE + (GT_M + tn) * GT_PITCH;
-        const int len = RAGGED ? k_to - (k_from + t * GT_K) : GT_K;
+        const int len = k_to - (k_from + t * GT_K);
+        if (!RAGGED || len >= GT_K) {
 #pragma unroll
-        for (int k = 0; k < GT_K; k += 4) {
-            if (RAGGED && k >= len) break;
-            float4 x[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) x[i] = *reinterpret_cast<const float4*>(xs + 8 * i * GT_PITCH + k);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float4 w = *reinterpret_cast<const float4*>(ws + 16 * j * GT_PITCH + k);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    float& a = acc[i][j];
-                    a = fmaf(x[i].x, w.x, a); a = fmaf(x[i].y, w.y, a);
-                    a = fmaf(x[i].z, w.z, a); a = fmaf(x[i].w, w.w, a);
-                }
-            }
+            for (int k = 0; k < GT_K; k += 4) gt_four(acc, xs, ws, k);
+        } else {
+#pragma unroll 1
+            for (int k = 0; k < len; k += 4) gt_four(acc, xs, ws, k);
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
