@@ -598,3 +598,44 @@ def test_scans_find_their_pieces_in_any_batch(B):
         got.append((out, S, y, s))
     for a, b in zip(*got):
         same(b, a)
+
+
+@pytest.mark.parametrize("inner,N", [(96, 16), (66, 4), (33, 128), (20, 200)])
+@pytest.mark.parametrize("counts", [[200], [1, 500, 96, 3], [192, 191]])
+@pytest.mark.parametrize("strong", [False, True])
+def test_selective_scan_in_64_bits(inner, N, counts, strong):
+    """Both forms against the recurrence in 64 bits, states that go on from another step, a padding entry, decays near
+    one and near zero: segments no further off than whole sequences (with room for the order of the sums)."""
+    from agave_b200 import kernels
+    T, B, Np = sum(counts), len(counts), kernels.selective_pad(N)
+    slots = [b if b != 2 else -1 for b in range(B)]
+    ctx = step(counts, [0] * B, slots)
+    u, dt, z = rnd(T, inner, seed=1), rnd(T, inner, seed=2) - 1.0, rnd(T, inner, seed=3)
+    bc = torch.zeros(T, 2, Np, device=DEV)
+    bc[:, :, :N] = rnd(T, 2, N, seed=4)
+    a2 = -torch.exp(rnd(inner, N, seed=5, scale=1.0) + (2.0 if strong else -4.0))
+    bias, d, state0 = rnd(inner, seed=6), rnd(inner, seed=7), rnd(B, 3 + inner * N, seed=8)
+    step8 = torch.nn.functional.softplus((dt + bias).double(), threshold=1e9)
+    want, ends, at = torch.zeros(T, inner, dtype=torch.float64, device=DEV), state0.double(), 0
+    for b, n in enumerate(counts):
+        S = state0[b, 3:].double().view(inner, N)
+        for t in range(at, at + n):
+            S = torch.exp2(step8[t][:, None] * a2.double()) * S + (step8[t] * u[t].double())[:, None] * bc[t, 0, :N].double()
+            want[t] = S @ bc[t, 1, :N].double() + d.double() * u[t].double()
+        if slots[b] >= 0:
+            ends[b, 3:] = S.reshape(-1)
+        else:
+            want[at:at + n] = 0.0
+        at += n
+    want = want * torch.nn.functional.silu(z.double())
+    err = {}
+    for form in ("whole", "segments"):
+        state, out = state0.clone(), torch.full((T, inner), float("nan"), device=DEV)
+        kernels.selective_scan(u, dt, bias, bc.view(T, -1), a2, d, z, None, inner, 0, out, ctx, state, 3, form=form)
+        err[form] = [float((g.double() - r).norm() / r.norm()) for g, r in ((out, want), (state, ends))]
+        assert torch.equal(state[:, :3], state0[:, :3])
+        if B > 2:
+            assert torch.equal(state[2], state0[2])
+    # (2^-22 a decay by the hardware's power of two, once a token, over states of some hundred tokens)
+    for whole, cut in zip(err["whole"], err["segments"]):
+        assert cut <= 1.5 * whole + 2e-7 and cut < 5e-6, err
