@@ -13,6 +13,19 @@ constexpr unsigned WAIT_LIMIT = 1u << 22;
 static __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
+// True in one lane of a warp that is here whole.  Code behind it is known to the compiler to run
+// in a single thread, so a TMA request or a product is one instruction with uniform operands;
+// behind a test of the lane number it becomes a loop over the lanes that might be there.
+static __device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+                 : "=r"(p));
+    return p != 0;
+}
+// The warp's number, known to be the same in all its lanes.
+static __device__ __forceinline__ int warp_number() {
+    return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+}
 static __device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
