@@ -154,7 +154,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
     // [rank][token][row of this CTA's slice]: what the cluster's CTAs push here
     float* inbox = (float*)(smem + TL::STAGES * TL::STAGE_BYTES + TL::XCHG_BYTES + 1024);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * (HALF ? TILE_M / 2 : TILE_M);   // first output feature
     const int n0 = blockIdx.y * BN;              // first token
     const int kb_total = (K + TILE_K - 1) / TILE_K;
@@ -189,7 +189,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
     if (TL::PUSH && cluster_reduce)
         asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
+        if (elect_one()) {
         // ------------------------------------------------------------ loader
         // The weights never change, so the first ring of weight boxes is requested
         // before this kernel waits for its predecessor (which produces x): the
@@ -232,7 +233,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
             for (int i = first; i < issued; ++i)
                 mbar_wait(&full[i % TL::STAGES], (i / TL::STAGES) & 1);
         }
-    } else if (warp == 1 && lane == 0) {
+        }
+    } else if (warp == 1) {
+        if (elect_one()) {
         // ------------------------------------------------------------ products
         constexpr uint32_t idesc = umma_idesc(TILE_M, BN);
         bool ok = true;
@@ -261,6 +264,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
             tc_commit(&empty[s]);          // the stage is free once these products have read it
         }
         tc_commit(acc_full);               // arrives when every product above is done
+        }
     } else if (warp >= 2) {
         // ------------------------------------------------------------ epilogue
         const int quarter = warp & 3;
@@ -789,7 +793,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w,
     uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     const int m_tiles = (N + M_STEP - 1) / M_STEP, n_tiles = (T + BN - 1) / BN;
     const int tiles = m_tiles * n_tiles, items = tiles * splits;
     const int kb_total = (K + TILE_K - 1) / TILE_K;
@@ -829,7 +833,8 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w,
         n_kb = min(kb_total, kb_begin + kb_per_split) - kb_begin;
     };
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
+        if (elect_one()) {
         // ------------------------------------------------------------ loader
         int it = 0;                       // k-blocks issued so far, over all tiles
         bool waited = false;
@@ -863,7 +868,9 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w,
             const int first = it > TL::STAGES ? it - TL::STAGES : 0;
             for (int i = first; i < it; ++i) mbar_wait(&full[i % TL::STAGES], (i / TL::STAGES) & 1);
         }
-    } else if (warp == 1 && lane == 0) {
+        }
+    } else if (warp == 1) {
+        if (elect_one()) {
         // ------------------------------------------------------------ products
         constexpr uint32_t idesc = TOKM ? umma_idesc(BN, 2 * TILE_M) : umma_idesc(TILE_M, BN);
         int it = 0, li = 0;
@@ -905,6 +912,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w,
                 tc_commit(&empty[s]);
             }
             tc_commit(&acc_full[as]);
+        }
         }
     } else if (warp >= 2) {
         // ------------------------------------------------------------ epilogue
@@ -1146,7 +1154,7 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
     uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();                // 0: issues the products
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int f_tiles = (N + TILE_M - 1) / TILE_M;          // tiles of 128 features
@@ -1187,7 +1195,8 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
         n0 = (item % t_tiles) * 2 * TILE_M + (int)rank * TILE_M;     // this CTA's first token
     };
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
+        if (elect_one()) {
         // ------------------------------------------------------------ loader (both CTAs)
         int it = 0;
         bool waited = false;
@@ -1216,7 +1225,9 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
                 tma_load_2d_pair(st, &map_x, kx, n0, bar);
             }
         }
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+        }
+    } else if (warp == 1 && rank == 0) {
+        if (elect_one()) {
         // ------------------------------------------------------------ products (even CTA)
         constexpr uint32_t idesc = umma_idesc(2 * TILE_M, 2 * TILE_M);
         int it = 0, li = 0;
@@ -1249,6 +1260,7 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
             }
             if (*abort_flag) break;
             tc_commit_pair(&acc_full[as]);
+        }
         }
     } else if (warp >= 2) {
         // ------------------------------------------------------------ epilogue (both CTAs)

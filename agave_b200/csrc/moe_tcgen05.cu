@@ -80,7 +80,7 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w,
     int* s_row = s_tok + MT_N;                     // [MT_N] output row
     float* s_scale = (float*)(s_row + MT_N);       // [MT_N]
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * MT_M;              // first output feature
     const int n0 = blockIdx.y * MT_N;              // first sorted row
     const int n_kb = (K + MT_K - 1) / MT_K;
@@ -112,7 +112,8 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w,
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
+        if (elect_one()) {
         // ------------------------------------------------------------ loader
         const int wrow = e * N + m0;               // the expert's rows in the stacked matrix
         int issued = 0;
@@ -139,7 +140,9 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w,
             for (int i = first; i < issued; ++i)
                 mbar_wait(&full[i % MT_STAGES], (i / MT_STAGES) & 1);
         }
-    } else if (warp == 1 && lane == 0) {
+        }
+    } else if (warp == 1) {
+        if (elect_one()) {
         // ------------------------------------------------------------ products
         constexpr uint32_t idesc = umma_idesc(MT_M, MT_N);
         bool ok = true;
@@ -168,6 +171,7 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w,
             tc_commit(&empty[s]);          // the stage is free once these products have read it
         }
         tc_commit(acc_full);               // arrives when every product above is done
+        }
     } else if (warp >= 2) {
         // ------------------------------------------------------------ epilogue
         const int quarter = warp & 3;      // the tensor-memory lanes this warp may read
