@@ -1,0 +1,66 @@
+"""Prompt kernels at the edges of their tiles, against sums written out in torch."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def rnd(*shape, dtype=torch.float32, seed=0, scale=1.0):
+    g = torch.Generator(device="cpu").manual_seed(seed)
+    return (torch.randn(*shape, generator=g) * scale).to(dtype).to(DEV)
+
+
+def rel_err(got, ref):
+    got, ref = got.double().cpu(), ref.double().cpu()
+    return ((got - ref).abs().max() / ref.abs().max().clamp_min(1e-30)).item()
+
+
+@pytest.mark.parametrize("nh,nkv,hd,hdv,window,keep", [
+    (4, 1, 256, 256, 0, 0), (4, 1, 256, 256, 130, 0), (8, 4, 128, 128, 65, 0),
+    (3, 3, 64, 192, 0, 0), (2, 1, 192, 48, 64, 0), (16, 1, 80, 144, 70, 5), (4, 2, 128, 128, 40, 130),
+    (2, 2, 16, 16, 1, 0)])
+def test_prompt_attention_at_the_edges_of_its_tiles(nh, nkv, hd, hdv, window, keep):
+    """Lengths round half tiles of 64 keys and tiles of 128, an odd number of halves, windows that
+    start inside one, kept first keys apart from the window, value heads of their own size (one
+    and two slots a tile).  Errors: P, the values and the result are bfloat16 (2^-9 each)."""
+    from agave_b200 import kernels
+    lens = [1, 63, 64, 65, 127, 128, 129, 191, 192, 193, 256, 257, 321]
+    T = sum(lens)
+    q, k = (rnd(T, n * hd, dtype=torch.bfloat16, seed=i, scale=0.5) for i, n in enumerate((nh, nkv)))
+    v = rnd(T, nkv * hdv, dtype=torch.bfloat16, seed=3)
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    out = torch.full((T, nh * hdv), float("nan"), dtype=torch.bfloat16, device=DEV)
+    kernels.attention_prefill_tc(q, k, v, out, cu, max(lens), nh, nkv, hd, 0.3, window,
+                                 value_dim=hdv, keep_first=keep)
+    assert kernels.attention_tc_status() == 0
+    o = 0
+    for n in lens:
+        at = slice(o, o + n)
+        qs = q[at].double().reshape(n, nh, hd).transpose(0, 1)
+        ks = k[at].double().reshape(n, nkv, hd).transpose(0, 1).repeat_interleave(nh // nkv, 0)
+        vs = v[at].double().reshape(n, nkv, hdv).transpose(0, 1).repeat_interleave(nh // nkv, 0)
+        p = torch.arange(n, device=DEV)[:, None]
+        j = torch.arange(n, device=DEV)[None, :]
+        see = (j <= p) & ((j > p - window) | (j < keep) if window else j >= 0)
+        s = ((qs @ ks.transpose(1, 2)) * 0.3).masked_fill(~see, float("-inf"))
+        ref = (torch.softmax(s, -1) @ vs).transpose(0, 1).reshape(n, nh * hdv)
+        assert rel_err(out[at], ref) < 6e-3, n
+        o += n
+
+
+@pytest.mark.parametrize("T", [65, 100, 128])
+@pytest.mark.parametrize("N,K", [(6912, 1152), (100, 72), (10240, 320), (4800, 64)])
+def test_gated_product_of_short_prompts(T, N, K):
+    """One or two tiles of features a CTA, a last tile that is not full, fewer and more k-blocks
+    than stages.  The result is rounded to bfloat16 (2^-9), the gate's tanh is within 2^-11."""
+    from agave_b200 import kernels
+    x = rnd(T, K, dtype=torch.bfloat16, seed=7)
+    wg, wu = (rnd(N, K, dtype=torch.bfloat16, seed=s, scale=K ** -0.5) for s in (8, 9))
+    out = torch.full((T + 1, N + 8), float("nan"), dtype=torch.bfloat16, device=DEV)
+    kernels.linear_tc(x, wg, out[:T, :N], w2=wu, activation="gelu_tanh")
+    assert kernels.linear_tc_status() == 0
+    ref = torch.nn.functional.gelu(x.double() @ wg.double().T, approximate="tanh") * (x.double() @ wu.double().T)
+    assert rel_err(out[:T, :N], ref) < 6e-3
+    assert torch.isnan(out[T]).all() and torch.isnan(out[:, N:]).all()
