@@ -174,21 +174,19 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 
 // Sum over a block of up to 1024 threads; every thread gets the result.
-// `scratch` holds 33 floats of shared memory; safe to call repeatedly.
-__device__ __forceinline__ float block_sum(float v, float* scratch) {
+// `scratch` holds 32 floats of shared memory.  The first form is for scratch that nobody has
+// used since the last barrier; the second is safe to call repeatedly.
+__device__ __forceinline__ float block_sum_fresh(float v, float* scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nwarps = (blockDim.x + 31) >> 5;
     v = warp_sum(v);
-    __syncthreads();
     if (lane == 0) scratch[warp] = v;
     __syncthreads();
-    if (warp == 0) {
-        float t = lane < nwarps ? scratch[lane] : 0.f;
-        t = warp_sum(t);
-        if (lane == 0) scratch[32] = t;
-    }
+    return warp_sum(lane < nwarps ? scratch[lane] : 0.f);      // (by every warp for itself)
+}
+__device__ __forceinline__ float block_sum(float v, float* scratch) {
     __syncthreads();
-    return scratch[32];
+    return block_sum_fresh(v, scratch);
 }
 __device__ __forceinline__ float block_max(float v, float* scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -197,11 +195,5 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
     __syncthreads();
     if (lane == 0) scratch[warp] = v;
     __syncthreads();
-    if (warp == 0) {
-        float t = lane < nwarps ? scratch[lane] : -INFINITY;
-        t = warp_max(t);
-        if (lane == 0) scratch[32] = t;
-    }
-    __syncthreads();
-    return scratch[32];
+    return warp_max(lane < nwarps ? scratch[lane] : -INFINITY);
 }

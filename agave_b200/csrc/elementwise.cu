@@ -184,21 +184,27 @@ norm_residual_small_kernel(float* __restrict__ h, const TY* __restrict__ y, int 
     // is a slow one, and here nothing else hides it)
     asm volatile("" ::"l"(h), "l"(y), "l"(w_post), "l"(w_next), "l"(x), "l"(rows), "r"(H),
                  "r"(n_splits), "l"(split_stride), "f"(eps_post), "f"(eps_next), "r"(add_residual));
-    pdl_wait();
-    pdl_launch_next();
-    __shared__ float red[33];
-    const int r = blockIdx.x;
-    const size_t src = (size_t)(rows ? rows[r] : r) * H;
-    const size_t dst = (size_t)r * H;
+    // The weights are nobody's output: they are on their way before the wait, from HBM where a
+    // step's other weights have pushed them out of L2.
     float v[EPT], hv[EPT], wp[EPT], wn[EPT];
 #pragma unroll
     for (int k = 0; k < EPT; ++k) {
         const int i = threadIdx.x + k * blockDim.x;
         const bool in = i < H;
-        v[k] = 0.f;
-        hv[k] = (in && (add_residual || !y)) ? h[src + i] : 0.f;
         wp[k] = (in && w_post) ? w_post[i] : 1.f;
         wn[k] = (in && w_next) ? w_next[i] : 1.f;
+    }
+    pdl_wait();
+    pdl_launch_next();
+    __shared__ float red[2][32];
+    const int r = blockIdx.x;
+    const size_t src = (size_t)(rows ? rows[r] : r) * H;
+    const size_t dst = (size_t)r * H;
+#pragma unroll
+    for (int k = 0; k < EPT; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        v[k] = 0.f;
+        hv[k] = (i < H && (add_residual || !y)) ? h[src + i] : 0.f;
     }
     if (y) {
         constexpr int U = EPT <= 2 ? 16 : (EPT <= 4 ? 8 : (EPT <= 8 ? 4 : (EPT <= 16 ? 2 : 1)));
@@ -231,7 +237,7 @@ norm_residual_small_kernel(float* __restrict__ h, const TY* __restrict__ y, int 
             float ss = 0.f;
 #pragma unroll
             for (int k = 0; k < EPT; ++k) ss += v[k] * v[k];
-            ss = block_sum(ss, red);
+            ss = block_sum_fresh(ss, red[0]);
             const float rs = 1.0f / sqrtf(ss / (float)H + eps_post);
 #pragma unroll
             for (int k = 0; k < EPT; ++k) v[k] = v[k] * rs * wp[k];
@@ -252,7 +258,7 @@ norm_residual_small_kernel(float* __restrict__ h, const TY* __restrict__ y, int 
         float ss = 0.f;
 #pragma unroll
         for (int k = 0; k < EPT; ++k) ss += v[k] * v[k];      // lanes beyond H hold 0
-        ss = block_sum(ss, red);
+        ss = block_sum_fresh(ss, red[1]);
         const float r2 = 1.0f / sqrtf(ss / (float)H + eps_next);
 #pragma unroll
         for (int k = 0; k < EPT; ++k) {
@@ -380,12 +386,26 @@ norm_residual_row_kernel(float* __restrict__ h, const float* __restrict__ y, int
                           size_t split_stride, const float* __restrict__ w_post,
                           const float* __restrict__ w_next, TX* __restrict__ x, int R, int H,
                           float eps_post, float eps_next, int add_residual) {
-    pdl_wait();
-    pdl_launch_next();
-    __shared__ float red[33];
+    __shared__ float red[2][32];
     const int lane = threadIdx.x, n = TH ? TH : blockDim.x;         // n threads share the row
     const int row = blockIdx.x;
     const int H4 = H >> 2;
+    // few rows: the weights are on their way before the wait (many rows find them in L1, and are
+    // better off with the registers)
+    constexpr bool EARLY = TH != 0 && NV <= 3;
+    float4 wp[EARLY ? NV : 1], wn[EARLY ? NV : 1];
+    auto weight = [&](const float* w, int idx) {
+        return w && idx < H4 ? reinterpret_cast<const float4*>(w)[idx] : make_float4(1.f, 1.f, 1.f, 1.f);
+    };
+    if constexpr (EARLY) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            wp[i] = weight(w_post, lane + n * i);
+            wn[i] = weight(w_next, lane + n * i);
+        }
+    }
+    pdl_wait();
+    pdl_launch_next();
     const size_t base = (size_t)row * H;
     float4 v[NV], hv[NV];
 #pragma unroll
@@ -427,7 +447,7 @@ norm_residual_row_kernel(float* __restrict__ h, const float* __restrict__ y, int
 #pragma unroll
         for (int i = 0; i < NV; ++i)
             ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
-        ss = block_sum(ss, red);
+        ss = block_sum_fresh(ss, red[0]);
         rs = 1.0f / sqrtf(ss / (float)H + eps_post);
     }
     float ss2 = 0.f;
@@ -436,7 +456,7 @@ norm_residual_row_kernel(float* __restrict__ h, const float* __restrict__ y, int
         const int idx = lane + n * i;
         if (idx < H4) {
             if (w_post) {
-                const float4 w = reinterpret_cast<const float4*>(w_post)[idx];
+                const float4 w = EARLY ? wp[EARLY ? i : 0] : reinterpret_cast<const float4*>(w_post)[idx];
                 v[i].x = v[i].x * rs * w.x; v[i].y = v[i].y * rs * w.y;
                 v[i].z = v[i].z * rs * w.z; v[i].w = v[i].w * rs * w.w;
             }
@@ -448,13 +468,13 @@ norm_residual_row_kernel(float* __restrict__ h, const float* __restrict__ y, int
         }
     }
     if (w_next) {
-        ss2 = block_sum(ss2, red);
+        ss2 = block_sum_fresh(ss2, red[1]);
         const float r2 = 1.0f / sqrtf(ss2 / (float)H + eps_next);
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int idx = lane + n * i;
             if (idx < H4) {
-                const float4 w = reinterpret_cast<const float4*>(w_next)[idx];
+                const float4 w = EARLY ? wn[EARLY ? i : 0] : reinterpret_cast<const float4*>(w_next)[idx];
                 Pack4<TX>::store(x + base + 4 * idx,
                                  make_float4(v[i].x * r2 * w.x, v[i].y * r2 * w.y,
                                              v[i].z * r2 * w.z, v[i].w * r2 * w.w));
