@@ -132,6 +132,19 @@ template <> __device__ __forceinline__ void store_out<__nv_bfloat16>(__nv_bfloat
     *p = __float2bfloat16_rn(v);
 }
 
+// four values in one store
+template <typename TO> struct Pack4To;
+template <> struct Pack4To<float> {
+    __device__ static void store(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+};
+template <> struct Pack4To<__nv_bfloat16> {
+    __device__ static void store(__nv_bfloat16* p, const float4& v) {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+        *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a),
+                                                  *reinterpret_cast<const uint32_t*>(&b));
+    }
+};
+
 template <int BN, int MODE, typename TO, int SLIM = 0, bool BOUNDED = false>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
@@ -1366,6 +1379,238 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
     }
 }
 
+// The plain product on CTA pairs: a tile is 256 tokens (the M operand, 128 a CTA) by BN weight
+// rows (the N operand, half of them in each CTA's shared memory), so that a CTA fetches
+// 128 + BN / 2 rows a k-block for a share of 128 x BN of the products, where one CTA alone fetches
+// 128 + BN.  Accumulator lanes are tokens, columns features: a warp's 32 x 32 values go through
+// its own staging, so that a row leaves in a line of 128 bytes.  Roles, barriers and K in `splits`
+// ranges as in the forms above.
+template <int BN>
+struct PairTile {
+    static constexpr int A_BYTES = TILE_M * TILE_K * 2;
+    static constexpr int STAGE_BYTES = A_BYTES + BN / 2 * TILE_K * 2;
+    static constexpr int STAGES = BN == 128 ? 8 : 6;
+    static constexpr int EPI_BYTES = PERSISTENT_EPI_WARPS * 32 * 32 * 4;
+    static constexpr int SMEM = STAGES * STAGE_BYTES + EPI_BYTES + 1024 + 256;
+    static_assert(SMEM <= 227 * 1024, "stages and staging must fit shared memory");
+};
+
+template <int BN, typename TO>
+__global__ void __launch_bounds__(PERSISTENT_THREADS, 1)
+gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w,
+                         const __grid_constant__ CUtensorMap map_x, TO* __restrict__ out, int T, int N,
+                         int K, long long ldc, long long split_stride, int splits, int kb_per_split,
+                         int act) {
+    pdl_launch_next();
+    using TL = PairTile<BN>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* epi = smem + TL::STAGES * TL::STAGE_BYTES;
+    uint64_t* full = (uint64_t*)(epi + TL::EPI_BYTES);      // used in the even CTA
+    uint64_t* empty = full + TL::STAGES;                    // one set per CTA
+    uint64_t* acc_full = empty + TL::STAGES;                // [2], one set per CTA
+    uint64_t* acc_empty = acc_full + 2;                     // [2], used in the even CTA
+    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+
+    const int warp = warp_number(), lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();                // 0: issues the products
+    const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    const int t_tiles = (T + 2 * TILE_M - 1) / (2 * TILE_M);
+    const int tiles = (N + BN - 1) / BN * t_tiles, items = tiles * splits;
+    const int kb_total = (K + TILE_K - 1) / TILE_K;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < TL::STAGES; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], 2 * PERSISTENT_EPI_WARPS);   // the epilogue warps of both CTAs
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(tmem_slot)),
+                     "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();          // the partner's barriers exist before anything is sent to them
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    // item -> (range of K, feature tile, token tile); token tiles vary fastest so that the pairs
+    // of a wave share weight tiles in L2
+    auto decode_item = [&](int item, int& m0, int& n0, int& kb_begin, int& n_kb, int& split) {
+        split = item / tiles;
+        const int t = item - split * tiles;
+        m0 = t / t_tiles * BN;
+        n0 = t % t_tiles * 2 * TILE_M + (int)rank * TILE_M;      // this CTA's first token
+        kb_begin = split * kb_per_split;
+        n_kb = min(kb_total, kb_begin + kb_per_split) - kb_begin;
+    };
+
+    if (warp == 0) {
+        if (elect_one()) {
+        // ------------------------------------------------------------ loader (both CTAs)
+        int s = 0;
+        uint32_t ph = 1;
+        bool waited = false;
+        for (int item = pair; item < items && !*abort_flag; item += n_pairs) {
+            int m0, n0, kb_begin, n_kb, split;
+            decode_item(item, m0, n0, kb_begin, n_kb, split);
+            for (int i = 0; i < n_kb; ++i) {
+                if (!mbar_wait(&empty[s], ph)) {
+                    atomicCAS(&g_gemm_status, 0, (5 << 8) | s);
+                    *abort_flag = 1;
+                    break;
+                }
+                uint8_t* st = smem + s * TL::STAGE_BYTES;
+                const uint32_t bar = mapa_u32(smem_u32(&full[s]), 0);
+                if (rank == 0) mbar_expect_tx(&full[s], 2 * TL::STAGE_BYTES);   // both CTAs' bytes
+                const int kx = (kb_begin + i) * TILE_K;
+                // the weights never change: their box is requested before the predecessor
+                // (which produces x) is known to have finished
+                tma_load_2d_pair(st + TL::A_BYTES, &map_w, kx, m0 + (int)rank * (BN / 2), bar);
+                if (!waited) {
+                    pdl_wait();
+                    waited = true;
+                }
+                tma_load_2d_pair(st, &map_x, kx, n0, bar);
+                if (++s == TL::STAGES) s = 0, ph ^= 1;
+            }
+        }
+        }
+    } else if (warp == 1 && rank == 0) {
+        if (elect_one()) {
+        // ------------------------------------------------------------ products (even CTA)
+        constexpr uint32_t idesc = umma_idesc(2 * TILE_M, BN);
+        int s = 0, li = 0;
+        uint32_t ph = 0;
+        for (int item = pair; item < items && !*abort_flag; item += n_pairs, ++li) {
+            int m0, n0, kb_begin, n_kb, split;
+            decode_item(item, m0, n0, kb_begin, n_kb, split);
+            const int as = li & 1;
+            if (!mbar_wait(&acc_empty[as], ((li >> 1) & 1) ^ 1)) {
+                atomicCAS(&g_gemm_status, 0, (6 << 8) | as);
+                *abort_flag = 1;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + as * BN;
+            for (int i = 0; i < n_kb; ++i) {
+                if (!mbar_wait(&full[s], ph)) {
+                    atomicCAS(&g_gemm_status, 0, (7 << 8) | s);
+                    *abort_flag = 1;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t a_addr = smem_u32(smem + s * TL::STAGE_BYTES);       // tokens
+                const uint32_t b_addr = a_addr + TL::A_BYTES;                       // weight rows
+#pragma unroll
+                for (int k = 0; k < TILE_K / UMMA_K; ++k)
+                    tc_mma_bf16_pair(d_tmem, umma_desc(a_addr + k * UMMA_K * 2),
+                                     umma_desc(b_addr + k * UMMA_K * 2), idesc,
+                                     (i > 0 || k > 0) ? 1u : 0u);
+                tc_commit_pair(&empty[s]);
+                if (++s == TL::STAGES) s = 0, ph ^= 1;
+            }
+            if (*abort_flag) break;
+            tc_commit_pair(&acc_full[as]);
+        }
+        }
+    } else if (warp >= 2) {
+        // ------------------------------------------------------------ epilogue (both CTAs)
+        // two warps share each quarter of the lanes, half of the columns each
+        pdl_wait();
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const uint32_t acc_empty_leader0 = mapa_u32(smem_u32(&acc_empty[0]), 0);
+        const uint32_t acc_empty_leader1 = mapa_u32(smem_u32(&acc_empty[1]), 0);
+        float4* st = reinterpret_cast<float4*>(epi) + (warp - 2) * (32 * 8);     // [32 rows][8 pieces]
+        // (pieces are swizzled by the row: no bank conflicts on either side)
+        const bool aligned = ldc % 4 == 0 && ((uintptr_t)out & 15) == 0;
+        int li = 0;
+        for (int item = pair; item < items; item += n_pairs, ++li) {
+            int m0, n0, kb_begin, n_kb, split;
+            decode_item(item, m0, n0, kb_begin, n_kb, split);
+            const int as = li & 1;
+            const bool ok = !*abort_flag && mbar_wait(&acc_full[as], (li >> 1) & 1);
+            if (!ok) {
+                if (!*abort_flag) atomicCAS(&g_gemm_status, 0, (8 << 8) | as);
+                *abort_flag = 1;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t lane_base = tmem_base + as * BN + half * (BN / 2) + ((uint32_t)(quarter * 32) << 16);
+            const int tok = n0 + quarter * 32, f0 = m0 + half * (BN / 2);
+            TO* obase = out + (size_t)split * split_stride + (size_t)tok * ldc + f0;
+            uint32_t a[16], b[16];
+            tc_ld16(lane_base, a);
+            tc_ld16(lane_base + 16, b);
+#pragma unroll 1
+            for (int c = 0; c < BN / 2; c += 32) {
+                tc_wait_ld();
+                if (act >= 2) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        a[j] = __float_as_uint(plain_act(__uint_as_float(a[j]), act));
+                        b[j] = __float_as_uint(plain_act(__uint_as_float(b[j]), act));
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    reinterpret_cast<uint4*>(st)[lane * 8 + (j ^ (lane & 7))] =
+                        make_uint4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
+                    reinterpret_cast<uint4*>(st)[lane * 8 + ((j + 4) ^ (lane & 7))] =
+                        make_uint4(b[4 * j], b[4 * j + 1], b[4 * j + 2], b[4 * j + 3]);
+                }
+                __syncwarp();
+                if (c + 32 < BN / 2) {
+                    tc_ld16(lane_base + c + 32, a);
+                    tc_ld16(lane_base + c + 48, b);
+                } else {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(as ? acc_empty_leader1 : acc_empty_leader0);
+                }
+                const int piece = lane & 7, f = f0 + c + piece * 4;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int row = q * 4 + (lane >> 3);
+                    const float4 v = st[row * 8 + (piece ^ (row & 7))];
+                    if (tok + row >= T) continue;
+                    TO* p = obase + (size_t)row * ldc + c + piece * 4;
+                    if (aligned && f + 4 <= N) {
+                        Pack4To<TO>::store(p, v);
+                    } else {
+                        const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (f + j < N) store_out<TO>(p + j, e[j]);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
+    // (as in the gated form above)
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();          // the partner has no product, commit or arrival left for us
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
+                     "r"(512u)
+                     : "memory");
+    }
+}
+
 int device_sms() {
     static const int sms = [] {
         int dev = 0, n = 0;
@@ -1480,6 +1725,29 @@ int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mw2, const CUten
     return 0;
 }
 
+template <int BN, typename TO>
+int launch_pair(const void* w, const CUtensorMap& mx, void* out, int T, int N, int K, long long ldc,
+                long long split_stride, int splits, int kb_per_split, int act, cudaStream_t stream) {
+    CUtensorMap mw;
+    if (int rc = make_map(&mw, w, N, K, K, BN / 2)) return rc;
+    auto kern = gemm_tcgen05_pair_kernel<BN, TO>;
+    static bool configured = false;
+    if (!configured) {
+        AGV_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         PairTile<BN>::SMEM));
+        configured = true;
+    }
+    const long long items =
+        (long long)((N + BN - 1) / BN) * ((T + 2 * TILE_M - 1) / (2 * TILE_M)) * splits;
+    long long pairs = device_sms() / 2;
+    if (items < pairs) pairs = items;
+    agv_launch_cluster(kern, dim3((unsigned)(2 * pairs)), PERSISTENT_THREADS, PairTile<BN>::SMEM, stream,
+                       dim3(2, 1, 1), mw, mx, (TO*)out, T, N, K, ldc, split_stride, splits, kb_per_split,
+                       act);
+    AGV_LAUNCH_OK("gemm_tcgen05_pair_kernel");
+    return 0;
+}
+
 template <bool BOUNDED>
 int launch_pair_gated(const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensorMap& mx,
                       void* out, int T, int N, int K, long long ldc, GateAct act, cudaStream_t stream) {
@@ -1502,6 +1770,40 @@ int launch_pair_gated(const CUtensorMap& mw, const CUtensorMap& mw2, const CUten
                        dim3(2, 1, 1), mw, mw2, mx, (__nv_bfloat16*)out, T, N, K, ldc, act);
     AGV_LAUNCH_OK("gemm_tcgen05_pair_gated_kernel");
     return 0;
+}
+
+// How a prompt's plain product is tiled: the form that needs the least time.  A k-block takes
+// `alone` cycles a round of the SMs (or pairs of them) when few of them are busy, and `each` and
+// `full` times their share when all are (they share L2, and the clock goes down with the power); a
+// pair takes 1,300 more to start.  One CTA: 128 weight rows by `tile` tokens.  A pair: 256 tokens by
+// `tile` weight rows, each CTA with half of these.  Fitted to shapes of 256 to 18,432 tokens, 1,152 to
+// 8,192 outputs and a K of 1,024 to 21,504 (56), of which 50 get the fastest form or one within 3 % of it,
+// the others within 7 %.  us, the best form of one CTA and of a pair: 8,696 x 1,152 x 6,912 122 and 111, 18,432
+// tokens 281 and 253, 2,048 29.5 and 27.0; 6,400 x 5,376 x 21,504 1,152 and 1,057; 4,001 x 2,560 x
+// 10,240 160 and 168.  Returns the tile and, in *cycles, the estimate.
+int prompt_plan(int T, int N, int kb, int splits, bool f32, bool* pair, long long* cycles = nullptr) {
+    struct Form { int tile; bool two; int alone, each, full; };
+    static const Form forms[] = {{256, true, 592, 400, 390},  {192, true, 448, 100, 580},
+                                 {128, true, 332, 200, 260},  {256, false, 622, 480, 390},
+                                 {192, false, 457, 160, 540}, {128, false, 385, 250, 260}};
+    static const bool pairs = getenv("AGAVE_B200_CTA_PAIRS") == nullptr ||
+                              getenv("AGAVE_B200_CTA_PAIRS")[0] != '0';
+    const int kb_per = (kb + splits - 1) / splits;
+    long long best = -1;
+    int bn = 256;
+    *pair = false;
+    for (const Form& f : forms) {
+        if (f.two ? !pairs : !f32 && f.tile != 256) continue;
+        const int units = f.two ? device_sms() / 2 : device_sms();
+        const int m = f.two ? f.tile : TILE_M, n = f.two ? 2 * TILE_M : f.tile;
+        const long long items = (long long)((N + m - 1) / m) * ((T + n - 1) / n) * splits;
+        const long long rounds = (items + units - 1) / units;
+        const long long alone = rounds * f.alone, busy = rounds * f.each + items * f.full / units;
+        const long long cost = kb_per * (alone > busy ? alone : busy) + (f.two ? 1300 : 0);
+        if (best < 0 || cost < best) best = cost, bn = f.tile, *pair = f.two;
+    }
+    if (cycles) *cycles = best;
+    return bn;
 }
 
 template <int MODE, typename TO>
@@ -1599,31 +1901,13 @@ AGV_API int agv_linear_tc(const void* x, const void* w, const void* w2, void* ou
     } else {
         mw2 = mw;
     }
+    bool pair = false;
     const bool persistent = T > 128 && !cluster && token_tile == 0 && getenv("AGV_GEMM_ONESHOT") == nullptr;
     if (persistent) {
         bn = w2 ? 128 : 256;
-        if (!w2 && out_dtype == AGV_F32) {
-            // the token tile that needs the least time: rounds of the SMs times the time
-            // of a k-block, which is the slower of its four products (2 cycles per token
-            // column, at least 256) and its bytes from L2 at the 69 B/clk an SM gets
-            // while all SMs ask (measured)
-            int sms = 148;
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-            const long long m_tiles = (N + TILE_M - 1) / TILE_M;
-            long long best = -1;
-            for (int cand : {256, 192, 128}) {
-                const long long items = m_tiles * ((T + cand - 1) / cand) * splits;
-                const long long products = cand * 2 < 256 ? 256 : cand * 2;
-                const long long feed = (long long)(TILE_M + cand) * TILE_K * 2 / 69;
-                const long long cost = ((items + sms - 1) / sms) * (products > feed ? products : feed);
-                if (best < 0 || cost < best) {
-                    best = cost;
-                    bn = cand;
-                }
-            }
-        }
+        if (!w2) bn = prompt_plan(T, N, kb_total, splits, out_dtype == AGV_F32, &pair);
     }
-    if (int rc = make_map(&mx, x, T, K, lda, bn)) return rc;
+    if (int rc = make_map(&mx, x, T, K, lda, pair ? TILE_M : bn)) return rc;
     const long long split_stride = (long long)T * ldc;
     const int creduce = splits > 1 ? cluster : 0;
     if (persistent) {
@@ -1637,6 +1921,20 @@ AGV_API int agv_linear_tc(const void* x, const void* w, const void* w2, void* ou
                            : launch_pair_gated<false>(mw, mw2, mx, out, T, N, K, ldc, act, stream);
             return launch_persistent<128, 1, __nv_bfloat16>(mw, mw2, mx, out, T, N, K, ldc, 0, 1,
                                                             kb_total, act, stream);
+        }
+        if (pair) {
+#define AGV_PAIR_CASE(B, TO)                                                                     \
+    if (bn == B)                                                                                 \
+        return launch_pair<B, TO>(w, mx, out, T, N, K, ldc, split_stride, splits, kb_per, act_kind, stream)
+            if (out_dtype == AGV_BF16) {
+                AGV_PAIR_CASE(256, __nv_bfloat16);
+                AGV_PAIR_CASE(192, __nv_bfloat16);
+                AGV_PAIR_CASE(128, __nv_bfloat16);
+            }
+            AGV_PAIR_CASE(256, float);
+            AGV_PAIR_CASE(192, float);
+            AGV_PAIR_CASE(128, float);
+#undef AGV_PAIR_CASE
         }
         if (out_dtype == AGV_BF16)
             return launch_persistent<256, 0, __nv_bfloat16>(mw, mw2, mx, out, T, N, K, ldc, 0, 1,
@@ -1774,6 +2072,18 @@ AGV_API int agv_linear_tc_splits(int K, int splits) {
     if (splits < 1) splits = 1;
     const int kb_per = (kb_total + splits - 1) / splits;
     return (kb_total + kb_per - 1) / kb_per;
+}
+
+// Into how many ranges of K (1 or 2) a prompt of more than 512 tokens is cut: two where the time they
+// save is more than the second partial sum's way out and back costs.
+AGV_API int agv_linear_tc_prompt_splits(int T, int N, int K) {
+    const int kb = (K + TILE_K - 1) / TILE_K;
+    if (kb < 32) return 1;
+    bool pair;
+    long long one, two;
+    prompt_plan(T, N, kb, 1, true, &pair, &one);
+    prompt_plan(T, N, kb, 2, true, &pair, &two);
+    return two + (long long)T * N * 8 / 3400 < one ? 2 : 1;         // (bytes at 3,400 a clock)
 }
 
 // Reads and clears the status word of the tensor-core kernels: 0, or

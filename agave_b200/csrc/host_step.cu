@@ -37,6 +37,7 @@ int agv_linear_simt(const void*, const void*, const void*, void*, int, int, int,
 int agv_linear_tc(const void*, const void*, const void*, void*, int, int, int, long long, long long,
                   int, int, float, float, int, int, int, cudaStream_t);
 int agv_linear_tc_splits(int, int);
+int agv_linear_tc_prompt_splits(int, int, int);
 int agv_gemv_few_supported(int, int, int, long long, int);
 int agv_gemv_few(const void*, const void*, int, int, int, const void*, long long, const float*, float*,
                  const float*, const float*, const float*, float, float, void*, long long, int,
@@ -177,7 +178,7 @@ struct Run {
 
     // (groups, cluster size) of the ranges K is cut into: about one CTA per SM when the
     // weight has few row tiles; the CTAs of a cluster add in the kernel, the groups are left
-    // to the consumer; prompts are cut in two only over a long K with few tiles
+    // to the consumer; prompts are cut in two only where that pays
     void plan_splits(int T, int N, int K, bool cheap, int* groups, int* csize) const {
         *groups = 1;
         *csize = 0;
@@ -195,7 +196,7 @@ struct Run {
                 if (want >= 2) *groups = agv_linear_tc_splits(K, (int)want);
                 return;
             }
-            if (ctas <= sms / 2 + 6 && kb >= 32) *groups = 2;
+            *groups = agv_linear_tc_prompt_splits(T, N, K);
             return;
         }
         const int tile = T <= 16 ? 16 : T <= 32 ? 32 : 64;

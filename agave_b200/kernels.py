@@ -1562,11 +1562,9 @@ def plan_splits(T: int, N: int, K: int, cheap_sum: bool = False):
             most = 16 if T <= 128 else 8 if T <= 256 else 4
             want = min(kb // 2, n_sms() // ctas, most)
             return (linear_tc_splits(K, want), 0) if want >= 2 else (1, 0)
-        # long prompts: only a long K over few tiles is cut, in two, with the partial
-        # sums left to the consumer (a cluster's exchange is slow for wide tiles)
-        if ctas <= n_sms() // 2 + 6 and kb >= 32:
-            return 2, 0
-        return 1, 0
+        # long prompts: cut in two where that pays, with the partial sums left to the
+        # consumer (a cluster's exchange is slow for wide tiles)
+        return library().agv_linear_tc_prompt_splits(T, N, K), 0
     tile = 16 if T <= 16 else 32 if T <= 32 else 64
     ctas = ((N + 127) // 128) * ((T + tile - 1) // tile)
     kb = (K + 63) // 64

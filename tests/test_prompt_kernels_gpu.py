@@ -64,3 +64,30 @@ def test_gated_product_of_short_prompts(T, N, K):
     ref = torch.nn.functional.gelu(x.double() @ wg.double().T, approximate="tanh") * (x.double() @ wu.double().T)
     assert rel_err(out[:T, :N], ref) < 6e-3
     assert torch.isnan(out[T]).all() and torch.isnan(out[:, N:]).all()
+
+
+@pytest.mark.parametrize("T,N,K,splits,act", [
+    (129, 130, 8192, 1, None), (300, 1150, 1096, 1, "relu2"), (2051, 2300, 2056, 1, "gelu_erf"),
+    (3000, 1541, 4104, 1, None), (5000, 4100, 1032, 1, "relu2"), (4100, 1000, 1160, 2, None)])
+def test_products_of_prompts_on_pairs_of_ctas(T, N, K, splits, act):
+    """Tiles of 256, 192 and 128 features a pair: tokens and features that end inside a tile, rows
+    whose stride is no multiple of four values, one and many rounds, K in two ranges and with a
+    ragged end.  32-bit sums of bfloat16 products: errors of a sum of K terms in 32 bits."""
+    from agave_b200 import kernels
+    x = rnd(T, K, dtype=torch.bfloat16, seed=1)
+    w = rnd(N, K, dtype=torch.bfloat16, seed=2, scale=K ** -0.5)
+    ref = x.double() @ w.double().T
+    for ld in (N + (-N) % 4, N + (-N) % 4 + 3):
+        if splits > 1 and ld != N:
+            continue
+        out = torch.full((splits, T, ld) if splits > 1 else (T + 1, ld), float("nan"), device=DEV)
+        kernels.linear_tc(x, w, out if splits > 1 else out[:T, :N], splits=splits)
+        assert kernels.linear_tc_status() == 0
+        assert rel_err(out.double().sum(0) if splits > 1 else out[:T, :N], ref) < 1e-5
+        assert splits > 1 or (torch.isnan(out[T]).all() and torch.isnan(out[:, N:]).all())
+    if act:
+        ob = torch.full((T, N + 4 + (-N) % 4), float("nan"), dtype=torch.bfloat16, device=DEV)
+        kernels.linear_activated(x, w, ob[:, :N], act)
+        assert kernels.linear_tc_status() == 0
+        want = torch.relu(ref) ** 2 if act == "relu2" else torch.nn.functional.gelu(ref)
+        assert rel_err(ob[:, :N], want) < 6e-3 and torch.isnan(ob[:, N:]).all()
