@@ -118,7 +118,12 @@ constexpr int GS_K = 32;                       // k of a piece
 constexpr int GS_PITCH = GS_K + 4;             // of a weight row in shared memory (no bank conflict)
 constexpr int GS_WARPS = 2;
 
-__host__ __device__ constexpr int gs_stages(int mats, int bm) { return mats * bm >= 64 ? 3 : 4; }
+// One range a warp (R = 1) is for weights with few warps (288 for 1152 x 6912): those keep eight pieces
+// under way, four are too few bytes for the SMs' trips to HBM (replay of three sequences, 13 layers of
+// the 1B sizes, 12.7 -> 11.7 ms).
+__host__ __device__ constexpr int gs_stages(int mats, int bm, int r) {
+    return mats * bm >= 64 ? 3 : r == 1 && mats * bm <= 16 ? 8 : 4;
+}
 __host__ __device__ constexpr int gs_stage_floats(int mats, int bm) {
     return mats * GS_ROWS * GS_PITCH + bm * GS_K;
 }
@@ -144,7 +149,7 @@ __global__ void __launch_bounds__(GS_WARPS * 32)
 gemm_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ W2,
                  float* __restrict__ C, int M, int N, int K, long long lda, long long ldc, GateAct act,
                  int m_tiles, int range) {
-    constexpr int MATS = GATED ? 2 : 1, STAGES = gs_stages(MATS, BM), CL = 4 / R;
+    constexpr int MATS = GATED ? 2 : 1, STAGES = gs_stages(MATS, BM, R), CL = 4 / R;
     constexpr int STAGE = gs_stage_floats(MATS, BM), PARTS = 8 / R;
     extern __shared__ __align__(16) float gs_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -427,7 +432,7 @@ static int launch_f32(const GsArgs& a) {
     constexpr int MATS = GATED ? 2 : 1, CL = TILE ? 8 : 4 / R;
     constexpr int WIDE = TILE ? GT_N / MATS : GS_ROWS;
     constexpr size_t smem = sizeof(float) * (TILE ? GT_STAGES * GT_STAGE
-                                                  : GS_WARPS * gs_stages(MATS, BM) * gs_stage_floats(MATS, BM));
+                                                  : GS_WARPS * gs_stages(MATS, BM, R) * gs_stage_floats(MATS, BM));
     const long long m_tiles = (a.M + BM - 1) / BM, n_tiles = (a.N + WIDE - 1) / WIDE;
     AGV_REQUIRE(m_tiles * n_tiles * CL <= 0x7fffffffLL, "linear: M=%d N=%d exceed the grid limit", a.M, a.N);
     const int range = ((a.K + 7) / 8 + 3) / 4 * 4;
