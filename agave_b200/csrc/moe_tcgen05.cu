@@ -36,12 +36,14 @@ __device__ int g_moe_status = 0;   // 0 ok; else (role << 8) | stage of the firs
 template <bool GATED, int MT_N>
 struct MTile {
     // The plain form (the down product: a short K, a large 32-bit tile to write) keeps its
-    // ring small enough for two CTAs to share an SM, so that one's epilogue runs under the
-    // other's products; the gated form has a long K and takes the SM alone.
+    // ring small enough for two or three CTAs to share an SM, so that one's epilogue runs under the
+    // others' products (three with tiles of 64 rows, where a decode step's CTAs are many and short: 21
+    // experts x 2,048 features are 336 of them); the gated form has a long K and takes the SM alone.
     static constexpr int STAGES = GATED ? (MT_N == 128 ? 2 : 4) : 3;
     static constexpr int A_BYTES = MT_M * MT_K * 2;
     static constexpr int B_BYTES = MT_N * MT_K * 2;
     static constexpr int STAGE_BYTES = A_BYTES * (GATED ? 2 : 1) + B_BYTES;
+    static constexpr int PER_SM = GATED ? (MT_N == 128 ? 2 : 1) : (MT_N == 128 ? 2 : 3);
     static constexpr int TMEM_COLS = GATED ? 2 * MT_N : MT_N;
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 2048 /*barriers, rows*/;
 };
@@ -56,7 +58,7 @@ __device__ __forceinline__ float mt_act(float g, float u, const GateAct& act) {
 }
 
 template <bool GATED, int MT_N>
-__global__ void __launch_bounds__(MT_THREADS, (GATED && MT_N != 128) ? 1 : 2)
+__global__ void __launch_bounds__(MT_THREADS, MTile<GATED, MT_N>::PER_SM)
 moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w,
                       const __grid_constant__ CUtensorMap map_w2,
                       const __grid_constant__ CUtensorMap map_a, void* __restrict__ out,
@@ -64,9 +66,6 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w,
                       const float* __restrict__ c_scale, const int* __restrict__ tile_e, int N,
                       int K, GateAct act) {
     pdl_launch_next();
-    pdl_wait();                                    // the plan is the work of kernels before
-    const int e = tile_e[blockIdx.y];
-    if (e < 0) return;
     using TL = MTile<GATED, MT_N>;
     constexpr int MT_STAGES = TL::STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -94,12 +93,6 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w,
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (threadIdx.x >= 64 && threadIdx.x < 64 + MT_N) {
-        const int i = threadIdx.x - 64, pos = n0 + i;
-        s_tok[i] = tok[pos];
-        s_row[i] = c_index ? c_index[pos] : pos;
-        s_scale[i] = c_scale ? c_scale[pos] : 1.f;
-    }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(tmem_slot)),
@@ -107,12 +100,23 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w,
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    // (barriers and tensor memory are ready; the plan is the work of kernels before)
+    pdl_wait();
+    const int e = tile_e[blockIdx.y];
+    if (e >= 0 && threadIdx.x >= 64 && threadIdx.x < 64 + MT_N) {
+        const int i = threadIdx.x - 64, pos = n0 + i;
+        s_tok[i] = tok[pos];
+        s_row[i] = c_index ? c_index[pos] : pos;
+        s_scale[i] = c_scale ? c_scale[pos] : 1.f;
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0) {
+    if (e < 0) {
+        // a tile beyond the plan's last
+    } else if (warp == 0) {
         if (elect_one()) {
         // ------------------------------------------------------------ loader
         const int wrow = e * N + m0;               // the expert's rows in the stacked matrix
@@ -271,22 +275,21 @@ int mt_map(CUtensorMap* out, const void* ptr, long long rows, long long K, long 
     return 0;
 }
 
-// xs[pos, :] = x[tok[pos], :] for the live rows of a plan, zeros for its padding.
+// xs[pos_of[p], :] = x[p / top, :] for the pairs of a plan; the plan's padding is left as it is (a
+// product's rows do not meet, and those of padding are dropped).  With zeros there, 8 tokens of 4
+// experts among 32 wrote 8.5 MB a layer for the 0.13 that count.
 __global__ void __launch_bounds__(256)
 moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
-                       const int* __restrict__ tok, __nv_bfloat16* __restrict__ xs, int rows,
-                       int H) {
+                       const int* __restrict__ pos_of, __nv_bfloat16* __restrict__ xs, int pairs,
+                       int top, int H) {
     pdl_wait();
     pdl_launch_next();
-    const int per_row = H / 8;                         // 16-byte pieces of a row
-    const long long total = (long long)rows * per_row;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int pos = (int)(i / per_row), c = (int)(i % per_row);
-        const int t = tok[pos];
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (t >= 0) v = *reinterpret_cast<const uint4*>(x + (size_t)t * ldx + c * 8);
-        *reinterpret_cast<uint4*>(xs + (size_t)pos * H + c * 8) = v;
+    for (int p = blockIdx.x; p < pairs; p += gridDim.x) {
+        const int pos = pos_of[p];
+        if (pos < 0) continue;
+        const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(p / top) * ldx);
+        uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)pos * H);
+        for (int c = threadIdx.x; c < H / 8; c += 256) dst[c] = src[c];
     }
 }
 
@@ -297,19 +300,18 @@ AGV_API int agv_moe_grouped_tc_supported(int N, int K, long long lda) {
     return (N > 0 && K > 0 && K % 8 == 0 && lda % 8 == 0) ? 1 : 0;
 }
 
-// x: [T, H] bfloat16 rows of stride ldx; xs: [rows, H] dense.  H a multiple of 8, both
+// x: [T, H] bfloat16 rows of stride ldx; pos_of [pairs]: the plan's row of pair p (token p / top), or
+// -1; xs: the plan's rows, [*, H] dense, of which those of pairs are written.  H a multiple of 8, both
 // 16-byte aligned.
-AGV_API int agv_moe_gather_rows(const void* x, long long ldx, const int* tok, void* xs, int rows,
-                                int H, cudaStream_t stream) {
-    AGV_REQUIRE(rows >= 0 && H > 0 && H % 8 == 0 && ldx % 8 == 0, "moe_gather: rows of %d values "
-                "with stride %lld do not move in 16-byte pieces", H, ldx);
+AGV_API int agv_moe_gather_rows(const void* x, long long ldx, const int* pos_of, void* xs, int pairs,
+                                int top, int H, cudaStream_t stream) {
+    AGV_REQUIRE(pairs >= 0 && top > 0 && H > 0 && H % 8 == 0 && ldx % 8 == 0, "moe_gather: rows of %d "
+                "values with stride %lld do not move in 16-byte pieces", H, ldx);
     AGV_REQUIRE(agv_aligned(x, 16) && agv_aligned(xs, 16), "moe_gather: operands must be 16-byte "
                 "aligned");
-    if (rows == 0) return 0;
-    long long blocks = ((long long)rows * (H / 8) + 255) / 256;
-    if (blocks > 148 * 8) blocks = 148 * 8;
-    agv_launch(moe_gather_rows_kernel, (unsigned)blocks, 256, 0, stream, (const __nv_bfloat16*)x,
-               ldx, tok, (__nv_bfloat16*)xs, rows, H);
+    if (pairs == 0) return 0;
+    agv_launch(moe_gather_rows_kernel, (unsigned)(pairs < 148 * 8 ? pairs : 148 * 8), 256, 0, stream,
+               (const __nv_bfloat16*)x, ldx, pos_of, (__nv_bfloat16*)xs, pairs, top, H);
     AGV_LAUNCH_OK("moe_gather_rows_kernel");
     return 0;
 }

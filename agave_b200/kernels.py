@@ -422,15 +422,16 @@ _MOE_TC = os.environ.get("AGAVE_B200_MOE_TENSOR_CORES", "1") != "0"
 
 
 def moe_gather_rows(x: torch.Tensor, plan: MoePlan, xs: torch.Tensor) -> None:
-    """xs [plan.rows, H] = the rows of x [T, H] in the plan's sorted order (zeros where the
-    plan pads), bfloat16."""
+    """xs [plan.rows, H] = the rows of x [T, H] in the plan's sorted order, bfloat16; rows where
+    the plan pads are left as they are."""
     T, H = x.shape
     assert x.dtype == torch.bfloat16 and xs.dtype == torch.bfloat16 and x.stride(1) == 1
     _dense(xs, "xs")
     assert xs.shape == (plan.rows, H)
-    with _span("experts_gather", _nbytes(xs) * 2):
+    with _span("experts_gather", 2 * T * plan.top * H * x.element_size()):
         _check(library().agv_moe_gather_rows(_ptr(x), ctypes.c_longlong(x.stride(0)),
-                                             _ptr(plan.tok), _ptr(xs), plan.rows, H, _stream()))
+                                             _ptr(plan.pos_of), _ptr(xs), T * plan.top, plan.top, H,
+                                             _stream()))
 
 
 def moe_grouped_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: MoePlan,
