@@ -231,6 +231,11 @@ __device__ __forceinline__ void st_run(__nv_bfloat16* p, const float* v) {
     }
 }
 
+// Value columns that a block transposes, of 64 tokens.  With several partial sums (short prompts) a
+// narrow tile, so that all of a thread's sums are a trip or two to memory: with 64 columns and the
+// sums one by one a 100-token step of the 1B sizes, nine sums, spent 8.8 us a layer in this kernel.
+constexpr int vt_columns(bool multi) { return multi ? 16 : 64; }
+
 template <typename T, int NE, bool MULTI>
 __global__ void __launch_bounds__(QK_WARPS * 32, MULTI ? 1 : 8)
 qk_norm_rope_store_reg_kernel(T* __restrict__ qkv, long long row_stride,
@@ -249,12 +254,13 @@ qk_norm_rope_store_reg_kernel(T* __restrict__ qkv, long long row_stride,
     const int heads = nh + 2 * nkv;
     if ((int)blockIdx.x < vt_blocks) {
         // ---- the first blocks write the values transposed (they take longest, so they
-        // start first): one tile of 64 tokens x 64 of the nkv * hd value columns each
+        // start first): one tile of 64 tokens x CB of the nkv * hd value columns each
         if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-            __shared__ __align__(16) __nv_bfloat16 tile[64][72];    // rows of 9 x 16 bytes
+            constexpr int CB = vt_columns(MULTI), TPR = CB / 4, ROWS = QK_WARPS * 32 / TPR, PASSES = 64 / ROWS;
+            __shared__ __align__(16) __nv_bfloat16 tile[CB][72];    // rows of 9 x 16 bytes
             __shared__ int cols[64], pads[64], pad_at[64], n_pads;
-            const int vb = blockIdx.x, ncb = nkv * hd / 64;
-            const int t0 = (vb / ncb) * 64, c0 = (vb % ncb) * 64;
+            const int vb = blockIdx.x, ncb = nkv * hd / CB;
+            const int t0 = (vb / ncb) * 64, c0 = (vb % ncb) * CB;
             if (threadIdx.x == 0) n_pads = 0;
             __syncthreads();
             if (threadIdx.x < 64) {
@@ -273,45 +279,57 @@ qk_norm_rope_store_reg_kernel(T* __restrict__ qkv, long long row_stride,
                 if (pad) pad_at[atomicAdd(&n_pads, 1)] = threadIdx.x;   // (ends of sequences)
             }
             pdl_wait();
-            // 16 threads per token row (4 columns each), 8 rows per pass
-            const int tr = threadIdx.x >> 4, tc = (threadIdx.x & 15) * 4;
+            // TPR threads per token row (4 columns each), ROWS rows per pass
+            const int tr = threadIdx.x / TPR, tc = threadIdx.x % TPR * 4;
             const size_t vcol = (size_t)(nh + nkv) * hd + c0 + tc;
-            float val[8][4];
+            float val[PASSES][4] = {};
+            if (MULTI && part) {
+                // the partial sums in order, eight at a time under way
+                for (int s0 = 0; s0 < n_splits; s0 += 8) {
+                    float x[8][PASSES][4];
 #pragma unroll
-            for (int ps = 0; ps < 8; ++ps) {
-                const int t = t0 + ps * 8 + tr;
-                val[ps][0] = val[ps][1] = val[ps][2] = val[ps][3] = 0.f;
-                if (t < n_tokens) {
-                    if (part) {
-                        for (int sp = 0; sp < (MULTI ? n_splits : 1); ++sp) {
-                            float x[4];
-                            ld_run<4>(part + (size_t)sp * split_stride +
-                                          (size_t)t * (size_t)(heads * hd) + vcol, x);
-                            val[ps][0] += x[0], val[ps][1] += x[1], val[ps][2] += x[2],
-                                val[ps][3] += x[3];
+                    for (int u = 0; u < 8; ++u)
+#pragma unroll
+                        for (int ps = 0; ps < PASSES; ++ps) {
+                            const int t = min(t0 + ps * ROWS + tr, n_tokens - 1);
+                            ld_run<4>(part + (size_t)min(s0 + u, n_splits - 1) * split_stride +
+                                          (size_t)t * (size_t)(heads * hd) + vcol, x[u][ps]);
                         }
-                    } else {
-                        ld_run<4>(qkv + (size_t)t * row_stride + vcol, val[ps]);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (s0 + u < n_splits)
+#pragma unroll
+                            for (int ps = 0; ps < PASSES; ++ps)
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) val[ps][e] += x[u][ps][e];
+                }
+            } else {
+#pragma unroll
+                for (int ps = 0; ps < PASSES; ++ps) {
+                    const int t = t0 + ps * ROWS + tr;
+                    if (t < n_tokens) {
+                        if (part) ld_run<4>(part + (size_t)t * (size_t)(heads * hd) + vcol, val[ps]);
+                        else ld_run<4>(qkv + (size_t)t * row_stride + vcol, val[ps]);
                     }
                 }
             }
 #pragma unroll
-            for (int ps = 0; ps < 8; ++ps)
+            for (int ps = 0; ps < PASSES; ++ps)
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    tile[tc + e][ps * 8 + tr] = __float2bfloat16(val[ps][e]);
+                    tile[tc + e][ps * ROWS + tr] = __float2bfloat16(val[ps][e]);
             __syncthreads();
             const int g = c0 / hd, d0 = c0 % hd;
             if (cols[0] >= 0 && (cols[0] & 7) == 0 && cols[63] == cols[0] + 63) {
                 // 64 tokens of one sequence at an aligned column: 16 bytes (8 tokens) a store
-                for (int i = threadIdx.x; i < 64 * 8; i += QK_WARPS * 32) {
+                for (int i = threadIdx.x; i < CB * 8; i += QK_WARPS * 32) {
                     const int d = i >> 3, ch = i & 7;
                     *reinterpret_cast<uint4*>(vw.vt + (size_t)(g * hd + d0 + d) * vw.ld + cols[0] +
                                               ch * 8) =
                         *reinterpret_cast<const uint4*>(&tile[d][ch * 8]);
                 }
             } else {
-                for (int d = warp; d < 64; d += QK_WARPS) {
+                for (int d = warp; d < CB; d += QK_WARPS) {
                     __nv_bfloat16* dst = vw.vt + (size_t)(g * hd + d0 + d) * vw.ld;
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
@@ -322,7 +340,7 @@ qk_norm_rope_store_reg_kernel(T* __restrict__ qkv, long long row_stride,
             }
             for (int k = 0; k < n_pads; ++k) {
                 const int tl = pad_at[k], pad = pads[tl];
-                for (int i = threadIdx.x; i < 64 * pad; i += QK_WARPS * 32) {
+                for (int i = threadIdx.x; i < CB * pad; i += QK_WARPS * 32) {
                     const int d = i / pad, pc = i % pad;
                     vw.vt[(size_t)(g * hd + d0 + d) * vw.ld + cols[tl] + 1 + pc] =
                         __float2bfloat16(0.f);
@@ -449,7 +467,7 @@ static bool launch_qk_reg(T* qkv, long long row_stride, const float* part, int n
         return false;
     if (vw.vt && !std::is_same<T, __nv_bfloat16>::value) return false;
     const unsigned vt_blocks =
-        vw.vt ? (unsigned)((n_tokens + 63) / 64) * (unsigned)(nkv * hd / 64) : 0u;
+        vw.vt ? (unsigned)((n_tokens + 63) / 64) * (unsigned)(nkv * hd / vt_columns(part && n_splits > 1)) : 0u;
     const unsigned grid = main_blocks + vt_blocks;
     // runs of hd / 64 elements move as single accesses: everything must sit on 16 bytes
     if (row_stride % 8 || !agv_aligned(qkv, 16) || !agv_aligned(part, 16) ||

@@ -91,3 +91,34 @@ def test_products_of_prompts_on_pairs_of_ctas(T, N, K, splits, act):
         assert kernels.linear_tc_status() == 0
         want = torch.relu(ref) ** 2 if act == "relu2" else torch.nn.functional.gelu(ref)
         assert rel_err(ob[:, :N], want) < 6e-3 and torch.isnan(ob[:, N:]).all()
+
+
+@pytest.mark.parametrize("nkv,hd", [(1, 256), (3, 64), (2, 192)])
+@pytest.mark.parametrize("splits", [2, 8, 9, 16])
+def test_transposed_values_of_short_prompts(nkv, hd, splits):
+    """The values from several partial sums, transposed: sequences that end inside a tile of 64
+    tokens or fill it, sums up to a batch of loads and beyond.  The sums are added in order in 32
+    bits and rounded once, so they are what torch gives bit for bit."""
+    from agave_b200 import kernels
+    nh, lens = nkv, [64, 1, 37, 63, 65]
+    T, W = sum(lens), (nh + 2 * nkv) * hd
+    part = rnd(splits, T, W, seed=4)
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    pos = torch.cat([torch.arange(n) for n in lens]).int().to(DEV)
+    seq = torch.cat([torch.full((n,), b) for b, n in enumerate(lens)]).int().to(DEV)
+    cols = [(n + 63) // 64 * 64 for n in lens]
+    vt = torch.full((nkv * hd, sum(cols) + 64), 7.0, dtype=torch.bfloat16, device=DEV)
+    qkv = torch.empty(T, W, dtype=torch.bfloat16, device=DEV)
+    kernels.qk_norm_rope_store(qkv, nh, nkv, hd, None, None, 1e-6, None, None, 0, pos, seq_index=seq,
+                               partial=part, vt=vt, cu_seqlens=cu, max_len=max(lens))
+    total = part[0].clone()
+    for s in range(1, splits):
+        total += part[s]
+    v = total.to(torch.bfloat16)
+    assert torch.equal(qkv, v)
+    at = o = 0
+    for n, c in zip(lens, cols):
+        assert torch.equal(vt[:, at:at + n], v[o:o + n, (nh + nkv) * hd:].T), n
+        assert not vt[:, at + n:at + c].any(), n
+        at, o = at + c, o + n
+    assert (vt[:, at:] == 7.0).all()
