@@ -258,7 +258,7 @@ struct Run {
             return !(v2 && strcmp(v2, "mma") == 0);
         }();
         if (!dry()) {
-            if (aligned && b.hd % 16 == 0 && prefill_tc)
+            if (aligned && b.hd % 16 == 0 && prefill_tc && b.scale > 0.f)
                 did(agv_attention_prefill_tc(q, width, k, v, width, out, vt, vt_cols, 1, s.cu_seqlens,
                                              s.B, T, s.max_new, b.nh, b.nkv, b.hd, b.scale,
                                              b.window, stream));
@@ -281,7 +281,7 @@ struct Run {
             return !(v2 && strcmp(v2, "mma") == 0);
         }();
         const long long width = (long long)(b.nh + 2 * b.nkv) * b.hd;
-        return prefill_tc && m.dtype == AGV_BF16 && b.hd % 16 == 0 &&
+        return prefill_tc && b.scale > 0.f && m.dtype == AGV_BF16 && b.hd % 16 == 0 &&
                b.hd <= 256 &&
                width % 8 == 0 && agv_aligned(qkv, 16);
     }
