@@ -185,7 +185,8 @@ norm_residual_small_kernel(float* __restrict__ h, const TY* __restrict__ y, int 
     asm volatile("" ::"l"(h), "l"(y), "l"(w_post), "l"(w_next), "l"(x), "l"(rows), "r"(H),
                  "r"(n_splits), "l"(split_stride), "f"(eps_post), "f"(eps_next), "r"(add_residual));
     // The weights are nobody's output: they are on their way before the wait, from HBM where a
-    // step's other weights have pushed them out of L2.
+    // step's other weights have pushed them out of L2 (with it and sums of one barrier a decode step of
+    // eight sequences takes 1.5 % less, one of 64 2.5 %).
     float v[EPT], hv[EPT], wp[EPT], wn[EPT];
 #pragma unroll
     for (int k = 0; k < EPT; ++k) {
