@@ -27,6 +27,7 @@
 #include "tcgen05.cuh"
 #include "act.cuh"
 #include "cache_write.cuh"
+#include "pair_drain.cuh"
 #include <stdlib.h>
 #include <map>
 #include <mutex>
@@ -1153,6 +1154,64 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
                  : "memory");
 }
 
+// Arrives on this CTA's barrier alone, once the pair products issued so far are done.
+__device__ __forceinline__ void tc_commit_pair_local(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                     smem_u32(bar))
+                 : "memory");
+}
+
+// What the roles of a pair's CTA share beside the rings.
+struct PairState {
+    uint64_t products_done;    // (even CTA) everything the issuer asked for has been multiplied
+    uint32_t tmem;
+    int issued;                // stages this CTA's loader has asked for
+    int abort;                 // set in both CTAs by whoever gives up in either
+};
+
+// A bounded wait ran out: both CTAs are to stop issuing.
+__device__ __forceinline__ void pair_give_up(volatile PairState* st, uint32_t rank, int code) {
+    atomicCAS(&g_gemm_status, 0, code);
+    st->abort = 1;
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(
+                     mapa_u32(smem_u32((const void*)&st->abort), rank ^ 1)), "r"(1)
+                 : "memory");
+}
+
+// The end of a pair kernel, for all threads of both CTAs.  After an abort the copies that either
+// loader issued are waited for (bounded) before anybody leaves: those of both count on the even
+// CTA's barriers, so that CTA waits and its partner stays for it.
+template <int STAGES, int STAGE_BYTES>
+__device__ __forceinline__ void pair_end(PairState* st, uint64_t* full, uint32_t rank, int warp,
+                                         uint32_t tmem_base) {
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();          // the partner has no product, commit or arrival left for us
+    if (((volatile PairState*)st)->abort) {
+        if (rank == 0 && threadIdx.x == 0) {
+            int other;
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(other) : "r"(mapa_u32(smem_u32(&st->issued), 1))
+                         : "memory");
+            pair_drain(
+                st->issued, other, STAGES, [&](int s) { mbar_expect_tx(&full[s], STAGE_BYTES); },
+                [&](int s) {
+                    asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(
+                                     smem_u32(&full[s])), "r"(STAGE_BYTES)
+                                 : "memory");
+                },
+                [&](int s, int parity) { mbar_wait(&full[s], parity); });
+        }
+        __syncthreads();
+        cluster_sync_all();
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
+                     "r"(512u)
+                     : "memory");
+    }
+}
+
 template <bool BOUNDED>
 __global__ void __launch_bounds__(PERSISTENT_THREADS, 1)
 gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
@@ -1169,8 +1228,8 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
     uint64_t* empty = full + PAIR_STAGES;                   // one set per CTA
     uint64_t* acc_full = empty + PAIR_STAGES;               // [2], one set per CTA
     uint64_t* acc_empty = acc_full + 2;                     // [2], used in the even CTA
-    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
-    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    PairState* const state = (PairState*)(acc_empty + 2);
+    volatile int* const abort_flag = &state->abort;
 
     const int warp = warp_number(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();                // 0: issues the products
@@ -1190,12 +1249,14 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
             mbar_init(&acc_full[s], 1);
             mbar_init(&acc_empty[s], 2 * PERSISTENT_EPI_WARPS);   // the epilogue warps of both CTAs
         }
+        mbar_init(&state->products_done, 1);
+        state->issued = 0;
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         smem_u32(tmem_slot)),
+                         smem_u32(&state->tmem)),
                      "r"(512u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -1204,7 +1265,7 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
     __syncthreads();
     cluster_sync_all();          // the partner's barriers exist before anything is sent to them
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = state->tmem;
 
     // item -> (feature tile, token tile); token tiles vary fastest so that the pairs of a
     // wave share weight tiles in L2
@@ -1225,8 +1286,7 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
                 const int s = it % PAIR_STAGES;
                 const uint32_t ph = (it / PAIR_STAGES) & 1;
                 if (!mbar_wait(&empty[s], ph ^ 1)) {
-                    atomicCAS(&g_gemm_status, 0, (5 << 8) | s);
-                    *abort_flag = 1;
+                    pair_give_up(state, rank, (5 << 8) | s);
                     break;
                 }
                 uint8_t* st = smem + s * PAIR_STAGE_BYTES;
@@ -1243,6 +1303,7 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
                 tma_load_2d_pair(st, &map_x, kx, n0, bar);
             }
         }
+        state->issued = it;
         }
     } else if (warp == 1 && rank == 0) {
         if (elect_one()) {
@@ -1252,8 +1313,7 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
         for (int item = pair; item < items && !*abort_flag; item += n_pairs, ++li) {
             const int as = li & 1;
             if (!mbar_wait(&acc_empty[as], ((li >> 1) & 1) ^ 1)) {
-                atomicCAS(&g_gemm_status, 0, (6 << 8) | as);
-                *abort_flag = 1;
+                pair_give_up(state, rank, (6 << 8) | as);
                 break;
             }
             tc_fence_after();
@@ -1262,8 +1322,7 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
                 const int s = it % PAIR_STAGES;
                 const uint32_t ph = (it / PAIR_STAGES) & 1;
                 if (!mbar_wait(&full[s], ph)) {
-                    atomicCAS(&g_gemm_status, 0, (7 << 8) | s);
-                    *abort_flag = 1;
+                    pair_give_up(state, rank, (7 << 8) | s);
                     break;
                 }
                 tc_fence_after();
@@ -1278,6 +1337,11 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
             }
             if (*abort_flag) break;
             tc_commit_pair(&acc_full[as]);
+        }
+        if (*abort_flag) {
+            // the products under way read both CTAs' stages
+            tc_commit_pair_local(&state->products_done);
+            mbar_wait(&state->products_done, 0);
         }
         }
     } else if (warp >= 2) {
@@ -1294,10 +1358,10 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
             int m0, n0;
             decode_item(item, m0, n0);
             const int as = li & 1;
-            bool ok = !*abort_flag && mbar_wait(&acc_full[as], (li >> 1) & 1);
+            // (one answer for the warp, whose loads of tensor memory take all its lanes)
+            const bool ok = __all_sync(0xffffffffu, !*abort_flag && mbar_wait(&acc_full[as], (li >> 1) & 1));
             if (!ok) {
-                if (!*abort_flag) atomicCAS(&g_gemm_status, 0, (8 << 8) | as);
-                *abort_flag = 1;
+                if (lane == 0) pair_give_up(state, rank, (8 << 8) | as);
                 break;
             }
             tc_fence_after();
@@ -1364,19 +1428,7 @@ gemm_tcgen05_pair_gated_kernel(const __grid_constant__ CUtensorMap map_w,
             }
         }
     }
-    // An abort in one CTA leaves the partner to run into its own bounded waits.  Copies
-    // still in flight into this CTA's shared memory land before the cluster barrier below
-    // lets anybody leave only in a run without an abort; after an abort the result is
-    // void anyway and the status word says so.
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();          // the partner has no product, commit or arrival left for us
-    if (warp == 1) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                     "r"(512u)
-                     : "memory");
-    }
+    pair_end<PAIR_STAGES, PAIR_STAGE_BYTES>(state, full, rank, warp, tmem_base);
 }
 
 // The plain product on CTA pairs: a tile is 256 tokens (the M operand, 128 a CTA) by BN weight
@@ -1410,8 +1462,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w,
     uint64_t* empty = full + TL::STAGES;                    // one set per CTA
     uint64_t* acc_full = empty + TL::STAGES;                // [2], one set per CTA
     uint64_t* acc_empty = acc_full + 2;                     // [2], used in the even CTA
-    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
-    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    PairState* const state = (PairState*)(acc_empty + 2);
+    volatile int* const abort_flag = &state->abort;
 
     const int warp = warp_number(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();                // 0: issues the products
@@ -1429,12 +1481,14 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w,
             mbar_init(&acc_full[s], 1);
             mbar_init(&acc_empty[s], 2 * PERSISTENT_EPI_WARPS);   // the epilogue warps of both CTAs
         }
+        mbar_init(&state->products_done, 1);
+        state->issued = 0;
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         smem_u32(tmem_slot)),
+                         smem_u32(&state->tmem)),
                      "r"(512u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -1443,7 +1497,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w,
     __syncthreads();
     cluster_sync_all();          // the partner's barriers exist before anything is sent to them
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = state->tmem;
 
     // item -> (range of K, feature tile, token tile); token tiles vary fastest so that the pairs
     // of a wave share weight tiles in L2
@@ -1459,7 +1513,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w,
     if (warp == 0) {
         if (elect_one()) {
         // ------------------------------------------------------------ loader (both CTAs)
-        int s = 0;
+        int s = 0, issued = 0;
         uint32_t ph = 1;
         bool waited = false;
         for (int item = pair; item < items && !*abort_flag; item += n_pairs) {
@@ -1467,8 +1521,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w,
             decode_item(item, m0, n0, kb_begin, n_kb, split);
             for (int i = 0; i < n_kb; ++i) {
                 if (!mbar_wait(&empty[s], ph)) {
-                    atomicCAS(&g_gemm_status, 0, (5 << 8) | s);
-                    *abort_flag = 1;
+                    pair_give_up(state, rank, (5 << 8) | s);
                     break;
                 }
                 uint8_t* st = smem + s * TL::STAGE_BYTES;
@@ -1483,9 +1536,11 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w,
                     waited = true;
                 }
                 tma_load_2d_pair(st, &map_x, kx, n0, bar);
+                ++issued;
                 if (++s == TL::STAGES) s = 0, ph ^= 1;
             }
         }
+        state->issued = issued;
         }
     } else if (warp == 1 && rank == 0) {
         if (elect_one()) {
@@ -1498,16 +1553,14 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w,
             decode_item(item, m0, n0, kb_begin, n_kb, split);
             const int as = li & 1;
             if (!mbar_wait(&acc_empty[as], ((li >> 1) & 1) ^ 1)) {
-                atomicCAS(&g_gemm_status, 0, (6 << 8) | as);
-                *abort_flag = 1;
+                pair_give_up(state, rank, (6 << 8) | as);
                 break;
             }
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + as * BN;
             for (int i = 0; i < n_kb; ++i) {
                 if (!mbar_wait(&full[s], ph)) {
-                    atomicCAS(&g_gemm_status, 0, (7 << 8) | s);
-                    *abort_flag = 1;
+                    pair_give_up(state, rank, (7 << 8) | s);
                     break;
                 }
                 tc_fence_after();
@@ -1523,6 +1576,11 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w,
             }
             if (*abort_flag) break;
             tc_commit_pair(&acc_full[as]);
+        }
+        if (*abort_flag) {
+            // the products under way read both CTAs' stages
+            tc_commit_pair_local(&state->products_done);
+            mbar_wait(&state->products_done, 0);
         }
         }
     } else if (warp >= 2) {
@@ -1540,10 +1598,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w,
             int m0, n0, kb_begin, n_kb, split;
             decode_item(item, m0, n0, kb_begin, n_kb, split);
             const int as = li & 1;
-            const bool ok = !*abort_flag && mbar_wait(&acc_full[as], (li >> 1) & 1);
+            // (one answer for the warp, whose loads of tensor memory take all its lanes)
+            const bool ok = __all_sync(0xffffffffu, !*abort_flag && mbar_wait(&acc_full[as], (li >> 1) & 1));
             if (!ok) {
-                if (!*abort_flag) atomicCAS(&g_gemm_status, 0, (8 << 8) | as);
-                *abort_flag = 1;
+                if (lane == 0) pair_give_up(state, rank, (8 << 8) | as);
                 break;
             }
             tc_fence_after();
@@ -1599,16 +1657,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w,
             }
         }
     }
-    // (as in the gated form above)
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();          // the partner has no product, commit or arrival left for us
-    if (warp == 1) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                     "r"(512u)
-                     : "memory");
-    }
+    pair_end<TL::STAGES, TL::STAGE_BYTES>(state, full, rank, warp, tmem_base);
 }
 
 int device_sms() {
