@@ -118,11 +118,9 @@ constexpr int GS_K = 32;                       // k of a piece
 constexpr int GS_PITCH = GS_K + 4;             // of a weight row in shared memory (no bank conflict)
 constexpr int GS_WARPS = 2;
 
-// One range a warp (R = 1) is for weights with few warps (288 for 1152 x 6912): those keep eight pieces
-// under way, four are too few bytes for the SMs' trips to HBM (replay of three sequences, 13 layers of
-// the 1B sizes, 12.7 -> 11.7 ms).
-__host__ __device__ constexpr int gs_stages(int mats, int bm, int r) {
-    return mats * bm >= 64 ? 3 : r == 1 && mats * bm <= 16 ? 8 : 4;
+// Pieces under way a warp (DEEP: see launch_rows).
+__host__ __device__ constexpr int gs_stages(int mats, int bm, bool deep) {
+    return mats * bm >= 64 ? 3 : deep ? 8 : 4;
 }
 __host__ __device__ constexpr int gs_stage_floats(int mats, int bm) {
     return mats * GS_ROWS * GS_PITCH + bm * GS_K;
@@ -144,12 +142,12 @@ __device__ __forceinline__ float gs_peer(const float* mine, int rank) {
     return v;
 }
 
-template <bool GATED, int BM, int R>
+template <bool GATED, int BM, int R, bool DEEP>
 __global__ void __launch_bounds__(GS_WARPS * 32)
 gemm_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ W2,
                  float* __restrict__ C, int M, int N, int K, long long lda, long long ldc, GateAct act,
                  int m_tiles, int range) {
-    constexpr int MATS = GATED ? 2 : 1, STAGES = gs_stages(MATS, BM, R), CL = 4 / R;
+    constexpr int MATS = GATED ? 2 : 1, STAGES = gs_stages(MATS, BM, DEEP), CL = 4 / R;
     constexpr int STAGE = gs_stage_floats(MATS, BM), PARTS = 8 / R;
     extern __shared__ __align__(16) float gs_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -426,20 +424,20 @@ struct GsArgs {
 };
 
 // BM == GT_M: tiles, else a warp's rows.
-template <bool GATED, int BM, int R>
+template <bool GATED, int BM, int R, bool DEEP = false>
 static int launch_f32(const GsArgs& a) {
     constexpr bool TILE = BM == GT_M;
     constexpr int MATS = GATED ? 2 : 1, CL = TILE ? 8 : 4 / R;
     constexpr int WIDE = TILE ? GT_N / MATS : GS_ROWS;
     constexpr size_t smem = sizeof(float) * (TILE ? GT_STAGES * GT_STAGE
-                                                  : GS_WARPS * gs_stages(MATS, BM, R) * gs_stage_floats(MATS, BM));
+                                                  : GS_WARPS * gs_stages(MATS, BM, DEEP) * gs_stage_floats(MATS, BM));
     const long long m_tiles = (a.M + BM - 1) / BM, n_tiles = (a.N + WIDE - 1) / WIDE;
     AGV_REQUIRE(m_tiles * n_tiles * CL <= 0x7fffffffLL, "linear: M=%d N=%d exceed the grid limit", a.M, a.N);
     const int range = ((a.K + 7) / 8 + 3) / 4 * 4;
     void (*kern)(const float*, const float*, const float*, float*, int, int, int, long long, long long, GateAct,
                  int, int);
     if constexpr (TILE) kern = range % GT_K ? gemm_tile_kernel<GATED, true> : gemm_tile_kernel<GATED, false>;
-    else kern = gemm_rows_kernel<GATED, BM, R>;
+    else kern = gemm_rows_kernel<GATED, BM, R, DEEP>;
     if (smem > 48 * 1024)
         AGV_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     agv_launch_cluster(kern, dim3((unsigned)(m_tiles * n_tiles * CL)), TILE ? GT_THREADS : GS_WARPS * 32, smem,
@@ -453,10 +451,20 @@ static int launch_f32(const GsArgs& a) {
 // warp's ring busy), else two or four ranges a warp.  3 rows of x, us for R = 1, 2, 4:
 // 1536 x 1152 12, 14, 19; 6912 x 1152 21, 18, 23; gated 35, 31, 27; 262144 x 1152 298, 258, 242;
 // 10240 x 2560 35, 37, 39; 1152 x 6912 23, 40, 80.
+// With up to four rows of x and 64 groups a warp keeps eight pieces under way instead of four: such a launch
+// is at most 256 CTAs, all resident with 82 KB each, and four pieces are too few bytes for their trips to HBM
+// (us, 1152 x 6912 19.1 -> 14.7, 1536 x 4096 12.0 -> 10.2, 2048 x 2304 8.0 -> 7.4, 256 x 10240 24.7 -> 18.5).
+// More groups would need a second round (2304 x 2304 1.46 times the time with eight, 8192 x 4096 1.28), a gated pair
+// takes 156 KB a CTA (1.6 to 2 times), eight rows gain nothing (0.96 to 1.08), and a walk of up to four pieces
+// (K of 1,024) does from 57 groups on (1.02 to 1.05).
 template <bool GATED, int BM>
 static int launch_rows(const GsArgs& a) {
     const int pieces = (a.N + GS_ROWS - 1) / GS_ROWS * (GATED ? 2 : 1);
-    if (pieces <= 128 || a.K >= 2304) return launch_f32<GATED, BM, 1>(a);
+    if (pieces <= 128 || a.K >= 2304) {
+        if constexpr (!GATED && BM == 4)
+            if (pieces <= (a.K > 1024 ? 64 : 56)) return launch_f32<GATED, BM, 1, true>(a);
+        return launch_f32<GATED, BM, 1>(a);
+    }
     if constexpr (BM <= 16)
         if (pieces > 400) return launch_f32<GATED, BM, 4>(a);
     return launch_f32<GATED, BM, 2>(a);

@@ -122,3 +122,19 @@ def test_transposed_values_of_short_prompts(nkv, hd, splits):
         assert not vt[:, at + n:at + c].any(), n
         at, o = at + c, o + n
     assert (vt[:, at:] == 7.0).all()
+
+
+@pytest.mark.parametrize("N,K", [(1152, 1024), (2048, 1152), (2080, 1152), (40, 2312), (2016, 6920)])
+@pytest.mark.parametrize("M", [1, 3, 4, 5])
+def test_32_bit_products_either_side_of_the_deep_rings(N, K, M):
+    """Weights of up to 64 groups of 32 rows and of more, walks shorter than a ring and with a ragged
+    last piece, more rows than a deep ring takes.  A row's sum has one order whatever its company."""
+    from agave_b200 import kernels
+    x, w = rnd(M, K, seed=1), rnd(N, K, seed=2, scale=K ** -0.5)
+    out = torch.full((M + 1, N), float("nan"), device=DEV)
+    kernels.linear_simt(x, w, out[:M])
+    ref = x.double() @ w.double().T
+    assert rel_err(out[:M], ref) < 1e-6 and torch.isnan(out[M]).all()
+    one = torch.empty(1, N, device=DEV)
+    kernels.linear_simt(x[:1], w, one)
+    assert torch.equal(one[0], out[0])
