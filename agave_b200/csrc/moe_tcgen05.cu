@@ -277,20 +277,49 @@ int mt_map(CUtensorMap* out, const void* ptr, long long rows, long long K, long 
 
 // xs[pos_of[p], :] = x[p / top, :] for the pairs of a plan; the plan's padding is left as it is (a
 // product's rows do not meet, and those of padding are dropped).  With zeros there, 8 tokens of 4
-// experts among 32 wrote 8.5 MB a layer for the 0.13 that count.
+// experts among 32 wrote 8.5 MB a layer for the 0.13 that count.  Few pairs: a CTA each.
 __global__ void __launch_bounds__(256)
 moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
-                       const int* __restrict__ pos_of, __nv_bfloat16* __restrict__ xs, int pairs,
-                       int top, int H) {
+                       const int* __restrict__ pos_of, __nv_bfloat16* __restrict__ xs, int top, int H) {
     pdl_wait();
     pdl_launch_next();
-    for (int p = blockIdx.x; p < pairs; p += gridDim.x) {
+    const int p = blockIdx.x, pos = pos_of[p];
+    if (pos < 0) return;
+    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(p / top) * ldx);
+    uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)pos * H);
+    for (int c = threadIdx.x; c < H / 8; c += 256) dst[c] = src[c];
+}
+
+// The same for many: the rows' 16-byte pieces are shared out one by one, U to a thread, all asked for at
+// once (four where that leaves more than a round of the SMs).  Bound by the bytes; a CTA a pair leaves threads
+// idle where rows are short, and is a chain of position, row and store.  us, a CTA a pair (1,184 of them in
+// turn) and in pieces: 131,072 pairs of 2,048 values 240 and 100, 65,536 of 512 59 and 16, 32,768 of 256 23
+// and 6.2; 1,024 of 512 2.3 and 1.9, 512 of 1,024 1.8 and 2.0, 2,048 of 4,096 4.6 and 5.3.
+template <int U>
+__global__ void __launch_bounds__(256)
+moe_gather_pieces_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
+                         const int* __restrict__ pos_of, __nv_bfloat16* __restrict__ xs,
+                         long long pieces, int top, int H) {
+    pdl_wait();
+    pdl_launch_next();
+    const unsigned per_row = H / 8;
+    const long long first = (long long)blockIdx.x * (U * 256);
+    const unsigned p0 = (unsigned)(first / per_row), c0 = (unsigned)(first % per_row);
+    uint4 v[U];
+    uint4* dst[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const unsigned i = u * 256 + threadIdx.x, p = p0 + (c0 + i) / per_row, c = (c0 + i) % per_row;
+        dst[u] = nullptr;
+        if (first + i >= pieces) continue;
         const int pos = pos_of[p];
         if (pos < 0) continue;
-        const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(p / top) * ldx);
-        uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)pos * H);
-        for (int c = threadIdx.x; c < H / 8; c += 256) dst[c] = src[c];
+        v[u] = reinterpret_cast<const uint4*>(x + (size_t)(p / (unsigned)top) * ldx)[c];
+        dst[u] = reinterpret_cast<uint4*>(xs + (size_t)pos * H) + c;
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (dst[u]) *dst[u] = v[u];
 }
 
 }  // namespace
@@ -310,8 +339,16 @@ AGV_API int agv_moe_gather_rows(const void* x, long long ldx, const int* pos_of,
     AGV_REQUIRE(agv_aligned(x, 16) && agv_aligned(xs, 16), "moe_gather: operands must be 16-byte "
                 "aligned");
     if (pairs == 0) return 0;
-    agv_launch(moe_gather_rows_kernel, (unsigned)(pairs < 148 * 8 ? pairs : 148 * 8), 256, 0, stream,
-               (const __nv_bfloat16*)x, ldx, pos_of, (__nv_bfloat16*)xs, pairs, top, H);
+    if (pairs <= (H >= 2048 ? 2048 : 512)) {
+        agv_launch(moe_gather_rows_kernel, (unsigned)pairs, 256, 0, stream, (const __nv_bfloat16*)x, ldx,
+                   pos_of, (__nv_bfloat16*)xs, top, H);
+    } else {
+        const long long pieces = (long long)pairs * (H / 8), blocks = (pieces + 255) / 256;
+        const bool many = blocks > 148 * 8;
+        agv_launch(many ? moe_gather_pieces_kernel<4> : moe_gather_pieces_kernel<1>,
+                   (unsigned)(many ? (blocks + 3) / 4 : blocks), 256, 0, stream, (const __nv_bfloat16*)x,
+                   ldx, pos_of, (__nv_bfloat16*)xs, pieces, top, H);
+    }
     AGV_LAUNCH_OK("moe_gather_rows_kernel");
     return 0;
 }

@@ -138,3 +138,56 @@ def test_32_bit_products_either_side_of_the_deep_rings(N, K, M):
     one = torch.empty(1, N, device=DEV)
     kernels.linear_simt(x[:1], w, one)
     assert torch.equal(one[0], out[0])
+
+
+@pytest.mark.parametrize("tile", [64, 128])
+@pytest.mark.parametrize("weigh_input", [False, True])
+@pytest.mark.parametrize("T,E,top,H,ff", [(9, 6, 3, 264, 200), (3, 40, 4, 64, 136), (300, 5, 2, 136, 264),
+                                          (1500, 7, 4, 1032, 72)])
+def test_padding_of_the_experts_rows_reaches_nothing(tile, weigh_input, T, E, top, H, ff):
+    """The plan's padding rows hold NaN before the rows are gathered and before both products: results
+    are finite and right, the padding is as it was; one expert has no tokens and some choices name no
+    expert at all.  A CTA a row, and pieces of rows that end inside a CTA.  z is rounded to bfloat16 (2^-9),
+    its gate is within 2^-11 and sums are in 32 bits."""
+    from agave_b200 import kernels
+    g = torch.Generator().manual_seed(T + E)
+    ids = torch.stack([torch.randperm(E + 2, generator=g)[:top] for _ in range(T)])
+    ids[ids == 1] = E                                  # (nobody goes to expert 1)
+    ids = ids.int().to(DEV)
+    wts = torch.rand(T, top, generator=g).to(DEV) + 0.1
+    x = rnd(T, H + 8, dtype=torch.bfloat16, seed=1)[:, :H]
+    wg, wu = (rnd(E, ff, H, dtype=torch.bfloat16, seed=s, scale=H ** -0.5) for s in (2, 3))
+    wd = rnd(E, H, ff, dtype=torch.bfloat16, seed=4, scale=ff ** -0.5)
+    plan = kernels.moe_plan(ids, wts, E, tile=tile)
+    nan = float("nan")
+    xs = torch.full((plan.rows, H), nan, dtype=torch.bfloat16, device=DEV)
+    z = torch.full((plan.rows, ff), nan, dtype=torch.bfloat16, device=DEV)
+    y = torch.full((top * T, H), nan, device=DEV)
+    kernels.moe_gather_rows(x, plan, xs)
+    kernels.moe_grouped_tc(xs, wg, z, plan, w2=wu, activation="silu", weigh=weigh_input)
+    kernels.moe_grouped_tc(z, wd, y, plan, scatter=True, weigh=not weigh_input)
+    assert kernels.moe_tc_status() == 0
+    pos = plan.pos_of.view(T, top).long()
+    assert torch.equal(pos < 0, ids >= E)
+    live = pos[pos >= 0]
+    padding = torch.ones(plan.rows, dtype=torch.bool, device=DEV)
+    padding[live] = False
+    assert padding.any()
+    for t in (xs, z):
+        assert torch.isnan(t[padding]).all() and torch.isfinite(t[live]).all()
+    want = torch.full((top, T, H), nan, dtype=torch.float64, device=DEV)
+    for e in range(E):
+        t, c = (ids == e).nonzero(as_tuple=True)
+        if not len(t):
+            continue
+        assert torch.equal(xs[pos[t, c]], x[t])
+        w = wts[t, c].double()[:, None]
+        u, v = x[t].double() @ wg[e].double().T, x[t].double() @ wu[e].double().T
+        if weigh_input:
+            u, v = u * w, v * w
+        r = (torch.nn.functional.silu(u) * v) @ wd[e].double().T
+        want[c, t] = r if weigh_input else r * w
+    got = y.view(top, T, H)
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    there = ~torch.isnan(want)
+    assert rel_err(got[there], want[there]) < 8e-3
