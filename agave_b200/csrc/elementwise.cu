@@ -119,7 +119,7 @@ __global__ void norm_residual_kernel(float* __restrict__ h, const TY* __restrict
     pdl_wait();
     pdl_launch_next();
     extern __shared__ float row[];
-    __shared__ float red[33];
+    __shared__ float red[32];
     const int r = blockIdx.x;
     const size_t src = (size_t)(rows ? rows[r] : r) * H;
     const size_t dst = (size_t)r * H;
@@ -185,8 +185,9 @@ norm_residual_small_kernel(float* __restrict__ h, const TY* __restrict__ y, int 
     asm volatile("" ::"l"(h), "l"(y), "l"(w_post), "l"(w_next), "l"(x), "l"(rows), "r"(H),
                  "r"(n_splits), "l"(split_stride), "f"(eps_post), "f"(eps_next), "r"(add_residual));
     // The weights are nobody's output: they are on their way before the wait, from HBM where a
-    // step's other weights have pushed them out of L2 (with it and sums of one barrier a decode step of
-    // eight sequences takes 1.5 % less, one of 64 2.5 %).
+    // step's other weights have pushed them out of L2 (with it and sums of one barrier, here and in the kernel of
+    // a CTA a row, a recorded decode step of eight sequences alone, 1B sizes, 1,078 -> 1,052 us, of 64 1,690 ->
+    // 1,640).
     float v[EPT], hv[EPT], wp[EPT], wn[EPT];
 #pragma unroll
     for (int k = 0; k < EPT; ++k) {
@@ -381,7 +382,7 @@ norm_residual_warp_kernel(float* __restrict__ h, const float* __restrict__ y, in
 // 6 us, against four partial sums at a time (a warp a row up to 2,048 values): 4,001 rows of 2,560, 22 us of
 // HBM, 43.0 -> 30.7; of 5,376, 46 us, 92.1 -> 59.4; 2,048 rows of 2,048 25.6 -> 18.5; 8,696 of 1,152
 // 31.7 -> 29.7, with two partial sums 42.0 -> 37.8.
-template <typename TX, int NV, int U, int TH>
+template <typename TX, int NV, int U, int TH, bool EARLY>
 __global__ void __launch_bounds__(256)
 norm_residual_row_kernel(float* __restrict__ h, const float* __restrict__ y, int n_splits,
                           size_t split_stride, const float* __restrict__ w_post,
@@ -391,9 +392,7 @@ norm_residual_row_kernel(float* __restrict__ h, const float* __restrict__ y, int
     const int lane = threadIdx.x, n = TH ? TH : blockDim.x;         // n threads share the row
     const int row = blockIdx.x;
     const int H4 = H >> 2;
-    // few rows: the weights are on their way before the wait (many rows find them in L1, and are
-    // better off with the registers)
-    constexpr bool EARLY = TH != 0 && NV <= 3;
+    // EARLY: the weights are on their way before the wait (see launch_norm_row)
     float4 wp[EARLY ? NV : 1], wn[EARLY ? NV : 1];
     auto weight = [&](const float* w, int idx) {
         return w && idx < H4 ? reinterpret_cast<const float4*>(w)[idx] : make_float4(1.f, 1.f, 1.f, 1.f);
@@ -513,13 +512,20 @@ static bool launch_norm_row(float* h, const float* y, int n_splits, size_t split
                             float eps_post, float eps_next, int add_residual,
                             cudaStream_t stream) {
     const int nv = (H / 4 + 255) / 256;
+    // The weights early, before the wait, where they cost no CTA that would be resident: up to 2,048 values they
+    // take 16 registers more, three CTAs an SM instead of four, so that more than 444 rows go two rounds (us,
+    // 512 rows of 1,152, five partial sums, 4.1 late and 5.1 early; 320 rows 3.8 and 3.2; 8,192 rows 52 and
+    // 60); wider rows run two either way (512 rows of 2,560 9.7 and 8.6).  Rows of up to 1,024 values in
+    // fewer threads than 256 gain up to 192 rows (0.85 to 0.95 of the time) and lose from 256 on (1.0 to 1.1).
+    const bool early = nv == 3 || R <= (H > 1024 ? 3 * 148 : 192);
 #define AGV_ROW(NV)                                                                             \
     do {                                                                                        \
         const bool whole = R <= 256 || (n_splits > 2 && H > 1024);                              \
         const int threads = whole ? 256 : ((H / 4 + NV - 1) / NV + 31) / 32 * 32;               \
-        auto kern = whole          ? norm_residual_row_kernel<TX, NV, 4, 256>                   \
-                    : n_splits > 2 ? norm_residual_row_kernel<TX, NV, 4, 0>                     \
-                                   : norm_residual_row_kernel<TX, NV, 1, 0>;                    \
+        auto kern = whole && early ? norm_residual_row_kernel<TX, NV, 4, 256, NV <= 3>          \
+                    : whole        ? norm_residual_row_kernel<TX, NV, 4, 256, false>            \
+                    : n_splits > 2 ? norm_residual_row_kernel<TX, NV, 4, 0, false>              \
+                                   : norm_residual_row_kernel<TX, NV, 1, 0, false>;             \
         agv_launch(kern, (unsigned)R, threads, 0, stream, h, y, n_splits, split_stride, w_post, w_next, x, R, H, \
                    eps_post, eps_next, add_residual);                                           \
     } while (0)

@@ -191,3 +191,19 @@ def test_padding_of_the_experts_rows_reaches_nothing(tile, weigh_input, T, E, to
     assert torch.equal(torch.isnan(got), torch.isnan(want))
     there = ~torch.isnan(want)
     assert rel_err(got[there], want[there]) < 8e-3
+
+
+@pytest.mark.parametrize("R", [192, 193, 444, 445])
+@pytest.mark.parametrize("H,S", [(512, 5), (1024, 1), (1152, 3), (2048, 5), (2560, 4)])
+def test_norm_with_its_weights_early_or_late(H, S, R):
+    """Rows either side of the lines at which the weights are asked for before the wait.  Sums of S
+    values and of H squares in 32 bits; the stream in 32 bits, the result rounded to bfloat16 (2^-9)."""
+    from agave_b200 import kernels
+    h0, y = rnd(R, H, seed=1), rnd(S, R, H, seed=2)
+    wp, wn = 1 + rnd(H, seed=3, scale=0.1), 1 + rnd(H, seed=4, scale=0.1)
+    h, x = h0.clone(), torch.empty(R, H, dtype=torch.bfloat16, device=DEV)
+    kernels.norm_residual(h, y if S > 1 else y[0], wp, wn, x, 1e-6, 1e-6)
+    b = y.double().sum(0)
+    want = h0.double() + b / (b.square().mean(1, keepdim=True) + 1e-6).sqrt() * wp.double()
+    assert rel_err(h, want) < 2e-6
+    assert rel_err(x, want / (want.square().mean(1, keepdim=True) + 1e-6).sqrt() * wn.double()) < 4e-3
