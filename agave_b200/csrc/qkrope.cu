@@ -231,13 +231,9 @@ __device__ __forceinline__ void st_run(__nv_bfloat16* p, const float* v) {
     }
 }
 
-// Value columns that a block transposes, of 64 tokens.  With several partial sums (short prompts) a
-// narrow tile, so that all of a thread's sums are a trip or two to memory: with 64 columns and the
-// sums one by one a 100-token step of the 1B sizes, nine sums, spent 8.8 us a layer in this kernel.
-constexpr int vt_columns(bool multi) { return multi ? 16 : 64; }
-
-template <typename T, int NE, bool MULTI>
-__global__ void __launch_bounds__(QK_WARPS * 32, MULTI ? 1 : 8)
+template <typename T, int NE, bool MULTI, int CB>
+// (with heads of 64 six blocks an SM, as many as its heads' own share of the registers allows)
+__global__ void __launch_bounds__(QK_WARPS * 32, !MULTI ? 8 : NE == 2 && CB == 64 ? 6 : 1)
 qk_norm_rope_store_reg_kernel(T* __restrict__ qkv, long long row_stride,
                               const float* __restrict__ part, int n_splits,
                               long long split_stride, int n_tokens, int nh, int nkv,
@@ -256,7 +252,7 @@ qk_norm_rope_store_reg_kernel(T* __restrict__ qkv, long long row_stride,
         // ---- the first blocks write the values transposed (they take longest, so they
         // start first): one tile of 64 tokens x CB of the nkv * hd value columns each
         if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-            constexpr int CB = vt_columns(MULTI), TPR = CB / 4, ROWS = QK_WARPS * 32 / TPR, PASSES = 64 / ROWS;
+            constexpr int TPR = CB / 4, ROWS = QK_WARPS * 32 / TPR, PASSES = 64 / ROWS;
             __shared__ __align__(16) __nv_bfloat16 tile[CB][72];    // rows of 9 x 16 bytes
             __shared__ int cols[64], pads[64], pad_at[64], n_pads;
             const int vb = blockIdx.x, ncb = nkv * hd / CB;
@@ -282,9 +278,11 @@ qk_norm_rope_store_reg_kernel(T* __restrict__ qkv, long long row_stride,
             // TPR threads per token row (4 columns each), ROWS rows per pass
             const int tr = threadIdx.x / TPR, tc = threadIdx.x % TPR * 4;
             const size_t vcol = (size_t)(nh + nkv) * hd + c0 + tc;
-            float val[PASSES][4] = {};
-            if (MULTI && part) {
+            float val[PASSES][4];
+            if constexpr (MULTI && CB == 16) {
                 // the partial sums in order, eight at a time under way
+#pragma unroll
+                for (int ps = 0; ps < PASSES; ++ps) val[ps][0] = val[ps][1] = val[ps][2] = val[ps][3] = 0.f;
                 for (int s0 = 0; s0 < n_splits; s0 += 8) {
                     float x[8][PASSES][4];
 #pragma unroll
@@ -303,10 +301,24 @@ qk_norm_rope_store_reg_kernel(T* __restrict__ qkv, long long row_stride,
 #pragma unroll
                                 for (int e = 0; e < 4; ++e) val[ps][e] += x[u][ps][e];
                 }
+            } else if constexpr (MULTI) {
+#pragma unroll
+                for (int ps = 0; ps < PASSES; ++ps) {
+                    const int t = t0 + ps * ROWS + tr;
+                    val[ps][0] = val[ps][1] = val[ps][2] = val[ps][3] = 0.f;
+                    if (t < n_tokens) {
+                        for (int sp = 0; sp < n_splits; ++sp) {
+                            float x[4];
+                            ld_run<4>(part + (size_t)sp * split_stride + (size_t)t * (size_t)(heads * hd) + vcol, x);
+                            val[ps][0] += x[0], val[ps][1] += x[1], val[ps][2] += x[2], val[ps][3] += x[3];
+                        }
+                    }
+                }
             } else {
 #pragma unroll
                 for (int ps = 0; ps < PASSES; ++ps) {
                     const int t = t0 + ps * ROWS + tr;
+                    val[ps][0] = val[ps][1] = val[ps][2] = val[ps][3] = 0.f;
                     if (t < n_tokens) {
                         if (part) ld_run<4>(part + (size_t)t * (size_t)(heads * hd) + vcol, val[ps]);
                         else ld_run<4>(qkv + (size_t)t * row_stride + vcol, val[ps]);
@@ -338,12 +350,15 @@ qk_norm_rope_store_reg_kernel(T* __restrict__ qkv, long long row_stride,
                     }
                 }
             }
-            for (int k = 0; k < n_pads; ++k) {
-                const int tl = pad_at[k], pad = pads[tl];
-                for (int i = threadIdx.x; i < CB * pad; i += QK_WARPS * 32) {
-                    const int d = i / pad, pc = i % pad;
-                    vw.vt[(size_t)(g * hd + d0 + d) * vw.ld + cols[tl] + 1 + pc] =
-                        __float2bfloat16(0.f);
+            // zeros behind the sequences that end here, up to a multiple of 64 columns, eight at a
+            // time where they are
+            for (int i = threadIdx.x; i < n_pads * CB * 8; i += QK_WARPS * 32) {
+                const int last = cols[pad_at[i / (CB * 8)]], at = (last & ~63) + (i & 7) * 8;
+                __nv_bfloat16* dst = vw.vt + (size_t)(g * hd + d0 + i / 8 % CB) * vw.ld + at;
+                if (at > last) {
+                    *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+                } else {
+                    for (int c = last + 1 - at; c < 8; ++c) dst[c] = __float2bfloat16(0.f);
                 }
             }
         } else {
@@ -461,13 +476,22 @@ static bool launch_qk_reg(T* qkv, long long row_stride, const float* part, int n
                           long long split_stride, int n_tokens, int nh, int nkv, int hd,
                           const float* wq, const float* wk, float eps, const float* cosv,
                           const float* sinv, int rotary_dim, const int* positions,
-                          const CacheWrite& cw, const VtWrite& vw, unsigned main_blocks,
+                          const CacheWrite& cw, const VtWrite& vw, int n_seq, unsigned main_blocks,
                           cudaStream_t stream, int hdv, QueryTemp qt) {
     if (hd % 64 != 0 || hd > 256 || (cosv && rotary_dim != hd) || (hdv != hd && nkv > 0))
         return false;
     if (vw.vt && !std::is_same<T, __nv_bfloat16>::value) return false;
-    const unsigned vt_blocks =
-        vw.vt ? (unsigned)((n_tokens + 63) / 64) * (unsigned)(nkv * hd / vt_columns(part && n_splits > 1)) : 0u;
+    // A block transposes 64 tokens of 64 value columns.  With several partial sums a narrow tile of 16,
+    // so that all of a thread's sums are a trip or two to memory, while the launch is about one round of the SMs
+    // (four heads of 256, 100 tokens, nine sums 6.7 -> 3.5 us; 300 tokens, four sums 6.8 -> 3.6); in larger
+    // ones its four times as many blocks and its rows of 64 bytes cost more than it hides (16 heads of 64,
+    // 512 tokens, four sums 18.2 us wide, 21.4 narrow).  Sequences shorter than the tile have single values
+    // and zeros to write, which the wide tile's blocks take long over (32 heads of 128 over 16, eight
+    // sequences of 186 tokens in all, with the attention 21.4 us wide, 14.9 narrow).
+    const bool multi = part && n_splits > 1;
+    const unsigned wide = (unsigned)((n_tokens + 63) / 64) * (unsigned)(nkv * hd / 64);
+    const bool narrow = multi && (4 * wide + main_blocks < 16 * 148 || n_tokens < 64LL * n_seq);
+    const unsigned vt_blocks = vw.vt ? wide * (narrow ? 4 : 1) : 0u;
     const unsigned grid = main_blocks + vt_blocks;
     // runs of hd / 64 elements move as single accesses: everything must sit on 16 bytes
     if (row_stride % 8 || !agv_aligned(qkv, 16) || !agv_aligned(part, 16) ||
@@ -475,14 +499,11 @@ static bool launch_qk_reg(T* qkv, long long row_stride, const float* part, int n
         !agv_aligned(sinv, 16) || !agv_aligned(cw.k_pool, 16) || !agv_aligned(cw.v_pool, 16))
         return false;
 #define AGV_QK_REG(NE)                                                                          \
-    if (part && n_splits > 1)                                                                   \
-        agv_launch(qk_norm_rope_store_reg_kernel<T, NE, true>, grid, QK_WARPS * 32, 0, stream,  \
-                   qkv, row_stride, part, n_splits, split_stride, n_tokens, nh, nkv, wq, wk,    \
-                   eps, cosv, sinv, positions, cw, vw, (int)vt_blocks, qt);                     \
-    else                                                                                        \
-        agv_launch(qk_norm_rope_store_reg_kernel<T, NE, false>, grid, QK_WARPS * 32, 0, stream, \
-                   qkv, row_stride, part, n_splits, split_stride, n_tokens, nh, nkv, wq, wk,    \
-                   eps, cosv, sinv, positions, cw, vw, (int)vt_blocks, qt)
+    agv_launch(narrow  ? qk_norm_rope_store_reg_kernel<T, NE, true, 16>                         \
+               : multi ? qk_norm_rope_store_reg_kernel<T, NE, true, 64>                         \
+                       : qk_norm_rope_store_reg_kernel<T, NE, false, 64>,                       \
+               grid, QK_WARPS * 32, 0, stream, qkv, row_stride, part, n_splits, split_stride,   \
+               n_tokens, nh, nkv, wq, wk, eps, cosv, sinv, positions, cw, vw, (int)vt_blocks, qt)
     if (hd == 64) { AGV_QK_REG(2); }
     else if (hd == 128) { AGV_QK_REG(4); }
     else if (hd == 192) { AGV_QK_REG(6); }
@@ -548,15 +569,15 @@ AGV_API int agv_qk_norm_rope_store_ex(void* qkv, int dtype, long long row_stride
     const bool simple = !bias && !(interleaved && cosv) && v_eps < 0.f;
     if (simple && dtype == AGV_F32 &&
         launch_qk_reg<float>((float*)qkv, row_stride, part, n_splits, split_stride, n_tokens, nh,
-                             nkv, hd, wq, wk, eps, cosv, sinv, rotary_dim, positions, cw, vw, grid,
-                             stream, hdv, qt)) {
+                             nkv, hd, wq, wk, eps, cosv, sinv, rotary_dim, positions, cw, vw, n_seq,
+                             grid, stream, hdv, qt)) {
         AGV_LAUNCH_OK("qk_norm_rope_store_reg_kernel");
         return 0;
     }
     if (simple && dtype == AGV_BF16 &&
         launch_qk_reg<__nv_bfloat16>((__nv_bfloat16*)qkv, row_stride, part, n_splits, split_stride,
                                      n_tokens, nh, nkv, hd, wq, wk, eps, cosv, sinv, rotary_dim,
-                                     positions, cw, vw, grid, stream, hdv, qt)) {
+                                     positions, cw, vw, n_seq, grid, stream, hdv, qt)) {
         AGV_LAUNCH_OK("qk_norm_rope_store_reg_kernel");
         return 0;
     }

@@ -207,3 +207,35 @@ def test_norm_with_its_weights_early_or_late(H, S, R):
     want = h0.double() + b / (b.square().mean(1, keepdim=True) + 1e-6).sqrt() * wp.double()
     assert rel_err(h, want) < 2e-6
     assert rel_err(x, want / (want.square().mean(1, keepdim=True) + 1e-6).sqrt() * wn.double()) < 4e-3
+
+
+@pytest.mark.parametrize("splits", [1, 2, 9])
+@pytest.mark.parametrize("nh,nkv,hd,lens", [
+    (8, 4, 64, [64, 1, 700, 63, 513, 128]), (3, 1, 256, [1200, 70]), (5, 2, 128, [3, 64, 1, 17] * 12 + [60]),
+    (16, 16, 64, [2] * 70)])
+def test_transposed_values_of_both_tiles(nh, nkv, hd, lens, splits):
+    """Steps whose values are transposed 64 columns a block, from one partial sum and from several, and
+    steps of many sequences that end inside a tile of 64 tokens, whose zeros begin at any column.  The
+    sums are added in order in 32 bits and rounded once: what torch gives bit for bit."""
+    from agave_b200 import kernels
+    T, W = sum(lens), (nh + 2 * nkv) * hd
+    part = rnd(splits, T, W, seed=4)
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    pos = torch.cat([torch.arange(n) for n in lens]).int().to(DEV)
+    seq = torch.cat([torch.full((n,), b) for b, n in enumerate(lens)]).int().to(DEV)
+    cols = [(n + 63) // 64 * 64 for n in lens]
+    vt = torch.full((nkv * hd, sum(cols) + 64), 7.0, dtype=torch.bfloat16, device=DEV)
+    qkv = torch.empty(T, W, dtype=torch.bfloat16, device=DEV)
+    kernels.qk_norm_rope_store(qkv, nh, nkv, hd, None, None, 1e-6, None, None, 0, pos, seq_index=seq,
+                               partial=part, vt=vt, cu_seqlens=cu, max_len=max(lens))
+    total = part[0].clone()
+    for s in range(1, splits):
+        total += part[s]
+    assert torch.equal(qkv, total.to(torch.bfloat16))
+    want = torch.zeros_like(vt)
+    want[:, sum(cols):] = 7.0
+    at = o = 0
+    for n, c in zip(lens, cols):
+        want[:, at:at + n] = qkv[o:o + n, (nh + nkv) * hd:].T
+        at, o = at + c, o + n
+    assert torch.equal(vt, want)
