@@ -88,8 +88,8 @@ __device__ __forceinline__ float plain_act(float t, int act) {
 // MODE 0: plain.  MODE 1: gated, gate and up tiles of 128 rows each with an
 // accumulator of their own (prompts).  MODE 2: gated, 64 gate rows and the 64 up
 // rows of the same features share one 128-row tile and one accumulator, and the
-// epilogue warps exchange the halves through shared memory (decoding: twice as
-// many CTAs stream the weights).
+// epilogue warps exchange the halves through shared memory (decoding, and prompts of
+// up to 128 tokens where twice as many CTAs bring the weights sooner).
 template <int BN, int MODE, int SLIM = 0>
 struct Tile {
     static constexpr bool DUAL = MODE == 1;
@@ -1821,20 +1821,29 @@ int launch_pair_gated(const CUtensorMap& mw, const CUtensorMap& mw2, const CUten
     return 0;
 }
 
-// How a prompt's plain product is tiled: the form that needs the least time.  A k-block takes
-// `alone` cycles a round of the SMs (or pairs of them) when few of them are busy, and `each` and
-// `full` times their share when all are (they share L2, and the clock goes down with the power); a
-// pair takes 1,300 more to start.  One CTA: 128 weight rows by `tile` tokens.  A pair: 256 tokens by
-// `tile` weight rows, each CTA with half of these.  Fitted to shapes of 256 to 18,432 tokens, 1,152 to
-// 8,192 outputs and a K of 1,024 to 21,504 (56), of which 50 get the fastest form or one within 3 % of it,
-// the others within 7 %.  us, the best form of one CTA and of a pair: 8,696 x 1,152 x 6,912 122 and 111, 18,432
-// tokens 281 and 253, 2,048 29.5 and 27.0; 6,400 x 5,376 x 21,504 1,152 and 1,057; 4,001 x 2,560 x
-// 10,240 160 and 168.  Returns the tile and, in *cycles, the estimate.
-int prompt_plan(int T, int N, int kb, int splits, bool f32, bool* pair, long long* cycles = nullptr) {
-    struct Form { int tile; bool two; int alone, each, full; };
-    static const Form forms[] = {{256, true, 592, 400, 390},  {192, true, 448, 100, 580},
-                                 {128, true, 332, 200, 260},  {256, false, 622, 480, 390},
-                                 {192, false, 457, 160, 540}, {128, false, 385, 250, 260}};
+// How a prompt's plain product is tiled: the form with the smallest estimate, in nanoseconds.  One CTA:
+// 128 weight rows by `tile` tokens.  A pair: 256 tokens by `tile` weight rows, each CTA with half of
+// these.  A k-block takes `alone` a round of the SMs (or pairs of them) when few of them are busy, and
+// `each` and `full` times their share when all are (they share L2, and the clock goes down with the
+// power); a tile takes no less than its way out (`out` a round, `share` times the SMs' share), and a
+// launch `start`.  Every form was timed on 3,317 products into 32 bits and 2,406 into bfloat16, of 129 to
+// 8,192 tokens, 32 to 8,192 outputs and a K of 64 to 21,504, and the constants chosen so that what they
+// pick is fast: 0.8 % (0.2 %) slower than the fastest form on the mean, 160 (24) of them by more than
+// 5 %.  Beside the rule of single CTAs alone (32 bits: the products or the bytes a tile needs; bfloat16: a
+// tile of 256) 3.4 % (21 %) faster on the mean; 25 (8) are slower by more than 7 %, nearly all with a K of
+// 64.  us, the best form of one CTA and of a pair: 8,696 x 1,152 x 6,912 122 and 111, 18,432 tokens
+// 281 and 253, 2,048 29.5 and 27.0; 6,400 x 5,376 x 21,504 1,152 and 1,057; 4,001 x 2,560 x 10,240 160 and
+// 168; 4,096 x 8,192 x 256 into bfloat16 25 and 32.  Returns the tile and, in *ns, the estimate.
+int prompt_plan(int T, int N, int kb, int splits, bool f32, bool* pair, long long* ns = nullptr) {
+    struct Cost { int alone, each, full, start, out, share; };
+    struct Form { int tile; bool two; Cost f32, bf16; };
+    static const Form forms[] = {
+        {256, true, {279, 235, 136, 6260, 0, 1868}, {332, 266, 81, 7224, 0, 4085}},
+        {192, true, {188, 205, 97, 5637, 30, 2237}, {218, 204, 64, 6202, 49, 2901}},
+        {128, true, {140, 142, 82, 4990, 22, 2541}, {157, 181, 70, 4323, 0, 2394}},
+        {256, false, {243, 269, 142, 4650, 270, 1507}, {242, 268, 120, 4571, 0, 2564}},
+        {192, false, {197, 198, 124, 4339, 0, 1601}, {}},
+        {128, false, {243, 184, 98, 3812, 37, 1555}, {}}};
     static const bool pairs = getenv("AGAVE_B200_CTA_PAIRS") == nullptr ||
                               getenv("AGAVE_B200_CTA_PAIRS")[0] != '0';
     const int kb_per = (kb + splits - 1) / splits;
@@ -1843,15 +1852,17 @@ int prompt_plan(int T, int N, int kb, int splits, bool f32, bool* pair, long lon
     *pair = false;
     for (const Form& f : forms) {
         if (f.two ? !pairs : !f32 && f.tile != 256) continue;
+        const Cost& c = f32 ? f.f32 : f.bf16;
         const int units = f.two ? device_sms() / 2 : device_sms();
         const int m = f.two ? f.tile : TILE_M, n = f.two ? 2 * TILE_M : f.tile;
         const long long items = (long long)((N + m - 1) / m) * ((T + n - 1) / n) * splits;
         const long long rounds = (items + units - 1) / units;
-        const long long alone = rounds * f.alone, busy = rounds * f.each + items * f.full / units;
-        const long long cost = kb_per * (alone > busy ? alone : busy) + (f.two ? 1300 : 0);
+        const long long alone = rounds * c.alone, busy = rounds * c.each + items * c.full / units;
+        const long long main = kb_per * (alone > busy ? alone : busy), out = rounds * c.out + items * c.share / units;
+        const long long cost = c.start + (main > out ? main : out);
         if (best < 0 || cost < best) best = cost, bn = f.tile, *pair = f.two;
     }
-    if (cycles) *cycles = best;
+    if (ns) *ns = best;
     return bn;
 }
 
@@ -1936,7 +1947,9 @@ AGV_API int agv_linear_tc(const void* x, const void* w, const void* w2, void* ou
     }
     // decoding through a gated layer: gate and up rows share a tile (see Tile)
     // (and in short prompts where twice the CTAs, each with 32 KB a k-block instead of 48, bring
-    // fewer bytes to an SM one after the other: 6,912 x 1,152 on 108 CTAs instead of 54)
+    // fewer bytes to an SM one after the other: 6,912 x 1,152 on 108 CTAs instead of 54.  Of 126 products of
+    // 65 to 128 tokens, 512 to 21,504 features and a K of 64 to 8,192 none is slower than the form before
+    // by more than 3 %, and on the mean they take 0.80 of its time)
     bool half = w2 && T <= 64;
     if (w2 && T > 64 && T <= 128 && token_tile == 0) {
         const int sms = device_sms();
@@ -2123,8 +2136,18 @@ AGV_API int agv_linear_tc_splits(int K, int splits) {
     return (kb_total + kb_per - 1) / kb_per;
 }
 
+// How a prompt's plain product of these sizes is tiled, for those who check it: the tile, negative
+// where a pair of CTAs takes one (see prompt_plan).
+AGV_API int agv_linear_tc_prompt_form(int T, int N, int K, int splits, int out_dtype) {
+    bool pair;
+    const int tile = prompt_plan(T, N, (K + TILE_K - 1) / TILE_K, splits, out_dtype == AGV_F32, &pair);
+    return pair ? -tile : tile;
+}
+
 // Into how many ranges of K (1 or 2) a prompt of more than 512 tokens is cut: two where the time they
-// save is more than the second partial sum's way out and back costs.
+// save is more than the second partial sum's way out and back costs, at 6,500 bytes a nanosecond.  Of 677
+// products of 513 to 8,192 tokens with a K of 2,048 to 21,504 the answer is within 5 % of the better one
+// for all but 11, and within 10 % for those.
 AGV_API int agv_linear_tc_prompt_splits(int T, int N, int K) {
     const int kb = (K + TILE_K - 1) / TILE_K;
     if (kb < 32) return 1;
@@ -2132,7 +2155,7 @@ AGV_API int agv_linear_tc_prompt_splits(int T, int N, int K) {
     long long one, two;
     prompt_plan(T, N, kb, 1, true, &pair, &one);
     prompt_plan(T, N, kb, 2, true, &pair, &two);
-    return two + (long long)T * N * 8 / 3400 < one ? 2 : 1;         // (bytes at 3,400 a clock)
+    return two + (long long)T * N * 8 / 6500 < one ? 2 : 1;
 }
 
 // Reads and clears the status word of the tensor-core kernels: 0, or

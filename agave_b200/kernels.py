@@ -1485,6 +1485,12 @@ def linear_tc_splits(K: int, splits: int) -> int:
     return library().agv_linear_tc_splits(K, splits)
 
 
+def linear_tc_prompt_form(T: int, N: int, K: int, splits: int = 1, dtype=torch.float32):
+    """(tile, whether on pairs of CTAs) of a prompt's plain product (T > 128)."""
+    tile = library().agv_linear_tc_prompt_form(T, N, K, splits, dtype_code(dtype))
+    return abs(tile), tile < 0
+
+
 def linear_tc_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
     return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and
             w.shape[1] % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and

@@ -239,3 +239,60 @@ def test_transposed_values_of_both_tiles(nh, nkv, hd, lens, splits):
         want[:, at:at + n] = qkv[o:o + n, (nh + nkv) * hd:].T
         at, o = at + c, o + n
     assert torch.equal(vt, want)
+
+
+@pytest.mark.parametrize("dtype,T,N,K,splits,form", [
+    (torch.float32, 1830, 2047, 4104, 1, (256, True)), (torch.float32, 5000, 4100, 1032, 1, (192, True)),
+    (torch.float32, 300, 1150, 4104, 1, (128, True)), (torch.float32, 4100, 1001, 1160, 2, (256, False)),
+    (torch.float32, 2051, 2301, 200, 1, (192, False)), (torch.float32, 400, 902, 2056, 2, (128, False)),
+    (torch.float32, 700, 513, 4104, 2, (128, True)),
+    (torch.bfloat16, 1030, 3001, 8200, 1, (256, True)), (torch.bfloat16, 700, 4100, 2056, 1, (192, True)),
+    (torch.bfloat16, 200, 131, 72, 1, (128, True)), (torch.bfloat16, 3000, 1543, 200, 1, (256, False))])
+def test_every_form_of_a_prompts_product(dtype, T, N, K, splits, form):
+    """Each tile of a pair and of a CTA alone, by the plan's own choice: tokens, features and K that end
+    inside a tile, rows whose stride is a multiple of four values and one that is not.  32-bit sums of
+    bfloat16 products; into bfloat16 rounded once (2^-9)."""
+    from agave_b200 import kernels
+    assert kernels.linear_tc_prompt_form(T, N, K, splits, dtype) == form
+    x = rnd(T, K, dtype=torch.bfloat16, seed=1)
+    w = rnd(N, K, dtype=torch.bfloat16, seed=2, scale=K ** -0.5)
+    ref = x.double() @ w.double().T
+    for ld in (N,) if splits > 1 else (N + (-N) % 4, N + (-N) % 4 + 1):
+        out = torch.full((splits, T, ld) if splits > 1 else (T + 1, ld), float("nan"), dtype=dtype, device=DEV)
+        kernels.linear_tc(x, w, out if splits > 1 else out[:T, :N], splits=splits)
+        assert kernels.linear_tc_status() == 0
+        got = out.double().sum(0) if splits > 1 else out[:T, :N]
+        assert rel_err(got, ref) < (1e-5 if dtype == torch.float32 else 4e-3)
+        assert splits > 1 or (torch.isnan(out[T]).all() and torch.isnan(out[:, N:]).all())
+
+
+@pytest.mark.parametrize("T,splits", [(600, 2), (3600, 1)])
+def test_a_step_whose_products_are_cut_in_two(T, splits, tmp_path):
+    """A prompt long enough for the rule of two ranges of K on the output and down products, and one
+    beyond it: the norm behind them meets two partial sums or one.  Logits against the plain
+    implementation in 32 bits; bfloat16 layers."""
+    import os
+    import sys
+    sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+    from plain import gemma3_plain as P
+    from agave_b200 import kernels
+    from agave_b200.engine.api import Engine
+    from agave_b200.weights import write_model_folder
+    cfg = {"architectures": ["Gemma3ForCausalLM"], "model_type": "gemma3_text", "num_hidden_layers": 2,
+           "hidden_size": 512, "num_attention_heads": 8, "num_key_value_heads": 2, "head_dim": 256,
+           "query_pre_attn_scalar": 256, "intermediate_size": 2304, "vocab_size": 384,
+           "sliding_window": 100, "sliding_window_pattern": 2, "rope_local_base_freq": 10000.0,
+           "rope_theta": 1000000.0, "rms_norm_eps": 1e-6, "max_position_embeddings": 4096,
+           "eos_token_id": 1}
+    for K in (2048, 2304):
+        assert kernels.plan_splits(T, 512, K)[0] == splits
+    write_model_folder(str(tmp_path), cfg, seed=3, dtype=torch.bfloat16)
+    g = torch.Generator().manual_seed(4)
+    tokens = torch.randint(2, 384, (T,), generator=g).tolist()
+    pcfg, w = P.read_config(str(tmp_path)), P.read_weights(str(tmp_path))
+    ref = P.forward_logits(pcfg, w, tokens)[-1].double()
+    eng = Engine(str(tmp_path), dtype="bfloat16", max_tokens=4096)
+    slot = eng.acquire()
+    got = eng.step([(slot, tokens)], [[T - 1]]).reshape(384).double().cpu()
+    assert kernels.linear_tc_status() == 0
+    assert float((got - ref).norm() / ref.norm()) < 2e-2
