@@ -654,6 +654,37 @@ AGV_API int agv_attention_prefill_tc_supported(int hd, long long q_stride, long 
     return (hd >= 16 && hd % 16 == 0 && hd <= 256 && q_stride % 8 == 0 && kv_stride % 8 == 0) ? 1 : 0;
 }
 
+// Whether a prompt step's attention should take this kernel and not the mma.sync one, where both can:
+// T tokens in B sequences of up to max_len; with_vt: the step's q/k/v kernel can write the values
+// transposed, else a kernel of its own would.  One CTA of this kernel has the SM, where the other has
+// several of 64 rows of one head.  Up to 64 keys that other one walks a single tile, and is ahead where
+//  - this kernel needs a second round of the SMs for about as many CTAs as the other has: 16 heads of 64, 16
+//    sequences of 12 tokens 9.6 us against 6.1, 64 of 32 tokens 33 against 13; up to twice as many with heads
+//    up to 64 (32 over 8, 16 sequences of 64 tokens 9.8 against 8.0); heads of 128 with as many 10.6
+//    against 8.3, with twice as many 10.7 against 15.0;
+//  - the values would cost a kernel (with the q/k/v kernel: four heads of 256, one kv head, a sequence of 64
+//    tokens 19.2 us against 15.0; 16 heads of 64 11.1 against 9.8), but for four and more heads packed into
+//    one of so many CTAs (16 over 4 of 128, 64 sequences of 12 tokens 21.7 against 34.1), and for heads
+//    that the other one pads (16 heads of 16, 64 tokens 8.8 against 11.2);
+//  - sequences have a few tokens each, and their values padded to 64 columns are what takes long: 8 of 4 tokens,
+//    16 heads of 64, with the q/k/v kernel 11.4 us against 9.3.
+// Everywhere else this kernel is ahead, from one token on: four heads of 256, with the q/k/v kernel 8.2 us
+// against 15.2 for 64 tokens, 8.9 against 22.0 for 128.  (1,072 steps of 1 to 4,096 tokens, 16 shapes of
+// heads, and 1,134 with ragged ones among them.)
+AGV_API int agv_attention_prefill_prefers_tc(int T, int B, int max_len, int nh, int nkv, int hd, int hdv,
+                                             int with_vt) {
+    const int widest = hd > hdv ? hd : hdv, G = packed_heads(nh, nkv), QT = AT_M / G, sms = 148;
+    const long long here = (long long)B * (G > 1 ? nkv : nh) * ((max_len + QT - 1) / QT);
+    const long long there = (long long)B * nh * ((max_len + 63) / 64);
+    with_vt = with_vt && hd % 64 == 0 && hd == hdv;       // (else the q/k/v kernel calls that of its own)
+    // (a few CTAs walking two tiles or three: a kernel for the values takes about what they gain)
+    if (max_len > 64) return with_vt || T > 192 || max_len > 128 || widest <= 128;
+    if (here > sms && there >= 4 * here) return !with_vt || max_len > 2;
+    if (!with_vt) return here <= sms && 8 * widest <= 5 * ((widest + 63) / 64 * 64);
+    if (T <= 6LL * B && B >= (widest <= 128 ? 8 : 16)) return 0;
+    return here <= sms || there > (widest <= 64 ? 2 : 1) * here;
+}
+
 // Columns the transposed-values scratch needs for B sequences of T tokens in all.
 AGV_API long long agv_attention_prefill_tc_vt_cols(int T, int B) {
     return ((long long)T + 63LL * B + 63) / 64 * 64;

@@ -38,6 +38,7 @@ int agv_linear_tc(const void*, const void*, const void*, void*, int, int, int, l
                   int, int, float, float, int, int, int, cudaStream_t);
 int agv_linear_tc_splits(int, int);
 int agv_linear_tc_prompt_splits(int, int, int);
+int agv_attention_prefill_prefers_tc(int, int, int, int, int, int, int, int);
 int agv_gemv_few_supported(int, int, int, long long, int);
 int agv_gemv_few(const void*, const void*, int, int, int, const void*, long long, const float*, float*,
                  const float*, const float*, const float*, float, float, void*, long long, int,
@@ -253,12 +254,8 @@ struct Run {
         void* out = ar.take((size_t)T * b.nh * b.hd * e);
         const bool aligned = m.dtype == AGV_BF16 && b.hd <= 256 && width % 8 == 0 &&
                              agv_aligned(q, 16) && agv_aligned(k, 16) && agv_aligned(v, 16);
-        static const bool prefill_tc = [] {
-            const char* v2 = getenv("AGAVE_B200_PREFILL_ATTENTION");
-            return !(v2 && strcmp(v2, "mma") == 0);
-        }();
         if (!dry()) {
-            if (aligned && b.hd % 16 == 0 && prefill_tc && b.scale > 0.f)
+            if (vt)
                 did(agv_attention_prefill_tc(q, width, k, v, width, out, vt, vt_cols, 1, s.cu_seqlens,
                                              s.B, T, s.max_new, b.nh, b.nkv, b.hd, b.scale,
                                              b.window, stream));
@@ -274,7 +271,7 @@ struct Run {
         return linear_partial(out, (long long)b.nh * b.hd, b.w_out, m.H, b.nh * b.hd, T, false);
     }
 
-    // whether a prompt step's attention will read the values transposed (the tcgen05 kernel)
+    // whether a prompt step's attention is the tcgen05 kernel, which reads the values transposed
     bool wants_vt(const AgvBlockDesc& b, const void* qkv) const {
         static const bool prefill_tc = [] {
             const char* v2 = getenv("AGAVE_B200_PREFILL_ATTENTION");
@@ -282,8 +279,8 @@ struct Run {
         }();
         const long long width = (long long)(b.nh + 2 * b.nkv) * b.hd;
         return prefill_tc && b.scale > 0.f && m.dtype == AGV_BF16 && b.hd % 16 == 0 &&
-               b.hd <= 256 &&
-               width % 8 == 0 && agv_aligned(qkv, 16);
+               b.hd <= 256 && width % 8 == 0 && agv_aligned(qkv, 16) &&
+               agv_attention_prefill_prefers_tc(s.T, s.B, s.max_new, b.nh, b.nkv, b.hd, b.hd, 1);
     }
 
     Partial mixer(const AgvBlockDesc& b, const AgvCacheDesc& c, const void* x,

@@ -1749,23 +1749,31 @@ def attention_tc_status() -> int:
     return library().agv_attention_tc_status()
 
 
-def attention_prefill_wants_transposed_values(qkv: torch.Tensor, head_dim: int,
-                                              value_dim: int = 0) -> bool:
+def _prefill_prefers_tc(ctx, T: int, n_heads: int, n_kv_heads: int, head_dim: int, hdv: int,
+                        with_vt: bool) -> bool:
+    return bool(library().agv_attention_prefill_prefers_tc(
+        T, ctx.cu_seqlens.numel() - 1, ctx.max_new, n_heads, n_kv_heads, head_dim, hdv, 1 if with_vt else 0))
+
+
+def attention_prefill_wants_transposed_values(qkv: torch.Tensor, ctx, n_heads: int, n_kv_heads: int,
+                                              head_dim: int, value_dim: int = 0) -> bool:
     """Whether ``attention_prefill`` on views of this projection output will take the
-    tcgen05 kernel, which reads the values transposed."""
+    tcgen05 kernel, which reads the values transposed, if it is given them."""
     hdv = value_dim or head_dim
     return (_PREFILL_TC and qkv.dtype == torch.bfloat16 and
             head_dim % 16 == 0 and head_dim <= 256 and hdv % 16 == 0 and hdv <= 256 and
-            qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0)
+            qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and
+            _prefill_prefers_tc(ctx, qkv.shape[0], n_heads, n_kv_heads, head_dim, hdv, True))
 
 
 def attention_prefill(q, k, v, out, ctx, n_heads, n_kv_heads, head_dim, scale, window,
                       vt=None, value_dim: int = 0, sinks=None, dist_bias=None,
                       op: str = "attention", keep_first: int = 0, softcap: float = 0.0) -> None:
     """Prompt attention of one layer in bfloat16: the tcgen05 kernel for key and value head
-    sizes in steps of 16 up to 256 (short prompts too: 100 tokens, four heads of 256, 8.1 us against
-    14.2 by mma.sync, 64 tokens 7.6 against 10.6), the mma.sync kernel for the other multiples of 8; else
-    the one-warp-per-(token, head) kernel.  ``sinks`` [nh]: a logit per query head that joins its denominator once."""
+    sizes in steps of 16 up to 256 (for many short sequences only where it is the faster one:
+    ``agv_attention_prefill_prefers_tc``), the mma.sync kernel for those and the other multiples of 8;
+    else the one-warp-per-(token, head) kernel.  ``sinks`` [nh]: a logit per query head that joins its
+    denominator once."""
     hdv = value_dim or head_dim
     aligned = (q.dtype == torch.bfloat16 and head_dim <= 256 and hdv <= 256 and
                q.stride(0) % 8 == 0 and k.stride(0) % 8 == 0 and v.stride(0) % 8 == 0 and
@@ -1775,7 +1783,9 @@ def attention_prefill(q, k, v, out, ctx, n_heads, n_kv_heads, head_dim, scale, w
     if not window:
         keep_first = 0                    # (without a window every key is visible anyway)
     with _span(op, *_attention_cost(ctx, q, k, v, out, n_heads, head_dim, window)):
-        if aligned and tc and _PREFILL_TC and scale > 0:
+        if (aligned and tc and _PREFILL_TC and scale > 0 and
+                (vt is not None or _prefill_prefers_tc(ctx, q.shape[0], n_heads, n_kv_heads, head_dim,
+                                                       hdv, False))):
             attention_prefill_tc(q, k, v, out, ctx.cu_seqlens, ctx.max_new, n_heads, n_kv_heads,
                                  head_dim, scale, window, vt=vt, sinks=sinks, dist_bias=dist_bias,
                                  keep_first=keep_first, value_dim=hdv, softcap=softcap)

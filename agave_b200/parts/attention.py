@@ -323,7 +323,8 @@ class AttentionMixer:
             # transposed values are the epilogue of the q/k/v product
             qkv = ctx.new(T, (nh + 2 * nkv) * hd)
             vt = None
-            if writes_cache and kernels.attention_prefill_wants_transposed_values(qkv, hd):
+            if writes_cache and kernels.attention_prefill_wants_transposed_values(
+                    qkv, ctx, nh, nkv, hd):
                 vt = kernels.prefill_values_scratch(T, ctx.batch, nkv, hd, qkv.device)
             pools = dict(k_pool=view.k_pool, v_pool=view.v_pool, page_table=view.page_table,
                          slots=ctx.slots, lens=ctx.lens, page=view.page,
@@ -348,7 +349,8 @@ class AttentionMixer:
             # a prompt step on the tcgen05 attention kernel reads the values transposed:
             # the same launch writes that copy
             vt = None
-            if ctx.mode == PREFILL and kernels.attention_prefill_wants_transposed_values(qkv, hd):
+            if ctx.mode == PREFILL and kernels.attention_prefill_wants_transposed_values(
+                    qkv, ctx, nh, nkv, hd):
                 vt = kernels.prefill_values_scratch(T, ctx.batch, nkv, hd, qkv.device)
             kernels.qk_norm_rope_store(
                 qkv, nh, nkv, hd, self.q_norm_weight, self.k_norm_weight, eps, cos, sin,
@@ -419,7 +421,7 @@ class AttentionMixer:
                 ctx.step_values[cache_entry] = qkv[:, (nh + nkv) * hd:]
         elif self.own_kv:
             if ctx.mode == PREFILL and kernels.attention_prefill_wants_transposed_values(
-                    qkv, hd, hdv):
+                    qkv, ctx, nh, nkv, hd, hdv):
                 vt = kernels.prefill_values_scratch(T, ctx.batch, nkv, hdv, qkv.device)
             kernels.qk_norm_rope_store(
                 qkv, nh, nkv, hd, self.q_norm_weight, self.k_norm_weight, eps, cos, sin,

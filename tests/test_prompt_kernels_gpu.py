@@ -296,3 +296,106 @@ def test_a_step_whose_products_are_cut_in_two(T, splits, tmp_path):
     got = eng.step([(slot, tokens)], [[T - 1]]).reshape(384).double().cpu()
     assert kernels.linear_tc_status() == 0
     assert float((got - ref).norm() / ref.norm()) < 2e-2
+
+
+@pytest.mark.parametrize("nh,nkv,hd,hdv", [(4, 1, 256, 256), (16, 16, 64, 64), (8, 2, 48, 80), (6, 6, 16, 16)])
+@pytest.mark.parametrize("form", ["bias", "cap", "sinks", "blocks"])
+def test_prompt_attention_of_many_short_sequences(nh, nkv, hd, hdv, form):
+    """Sequences of a few tokens and of up to two half tiles of 64 keys in one step, with a bias by
+    distance, a soft cap, a sink and blocks of positions, by either kernel.  Errors: P, the values and
+    the result are bfloat16 (2^-9 each)."""
+    from agave_b200 import kernels
+    lens = [3, 1, 63, 7, 64, 2, 65, 31, 33, 127, 12, 5, 128, 4, 4, 4, 1, 1, 30]
+    T, nan = sum(lens), float("nan")
+    window = -40 if form == "blocks" else 0
+    q, k = (rnd(T, n * hd, dtype=torch.bfloat16, seed=i, scale=0.5) for i, n in enumerate((nh, nkv)))
+    v = rnd(T, nkv * hdv, dtype=torch.bfloat16, seed=3)
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=DEV)
+    sinks = rnd(nh, seed=5) if form == "sinks" else None
+    bias = rnd(nh, 50, seed=6) if form == "bias" else None
+    cap = 2.0 if form == "cap" else 0.0
+    for attend in (kernels.attention_prefill_tc, kernels.attention_prefill_mma):
+        out = torch.full((T, nh * hdv), nan, dtype=torch.bfloat16, device=DEV)
+        attend(q, k, v, out, cu, max(lens), nh, nkv, hd, 0.3, window, value_dim=hdv, sinks=sinks,
+               dist_bias=bias, softcap=cap)
+        assert kernels.attention_tc_status() == 0
+        o = 0
+        for n in lens:
+            at = slice(o, o + n)
+            qs = q[at].double().reshape(n, nh, hd).transpose(0, 1)
+            ks = k[at].double().reshape(n, nkv, hd).transpose(0, 1).repeat_interleave(nh // nkv, 0)
+            vs = v[at].double().reshape(n, nkv, hdv).transpose(0, 1).repeat_interleave(nh // nkv, 0)
+            p = torch.arange(n, device=DEV)[:, None]
+            j = torch.arange(n, device=DEV)[None, :]
+            s = (qs @ ks.transpose(1, 2)) * 0.3
+            if cap:
+                s = cap * torch.tanh(s / cap)
+            if bias is not None:
+                s = s + bias.double()[:, (p - j).clamp(0, 49)]
+            see = (j <= p) & (p // 40 == j // 40 if window else j >= 0)
+            s = s.masked_fill(~see, float("-inf"))
+            if sinks is not None:
+                s = torch.cat([s, sinks.double()[:, None, None].expand(nh, n, 1)], -1)
+            w = torch.softmax(s, -1)[..., :n]
+            ref = (w @ vs).transpose(0, 1).reshape(n, nh * hdv)
+            assert rel_err(out[at], ref) < 6e-3, n
+            o += n
+
+
+@pytest.mark.parametrize("lens", [[100], [300, 7], [12] * 12])
+def test_a_score_scale_that_is_not_positive(lens, monkeypatch):
+    """A negative scale with queries of the other sign is the same step: the tcgen05 attention, which
+    takes positive scales alone, against the kernel that a negative one goes to, each launched by the
+    C++ step function.  bfloat16 probabilities and results (2^-9) through two layers."""
+    from dataclasses import replace
+    from agave_b200 import Engine
+    from agave_b200.config import resolve_architecture
+    from agave_b200.models.decoder import decoder_param_specs
+    from agave_b200.weights import random_tensors
+    cfg = {"architectures": ["Gemma3ForCausalLM"], "model_type": "gemma3_text", "num_hidden_layers": 2,
+           "hidden_size": 256, "num_attention_heads": 4, "num_key_value_heads": 2, "head_dim": 64,
+           "query_pre_attn_scalar": 64, "intermediate_size": 512, "vocab_size": 384, "sliding_window": 100,
+           "sliding_window_pattern": 2, "rope_local_base_freq": 10000.0, "rope_theta": 1000000.0,
+           "rms_norm_eps": 1e-6, "max_position_embeddings": 1024, "eos_token_id": 1}
+    made = resolve_architecture(cfg).config_class
+    plain = made.to_model_spec
+    tensors = random_tensors(decoder_param_specs(made.from_dict(cfg).to_model_spec()), 5, 0.05, 0.1,
+                             torch.bfloat16, DEV)
+    g = torch.Generator().manual_seed(6)
+    prompts = [torch.randint(2, 384, (n,), generator=g).tolist() for n in lens]
+
+    def logits(sign):
+        t = {k: v.clone() for k, v in tensors.items()}
+        if sign < 0:
+            for k in t:
+                if k.endswith("q_norm.weight"):
+                    t[k] = -2 - t[k].float()           # (the norm's factor is 1 + w)
+
+        def spec_of(self):
+            spec = plain(self)
+            return replace(spec, blocks=[replace(b, mixer=replace(b.mixer, scale=sign * b.mixer.scale))
+                                         for b in spec.blocks])
+        monkeypatch.setattr(made, "to_model_spec", spec_of)
+        eng = Engine(None, _raw_config=cfg, _tensors=t, dtype="bfloat16", max_tokens=2048, max_batch=16)
+        slots = [eng.acquire() for _ in prompts]
+        return eng.step(list(zip(slots, prompts)), [list(range(n)) for n in lens]).double()
+
+    a, b = logits(1), logits(-1)
+    assert torch.isfinite(b).all()
+    assert float((a - b).norm() / a.norm()) < 2e-2
+
+
+@pytest.mark.parametrize("T,B,longest,nh,nkv,hd,fused,alone", [
+    (1, 1, 1, 4, 1, 256, True, False), (100, 1, 100, 4, 1, 256, True, False), (100, 1, 100, 16, 16, 64, True, True),
+    (300, 1, 300, 4, 1, 256, True, True), (192, 16, 12, 16, 16, 64, False, False),
+    (1024, 16, 64, 32, 8, 64, False, False), (512, 16, 32, 32, 16, 128, True, False),
+    (768, 64, 12, 16, 4, 128, True, True), (32, 8, 4, 16, 16, 64, False, False),
+    (32, 8, 4, 4, 1, 256, True, False), (64, 1, 64, 16, 16, 16, True, True),
+    (4096, 64, 64, 64, 8, 64, False, False)])
+def test_which_kernel_attends_for_a_prompt(T, B, longest, nh, nkv, hd, fused, alone):
+    """Either side of each line of the rule, with the values transposed by the q/k/v kernel and by one
+    of their own."""
+    from agave_b200 import kernels
+    got = [bool(kernels.library().agv_attention_prefill_prefers_tc(T, B, longest, nh, nkv, hd, hd, vt))
+           for vt in (1, 0)]
+    assert got == [fused, alone]
