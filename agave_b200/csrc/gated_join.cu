@@ -90,7 +90,7 @@ gated_join_kernel(float* __restrict__ h, JoinArgs a, RowIn<float> gates,
     pdl_wait();
     pdl_launch_next();
     extern __shared__ __align__(16) float row[];
-    __shared__ float red[33];
+    __shared__ float red[32];
     const int t = blockIdx.x;
     float ss = 0.f;
     for (int i = threadIdx.x * V; i < H; i += blockDim.x * V) {

@@ -65,7 +65,7 @@ proj_norm_store_kernel(RowIn<T> in, T* __restrict__ out, long long ldo, int n_to
     pdl_wait();
     pdl_launch_next();
     extern __shared__ float buf[];           // the row, 32-bit
-    __shared__ float red[33];
+    __shared__ float red[32];
     const int t = blockIdx.x;
     const int W = nq + nk + nv;
     float sq = 0.f, sk = 0.f;
@@ -332,7 +332,7 @@ latent_prepare_kernel(RowIn<T> in, T* __restrict__ out, long long ldo, int n_tok
     pdl_wait();
     pdl_launch_next();
     extern __shared__ float buf[];
-    __shared__ float red[33];
+    __shared__ float red[32];
     const int t = blockIdx.x;
     const int c_at = q_width, kr_at = q_width + R, g_at = q_width + R + r;
     float sq = 0.f, sc = 0.f;

@@ -53,7 +53,7 @@ layer_norm_join_kernel(float* __restrict__ h, const TY* __restrict__ y, int n_sp
                        size_t split_stride, NormSide post, NormSide next, TX* __restrict__ x,
                        const int* __restrict__ rows, int H, float mult, int add_residual,
                        int rms) {
-    __shared__ float red[33];
+    __shared__ float red[32];
     const int r = blockIdx.x;
     // weights and the row gather do not depend on the kernel before
     float wp[EPT], bp[EPT], wn[EPT], bn[EPT];
@@ -170,7 +170,7 @@ layer_norm_rows_kernel(float* __restrict__ h, const float* __restrict__ y, int n
                        int R, int H, float mult, int add_residual, int rms) {
     pdl_wait();
     pdl_launch_next();
-    __shared__ float red[33];
+    __shared__ float red[32];
     const int lane = GT == 32 ? (threadIdx.x & 31) : threadIdx.x;
     const int row = GT == 32 ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
     if (row >= R) return;                          // (whole warps, or nobody, leave)

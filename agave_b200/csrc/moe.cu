@@ -632,7 +632,7 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 row_gate_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ w,
                 float* __restrict__ y, int K, int H) {
-    __shared__ float red[33];
+    __shared__ float red[32];
     const int t = blockIdx.x, tid = threadIdx.x;
     const T* xr = x + (size_t)t * ldx;
     float* yr = y + (size_t)t * H;

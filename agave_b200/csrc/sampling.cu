@@ -285,7 +285,7 @@ struct SampleShared : RadixShared {
     unsigned long long wsum[SM_THREADS / 32];  // kept weight of every warp's range
     unsigned long long slice_sum;              // read by the whole cluster
     unsigned long long total_mass;             // read by the whole cluster
-    float red[33];
+    float red[32];
     float mx;                                  // read by the whole cluster
     unsigned bound;                            // read by the whole cluster
     int n_list;                                // read by the whole cluster

@@ -476,7 +476,7 @@ ssd_out_kernel(const float* __restrict__ num, const float* __restrict__ u, long 
     pdl_wait();
     pdl_launch_next();
     extern __shared__ __align__(16) float buf[]; // [inner / groups]
-    __shared__ float red[33];
+    __shared__ float red[32];
     const int t = blockIdx.x, width = inner / gridDim.y, c0 = blockIdx.y * width;
     float ss = 0.f;
     for (int i = threadIdx.x * V; i < width; i += blockDim.x * V) {

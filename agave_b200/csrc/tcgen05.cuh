@@ -17,7 +17,8 @@ static __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // in a single thread, so a TMA request or a product is one instruction with uniform operands;
 // behind a test of the lane number it becomes a loop over the lanes that might be there (with the
 // products' loaders and issuers found this way documents of eight sequences, 1B sizes, take 14.1 ms
-// instead of 14.9, a decode step of eight 4 % less).
+// instead of 14.9, a recorded decode step of eight alone 1,052 us instead of 1,101, of 64 1,645 instead
+// of 1,660).
 static __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.b32 %0, 1, 0, q;\n\t}"

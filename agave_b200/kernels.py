@@ -1557,7 +1557,8 @@ def plan_splits(T: int, N: int, K: int, cheap_sum: bool = False):
     layers).  The CTAs of a cluster add their sums in the kernel; the groups are
     left to the consumer.  ``cheap_sum``: the consumer adds partial sums in the
     loads it makes anyway (the q/k norm kernel), so up to eight groups are better
-    than a cluster, whose exchange costs about 2 us.  Prompts are not cut."""
+    than a cluster, whose exchange costs about 2 us.  Prompts of up to 512 tokens are cut into
+    up to 16 ranges, longer ones in two where that pays."""
     if T > 64:
         tile = 128 if T <= 128 else 256
         ctas = ((N + 127) // 128) * ((T + tile - 1) // tile)
